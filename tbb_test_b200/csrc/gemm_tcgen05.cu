@@ -39,19 +39,10 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace b2 {
 namespace {
-
-constexpr int BLOCK_M = 128;
-constexpr int SLAB_BYTES = 128;          // bytes of the contiguous dimension per smem row
-constexpr int KSTEP_BYTES = 32;          // bytes of K one tcgen05.mma consumes
-constexpr int KSTEPS = SLAB_BYTES / KSTEP_BYTES;
-constexpr int MAX_STAGES = 8;
-constexpr int NUM_THREADS = 192;       // producer warp + MMA warp + 4 epilogue warps
-constexpr int NUM_THREADS_SUB2 = 320;  // 256-row tiles: one group of 4 epilogue warps per 128-row accumulator
-constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
-constexpr uint32_t X3_CORR_COLS = 256;  // fp32-class mode: TMEM column offset of the correction accumulators
 
 struct TcParams {
   int M, N, K;
@@ -82,9 +73,10 @@ struct TcParams {
   uint32_t a_lbo, a_sbo, a_kstep;  // shared-memory descriptor strides / per-k-step advance (bytes)
   uint32_t b_lbo, b_sbo, b_kstep;
   uint32_t a_layout, b_layout;     // descriptor swizzle code: 2 = 128 B, 1 = 128 B with 32-byte atoms
-  int a_boxes, b_boxes;            // TMA boxes per stage
+  int a_form, b_form;              // SlabForm
+  int a_boxes, b_boxes;            // 2-D TMA boxes per slab (SLAB_MN2)
   uint32_t a_box_bytes, b_box_bytes;
-  int a_box_mn, b_box_mn;          // M/N elements covered by one box
+  int box_mn_log2;                 // M/N elements of a 128-byte column, as a power of two
   uint32_t a_stage_bytes, b_stage_bytes;
   void* C;
   long long ldc;
@@ -111,209 +103,6 @@ struct TcParams {
   void* C_lo;
   unsigned long long* trace;  // see GemmDesc::trace
 };
-
-// ------------------------------------------------------------------ PTX wrappers
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait. Returns false when it gave up or another role raised the abort flag.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned int* status, unsigned int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer();
-  unsigned int spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 0xFF) == 0) {
-      if (*abort_flag) return false;
-      if (globaltimer() - t0 > WAIT_LIMIT_NS) {
-        *abort_flag = 1;
-        atomicCAS(status, 0u, code);
-        return false;
-      }
-    }
-  }
-  return true;
-}
-__device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(map), "r"(smem_u32(src)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// waits until at most N of this thread's bulk groups still READ their shared-memory source
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// ---- CTA-pair (cta_group::2) forms
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// shared::cluster address of `local_addr` (a shared::cta address) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// TMA load whose completion bytes are credited to an mbarrier that may live in the peer
-// CTA of the pair (`mbar_cluster_addr` is a shared::cluster address). No multicast: the
-// data lands in the issuing CTA's own shared memory only.
-__device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_t mbar_cluster_addr, void* dst,
-                                                 int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(mbar_cluster_addr), "r"(x), "r"(y)
-      : "memory");
-}
-// commit of a pair's MMAs: arrives on the barrier at the same offset in both CTAs
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-      : "memory");
-}
-// One k-block (KSTEPS MMAs per 128-row sub-block) issued from precomputed descriptor
-// templates. A single thread issues every MMA of the CTA, so the instruction count
-// between two MMAs is what bounds the tensor pipe's duty cycle: the constant descriptor
-// fields are assembled once per kernel, and per MMA only the 14-bit start-address field
-// (address >> 4) is added in.
-template <bool TF32, bool PAIR>
-__device__ __forceinline__ void mma_issue(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  if (PAIR) {
-    if (TF32)
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                   ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-    else
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                   ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-  } else {
-    if (TF32)
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                   ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-    else
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                   ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-  }
-}
-// With alo16 / blo16 != 0 (fp32-class mode, tf32 only) the stage also holds the low-order
-// twins of both slabs, alo16 / blo16 sixteen-byte units behind the slabs themselves, and every
-// k-step issues three MMAs: A*B, A*B_lo and A_lo*B (the tensor core truncates fp32 operands
-// to tf32, so A and B stand for their own high parts; A_lo*B_lo, 2^-22 of the product, is dropped).
-// The two correction products go to an accumulator of their own, X3_CORR_COLS TMEM columns
-// behind the main one, and the epilogue adds the two: the tensor core truncates when it adds
-// into an accumulator, a bias that grows with the number of additions, so the main sum should
-// see K/8 of them, not 3K/8 (measured at K = 4096: 3.0e-5 relative with one accumulator).
-template <int SUB_M, bool TF32, bool PAIR>
-__device__ __forceinline__ void issue_kblock(uint32_t tmem_d, uint64_t a_tmpl, uint64_t b_tmpl, uint32_t sa16,
-                                             uint32_t sb16, uint32_t a_step16, uint32_t b_step16, uint32_t idesc,
-                                             uint32_t block_n, int sub, bool first_kblock, int ksteps,
-                                             uint32_t a_sub16, uint32_t alo16 = 0, uint32_t blo16 = 0) {
-#pragma unroll
-  for (int ks = 0; ks < KSTEPS; ++ks) {
-    if (ks >= ksteps) break;
-    const uint64_t bdesc = b_tmpl + (uint64_t)(sb16 + ks * b_step16);
-    const uint32_t accumulate = (ks == 0) ? (first_kblock ? 0u : 1u) : 1u;
-#pragma unroll
-    for (int i = 0; i < SUB_M; ++i) {  // the 128-row sub-blocks share the B slab
-      if (i < sub) {
-        const uint64_t adesc = a_tmpl + (uint64_t)(sa16 + i * a_sub16 + ks * a_step16);
-        const uint32_t d = tmem_d + (uint32_t)i * block_n;
-        mma_issue<TF32, PAIR>(d, adesc, bdesc, idesc, accumulate);
-        if (TF32 && !PAIR && SUB_M == 1 && alo16 != 0) {
-          mma_issue<TF32, PAIR>(d + X3_CORR_COLS, adesc, bdesc + (uint64_t)blo16, idesc, accumulate);
-          mma_issue<TF32, PAIR>(d + X3_CORR_COLS, adesc + (uint64_t)alo16, bdesc, idesc, 1u);
-        }
-      }
-    }
-  }
-}
-
-// 64-bit shared-memory matrix descriptor (version 1) for a 128-byte-swizzled slab.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version (Blackwell)
-  d |= (uint64_t)layout << 61;
-  return d;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
 
 // Work item -> (first row, number of 128-row sub-blocks, column block). Tiles are
 // numbered band by band: a band is `raster_m` row blocks tall and spans all column
@@ -715,11 +504,6 @@ __device__ __forceinline__ bool work_next(const TcParams& p, WorkIter& wi, Work&
   wi.w += gridDim.x;
   return true;
 }
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* ptr) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
-  return v;
-}
 __device__ __forceinline__ void epilogue_bar_sync(int nthreads) {
   asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
 }
@@ -729,7 +513,8 @@ __device__ __forceinline__ void epilogue_bar_sync(int nthreads) {
 // Register budget: the 320 threads of the 256-row mode get 168 registers each (the register file is
 // handed out as if the CTA had 384 threads: 192 per thread was refused at launch), the 192
 // threads of the other modes 255.
-template <int SUB_M>
+// KIND: how operands are multiplied (KIND_BF16, KIND_TF32, or KIND_X3: three tf32 MMAs per k-step).
+template <int SUB_M, int KIND>
 __global__ void __launch_bounds__(SUB_M == 2 ? NUM_THREADS_SUB2 : NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_a_lo,
@@ -745,8 +530,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // stage layout: A [A_lo] B [B_lo] (the low-order twins only in the fp32-class mode)
-  const uint32_t lo_mul = p.x3 ? 2u : 1u;
-  const uint32_t stage_bytes = (p.a_stage_bytes + p.b_stage_bytes) * lo_mul;
+  constexpr bool X3 = KIND == KIND_X3;
+  const uint32_t stage_bytes = (p.a_stage_bytes + p.b_stage_bytes) * (X3 ? 2u : 1u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &abort_s;
 
@@ -781,7 +566,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -789,40 +574,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       Work it;
       work_begin(p, wi);
       int load_tile = 0;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), ring0 = smem_u32(smem);
+      const int block_k = p.block_k, stages = p.stages, a_form = p.a_form, b_form = p.b_form;
+      const uint32_t a_slab = p.a_stage_bytes, b_slab = p.b_stage_bytes;
+      const bool tracing = p.trace && blockIdx.x == 0;
       while (ok && work_next<SUB_M>(p, wi, it)) {
-        const uint32_t a_bytes = (uint32_t)it.sub * p.a_sub_bytes;
+        const uint32_t tx_bytes = ((uint32_t)it.sub * p.a_sub_bytes + b_slab) * (X3 ? 2u : 1u);
+        const int n0 = it.n_blk * p.block_n;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
-          if (p.trace && blockIdx.x == 0 && load_tile == 1 && kb - it.kb0 < TC_TRACE_KBLOCKS)
+          if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
+          if (tracing && load_tile == 1 && kb - it.kb0 < TC_TRACE_KBLOCKS)
             p.trace[TC_TRACE_TILES * 4 + TC_TRACE_KBLOCKS + (kb - it.kb0)] = globaltimer();
-          uint8_t* sa = smem + (size_t)stage * stage_bytes;
-          uint8_t* sb = sa + p.a_stage_bytes * lo_mul;
-          mbar_expect_tx(&full_bar[stage], (a_bytes + p.b_stage_bytes) * lo_mul);
-          const int k0 = kb * p.block_k;
-          for (uint32_t part = 0; part < lo_mul; ++part) {  // the operands, then their low-order twins
-            const CUtensorMap* ma = part ? &tma_a_lo : &tma_a;
-            const CUtensorMap* mb = part ? &tma_b_lo : &tma_b;
-            uint8_t* da = sa + part * p.a_stage_bytes;
-            uint8_t* db = sb + part * p.b_stage_bytes;
-            if (p.a_mn) {
-              const int nbox = it.sub * p.a_boxes;  // a_boxes per 128 rows
-              for (int b = 0; b < nbox; ++b)
-                tma_load_2d(ma, &full_bar[stage], da + (size_t)b * p.a_box_bytes, it.m0 + b * p.a_box_mn, k0);
-            } else {
+          const uint32_t full = full0 + 8u * stage;
+          const uint32_t sa = ring0 + (uint32_t)stage * stage_bytes;
+          mbar_expect_tx(full, tx_bytes);
+          const int k0 = kb * block_k;
 #pragma unroll
-              for (int i = 0; i < SUB_M; ++i)
-                if (i < it.sub)
-                  tma_load_2d(ma, &full_bar[stage], da + (size_t)i * p.a_sub_bytes, k0, it.m0 + i * BLOCK_M);
-            }
-            if (p.b_mn) {
-              for (int b = 0; b < p.b_boxes; ++b)
-                tma_load_2d(mb, &full_bar[stage], db + (size_t)b * p.b_box_bytes, it.n_blk * p.block_n + b * p.b_box_mn,
-                            k0);
-            } else {
-              tma_load_2d(mb, &full_bar[stage], db, k0, it.n_blk * p.block_n);
-            }
+          for (int i = 0; i < SUB_M; ++i)
+            if (i < it.sub)
+              load_slab<false>(&tma_a, full, sa + (uint32_t)i * p.a_sub_bytes, a_form, k0, it.m0 + i * BLOCK_M,
+                               p.a_boxes, p.a_box_bytes, p.box_mn_log2);
+          const uint32_t sb = sa + a_slab * (X3 ? 2u : 1u);
+          load_slab<false>(&tma_b, full, sb, b_form, k0, n0, p.b_boxes, p.b_box_bytes, p.box_mn_log2);
+          if (X3) {  // the low-order twins
+            load_slab<false>(&tma_a_lo, full, sa + a_slab, a_form, k0, it.m0, p.a_boxes, p.a_box_bytes, p.box_mn_log2);
+            load_slab<false>(&tma_b_lo, full, sb + b_slab, b_form, k0, n0, p.b_boxes, p.b_box_bytes, p.box_mn_log2);
           }
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          if (++stage == stages) { stage = 0; phase ^= 1; }
         }
         ++load_tile;
       }
@@ -834,21 +612,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      const uint64_t a_tmpl = make_smem_desc(0, p.a_lbo, p.a_sbo, p.a_layout);
-      const uint64_t b_tmpl = make_smem_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
-      const uint32_t smem16 = smem_u32(smem) >> 4, stage16 = stage_bytes >> 4, a_stage16 = p.a_stage_bytes >> 4;
+      const uint64_t a_tmpl = make_smem_desc(smem_u32(smem), p.a_lbo, p.a_sbo, p.a_layout);
+      const uint64_t b_tmpl =
+          make_smem_desc(smem_u32(smem) + p.a_stage_bytes * (X3 ? 2u : 1u), p.b_lbo, p.b_sbo, p.b_layout);
+      const uint32_t stage16 = stage_bytes >> 4;
       const uint32_t a_step16 = p.a_kstep >> 4, b_step16 = p.b_kstep >> 4, idesc = p.idesc;
       const uint32_t block_n = (uint32_t)p.block_n;
-      const bool tf32 = p.kind_tf32 != 0;
-      const uint32_t alo16 = p.x3 ? a_stage16 : 0u, blo16 = p.x3 ? (p.b_stage_bytes >> 4) : 0u;
-      const int ksteps = p.ksteps;
+      const uint32_t alo16 = p.a_stage_bytes >> 4, blo16 = p.b_stage_bytes >> 4;
+      const int ksteps = p.ksteps, stages = p.stages;
       const uint32_t a_sub16 = p.a_sub_bytes >> 4;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full_bar);
+      const bool tracing = p.trace && blockIdx.x == 0;
       int trace_tile = 0;
       WorkIter wi;
       Work it;
@@ -858,24 +638,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)acc * acc_cols;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 3u)) { ok = false; break; }
+          if (!mbar_wait(full0 + 8u * stage, phase, abort_flag, p.status, 3u)) { ok = false; break; }
           tc_fence_after();
-          if (p.trace && blockIdx.x == 0) {
+          if (tracing) {
             if (kb == it.kb0 && trace_tile < TC_TRACE_TILES) p.trace[trace_tile * 4 + 0] = globaltimer();
             if (trace_tile == 1 && kb - it.kb0 < TC_TRACE_KBLOCKS) p.trace[TC_TRACE_TILES * 4 + (kb - it.kb0)] = globaltimer();
           }
-          const uint32_t sa16 = smem16 + (uint32_t)stage * stage16;
-          if (tf32)
-            issue_kblock<SUB_M, true, false>(tmem_d, a_tmpl, b_tmpl, sa16, sa16 + a_stage16 * lo_mul, a_step16, b_step16,
-                                             idesc, block_n, it.sub, kb == it.kb0, ksteps, a_sub16, alo16, blo16);
-          else
-            issue_kblock<SUB_M, false, false>(tmem_d, a_tmpl, b_tmpl, sa16, sa16 + a_stage16, a_step16, b_step16,
-                                              idesc, block_n, it.sub, kb == it.kb0, ksteps, a_sub16);
-          tc_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          const uint32_t off16 = (uint32_t)stage * stage16;
+          issue_kblock<SUB_M, KIND != KIND_BF16, false, X3>(tmem_d, a_tmpl + off16, b_tmpl + off16, a_step16, b_step16,
+                                                            idesc, block_n, it.sub, kb == it.kb0, ksteps, a_sub16,
+                                                            alo16, blo16);
+          tc_commit(empty0 + 8u * stage);  // frees the stage once these MMAs have read it
+          if (++stage == stages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit(&acc_full_bar[acc]);   // accumulator complete -> epilogue
+        tc_commit(acc_full0 + 8u * acc);   // accumulator complete -> epilogue
         ++trace_tile;
         if (++acc == ACC_STAGES) { acc = 0; acc_phase ^= 1; }
       }
@@ -1023,6 +800,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 // both CTAs (the peer's arrive remotely). A cluster barrier after initialisation keeps
 // remote signals away from uninitialised barriers, one before exit keeps either CTA's
 // shared memory and TMEM alive while the other may still touch it.
+template <int KIND>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                     const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ TcParams p) {
@@ -1071,37 +849,30 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int load_tile = 0;
+      const uint32_t full0 = map_to_cta(smem_u32(full_bar), 0), empty0 = smem_u32(empty_bar), ring0 = smem_u32(smem);
+      const int block_k = p.block_k, stages = p.stages, a_form = p.a_form, b_form = p.b_form;
+      const uint32_t a_slab = p.a_stage_bytes;
+      const bool tracing = p.trace && blockIdx.x < 2;
       for (int t = pair; t < num_tiles && ok; t += num_pairs, ++load_tile) {
         const Item it = decode_item<2>(t, num_tiles, p.num_m_blocks, p.num_n_blocks, p.raster_m, 1 << 30);
         const int m0 = it.m0 + (int)rank * BLOCK_M;                   // this CTA's rows of A
         const int n0 = it.n_blk * p.block_n + (int)rank * (p.block_n / 2);  // this CTA's half of B
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
-          if (p.trace && blockIdx.x < 2 && load_tile == 1 && kb < TC_TRACE_KBLOCKS)  // leader and peer of pair 0
+          if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
+          if (tracing && load_tile == 1 && kb < TC_TRACE_KBLOCKS)  // leader and peer of pair 0
             p.trace[TC_TRACE_TILES * 4 + (1 + blockIdx.x) * TC_TRACE_KBLOCKS + kb] = globaltimer();
-          uint8_t* sa = smem + (size_t)stage * stage_bytes;
-          uint8_t* sb = sa + p.a_stage_bytes;
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * stage_bytes);  // both CTAs' bytes
-          const uint32_t full_addr = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          const int k0 = kb * p.block_k;
-          if (p.a_mn) {
-            for (int b = 0; b < p.a_boxes; ++b)
-              tma_load_2d_pair(&tma_a, full_addr, sa + (size_t)b * p.a_box_bytes, m0 + b * p.a_box_mn, k0);
-          } else {
-            tma_load_2d_pair(&tma_a, full_addr, sa, k0, m0);
-          }
-          if (p.b_mn) {
-            for (int b = 0; b < p.b_boxes; ++b)
-              tma_load_2d_pair(&tma_b, full_addr, sb + (size_t)b * p.b_box_bytes, n0 + b * p.b_box_mn, k0);
-          } else {
-            tma_load_2d_pair(&tma_b, full_addr, sb, k0, n0);
-          }
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          const uint32_t sa = ring0 + (uint32_t)stage * stage_bytes;
+          if (rank == 0) mbar_expect_tx(smem_u32(full_bar) + 8u * stage, 2 * stage_bytes);  // both CTAs' bytes
+          const uint32_t full = full0 + 8u * stage;
+          const int k0 = kb * block_k;
+          load_slab<true>(&tma_a, full, sa, a_form, k0, m0, p.a_boxes, p.a_box_bytes, p.box_mn_log2);
+          load_slab<true>(&tma_b, full, sa + a_slab, b_form, k0, n0, p.b_boxes, p.b_box_bytes, p.box_mn_log2);
+          if (++stage == stages) { stage = 0; phase ^= 1; }
         }
       }
       if (!ok) {
@@ -1111,41 +882,39 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ----------------------------------------------- MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      const uint64_t a_tmpl = make_smem_desc(0, p.a_lbo, p.a_sbo, p.a_layout);
-      const uint64_t b_tmpl = make_smem_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
-      const uint32_t smem16 = smem_u32(smem) >> 4, stage16 = stage_bytes >> 4, a_stage16 = p.a_stage_bytes >> 4;
+      const uint64_t a_tmpl = make_smem_desc(smem_u32(smem), p.a_lbo, p.a_sbo, p.a_layout);
+      const uint64_t b_tmpl = make_smem_desc(smem_u32(smem) + p.a_stage_bytes, p.b_lbo, p.b_sbo, p.b_layout);
+      const uint32_t stage16 = stage_bytes >> 4;
       const uint32_t a_step16 = p.a_kstep >> 4, b_step16 = p.b_kstep >> 4, idesc = p.idesc;
-      const bool tf32 = p.kind_tf32 != 0;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full_bar);
+      const int ksteps = p.ksteps, stages = p.stages;
+      const bool tracing = p.trace && blockIdx.x == 0;
       int trace_tile = 0;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
         if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 2u)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * p.block_n);
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 3u)) { ok = false; break; }
+          if (!mbar_wait(full0 + 8u * stage, phase, abort_flag, p.status, 3u)) { ok = false; break; }
           tc_fence_after();
-          if (p.trace && blockIdx.x == 0) {
+          if (tracing) {
             if (kb == 0 && trace_tile < TC_TRACE_TILES) p.trace[trace_tile * 4 + 0] = globaltimer();
             if (trace_tile == 1 && kb < TC_TRACE_KBLOCKS) p.trace[TC_TRACE_TILES * 4 + kb] = globaltimer();
           }
-          const uint32_t sa16 = smem16 + (uint32_t)stage * stage16;
-          if (tf32)
-            issue_kblock<1, true, true>(tmem_d, a_tmpl, b_tmpl, sa16, sa16 + a_stage16, a_step16, b_step16, idesc,
-                                        0u, 1, kb == 0, p.ksteps, 0u);
-          else
-            issue_kblock<1, false, true>(tmem_d, a_tmpl, b_tmpl, sa16, sa16 + a_stage16, a_step16, b_step16, idesc,
-                                         0u, 1, kb == 0, p.ksteps, 0u);
-          tc_commit_pair(&empty_bar[stage]);
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          const uint32_t off16 = (uint32_t)stage * stage16;
+          issue_kblock<1, KIND != KIND_BF16, true, false>(tmem_d, a_tmpl + off16, b_tmpl + off16, a_step16, b_step16,
+                                                          idesc, 0u, 1, kb == 0, ksteps, 0u);
+          tc_commit_pair(empty0 + 8u * stage);
+          if (++stage == stages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit_pair(&acc_full_bar[acc]);
+        tc_commit_pair(acc_full0 + 8u * acc);
         ++trace_tile;
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
@@ -1209,41 +978,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
 }
 
 // ------------------------------------------------------------------ host side
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
-// 2-D tensor map over a row-major matrix: `inner` contiguous elements per row,
-// `outer` rows, `ld` elements between rows; box = box_inner x box_outer.
-// swizzle: 0 = 128 bytes, 1 = 128 bytes in 32-byte atoms, 2 = 64 bytes
-bool make_map(CUtensorMap* map, const void* base, int elem_bytes, long long inner, long long outer, long long ld,
-              int box_inner, int box_outer, int swizzle) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * elem_bytes};
-  cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  CUresult r = enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   swizzle == 1 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
-                   : swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
 
 }  // namespace
 
@@ -1320,12 +1054,12 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
     p.sub_m = cands[best_i].sub_m;
   }
   p.block_n = bn;
-  const char* force = getenv("B2_TC_SUB_M");
-  if (force && (force[0] == '1' || (force[0] == '2' && bn == 256))) p.sub_m = force[0] - '0';
   if (const char* fb = getenv("B2_TC_BN")) {  // experiments: force the tile width
     const int v = atoi(fb);
     if (v == 64 || v == 128 || v == 256) { bn = v; p.block_n = v; if (v != 256) p.sub_m = 1; }
   }
+  const char* force = getenv("B2_TC_SUB_M");
+  if (force && (force[0] == '1' || (force[0] == '2' && bn == 256))) p.sub_m = force[0] - '0';
   if (x3 && (bn == 256 || p.sub_m == 2)) { bn = 128; p.block_n = 128; p.sub_m = 1; }
   // CTA pairs: a 256 x 256 tile per pair of SMs once there is a tile for every pair
   {
@@ -1388,6 +1122,7 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
             ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((p.pair ? 2 * BLOCK_M : BLOCK_M) >> 4) << 24);
   const int slab_elems = SLAB_BYTES / eb;
+  p.box_mn_log2 = eb == 2 ? 6 : 5;
   const int cta_bn = p.pair ? bn / 2 : bn;  // B rows (columns of C) held by one CTA
   // K-contiguous slabs: rows of kb_bytes, 128-byte swizzle (8-row groups of 1024 B) or, for
   // half k-blocks, 64-byte swizzle (8-row groups of 512 B, descriptor layout code 4).
@@ -1405,17 +1140,25 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
   const uint32_t mn_group_bytes = mn_atom32 ? 512 : 1024;
   const uint32_t mn_layout = mn_atom32 ? 1 : 2;
   if (a_mn) {
-    // boxes of {128 bytes of M, block_k k-rows}; 8-row groups 1024 B apart, M atoms one box apart
+    // columns of {128 bytes of M, block_k k-rows}; 8-row groups 1024 B apart, columns block_k rows apart
     p.a_boxes = BLOCK_M / slab_elems;
-    p.a_box_mn = slab_elems;
     p.a_box_bytes = p.block_k * SLAB_BYTES;
     p.a_lbo = p.a_box_bytes;
     p.a_sbo = mn_group_bytes;
     p.a_layout = mn_layout;
     p.a_kstep = (KSTEP_BYTES / eb) * SLAB_BYTES;
-    ok = ok && make_map(&plan->map_a, g.A, eb, g.M, g.K, lda, slab_elems, p.block_k, mn_atom32 ? 1 : 0);
-    if (x3) ok = ok && make_map(&plan->map_a_lo, g.A_lo, eb, g.M, g.K, lda, slab_elems, p.block_k, mn_atom32 ? 1 : 0);
+    const int swz = mn_atom32 ? 1 : 0;
+    p.a_form = SLAB_MN2;
+    if (g.M % slab_elems == 0 &&
+        make_map_columns(&plan->map_a, g.A, eb, g.M, g.K, lda, p.block_k, p.a_boxes, swz) &&
+        (!x3 || make_map_columns(&plan->map_a_lo, g.A_lo, eb, g.M, g.K, lda, p.block_k, p.a_boxes, swz)))
+      p.a_form = SLAB_MN3;
+    if (p.a_form == SLAB_MN2) {
+      ok = ok && make_map(&plan->map_a, g.A, eb, g.M, g.K, lda, slab_elems, p.block_k, swz);
+      if (x3) ok = ok && make_map(&plan->map_a_lo, g.A_lo, eb, g.M, g.K, lda, slab_elems, p.block_k, swz);
+    }
   } else {
+    p.a_form = SLAB_K;
     p.a_boxes = 1;
     p.a_box_bytes = p.a_sub_bytes;
     p.a_lbo = 16;
@@ -1427,15 +1170,23 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
   }
   if (b_mn) {
     p.b_boxes = cta_bn / slab_elems;
-    p.b_box_mn = slab_elems;
     p.b_box_bytes = p.block_k * SLAB_BYTES;
     p.b_lbo = p.b_box_bytes;
     p.b_sbo = mn_group_bytes;
     p.b_layout = mn_layout;
     p.b_kstep = (KSTEP_BYTES / eb) * SLAB_BYTES;
-    ok = ok && make_map(&plan->map_b, g.B, eb, g.N, g.K, ldb, slab_elems, p.block_k, mn_atom32 ? 1 : 0);
-    if (x3) ok = ok && make_map(&plan->map_b_lo, g.B_lo, eb, g.N, g.K, ldb, slab_elems, p.block_k, mn_atom32 ? 1 : 0);
+    const int swz = mn_atom32 ? 1 : 0;
+    p.b_form = SLAB_MN2;
+    if (g.N % slab_elems == 0 &&
+        make_map_columns(&plan->map_b, g.B, eb, g.N, g.K, ldb, p.block_k, p.b_boxes, swz) &&
+        (!x3 || make_map_columns(&plan->map_b_lo, g.B_lo, eb, g.N, g.K, ldb, p.block_k, p.b_boxes, swz)))
+      p.b_form = SLAB_MN3;
+    if (p.b_form == SLAB_MN2) {
+      ok = ok && make_map(&plan->map_b, g.B, eb, g.N, g.K, ldb, slab_elems, p.block_k, swz);
+      if (x3) ok = ok && make_map(&plan->map_b_lo, g.B_lo, eb, g.N, g.K, ldb, slab_elems, p.block_k, swz);
+    }
   } else {
+    p.b_form = SLAB_K;
     p.b_boxes = 1;
     p.b_box_bytes = p.b_stage_bytes;
     p.b_lbo = 16;
@@ -1532,7 +1283,8 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
 void gemm_tc_plan_destroy(TcPlan* p) { delete p; }
 
 bool gemm_tc_plan_set_mask(TcPlan* plan, uint32_t* mask_out, const uint32_t* mask_in, long long ld_words) {
-  if (!plan || !plan->p.tma_store || plan->p.N % 32 != 0 || ld_words * 32 < plan->p.N) return false;
+  if (!plan || !plan->p.tma_store || ld_words * 32 < plan->p.N) return false;
+  // a last word of fewer than 32 columns: the accumulator columns beyond N are zero, so its spare bits are too
   if (mask_out && plan->p.epilogue != EPI_RELU) return false;
   if (mask_in && plan->p.epilogue != EPI_MASK) return false;
   plan->p.mask_out = mask_out;
@@ -1551,12 +1303,15 @@ cudaError_t gemm_tc_launch(const TcPlan* plan, cudaStream_t stream, unsigned int
   {
     std::lock_guard<std::mutex> attr_lock(attr_mutex);
     if (!(attr_set >> (dev & 63) & 1ull)) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-      if (e != cudaSuccess) return e;
+      const void* kernels[] = {
+          (const void*)gemm_tc_kernel<1, KIND_BF16>, (const void*)gemm_tc_kernel<1, KIND_TF32>,
+          (const void*)gemm_tc_kernel<1, KIND_X3>,   (const void*)gemm_tc_kernel<2, KIND_BF16>,
+          (const void*)gemm_tc_kernel<2, KIND_TF32>, (const void*)gemm_tc_pair_kernel<KIND_BF16>,
+          (const void*)gemm_tc_pair_kernel<KIND_TF32>};
+      for (const void* k : kernels) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        if (e != cudaSuccess) return e;
+      }
       attr_set |= 1ull << (dev & 63);
     }
   }
@@ -1575,14 +1330,14 @@ cudaError_t gemm_tc_launch(const TcPlan* plan, cudaStream_t stream, unsigned int
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel, plan->map_a, plan->map_b, plan->map_c, p);
+    return cudaLaunchKernelEx(&cfg, p.kind_tf32 ? gemm_tc_pair_kernel<KIND_TF32> : gemm_tc_pair_kernel<KIND_BF16>,
+                              plan->map_a, plan->map_b, plan->map_c, p);
   }
-  if (p.sub_m == 2)
-    gemm_tc_kernel<2><<<plan->grid, NUM_THREADS_SUB2, plan->smem, stream>>>(
-        plan->map_a, plan->map_b, plan->map_c, plan->map_a_lo, plan->map_b_lo, plan->map_c_lo, p);
-  else
-    gemm_tc_kernel<1><<<plan->grid, NUM_THREADS, plan->smem, stream>>>(
-        plan->map_a, plan->map_b, plan->map_c, plan->map_a_lo, plan->map_b_lo, plan->map_c_lo, p);
+  auto kernel = p.sub_m == 2 ? (p.kind_tf32 ? gemm_tc_kernel<2, KIND_TF32> : gemm_tc_kernel<2, KIND_BF16>)
+                : p.x3       ? gemm_tc_kernel<1, KIND_X3>
+                : p.kind_tf32 ? gemm_tc_kernel<1, KIND_TF32> : gemm_tc_kernel<1, KIND_BF16>;
+  kernel<<<plan->grid, p.sub_m == 2 ? NUM_THREADS_SUB2 : NUM_THREADS, plan->smem, stream>>>(
+      plan->map_a, plan->map_b, plan->map_c, plan->map_a_lo, plan->map_b_lo, plan->map_c_lo, p);
   return cudaGetLastError();
 }
 
