@@ -175,3 +175,24 @@ def test_optional_tile_schedules(dev, oracle, variant, monkeypatch):
                     assert row_err.max() <= 1e-4
     finally:
         oracle.use_builtin_gemm()
+
+
+# CUDA-core kernels at the edges of their dispatch: 128/64/32-wide tiles with remainders, rows that are and are
+# not whole 16-byte pieces, the narrow (N <= 16) and short (M <= 16) forms on both sides of their limits.
+# Bound: the oracle adds in k order in fp32 as the tile kernel does (2e-5 covers the other order of the two
+# split-K forms: K terms, unit roundoff 6e-8, observed growth sqrt(K)).
+@pytest.mark.parametrize("shape", [(33, 65, 31), (129, 64, 64), (70, 1, 64), (70, 2, 63), (77, 16, 200), (77, 17, 200),
+                                   (1, 70, 64), (2, 96, 129), (16, 100, 321), (17, 100, 321), (1300, 1100, 20),
+                                   (5, 3, 1), (1000, 10, 300), (10, 300, 1000)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("form", list(FORMS))
+def test_cuda_core_dispatch_edges(dev, oracle, form, shape):
+    from tbb_test_b200 import _capi as K
+    m, n, k = shape
+    ta, tb, a, b = operands(oracle, form, m, n, k, 101)
+    ref = oracle.sgemm(ta, tb, a, b)
+    c = dev.sgemm_host(K.PREC_FP32, ta, tb, a, b)
+    assert rel_fro(c, ref) <= TOL["fp32"]
+    aux = oracle.fill_uniform(m, n, 102, -1.0, 1.0)
+    assert rel_fro(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_RELU), np.maximum(ref, 0)) <= 2 * TOL["fp32"]
+    assert rel_fro(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_MASK, aux=aux),
+                   ref * (aux > 0)) <= 2 * TOL["fp32"]
