@@ -112,6 +112,10 @@ cudaError_t sgd_launch(float* w, const void* g, int g_type, __nv_bfloat16* w_bf1
                        int sm_count, cudaStream_t s, float* w_lo = nullptr);
 // *out += sum of the 32-bit words of buf modulo 2^64 (out must be zeroed by the caller)
 cudaError_t fingerprint_launch(const void* buf, size_t bytes, unsigned long long* out, cudaStream_t s);
+// The same for rows x cols 16-bit elements stored with a row pitch of ld elements, paired into words as if
+// the rows were dense (a last unpaired element is left out, as by fingerprint_launch)
+cudaError_t fingerprint_rows16_launch(const void* buf, int rows, int cols, int ld, unsigned long long* out,
+                                      cudaStream_t s);
 // dst = src - tf32(src): the part of an fp32 value the tensor core drops when it reads it as tf32
 cudaError_t split_lo_launch(const float* src, float* dst, size_t n, cudaStream_t s);
 cudaError_t fill_uniform_launch(void* buf, int type, size_t n, uint64_t seed, float lo, float hi,

@@ -189,6 +189,15 @@ __global__ void __launch_bounds__(256) fingerprint_kernel(const uint32_t* __rest
   if (threadIdx.x == 0) atomicAdd(out, red[0]);
 }
 
+__global__ void __launch_bounds__(256) fingerprint_rows16_kernel(const unsigned short* __restrict__ buf, int cols,
+                                                                 int ld, size_t n, unsigned long long* __restrict__ out) {
+  unsigned long long local = 0;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+    local += (unsigned long long)buf[i / cols * ld + i % cols] << ((i & 1) * 16);
+  atomicAdd(out, local);
+}
+
 int grid_for(size_t work_items, int sm_count, int per_sm) {
   size_t blocks = (work_items + 255) / 256;
   size_t cap = (size_t)sm_count * per_sm;
@@ -264,6 +273,15 @@ cudaError_t fingerprint_launch(const void* buf, size_t bytes, unsigned long long
   const size_t n = bytes / 4;  // whole 32-bit words (the buffers fingerprinted here are multiples of 4 bytes)
   if (n == 0) return cudaSuccess;
   fingerprint_kernel<<<grid_for(n, device_sms(), 8), 256, 0, s>>>(static_cast<const uint32_t*>(buf), n, out);
+  return cudaGetLastError();
+}
+
+cudaError_t fingerprint_rows16_launch(const void* buf, int rows, int cols, int ld, unsigned long long* out,
+                                      cudaStream_t s) {
+  const size_t n = (size_t)rows * cols / 2 * 2;
+  if (n == 0) return cudaSuccess;
+  fingerprint_rows16_kernel<<<grid_for(n, device_sms(), 8), 256, 0, s>>>(static_cast<const unsigned short*>(buf), cols,
+                                                                         ld, n, out);
   return cudaGetLastError();
 }
 

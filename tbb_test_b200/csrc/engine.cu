@@ -47,6 +47,11 @@ struct Site {
 struct b2_handle {
   b2_config cfg;
   std::vector<int> nf;
+  // Row pitch (elements) of every matrix with nf[l] columns: activations, gradients, weights of layer l.
+  // With bf16 operands on the tensor cores it is nf[l] rounded up to 8, whole 16-byte pieces, which is what
+  // TMA can address; else rows are dense. The padding is zero from the allocation on and no kernel
+  // gives it another value (stores are clipped at nf[l]; 0 - lr * 0 in the updates), or it is never read.
+  std::vector<int> ld;
   int L = 0, b0 = 0, b1 = 0, bl = 0, sms = 148;
   int gemm_sms = 148;  // SMs the persistent GEMM kernels of the step occupy (sms - comm_sms)
   int op_type = T_F32;    // element type of GEMM operands held on the device
@@ -191,6 +196,8 @@ void batch_range(int batch, int world, int rank, int* b, int* e) {
   *e = hi;
 }
 
+size_t layer_elems(const b2_handle* h, int l) { return (size_t)h->nf[l + 1] * h->ld[l]; }
+
 int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
   s.d.ws = h->tc_ws;
   s.d.ws_flags = h->tc_ws_flags;
@@ -281,31 +288,32 @@ cudaError_t copy_rows(void* dst, size_t dpitch, const void* src, size_t spitch, 
 
 // Host (ld) <-> dense device matrix of `type`, through the fp32 staging buffer when
 // the device holds bf16.
-int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t ld, int rows, int cols) {
+int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t ld, int rows, int cols, int pitch) {
   if (rows <= 0 || cols <= 0) return B2_OK;
   if (type == T_F32) {
-    CK(h, copy_rows(dev, (size_t)cols * 4, host, ld * 4, (size_t)cols * 4, (size_t)rows, cudaMemcpyHostToDevice,
+    CK(h, copy_rows(dev, (size_t)pitch * 4, host, ld * 4, (size_t)cols * 4, (size_t)rows, cudaMemcpyHostToDevice,
                     h->s_main));
   } else {
-    if ((size_t)rows * cols > h->stage_elems) return fail(h, B2_ERR_INVALID, "staging buffer too small");
-    CK(h, copy_rows(h->stage, (size_t)cols * 4, host, ld * 4, (size_t)cols * 4, (size_t)rows,
+    if ((size_t)rows * pitch > h->stage_elems) return fail(h, B2_ERR_INVALID, "staging buffer too small");
+    if (pitch != cols) CK(h, cudaMemsetAsync(h->stage, 0, (size_t)rows * pitch * 4, h->s_main));
+    CK(h, copy_rows(h->stage, (size_t)pitch * 4, host, ld * 4, (size_t)cols * 4, (size_t)rows,
                     cudaMemcpyHostToDevice, h->s_main));
-    CK(h, convert_f32_to_bf16(h->stage, (__nv_bfloat16*)dev, (size_t)rows * cols, h->s_main));
+    CK(h, convert_f32_to_bf16(h->stage, (__nv_bfloat16*)dev, (size_t)rows * pitch, h->s_main));
     ++h->launches;
   }
   return B2_OK;
 }
 
-int download_matrix(b2_handle* h, const void* dev, int type, float* host, size_t ld, int rows, int cols) {
+int download_matrix(b2_handle* h, const void* dev, int type, float* host, size_t ld, int rows, int cols, int pitch) {
   if (rows <= 0 || cols <= 0) return B2_OK;
   const void* src = dev;
   if (type == T_BF16) {
-    if ((size_t)rows * cols > h->stage_elems) return fail(h, B2_ERR_INVALID, "staging buffer too small");
-    CK(h, convert_bf16_to_f32((const __nv_bfloat16*)dev, h->stage, (size_t)rows * cols, h->s_main));
+    if ((size_t)rows * pitch > h->stage_elems) return fail(h, B2_ERR_INVALID, "staging buffer too small");
+    CK(h, convert_bf16_to_f32((const __nv_bfloat16*)dev, h->stage, (size_t)rows * pitch, h->s_main));
     ++h->launches;
     src = h->stage;
   }
-  CK(h, cudaMemcpy2DAsync(host, ld * 4, src, (size_t)cols * 4, (size_t)cols * 4, rows, cudaMemcpyDeviceToHost,
+  CK(h, cudaMemcpy2DAsync(host, ld * 4, src, (size_t)pitch * 4, (size_t)cols * 4, rows, cudaMemcpyDeviceToHost,
                           h->s_main));
   CK(h, cudaStreamSynchronize(h->s_main));
   return B2_OK;
@@ -332,15 +340,15 @@ int build_sites(b2_handle* h) {
     }
   }
   for (int l = 0; l < L; ++l) {
-    const int fi = h->nf[l], fo = h->nf[l + 1];
+    const int fi = h->nf[l], fo = h->nf[l + 1], li = h->ld[l], lo = h->ld[l + 1];
     const void* wop = h->op_type == T_BF16 ? (const void*)h->w16[l] : (const void*)h->w[l];
     // forward: A[l+1] = A[l] * W[l]^T (mlp_omp.cc:474-488)
     GemmDesc f{};
     f.M = bl; f.N = fo; f.K = fi;
-    f.A = h->act[l]; f.sAm = fi; f.sAk = 1;
-    f.B = wop; f.sBk = 1; f.sBn = fi;
+    f.A = h->act[l]; f.sAm = li; f.sAk = 1;
+    f.B = wop; f.sBk = 1; f.sBn = li;
     f.C = (l == L - 1) ? (void*)h->y : h->act[l + 1];
-    f.ldc = fo;
+    f.ldc = lo;
     f.alpha = 1.f; f.beta = 0.f;
     f.epilogue = (baseline && l < L - 1) ? EPI_RELU : EPI_NONE;
     f.in_type = h->op_type;
@@ -355,9 +363,9 @@ int build_sites(b2_handle* h) {
     // weight gradient: dW[l] = dZ[l]^T * A[l] over this rank's rows (mlp_omp.cc:565-580)
     GemmDesc g{};
     g.M = fo; g.N = fi; g.K = bl;
-    g.A = h->dz[l]; g.sAm = 1; g.sAk = fo;
-    g.B = h->act[l]; g.sBk = fi; g.sBn = 1;
-    g.C = h->dw[l]; g.ldc = fi;
+    g.A = h->dz[l]; g.sAm = 1; g.sAk = lo;
+    g.B = h->act[l]; g.sBk = li; g.sBn = 1;
+    g.C = h->dw[l]; g.ldc = li;
     g.alpha = 1.f; g.beta = 0.f;
     g.epilogue = EPI_NONE;
     g.in_type = h->op_type;
@@ -371,13 +379,13 @@ int build_sites(b2_handle* h) {
     // input gradient: dA[l] = dZ[l] * W[l] (mlp_omp.cc:655-671), masked by ReLU'(A[l])
     GemmDesc b{};
     b.M = bl; b.N = fi; b.K = fo;
-    b.A = h->dz[l]; b.sAm = fo; b.sAk = 1;
-    b.B = wop; b.sBk = fi; b.sBn = 1;
+    b.A = h->dz[l]; b.sAm = lo; b.sAk = 1;
+    b.B = wop; b.sBk = li; b.sBn = 1;
     b.C = (l == 0) ? h->dinput : h->dz[l - 1];
-    b.ldc = fi;
+    b.ldc = li;
     b.alpha = 1.f; b.beta = 0.f;
     b.epilogue = (baseline && l > 0) ? EPI_MASK : EPI_NONE;
-    b.aux = h->act[l]; b.ldaux = fi;
+    b.aux = h->act[l]; b.ldaux = li;
     b.in_type = h->op_type;
     b.out_type = h->op_type;
     if (h->x3) {
@@ -403,7 +411,7 @@ int build_sites(b2_handle* h) {
   // its consumer (input gradient of the layer itself) run on the tensor-core kernel
   for (int l = 1; l < L; ++l) {
     if (!h->relu_bits[l] || !h->fwd[l - 1].plan || !h->dgrad[l].plan) continue;
-    const long long ldw = h->nf[l] / 32;
+    const long long ldw = (h->nf[l] + 31) / 32;
     if (l == 1 && !h->fwd0_alt.plan) continue;
     if (!gemm_tc_plan_set_mask(h->fwd[l - 1].plan, h->relu_bits[l], nullptr, ldw)) continue;
     if (!gemm_tc_plan_set_mask(h->dgrad[l].plan, nullptr, h->relu_bits[l], ldw)) {
@@ -444,7 +452,7 @@ int sum_gradients(b2_handle* h, size_t begin, size_t count, cudaStream_t st) {
 }
 
 int layer_update(b2_handle* h, int l, cudaStream_t st, bool timed) {
-  const size_t n = (size_t)h->nf[l + 1] * h->nf[l];
+  const size_t n = layer_elems(h, l);
   if (h->cfg.world_size > 1 && h->cfg.allreduce) {
     if (timed) CK(h, cudaEventRecord(phase_ev(h, l, B2_T_ALLREDUCE, 0), st));
     int rc = sum_gradients(h, h->dw_off[l], n, st);
@@ -464,7 +472,7 @@ void bucket_range(const b2_handle* h, int low, int high, size_t* begin, size_t* 
 int bucket_allreduce(b2_handle* h, int low, int high, cudaStream_t st, bool timed) {
   if (!(h->cfg.world_size > 1 && h->cfg.allreduce)) return B2_OK;
   const size_t begin = h->dw_off[high];
-  const size_t end = h->dw_off[low] + (size_t)h->nf[low + 1] * h->nf[low];
+  const size_t end = h->dw_off[low] + layer_elems(h, low);
   if (timed) CK(h, cudaEventRecord(phase_ev(h, low, B2_T_ALLREDUCE, 0), st));
   int rc = sum_gradients(h, begin, end - begin, st);
   if (rc) return rc;
@@ -578,7 +586,7 @@ int gather_masters(b2_handle* h) {
 }
 
 int layer_sgd(b2_handle* h, int l, cudaStream_t st, bool timed) {
-  const size_t n = (size_t)h->nf[l + 1] * h->nf[l];
+  const size_t n = layer_elems(h, l);
   if (timed) CK(h, cudaEventRecord(phase_ev(h, l, B2_T_WGT_UPDATE, 0), st));
   CK(h, sgd_launch(h->w[l], h->dw[l], h->grad_type, h->op_type == T_BF16 ? h->w16[l] : nullptr, n, h->cfg.lr,
                    h->sms, st, h->x3 ? h->w_lo[l] : nullptr));
@@ -621,7 +629,7 @@ int enqueue_step(b2_handle* h, bool timed, int slot = 0) {
     if (timed) CK(h, cudaEventRecord(phase_ev(h, l, B2_T_FWD, 1), sm));
   }
   {
-    const size_t n = (size_t)h->bl * h->nf[L];
+    const size_t n = (size_t)h->bl * h->ld[L];
     const bool baseline = h->cfg.mode == B2_MODE_BASELINE;
     CK(h, loss_grad_launch(h->y, target, h->dz[L - 1], h->op_type, n, baseline ? 1 : 0,
                            1.0f / (float)h->cfg.batch, baseline ? 1.0 / (double)h->cfg.batch : 1.0, loss_acc, sm,
@@ -636,7 +644,7 @@ int enqueue_step(b2_handle* h, bool timed, int slot = 0) {
     if (h->wgrad[l].active) {
       if ((rc = run_site(h, (l == 0 && slot) ? h->wgrad0_alt : h->wgrad[l], sw))) return rc;
     } else {  // a rank without batch rows contributes a zero gradient
-      CK(h, cudaMemsetAsync(h->dw[l], 0, (size_t)h->nf[l + 1] * h->nf[l] * esize(h->grad_type), sw));
+      CK(h, cudaMemsetAsync(h->dw[l], 0, layer_elems(h, l) * esize(h->grad_type), sw));
     }
     if (timed) CK(h, cudaEventRecord(phase_ev(h, l, B2_T_WGT_GRAD, 1), sw));
     const bool closes_bucket = (h->bucket_low[l] == l);
@@ -984,20 +992,22 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
   h->act_lo.assign(L + 1, nullptr);
   h->dz_lo.assign(L, nullptr);
   size_t max_elems = 16;
+  h->ld = h->nf;
+  if (h->op_type == T_BF16 && use_tc(h))
+    for (int& v : h->ld) v = (v + 7) / 8 * 8;
   for (int l = 0; l < L; ++l) {
-    const size_t nw = (size_t)h->nf[l + 1] * h->nf[l];
-    TRY(dev_alloc(h, &h->dz[l], bl * h->nf[l + 1] * esize(h->op_type)));
-    TRY(dev_alloc(h, &h->act[l], bl * h->nf[l] * esize(h->op_type)));
+    const size_t nw = layer_elems(h, l);
+    TRY(dev_alloc(h, &h->dz[l], bl * h->ld[l + 1] * esize(h->op_type)));
+    TRY(dev_alloc(h, &h->act[l], bl * h->ld[l] * esize(h->op_type)));
     if (h->x3) {
-      TRY(dev_alloc(h, &h->dz_lo[l], bl * h->nf[l + 1] * 4));
-      TRY(dev_alloc(h, &h->act_lo[l], bl * h->nf[l] * 4));
+      TRY(dev_alloc(h, &h->dz_lo[l], bl * h->ld[l + 1] * 4));
+      TRY(dev_alloc(h, &h->act_lo[l], bl * h->ld[l] * 4));
     }
-    if (l > 0 && cfg->mode == B2_MODE_BASELINE && cfg->precision != B2_PREC_FP32 && !cfg->force_simt &&
-        h->nf[l] % 32 == 0)
-      TRY(dev_alloc(h, &h->relu_bits[l], bl * (size_t)(h->nf[l] / 32) * sizeof(uint32_t)));
+    if (l > 0 && cfg->mode == B2_MODE_BASELINE && use_tc(h))
+      TRY(dev_alloc(h, &h->relu_bits[l], bl * (size_t)((h->nf[l] + 31) / 32) * sizeof(uint32_t)));
     if (nw > max_elems) max_elems = nw;
-    if (bl * h->nf[l] > max_elems) max_elems = bl * h->nf[l];
-    if (bl * h->nf[l + 1] > max_elems) max_elems = bl * h->nf[l + 1];
+    if (bl * h->ld[l] > max_elems) max_elems = bl * h->ld[l];
+    if (bl * h->ld[l + 1] > max_elems) max_elems = bl * h->ld[l + 1];
   }
   {
     // gradient and weight slabs, last layer first; every layer is padded to a multiple of
@@ -1006,9 +1016,9 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     h->dw_off.assign(L, 0);
     h->dw_pad.assign(L, 0);
     const size_t es = esize(h->grad_type);
-    std::vector<size_t> layer_elems(L);
-    for (int l = 0; l < L; ++l) layer_elems[l] = (size_t)h->nf[l + 1] * h->nf[l];
-    const size_t total = plan_slab_layout(layer_elems.data(), L, cfg->world_size, h->dw_off.data(), h->dw_pad.data());
+    std::vector<size_t> elems(L);
+    for (int l = 0; l < L; ++l) elems[l] = layer_elems(h, l);
+    const size_t total = plan_slab_layout(elems.data(), L, cfg->world_size, h->dw_off.data(), h->dw_pad.data());
     {
       const char* ub = getenv("B2_NCCL_UB");
       h->nccl_ub = ub && ub[0] == '1' && cfg->world_size > 1 && cfg->allreduce && nccl_api().ok &&
@@ -1038,7 +1048,7 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     // buckets of consecutive layers (rule and rationale: bucket_plan.h); B2_BUCKET_GROWTH
     // overrides the factor between consecutive buckets
     std::vector<size_t> layer_bytes(L);
-    for (int l = 0; l < L; ++l) layer_bytes[l] = (size_t)h->nf[l + 1] * h->nf[l] * es;
+    for (int l = 0; l < L; ++l) layer_bytes[l] = elems[l] * es;
     double growth = 0.0;
     if (const char* e = getenv("B2_BUCKET_GROWTH")) growth = atof(e);
     h->bucket_low.assign(L, 0);
@@ -1081,18 +1091,18 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
       }
     }
   }
-  TRY(dev_alloc(h, &h->y, bl * h->nf[L] * 4));
-  TRY(dev_alloc(h, &h->target, bl * h->nf[L] * 4));
-  TRY(dev_alloc(h, &h->dinput, bl * h->nf[0] * esize(h->op_type)));
+  TRY(dev_alloc(h, &h->y, bl * h->ld[L] * 4));
+  TRY(dev_alloc(h, &h->target, bl * h->ld[L] * 4));
+  TRY(dev_alloc(h, &h->dinput, bl * h->ld[0] * esize(h->op_type)));
   if (h->op_type == T_BF16 || h->grad_type == T_BF16) {
     h->stage_elems = max_elems;
     TRY(dev_alloc(h, &h->stage, max_elems * 4));
   }
-  TRY(dev_alloc(h, &h->act0_alt, bl * h->nf[0] * esize(h->op_type)));
-  if (h->x3) TRY(dev_alloc(h, &h->act0_alt_lo, bl * h->nf[0] * 4));
-  TRY(dev_alloc(h, &h->target_alt, bl * h->nf[L] * 4));
+  TRY(dev_alloc(h, &h->act0_alt, bl * h->ld[0] * esize(h->op_type)));
+  if (h->x3) TRY(dev_alloc(h, &h->act0_alt_lo, bl * h->ld[0] * 4));
+  TRY(dev_alloc(h, &h->target_alt, bl * h->ld[L] * 4));
   if (h->op_type == T_BF16)
-    for (int i = 0; i < 2; ++i) TRY(dev_alloc(h, &h->xstage[i], bl * h->nf[0] * 4));
+    for (int i = 0; i < 2; ++i) TRY(dev_alloc(h, &h->xstage[i], bl * h->ld[0] * 4));
   TRY(dev_alloc(h, &h->loss_dev, 2 * sizeof(double)));
   TRYCK(cudaHostAlloc((void**)&h->loss_host, 2 * sizeof(double), cudaHostAllocDefault));
   TRYCK(cudaStreamCreateWithFlags(&h->s_copy, cudaStreamNonBlocking));
@@ -1195,14 +1205,14 @@ int b2_upload_weights(b2_handle* h, int l, const float* host, size_t ld) {
   LAYER_OK(h, l, h->L - 1);
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
   const int rows = h->nf[l + 1], cols = h->nf[l];
-  CK(h, cudaMemcpy2DAsync(h->w[l], (size_t)cols * 4, host, ld * 4, (size_t)cols * 4, rows, cudaMemcpyHostToDevice,
+  CK(h, cudaMemcpy2DAsync(h->w[l], (size_t)h->ld[l] * 4, host, ld * 4, (size_t)cols * 4, rows, cudaMemcpyHostToDevice,
                           h->s_main));
   if (h->op_type == T_BF16) {
-    CK(h, convert_f32_to_bf16(h->w[l], h->w16[l], (size_t)rows * cols, h->s_main));
+    CK(h, convert_f32_to_bf16(h->w[l], h->w16[l], layer_elems(h, l), h->s_main));
     ++h->launches;
   }
   if (h->x3) {
-    CK(h, split_lo_launch(h->w[l], h->w_lo[l], (size_t)rows * cols, h->s_main));
+    CK(h, split_lo_launch(h->w[l], h->w_lo[l], layer_elems(h, l), h->s_main));
     ++h->launches;
   }
   CK(h, cudaStreamSynchronize(h->s_main));
@@ -1215,16 +1225,16 @@ int b2_download_weights(b2_handle* h, int l, float* host, size_t ld) {
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
   int rc = gather_masters(h);  // collective when ranks hold current masters only for their own slices
   if (rc) return rc;
-  return download_matrix(h, h->w[l], T_F32, host, ld, h->nf[l + 1], h->nf[l]);
+  return download_matrix(h, h->w[l], T_F32, host, ld, h->nf[l + 1], h->nf[l], h->ld[l]);
 }
 
 int b2_upload_input(b2_handle* h, const float* host, size_t ld) {
   ENTER(h);
   if (!host || ld < (size_t)h->nf[0]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  int rc = upload_matrix(h, h->act[0], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[0]);
+  int rc = upload_matrix(h, h->act[0], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[0], h->ld[0]);
   if (rc) return rc;
   if (h->x3 && h->bl > 0) {
-    CK(h, split_lo_launch(static_cast<const float*>(h->act[0]), h->act_lo[0], (size_t)h->bl * h->nf[0], h->s_main));
+    CK(h, split_lo_launch(static_cast<const float*>(h->act[0]), h->act_lo[0], (size_t)h->bl * h->ld[0], h->s_main));
     ++h->launches;
   }
   CK(h, cudaStreamSynchronize(h->s_main));
@@ -1234,7 +1244,7 @@ int b2_upload_input(b2_handle* h, const float* host, size_t ld) {
 int b2_upload_target(b2_handle* h, const float* host, size_t ld) {
   ENTER(h);
   if (!host || ld < (size_t)h->nf[h->L]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  int rc = upload_matrix(h, h->target, T_F32, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[h->L]);
+  int rc = upload_matrix(h, h->target, T_F32, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[h->L], h->ld[h->L]);
   if (rc) return rc;
   CK(h, cudaStreamSynchronize(h->s_main));
   return B2_OK;
@@ -1244,35 +1254,35 @@ int b2_download_activation(b2_handle* h, int l, float* host, size_t ld) {
   ENTER(h);
   LAYER_OK(h, l, h->L);
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  if (l == h->L) return download_matrix(h, h->y, T_F32, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l]);
-  return download_matrix(h, h->act[l], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l]);
+  if (l == h->L) return download_matrix(h, h->y, T_F32, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l], h->ld[l]);
+  return download_matrix(h, h->act[l], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l], h->ld[l]);
 }
 
 int b2_download_dz(b2_handle* h, int l, float* host, size_t ld) {
   ENTER(h);
   LAYER_OK(h, l, h->L - 1);
   if (!host || ld < (size_t)h->nf[l + 1]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  return download_matrix(h, h->dz[l], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l + 1]);
+  return download_matrix(h, h->dz[l], h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[l + 1], h->ld[l + 1]);
 }
 
 int b2_download_input_grad(b2_handle* h, float* host, size_t ld) {
   ENTER(h);
   if (!host || ld < (size_t)h->nf[0]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  return download_matrix(h, h->dinput, h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[0]);
+  return download_matrix(h, h->dinput, h->op_type, host + (size_t)h->b0 * ld, ld, h->bl, h->nf[0], h->ld[0]);
 }
 
 int b2_download_weight_grad(b2_handle* h, int l, float* host, size_t ld) {
   ENTER(h);
   LAYER_OK(h, l, h->L - 1);
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  return download_matrix(h, h->dw[l], h->grad_type, host, ld, h->nf[l + 1], h->nf[l]);
+  return download_matrix(h, h->dw[l], h->grad_type, host, ld, h->nf[l + 1], h->nf[l], h->ld[l]);
 }
 
 int b2_upload_weight_grad(b2_handle* h, int l, const float* host, size_t ld) {
   ENTER(h);
   LAYER_OK(h, l, h->L - 1);
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  int rc = upload_matrix(h, h->dw[l], h->grad_type, host, ld, h->nf[l + 1], h->nf[l]);
+  int rc = upload_matrix(h, h->dw[l], h->grad_type, host, ld, h->nf[l + 1], h->nf[l], h->ld[l]);
   if (rc) return rc;
   CK(h, cudaStreamSynchronize(h->s_main));
   return B2_OK;
@@ -1442,14 +1452,16 @@ int b2_train_step_host(b2_handle* h, const float* x, size_t ldx, const float* t,
   int rc;
   // fwd(0) of this step must not start before the copy; the copy must not start
   // before the previous step stopped reading act[0] - both hold on the main stream.
-  if ((rc = upload_matrix(h, h->act[0], h->op_type, x + (size_t)h->b0 * ldx, ldx, h->bl, h->nf[0]))) return rc;
+  if ((rc = upload_matrix(h, h->act[0], h->op_type, x + (size_t)h->b0 * ldx, ldx, h->bl, h->nf[0], h->ld[0])))
+    return rc;
   if (h->x3 && h->bl > 0) {
-    CK(h, split_lo_launch(static_cast<const float*>(h->act[0]), h->act_lo[0], (size_t)h->bl * h->nf[0], h->s_main));
+    CK(h, split_lo_launch(static_cast<const float*>(h->act[0]), h->act_lo[0], (size_t)h->bl * h->ld[0], h->s_main));
     ++h->launches;
   }
   if (t) {
     if (ldt < (size_t)h->nf[h->L]) return fail(h, B2_ERR_INVALID, "bad target matrix");
-    if ((rc = upload_matrix(h, h->target, T_F32, t + (size_t)h->b0 * ldt, ldt, h->bl, h->nf[h->L]))) return rc;
+    if ((rc = upload_matrix(h, h->target, T_F32, t + (size_t)h->b0 * ldt, ldt, h->bl, h->nf[h->L], h->ld[h->L])))
+      return rc;
   }
   if ((rc = b2_step(h, 1))) return rc;
   if (loss) return b2_loss(h, loss);
@@ -1466,26 +1478,27 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
     return fail(h, B2_ERR_STATE, "two steps already in flight: call b2_wait_loss first");
   const int slot = (int)(h->async_issued & 1);
   const int rows = h->bl, f0 = h->nf[0], fl = h->nf[h->L];
+  const size_t p0 = (size_t)h->ld[0], pl = (size_t)h->ld[h->L];
   int rc;
   // the copy may start once the step that last computed on this slot is done with it
   if (h->slot_used[slot]) CK(h, cudaStreamWaitEvent(h->s_copy, h->ev_slot_free[slot], 0));
   if (rows > 0) {
     void* act0 = slot ? h->act0_alt : h->act[0];
     void* land = h->op_type == T_BF16 ? (void*)h->xstage[slot] : act0;
-    CK(h, copy_rows(land, (size_t)f0 * 4, x + (size_t)h->b0 * ldx, ldx * 4, (size_t)f0 * 4, (size_t)rows,
+    CK(h, copy_rows(land, p0 * 4, x + (size_t)h->b0 * ldx, ldx * 4, (size_t)f0 * 4, (size_t)rows,
                     cudaMemcpyHostToDevice, h->s_copy));
     if (h->op_type == T_BF16) {
-      CK(h, convert_f32_to_bf16(h->xstage[slot], (__nv_bfloat16*)act0, (size_t)rows * f0, h->s_copy));
+      CK(h, convert_f32_to_bf16(h->xstage[slot], (__nv_bfloat16*)act0, (size_t)rows * p0, h->s_copy));
       ++h->launches;
     }
     if (h->x3) {
-      CK(h, split_lo_launch(static_cast<const float*>(act0), slot ? h->act0_alt_lo : h->act_lo[0], (size_t)rows * f0,
+      CK(h, split_lo_launch(static_cast<const float*>(act0), slot ? h->act0_alt_lo : h->act_lo[0], (size_t)rows * p0,
                             h->s_copy));
       ++h->launches;
     }
     if (t)
-      CK(h, copy_rows(slot ? h->target_alt : h->target, (size_t)fl * 4, t + (size_t)h->b0 * ldt, ldt * 4,
-                      (size_t)fl * 4, (size_t)rows, cudaMemcpyHostToDevice, h->s_copy));
+      CK(h, copy_rows(slot ? h->target_alt : h->target, pl * 4, t + (size_t)h->b0 * ldt, ldt * 4, (size_t)fl * 4,
+                      (size_t)rows, cudaMemcpyHostToDevice, h->s_copy));
   }
   CK(h, cudaEventRecord(h->ev_copied[slot], h->s_copy));
   CK(h, cudaStreamWaitEvent(h->s_main, h->ev_copied[slot], 0));
@@ -1701,7 +1714,7 @@ int b2_p2p_connect(b2_handle* h, const void* descs, size_t max_bytes) {
   const size_t es = esize(h->grad_type);
   for (int l = 0; l < h->L; ++l) {
     if (h->bucket_low[l] != l) continue;
-    const size_t bytes = (h->dw_off[l] + (size_t)h->nf[l + 1] * h->nf[l] - h->dw_off[h->bucket_high[l]]) * es;
+    const size_t bytes = (h->dw_off[l] + layer_elems(h, l) - h->dw_off[h->bucket_high[l]]) * es;
     h->bucket_full[l] = (max_bytes > 0 && bytes <= max_bytes) ? 1 : 0;
   }
   h->p2p_max_bytes = max_bytes;
@@ -1921,10 +1934,12 @@ int b2_weights_fingerprint(b2_handle* h, int l, unsigned long long* out) {
   LAYER_OK(h, l, h->L - 1);
   if (!out) return fail(h, B2_ERR_INVALID, "null output");
   unsigned long long* acc = h->fp_dev;
-  const size_t n = (size_t)h->nf[l + 1] * h->nf[l];
+  const size_t n = layer_elems(h, l);
   CK(h, cudaStreamSynchronize(h->s_main));
   CK(h, cudaMemsetAsync(acc, 0, sizeof *acc, h->s_main));
-  if (h->op_type == T_BF16)
+  if (h->op_type == T_BF16 && (h->nf[l] & 1))  // padded rows of odd length: pair the elements as in dense rows
+    CK(h, fingerprint_rows16_launch(h->w16[l], h->nf[l + 1], h->nf[l], h->ld[l], acc, h->s_main));
+  else if (h->op_type == T_BF16)
     CK(h, fingerprint_launch(h->w16[l], n * 2, acc, h->s_main));
   else
     CK(h, fingerprint_launch(h->w[l], n * 4, acc, h->s_main));

@@ -446,3 +446,44 @@ def test_pinned_memory_near_the_gpu(native):
         losses.append(dev.train_step_host(xs.ctypes.data_as(K._fp), 128, ts.ctypes.data_as(K._fp), 64))
         dev.close()
     assert losses[0] == losses[1] and np.isfinite(losses[0])
+
+
+@pytest.mark.parametrize("nf,batch", [([123, 77, 201, 33], 130), ([784, 500, 300, 10], 200), ([65, 17, 16], 129),
+                                      ([40, 24, 1], 33)], ids=lambda v: "x".join(map(str, v)) if isinstance(v, list) else str(v))
+def test_bf16_padded_rows(native, oracle, nf, batch):
+    """Widths whose bf16 rows are not whole 16-byte pieces are stored with padded rows and run on the tensor
+    cores: every tensor of one step against the oracle that rounds at the same points (bound as above), the
+    same step through the pipelined host-fed call on both input slots, and the fingerprint of dense rows."""
+    import ctypes as C
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    out, (total, tc) = run_pair(oracle, nf, batch, "bf16", K.MODE_BASELINE, 1, 0.01, rounding=oracle.ROUND_BF16)
+    assert tc > 0
+    check(out, SAME_ROUNDING_TOL)
+    fp = C.POINTER(C.c_float)
+    x = np.ascontiguousarray(oracle.fill_normal(batch, nf[0], 7))
+    t = np.ascontiguousarray(oracle.fill_sign(batch, nf[-1], 8))
+    ws = [oracle.fill_uniform(nf[l + 1], nf[l], 20 + l, -0.3, 0.3) for l in range(len(nf) - 1)]
+    got = []
+    for fed in (False, True):
+        m = MLP(nf, batch, precision=K.PREC_BF16, lr=0.01)
+        for l, w in enumerate(ws):
+            m.upload_weights(l, w)
+        if fed:
+            for i in range(3):
+                m.train_step_host_async(x.ctypes.data_as(fp), nf[0], t.ctypes.data_as(fp), nf[-1])
+                if i:
+                    m.wait_loss()
+            m.wait_loss()
+        else:
+            m.upload_input(x)
+            m.upload_target(t)
+            m.step(3)
+        got.append([m.weights(l) for l in range(len(ws))])
+        bits = [oracle.round_bf16(w).view(np.uint32) >> 16 for w in got[-1]]
+        for l, b in enumerate(bits):
+            b = b.ravel()[: b.size // 2 * 2].astype(np.uint64)
+            assert m.weights_fingerprint(l) == int((b[0::2] + (b[1::2] << np.uint64(16))).sum(dtype=np.uint64))
+        m.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
