@@ -356,7 +356,8 @@ int b2_site_report(const b2_handle* h, int* tensor_core_sites, int* cuda_core_si
                    size_t reason_len);
 
 /* Number of kernels of this library launched on the handle since creation, and
- * how many of them were tensor-core (tcgen05) GEMMs. */
+ * the number of GEMMs run by its tensor-core (tcgen05) kernels: one per GEMM launch; a
+ * launch that computes whole training steps counts all tensor-core GEMMs of its steps. */
 int b2_launch_counts(const b2_handle* h, long long* total, long long* tensor_core);
 
 #ifdef __cplusplus

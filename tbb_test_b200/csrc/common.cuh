@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace b2 {
 
 enum Epilogue : int {
@@ -74,6 +76,41 @@ void gemm_tc_plan_destroy(TcPlan* p);
 // the mask epilogue (read instead of the activation). False when the plan cannot use one.
 bool gemm_tc_plan_set_mask(TcPlan* plan, uint32_t* mask_out, const uint32_t* mask_in, long long ld_words);
 cudaError_t gemm_tc_launch(const TcPlan* p, cudaStream_t stream, unsigned int* status);
+
+// Whole training steps as one launch (step_kernel.cu). The GEMMs of a step in an order in which each depends
+// only on earlier ones, with what its tiles wait for (indices into `gemms`, -1: nothing).
+enum StepRole : int { STEP_GEMM = 0, STEP_LAST_FWD = 1, STEP_WGRAD = 2 };
+struct StepGemm {
+  GemmDesc d;
+  int role;          // STEP_LAST_FWD: the epilogue also writes dz and the loss; STEP_WGRAD: it also updates w
+  int block_n;       // tile width, 64 or 128
+  int rows_of;       // a tile needs the same row block of that GEMM's result
+  int all_of;        // a tile needs that GEMM's whole result
+  int update_after;  // STEP_WGRAD: w may change once that GEMM (which reads it) is done
+  int prev_step[2];  // weight gradients of the previous step that must be done, update included
+  uint32_t* mask_out;
+  const uint32_t* mask_in;
+  long long ld_mask;
+  float* w;
+  __nv_bfloat16* w16;
+  float* w_lo;
+};
+struct StepSpec {
+  std::vector<StepGemm> gemms;
+  const float* target;
+  void* dz;
+  float* dz_lo;
+  int baseline;
+  float inv_batch;
+  double loss_scale;
+  double* loss;
+};
+struct StepPlan;
+int step_plan_counters(const StepSpec& s);  // counter words a launch needs, zeroed by the caller before it
+StepPlan* step_plan_create(const StepSpec& s, int sm_count);  // null: cannot be served
+void step_plan_destroy(StepPlan* p);
+cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
+                        cudaStream_t stream);
 
 // Small-message allreduce over peer memory (p2p_allreduce.cu). Every rank's gradient slab and
 // flag block are addressable from every rank (peer access within a process, IPC mappings

@@ -118,7 +118,12 @@ struct b2_handle {
   void* dinput = nullptr;
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
-  double* loss_dev = nullptr;  // [2]: one accumulator per input slot
+  // Per input slot: the loss accumulator (double) and, 16 bytes behind it, the tile counters of the step
+  // kernel, so that one memset readies both.
+  char* sync_dev = nullptr;
+  size_t sync_bytes = 0;
+  // Whole steps in one launch (step_kernel.cu), one plan per input slot; null: one launch per GEMM
+  StepPlan* step_plan[2] = {nullptr, nullptr};
   unsigned int* status_dev = nullptr;
   unsigned long long* fp_dev = nullptr;  // accumulator of b2_weights_fingerprint
   float* tc_ws = nullptr;           // stream-K workspace shared by this handle's GEMMs (they
@@ -194,6 +199,10 @@ void batch_range(int batch, int world, int rank, int* b, int* e) {
   int hi = lo + per < batch ? lo + per : batch;
   *b = lo;
   *e = hi;
+}
+
+double* loss_ptr(const b2_handle* h, int slot) {
+  return reinterpret_cast<double*>(h->sync_dev + (size_t)slot * h->sync_bytes);
 }
 
 size_t layer_elems(const b2_handle* h, int l) { return (size_t)h->nf[l + 1] * h->ld[l]; }
@@ -423,6 +432,110 @@ int build_sites(b2_handle* h) {
   return B2_OK;
 }
 
+// Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken when every GEMM of the step
+// is at most two rounds of 128 x 128 tiles over the SMs, where the chain of layers is bound by latency; wider
+// layers keep the larger tiles of gemm_tc_kernel (per step, one launch per GEMM against one per step: 4 x 2048,
+// batch 2048, bf16 283 -> 256 us; 1536-768-1536-1024, batch 3000, tf32 240 -> 172 us; but 3 x 4096, batch 1024,
+// bf16 433 -> 473 us and tf32 612 -> 709 us).
+int build_step_plans(b2_handle* h) {
+  const int L = h->L;
+  const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
+  if (e && e[0] == '0') return B2_OK;
+  const bool has_ar = h->cfg.world_size > 1 && h->cfg.allreduce;
+  if (!use_tc(h) || has_ar || !h->cfg.overlap || h->bl < 1) return B2_OK;
+  auto tiles = [](const GemmDesc& d, int bn) { return (long long)((d.M + 127) / 128) * ((d.N + bn - 1) / bn); };
+  for (int l = 0; l < L; ++l) {
+    for (const Site* s : {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]}) {
+      if (!s->active) {
+        if (s == &h->dgrad[0]) continue;  // no input gradient asked for
+        return B2_OK;
+      }
+      // a last layer of fewer than 16 outputs stays on the CUDA cores, inside the step kernel
+      const bool narrow = s == &h->fwd[L - 1] && s->d.N < 16 && s->d.sAm % (16 / (int)esize(s->d.in_type)) == 0;
+      if (!s->plan && !narrow) return B2_OK;
+      if (!(e && e[0] == '1') && tiles(s->d, 128) > 2 * h->sms) return B2_OK;
+    }
+  }
+  for (int slot = 0; slot < 2; ++slot) {
+    StepSpec spec;
+    std::vector<int> wg(L, -1);
+    auto add = [&](const Site& s, int role) -> StepGemm& {
+      StepGemm g{};
+      g.d = s.d;
+      g.role = role;
+      g.rows_of = g.all_of = g.update_after = g.prev_step[0] = g.prev_step[1] = -1;
+      // narrow tiles as long as the GEMM fits one round of the grid: shorter tiles, more SMs at work
+      g.block_n = tiles(s.d, 64) <= h->sms ? 64 : 128;
+      spec.gemms.push_back(g);
+      return spec.gemms.back();
+    };
+    for (int l = 0; l < L; ++l) {
+      StepGemm& g = add((l == 0 && slot) ? h->fwd0_alt : h->fwd[l], l == L - 1 ? STEP_LAST_FWD : STEP_GEMM);
+      g.rows_of = l - 1;  // the list starts with fwd(0) .. fwd(L-1)
+      if (l + 1 < L) {
+        g.mask_out = h->relu_bits[l + 1];
+        g.ld_mask = (h->nf[l + 1] + 31) / 32;
+      }
+    }
+    // Backward: the chain of input gradients, and the weight gradients one layer behind it, so that an SM
+    // does not hold a chain tile back behind a weight gradient that became ready at the same moment
+    // (20 x 512, batch 2048: 313 us per step against 388 side by side; 4 x 2048: 275 against 291).
+    const int lag = 1;
+    std::vector<int> dz_of(L, L - 1), dg(L, -1);  // the GEMMs that produced dz[l] and that read W[l]
+    for (int t = L - 1; t >= -lag; --t) {
+      if (t >= 0 && h->dgrad[t].active) {
+        StepGemm& g = add(h->dgrad[t], STEP_GEMM);
+        g.rows_of = dz_of[t];
+        g.mask_in = h->relu_bits[t];
+        g.ld_mask = (h->nf[t] + 31) / 32;
+        dg[t] = (int)spec.gemms.size() - 1;
+        if (t > 0) dz_of[t - 1] = dg[t];
+      }
+      const int l = t + lag;
+      if (l < 0 || l >= L) continue;
+      StepGemm& g = add((l == 0 && slot) ? h->wgrad0_alt : h->wgrad[l], STEP_WGRAD);
+      g.all_of = dz_of[l];
+      g.update_after = dg[l];
+      g.w = h->w[l];
+      g.w16 = h->op_type == T_BF16 ? h->w16[l] : nullptr;
+      g.w_lo = h->x3 ? h->w_lo[l] : nullptr;
+      wg[l] = (int)spec.gemms.size() - 1;
+    }
+    for (int l = 0; l < L; ++l) {
+      spec.gemms[l].prev_step[0] = wg[l];
+      if (l + 1 < L) spec.gemms[l].prev_step[1] = wg[l + 1];
+    }
+    const bool baseline = h->cfg.mode == B2_MODE_BASELINE;
+    spec.target = slot ? h->target_alt : h->target;
+    spec.dz = h->dz[L - 1];
+    spec.dz_lo = h->x3 ? h->dz_lo[L - 1] : nullptr;
+    spec.baseline = baseline ? 1 : 0;
+    spec.inv_batch = 1.0f / (float)h->cfg.batch;
+    spec.loss_scale = baseline ? 1.0 / (double)h->cfg.batch : 1.0;
+    spec.loss = loss_ptr(h, slot);
+    if (16 + (size_t)step_plan_counters(spec) * sizeof(unsigned int) > h->sync_bytes)
+      return fail(h, B2_ERR_STATE, "counter block too small");
+    h->step_plan[slot] = step_plan_create(spec, h->sms);
+    if (!h->step_plan[slot]) {  // e.g. more layers than the kernel's table holds
+      step_plan_destroy(h->step_plan[0]);
+      h->step_plan[0] = nullptr;
+      return B2_OK;
+    }
+  }
+  return B2_OK;
+}
+
+// `steps` training steps on the main stream as one launch.
+int enqueue_fused(b2_handle* h, int slot, int steps) {
+  char* sync = h->sync_dev + (size_t)slot * h->sync_bytes;
+  CK(h, cudaMemsetAsync(sync, 0, h->sync_bytes, h->s_main));
+  CK(h, step_launch(h->step_plan[slot], steps, h->cfg.lr, reinterpret_cast<unsigned int*>(sync + 16), h->status_dev,
+                    h->s_main));
+  ++h->launches;
+  h->tc_launches += (long long)steps * (3 * h->L - (h->dgrad[0].active ? 0 : 1) - (h->fwd[h->L - 1].plan ? 0 : 1));
+  return B2_OK;
+}
+
 // Sum of `count` gradient elements starting `begin` elements into the slab, over all ranks:
 // through peer memory when the ranks are connected and the message is small, else NCCL.
 int sum_gradients(b2_handle* h, size_t begin, size_t count, cudaStream_t st) {
@@ -598,7 +711,7 @@ int layer_sgd(b2_handle* h, int l, cudaStream_t st, bool timed) {
 // Enqueue one training step on the two streams (no host synchronisation).
 int enqueue_step(b2_handle* h, bool timed, int slot = 0) {
   const int L = h->L;
-  double* loss_acc = h->loss_dev + slot;
+  double* loss_acc = loss_ptr(h, slot);
   const float* target = slot ? h->target_alt : h->target;
   const bool overlap = h->cfg.overlap != 0;
   const bool wg = overlap && h->wg_stream;
@@ -806,7 +919,8 @@ void free_all(b2_handle* h) {
   cudaFree(h->target);
   cudaFree(h->dinput);
   cudaFree(h->stage);
-  cudaFree(h->loss_dev);
+  cudaFree(h->sync_dev);
+  for (StepPlan* p : h->step_plan) step_plan_destroy(p);
   cudaFree(h->act0_alt);
   cudaFree(h->target_alt);
   cudaFree(h->xstage[0]);
@@ -1103,7 +1217,12 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
   TRY(dev_alloc(h, &h->target_alt, bl * h->ld[L] * 4));
   if (h->op_type == T_BF16)
     for (int i = 0; i < 2; ++i) TRY(dev_alloc(h, &h->xstage[i], bl * h->ld[0] * 4));
-  TRY(dev_alloc(h, &h->loss_dev, 2 * sizeof(double)));
+  {
+    size_t words = 0;  // a counter per 128-row block and one per GEMM: fwd, dgrad (batch rows), wgrad (weight rows)
+    for (int l = 0; l < L; ++l) words += 2 * ((bl + 127) / 128 + 1) + ((size_t)h->nf[l + 1] + 127) / 128 + 1;
+    h->sync_bytes = (16 + words * sizeof(unsigned int) + 255) / 256 * 256;
+    TRY(dev_alloc(h, &h->sync_dev, 2 * h->sync_bytes));
+  }
   TRYCK(cudaHostAlloc((void**)&h->loss_host, 2 * sizeof(double), cudaHostAllocDefault));
   TRYCK(cudaStreamCreateWithFlags(&h->s_copy, cudaStreamNonBlocking));
   for (int i = 0; i < 2; ++i) {
@@ -1174,6 +1293,7 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     }
   }
   TRY(build_sites(h));
+  TRY(build_step_plans(h));
   TRYCK(cudaDeviceSynchronize());
 #undef TRY
 #undef TRYCK
@@ -1354,7 +1474,8 @@ int b2_step(b2_handle* h, int iters) {
   if (h->async_issued != h->async_waited) return fail(h, B2_ERR_STATE, "pipelined steps in flight: b2_wait_loss first");
   if (iters == 0) return B2_OK;
   const bool timed = h->cfg.collect_timing != 0;
-  const bool graph = h->cfg.use_graph && !timed;
+  const bool fused = h->step_plan[0] && !timed;
+  const bool graph = h->cfg.use_graph && !timed && !fused;
   int rc;
   if (graph && !h->graph_exec) {
     CK(h, cudaStreamSynchronize(h->s_main));
@@ -1381,7 +1502,12 @@ int b2_step(b2_handle* h, int iters) {
     for (auto& ev : h->ev_phase) CK(h, cudaEventCreate(&ev));
   }
   CK(h, cudaEventRecord(h->ev_t0, h->s_main));
-  for (int it = 0; it < iters; ++it) {
+  if (fused) {
+    // launches of a bounded number of steps, so that other work on the GPU gets its turn in between
+    for (int it = 0; it < iters; it += 64)
+      if ((rc = enqueue_fused(h, 0, iters - it < 64 ? iters - it : 64))) return rc;
+  }
+  for (int it = 0; it < iters && !fused; ++it) {
     if (graph) {
       CK(h, cudaGraphLaunch(h->graph_exec, h->s_main));
       long long t = 0;
@@ -1392,7 +1518,7 @@ int b2_step(b2_handle* h, int iters) {
       if ((rc = enqueue_step(h, timed))) return rc;
     }
   }
-  if (!graph && (rc = join_streams(h))) return rc;
+  if (!graph && !fused && (rc = join_streams(h))) return rc;
   CK(h, cudaEventRecord(h->ev_t1, h->s_main));
   CK(h, cudaStreamSynchronize(h->s_main));
   CK(h, cudaStreamSynchronize(h->s_comm));
@@ -1441,7 +1567,7 @@ int b2_step(b2_handle* h, int iters) {
 int b2_loss(b2_handle* h, double* loss) {
   ENTER(h);
   if (!loss) return fail(h, B2_ERR_INVALID, "null output");
-  CK(h, cudaMemcpyAsync(loss, h->loss_dev, sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
+  CK(h, cudaMemcpyAsync(loss, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
   CK(h, cudaStreamSynchronize(h->s_main));
   return B2_OK;
 }
@@ -1502,10 +1628,10 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
   }
   CK(h, cudaEventRecord(h->ev_copied[slot], h->s_copy));
   CK(h, cudaStreamWaitEvent(h->s_main, h->ev_copied[slot], 0));
-  if ((rc = enqueue_step(h, false, slot))) return rc;
+  if ((rc = h->step_plan[slot] ? enqueue_fused(h, slot, 1) : enqueue_step(h, false, slot))) return rc;
   CK(h, cudaEventRecord(h->ev_slot_free[slot], h->s_main));
   h->slot_used[slot] = true;
-  CK(h, cudaMemcpyAsync(h->loss_host + slot, h->loss_dev + slot, sizeof(double), cudaMemcpyDeviceToHost,
+  CK(h, cudaMemcpyAsync(h->loss_host + slot, loss_ptr(h, slot), sizeof(double), cudaMemcpyDeviceToHost,
                         h->s_main));
   CK(h, cudaEventRecord(h->ev_loss[slot], h->s_main));
   ++h->async_issued;

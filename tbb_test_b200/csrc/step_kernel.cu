@@ -1,0 +1,891 @@
+// A whole training step - or several - in one launch, for networks whose GEMMs are too small to fill
+// the GPU for long.
+//
+// As one launch per GEMM such a step is a chain of 2L kernels (forward, then input gradients) of
+// which each pays launch, pipeline fill, an exposed epilogue and drain before the next may start, with
+// most SMs idle (a 1024 x 1024 layer is 64 tiles of 128 x 128). Here one persistent CTA per SM walks a
+// fixed list of output tiles of all GEMMs of the step:
+//
+//   fwd(0) .. fwd(L-1), then for l = L-1 .. 0: dgrad(l) and, one layer behind, wgrad(l+1)
+//
+// round-robin over the grid, and a tile starts as soon as the tiles that produce its operands are
+// done: a forward or input-gradient tile waits for the row block it reads, a weight-gradient tile for
+// the whole gradient matrix. So layers overlap row block by row block, and the weight gradients fill the
+// SMs that the chain of input gradients leaves free. The element-wise kernels are gone: the epilogue of
+// the last forward GEMM computes the output gradient and the loss, the epilogue of a weight-gradient
+// tile updates the weights (after every input-gradient tile that reads them).
+//
+// Every tile waits only for tiles earlier in the list and every CTA takes its tiles in list order, so with
+// all CTAs resident (cooperative launch, at most one per SM) some CTA can always proceed. All waits are
+// bounded as in gemm_tc_kernel.
+//
+// Roles per CTA as in gemm_tc_kernel: warp 0 TMA producer (also waits for the dependencies), warp 1 MMA
+// issuer, warps 2-5 epilogue; two TMEM accumulators. A stage holds two 128-byte slabs of K (one in the
+// fp32-class mode): the issuing threads' instructions per stage bound these short k-loops.
+//
+// What bounds it: the latency of one layer after another. In-kernel stamps of a 1024 x 1024 layer at batch
+// 1024: 1.2 us from "dependency met" to the first operands, 2.8 us for 16 k-blocks (137 GB/s into each SM),
+// 1.3 us epilogue, 1.0 us until the stores are visible to the other SMs. bf16, per step, launch per GEMM ->
+// here: 5 x 1024, batch 1024 174 -> 106 us; 20 x 512, batch 2048 628 -> 291 us; 784-500-300-40,
+// batch 1000 83 -> 48 us.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "common.cuh"
+#include "tcgen05.cuh"
+
+namespace b2 {
+namespace {
+
+enum StepEpi : int { SE_NONE = 0, SE_RELU = 1, SE_MASK = 2, SE_LOSS = 3, SE_SGD = 4, SE_NARROW = 5 };
+enum OpForm : int { OP_K2D = 0, OP_K3D = 1, OP_MN3D = 2, OP_MN2D = 3 };
+constexpr int MAX_OPS = 64;
+constexpr int EPI_BYTES = 4 * 2 * 4096;  // two chunk buffers of 32 rows x 128 bytes per epilogue warp
+
+// One operand of a GEMM: how its slabs are fetched and described to the tensor core.
+struct Operand {
+  int form, boxes;        // boxes: 128-byte columns per slab (OP_MN2D)
+  uint32_t col_bytes;     // distance of those columns in shared memory
+  uint32_t bytes;         // bytes of a stage taken by this operand (without its twin)
+  uint32_t kstep16, slab16;  // descriptor advance per k-step and per 128-byte slab of K, in 16-byte units
+  uint64_t desc;          // descriptor without its address
+};
+struct StepMaps {
+  CUtensorMap a, b, c, a_lo, b_lo, c_lo;
+};
+struct StepOp {
+  Operand a, b;
+  int M, N, num_n, num_kb, block_n;
+  int first_item;
+  uint32_t idesc, tx_bytes;
+  int epi, out_bf16, c_lo;
+  int ld;                           // row pitch of C and, element for element, of w, w16, w_lo, target, dz
+  int ld_mask;
+  uint32_t* mask_out;
+  const uint32_t* mask_in;
+  float* w;                         // weight update
+  __nv_bfloat16* w16;
+  float* w_lo;
+  // What has to be finished before a tile may load: indices into the counters (-1: nothing) and the counts a
+  // step adds to them (every epilogue warp of a tile adds one).
+  int row_cnt, row_target;          // counter of row block 0 of the operand's producer
+  int all_cnt, all_target;          // all tiles of the producer (weight gradient)
+  int prev_cnt[2], prev_target[2];  // weight updates of the previous step: this layer's and the next one's
+  int upd_cnt, upd_target;          // weight gradient: input gradient of the same layer (reads the old weights)
+  int sig_row, sig_all, own_target; // counters this op raises (-1: nobody waits for them)
+};
+
+// The scalars travel as kernel parameters, in the constant bank: read from global memory they cost an L2
+// round trip per cache line and tile, because every acquiring load of a counter drops the L1.
+struct StepArgs {
+  const StepMaps* maps;
+  unsigned int* counters;
+  unsigned int* status;
+  int nops, items, steps;
+  int stages;
+  uint32_t slot_bytes;
+  int tmem_cols;
+  float neg_lr;
+  // output gradient and loss
+  int baseline;
+  float inv_batch;
+  const float* target;
+  void* dz;
+  float* dz_lo;
+  double* loss;
+  double loss_scale;
+  // narrow last layer (SE_NARROW): activation, weights, result
+  const void* nar_a;
+  const void* nar_w;
+  float* nar_y;
+  int nar_k, nar_lda;
+  StepOp op[MAX_OPS];
+};
+
+__device__ __forceinline__ float lo_part(float v) {
+  return v - __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+}
+
+// Walks this CTA's items: step `it`, op `op`, item `w` of the step's list.
+struct Walk {
+  int w, it, op;
+  __device__ __forceinline__ void begin() { w = blockIdx.x; it = 0; op = 0; }
+  __device__ __forceinline__ bool settle(const StepArgs& p) {
+    while (w >= p.items) { w -= p.items; ++it; op = 0; }
+    if (it >= p.steps) return false;
+    while (op + 1 < p.nops && w >= p.op[op + 1].first_item) ++op;
+    return true;
+  }
+  __device__ __forceinline__ void advance() { w += gridDim.x; }
+};
+
+__device__ __forceinline__ bool wait_counter(const unsigned int* c, unsigned int target, volatile int* abort_flag,
+                                             unsigned int* status, unsigned int code) {
+  if (ld_acquire_u32(c) >= target) return true;
+  unsigned long long t0 = 0;
+  unsigned int spins = 0;
+  while (ld_acquire_u32(c) < target) {
+    if ((++spins & 0xFF) == 0) {
+      if (*abort_flag) return false;
+      const unsigned long long now = globaltimer();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > WAIT_LIMIT_NS) {
+        *abort_flag = 1;
+        atomicCAS(status, 0u, code);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void count_up(unsigned int* c) {  // after a fence
+  asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
+}
+
+template <int SLABS>
+__device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap* map, uint32_t bar, uint32_t dst,
+                                             int kb, int slab_k, int mn0, int col_log2) {
+  const int k0 = kb * SLABS * slab_k;
+  if (o.form == OP_K3D) {
+    tma_load_3d<false>(map, bar, dst, 0, mn0, kb * SLABS);
+  } else if (o.form == OP_MN3D) {
+    tma_load_3d<false>(map, bar, dst, 0, k0, mn0 >> col_log2);
+  } else if (o.form == OP_K2D) {
+#pragma unroll
+    for (int s = 0; s < SLABS; ++s)
+      tma_load_2d<false>(map, bar, dst + (uint32_t)s * (o.bytes / SLABS), k0 + s * slab_k, mn0);
+  } else {
+    for (int c = 0; c < o.boxes; ++c)
+      tma_load_2d<false>(map, bar, dst + (uint32_t)c * o.col_bytes, mn0 + (c << col_log2), k0);
+  }
+}
+
+// Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic); t = targets.
+template <bool BF16>
+__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t) {
+  float4 d = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+  float4 g = d;
+  if (p.baseline) {
+    d.x -= t.x; d.y -= t.y; d.z -= t.z; d.w -= t.w;
+    g.x = d.x * p.inv_batch; g.y = d.y * p.inv_batch; g.z = d.z * p.inv_batch; g.w = d.w * p.inv_batch;
+  }
+  if (BF16) {
+    *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.dz) + at) =
+        make_uint2(pack_bf16(g.x, g.y), pack_bf16(g.z, g.w));
+  } else {
+    *reinterpret_cast<float4*>(static_cast<float*>(p.dz) + at) = g;
+    if (p.dz_lo)
+      *reinterpret_cast<float4*>(p.dz_lo + at) = make_float4(lo_part(g.x), lo_part(g.y), lo_part(g.z), lo_part(g.w));
+  }
+  return 0.5f * (d.x * d.x + d.y * d.y + d.z * d.z + d.w * d.w);
+}
+
+// w = fma(-lr, g, w) for four consecutive columns (sgd_kernel's arithmetic).
+__device__ __forceinline__ float4 sgd4(float4 w, float g0, float g1, float g2, float g3, float neg_lr) {
+  return make_float4(fmaf(neg_lr, g0, w.x), fmaf(neg_lr, g1, w.y), fmaf(neg_lr, g2, w.z), fmaf(neg_lr, g3, w.w));
+}
+__device__ __forceinline__ void sgd_store(const StepOp& o, size_t at, float4 v) {
+  *reinterpret_cast<float4*>(o.w + at) = v;
+  if (o.w16) *reinterpret_cast<uint2*>(o.w16 + at) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  if (o.w_lo)
+    *reinterpret_cast<float4*>(o.w_lo + at) = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
+}
+// The fp32 values (weights or targets) that belong to a chunk of 32 rows x 32 columns, in the order in which
+// the element-wise part of the epilogue takes the chunk's pieces: lanes 8i .. 8i+7 cover one row.
+__device__ __forceinline__ void load_chunk(float4 (&v)[8], const float* base, size_t ld, int row0, int M, int gcol, int N,
+                                           int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = row0 + 4 * i + (lane >> 3);
+    v[i] = (r < M && gcol < N) ? __ldcg(reinterpret_cast<const float4*>(base + (size_t)r * ld + gcol))
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats. Written by other SMs during this
+// launch: read past the L1.
+template <bool BF16>
+__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k) {
+  if (BF16) {
+    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(row) + k));
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < (BF16 ? 4 : 2); ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  } else {
+    const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k));
+    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+  }
+}
+
+// Last layer with fewer than 16 outputs, too narrow for a tensor-core tile: eight rows per epilogue warp on the
+// CUDA cores, lanes split K (row padding is zero on both sides). Weight rows are loaded four at a time: one at
+// a time the L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
+template <bool BF16, int NMAX>
+__device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, int N, int ld, int lane) {
+  constexpr int V = BF16 ? 8 : 4, R = NMAX <= 4 ? 8 : 4;  // rows at a time, as registers allow
+  const size_t row_bytes = (size_t)p.nar_lda * (BF16 ? 2 : 4);
+  float loss = 0.f;
+  for (int g = 0; g < 8 && row0 + g < M; g += R) {
+    float acc[R][NMAX];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int n = 0; n < NMAX; ++n) acc[r][n] = 0.f;
+    for (int k = lane * V; k < p.nar_k; k += 32 * V) {
+      float a[R][V];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k);
+#pragma unroll
+      for (int n0 = 0; n0 < NMAX; n0 += 4) {
+        if (n0 >= N) break;
+        float b[4][V];
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k);
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[r][n0 + n] = fmaf(a[r][i], b[n][i], acc[r][n0 + n]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NMAX; ++n) {
+      if (n >= N) break;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r][n] += __shfl_xor_sync(0xFFFFFFFFu, acc[r][n], s);
+      float y = acc[0][n];  // lane r finishes row r
+#pragma unroll
+      for (int r = 1; r < R; ++r) y = lane == r ? acc[r][n] : y;
+      const int row = row0 + g + lane;
+      if (lane < R && row < M) {
+        const size_t at = (size_t)row * ld + n;
+        p.nar_y[at] = y;
+        const float d = p.baseline ? y - __ldg(p.target + at) : y;
+        const float gr = p.baseline ? d * p.inv_batch : y;
+        if (BF16) {
+          static_cast<__nv_bfloat16*>(p.dz)[at] = __float2bfloat16_rn(gr);
+        } else {
+          static_cast<float*>(p.dz)[at] = gr;
+          if (p.dz_lo) p.dz_lo[at] = lo_part(gr);
+        }
+        loss += 0.5f * d * d;
+      }
+    }
+  }
+  return loss;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_constant__ StepArgs p) {
+  constexpr bool TF32 = KIND != KIND_BF16, X3 = KIND == KIND_X3;
+  constexpr int SLABS = X3 ? 1 : 2;
+  constexpr int SLAB_K = TF32 ? 32 : 64, COL_LOG2 = TF32 ? 5 : 6;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[MAX_STAGES];
+  __shared__ __align__(8) uint64_t acc_full_bar[2];
+  __shared__ __align__(8) uint64_t acc_empty_bar[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s;
+
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* abort_flag = &abort_s;
+  if (threadIdx.x == 0) {
+    abort_s = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&acc_full_bar[a], 1);
+      mbar_init(&acc_empty_bar[a], 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"((uint32_t)p.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+  const uint32_t acc_cols = X3 ? 128u : (uint32_t)p.tmem_cols / 2;  // TMEM columns of one accumulator
+  Walk wk;
+  wk.begin();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), ring0 = smem_u32(smem);
+      const int stages = p.stages;
+      const uint32_t slot = p.slot_bytes;
+      while (ok && wk.settle(p)) {
+        const StepOp& o = p.op[wk.op];
+        if (o.epi == SE_NARROW) { wk.advance(); continue; }
+        const StepMaps* mp = p.maps + wk.op;
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->b) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->c) : "memory");
+        const int idx = wk.w - o.first_item;
+        const int num_n = o.num_n, nkb = o.num_kb;
+        const int mb = idx / num_n, nb = idx - mb * num_n;
+        const int m0 = mb * BLOCK_M, n0 = nb * o.block_n;
+        const uint32_t tx = o.tx_bytes;
+        const Operand oa = o.a, ob = o.b;
+        const uint32_t a_bytes = oa.bytes, b_bytes = ob.bytes;
+        const unsigned int it = (unsigned int)wk.it;
+        // operands of this step
+        if (o.row_cnt >= 0)
+          ok = wait_counter(p.counters + o.row_cnt + mb, (it + 1) * (unsigned int)o.row_target, abort_flag, p.status, 6u);
+        if (ok && o.all_cnt >= 0)
+          ok = wait_counter(p.counters + o.all_cnt, (it + 1) * (unsigned int)o.all_target, abort_flag, p.status, 7u);
+        if (it > 0) {
+          // weights updated by the previous step; with them all readers of the buffers this tile overwrites are done
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (ok && o.prev_cnt[i] >= 0)
+              ok = wait_counter(p.counters + o.prev_cnt[i], it * (unsigned int)o.prev_target[i], abort_flag, p.status, 8u);
+        }
+        if (!ok) break;
+        fence_proxy_async_all();  // the acquired data is read through the async proxy next
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
+          const uint32_t full = full0 + 8u * stage;
+          const uint32_t sa = ring0 + (uint32_t)stage * slot;
+          const uint32_t sb = sa + a_bytes * (X3 ? 2u : 1u);
+          mbar_expect_tx(full, tx);
+          load_operand<SLABS>(oa, &mp->a, full, sa, kb, SLAB_K, m0, COL_LOG2);
+          load_operand<SLABS>(ob, &mp->b, full, sb, kb, SLAB_K, n0, COL_LOG2);
+          if (X3) {  // the low-order twins
+            load_operand<SLABS>(oa, &mp->a_lo, full, sa + a_bytes, kb, SLAB_K, m0, COL_LOG2);
+            load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, kb, SLAB_K, n0, COL_LOG2);
+          }
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+        wk.advance();
+      }
+      if (!ok) {  // give copies already in flight a bounded time to land before the CTA retires
+        const unsigned long long t0 = globaltimer();
+        while (globaltimer() - t0 < 2000000ull) __nanosleep(1000);
+      }
+    }
+  } else if (warp == 1) {
+    // -------------------------------------------------------------- MMA issuer
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      bool ok = true;
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full_bar);
+      const uint32_t ring16 = smem_u32(smem) >> 4, slot16 = p.slot_bytes >> 4;
+      const int stages = p.stages;
+      while (ok && wk.settle(p)) {
+        const StepOp& o = p.op[wk.op];
+        if (o.epi == SE_NARROW) { wk.advance(); continue; }
+        const int nkb = o.num_kb;
+        const uint32_t idesc = o.idesc;
+        const uint32_t a16 = o.a.bytes >> 4, b16 = o.b.bytes >> 4;
+        const uint32_t a_step = o.a.kstep16, b_step = o.b.kstep16, a_slab = o.a.slab16, b_slab = o.b.slab16;
+        const uint64_t a0 = o.a.desc + ring16, b0 = o.b.desc + ring16 + a16 * (X3 ? 2u : 1u);
+        if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 2u)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t tmem_d = tmem_base + (uint32_t)acc * acc_cols;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(full0 + 8u * stage, phase, abort_flag, p.status, 3u)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t off = (uint32_t)stage * slot16;
+#pragma unroll
+          for (int s = 0; s < SLABS; ++s)
+            issue_ksteps<1, TF32, false, X3, KSTEPS>(tmem_d, a0 + off + s * a_slab, b0 + off + s * b_slab, a_step, b_step,
+                                                     idesc, 0u, (s == 0 && kb == 0) ? 0u : 1u, 0u, a16, b16);
+          tc_commit(empty0 + 8u * stage);
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        tc_commit(acc_full0 + 8u * acc);
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        wk.advance();
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue
+    const int q = warp & 3;  // TMEM lane quarter this warp may read
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    uint8_t* ebuf = smem + (size_t)p.stages * p.slot_bytes + (size_t)(warp - 2) * (2 * 4096);
+    int ebuf_i = 0;
+    const uint32_t swz = (uint32_t)(lane & 7);
+    // the loss reported is the last step's
+    auto add_loss = [&](float loss) {
+      double sum = (double)loss;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, s);
+      if (lane == 0) atomicAdd(p.loss, sum * p.loss_scale);
+    };
+    // this warp's part of a tile is stored: complete the stores, then the counters
+    auto publish = [&](int sig_row, int sig_all) {
+      __syncwarp();
+      if (lane == 0) {
+        bulk_wait_all();
+        fence_proxy_async_all();
+        __threadfence();  // one fence for both counters
+        if (sig_row >= 0) count_up(p.counters + sig_row);
+        if (sig_all >= 0) count_up(p.counters + sig_all);
+      }
+    };
+    while (wk.settle(p)) {
+      const StepOp& o = p.op[wk.op];
+      const int idx = wk.w - o.first_item;
+      const int num_n = o.num_n, M = o.M, N = o.N, epi = o.epi;
+      if (epi == SE_NARROW) {  // an item is 32 rows here, four to a row block
+        bool ok = o.row_cnt < 0 || wait_counter(p.counters + o.row_cnt + (idx >> 2), (wk.it + 1u) * o.row_target,
+                                                abort_flag, p.status, 6u);
+        if (ok && wk.it > 0 && o.prev_cnt[0] >= 0)
+          ok = wait_counter(p.counters + o.prev_cnt[0], (unsigned int)wk.it * o.prev_target[0], abort_flag, p.status, 8u);
+        if (!__all_sync(0xFFFFFFFFu, ok)) break;
+        const int r8 = idx * 32 + (warp - 2) * 8;
+        const float part = N <= 4 ? narrow_rows<!TF32, 4>(p, r8, M, N, o.ld, lane) : narrow_rows<!TF32, 16>(p, r8, M, N, o.ld, lane);
+        if (wk.it + 1 == p.steps) add_loss(part);
+        publish(o.sig_row >= 0 ? o.sig_row + (idx >> 2) : -1, o.sig_all);
+        wk.advance();
+        continue;
+      }
+      const int mb = idx / num_n, nb = idx - mb * num_n;
+      const int row0 = mb * BLOCK_M + q * 32, row = row0 + lane, n0 = nb * o.block_n;
+      const bool out_bf16 = o.out_bf16 != 0;
+      const int chunk_cols = out_bf16 ? 64 : 32;  // 128 bytes of C per row and chunk
+      const int nchunks = o.block_n / chunk_cols;
+      const size_t ld = (size_t)o.ld;
+      const StepMaps* mp = p.maps + wk.op;
+      const int piece = lane & 7;  // 16-byte piece of a row this lane takes in the element-wise part
+      const unsigned int it = (unsigned int)wk.it;
+      float loss = 0.f;
+      uint32_t* const mask_out = epi == SE_RELU ? o.mask_out : nullptr;
+      const uint32_t* const mask_in = o.mask_in;
+      const long long ld_mask = o.ld_mask;
+      const float* const extra = epi == SE_SGD ? o.w : epi == SE_LOSS && p.baseline ? p.target : nullptr;
+      const bool fetch = extra && !out_bf16;
+      float4 pre[8];  // weights or targets of the next chunk, on their way while the MMAs run
+      bool ok = true;
+      if (epi == SE_SGD && it > 0)  // the update of the step before, possibly by another SM
+        ok = wait_counter(p.counters + o.sig_all, it * (unsigned int)o.own_target, abort_flag, p.status, 10u);
+      if (fetch) load_chunk(pre, extra, ld, row0, M, n0 + piece * 4, N, lane);
+      if (ok && epi == SE_SGD && o.upd_cnt >= 0)
+        ok = wait_counter(p.counters + o.upd_cnt, (it + 1) * (unsigned int)o.upd_target, abort_flag, p.status, 9u);
+      ok = ok && mbar_wait(&acc_full_bar[acc], acc_phase, abort_flag, p.status, 4u);
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols;
+      for (int ch = 0; ch < nchunks; ++ch) {
+        const int col0 = n0 + ch * chunk_cols;
+        if (col0 >= N) break;  // uniform across the warp; the first chunk of a tile always lies inside
+        const bool last = (ch == nchunks - 1) || (col0 + chunk_cols >= N);
+        uint32_t words[32];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          if (half == 1 && !out_bf16) break;
+          const int c0 = col0 + half * 32;
+          uint32_t r[32];
+          tmem_ld32(taddr + (uint32_t)(ch * chunk_cols + half * 32), r);
+          if (X3) {
+            uint32_t r2[32];
+            tmem_ld32(taddr + X3_CORR_COLS + (uint32_t)(ch * chunk_cols + half * 32), r2);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+          }
+          if (last && (half == 1 || !out_bf16)) {  // last read of the accumulator: the next tile may have it
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
+          }
+          if (epi == SE_RELU) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(fmaxf(__uint_as_float(r[j]), 0.f));
+          } else if (epi == SE_MASK) {
+            // written by other SMs during this launch: read past the L1
+            const uint32_t mask = (row < M && c0 < N) ? __ldcg(mask_in + (long long)row * ld_mask + (c0 >> 5)) : 0u;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = (mask >> j) & 1u ? r[j] : 0u;
+          }
+          uint32_t part[4] = {0, 0, 0, 0};
+          if (out_bf16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              words[half * 16 + j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            if (mask_out) {  // bit = the stored half is non-zero (it is not negative)
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint32_t m = ((words[half * 16 + j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u;
+                part[j & 3] |= (((m >> 15) | (m >> 30)) & 3u) << (2 * j);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) words[j] = r[j];
+            if (mask_out) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (__uint_as_float(r[j]) > 0.f) part[j & 3] |= 1u << j;
+            }
+          }
+          if (mask_out && row < M && c0 < N)
+            mask_out[(long long)row * ld_mask + (c0 >> 5)] = (part[0] | part[1]) | (part[2] | part[3]);
+        }
+        if (lane == 0) bulk_wait_read<1>();  // the store issued two chunks ago has read its buffer
+        __syncwarp();
+        uint8_t* cbuf = ebuf + (size_t)ebuf_i * 4096;
+        {
+          uint8_t* dst = cbuf + (size_t)lane * 128;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)  // 128-byte swizzle: piece j of row `lane` at slot j ^ (lane & 7)
+            *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) =
+                make_uint4(words[4 * j], words[4 * j + 1], words[4 * j + 2], words[4 * j + 3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < M) {
+          tma_store_2d(&mp->c, cbuf, col0, row0);
+          bulk_commit();
+        }
+        ebuf_i ^= 1;
+        if (epi >= SE_LOSS) {
+          // element-wise work on the finished chunk, read back so that a warp instruction covers four whole
+          // 128-byte rows: lanes 8i .. 8i+7 take the 16-byte pieces of one row
+          const int gcol = col0 + piece * (out_bf16 ? 8 : 4);
+          if (!out_bf16) {
+            float4 cur[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cur[i] = pre[i];
+            if (fetch && !last) load_chunk(pre, extra, ld, row0, M, gcol + 32, N, lane);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int rr = 4 * i + (lane >> 3);
+              const uint4 v = *reinterpret_cast<const uint4*>(cbuf + rr * 128 + ((piece ^ (rr & 7)) << 4));
+              if (row0 + rr < M && gcol < N) {
+                const size_t at = (size_t)(row0 + rr) * ld + gcol;
+                if (epi == SE_LOSS)
+                  loss += loss_piece<!TF32>(p, at, v, cur[i]);
+                else
+                  sgd_store(o, at,
+                            sgd4(cur[i], __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),
+                                 __uint_as_float(v.w), p.neg_lr));
+              }
+            }
+          } else {  // bf16 gradients: the update uses the stored (rounded) values
+            float4 w0[8], w1[8];
+            load_chunk(w0, o.w, ld, row0, M, gcol, N, lane);
+            load_chunk(w1, o.w + 4, ld, row0, M, gcol, N, lane);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int rr = 4 * i + (lane >> 3);
+              const uint4 v = *reinterpret_cast<const uint4*>(cbuf + rr * 128 + ((piece ^ (rr & 7)) << 4));
+              if (row0 + rr < M && gcol < N) {
+                const size_t at = (size_t)(row0 + rr) * ld + gcol;
+                sgd_store(o, at,
+                          sgd4(w0[i], __uint_as_float(v.x << 16), __uint_as_float(v.x & 0xFFFF0000u),
+                               __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xFFFF0000u), p.neg_lr));
+                sgd_store(o, at + 4,
+                          sgd4(w1[i], __uint_as_float(v.z << 16), __uint_as_float(v.z & 0xFFFF0000u),
+                               __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xFFFF0000u), p.neg_lr));
+              }
+            }
+          }
+        }
+        if (X3 && o.c_lo) {  // the low-order twin of the chunk
+          if (lane == 0) bulk_wait_read<1>();
+          __syncwarp();
+          uint8_t* lbuf = ebuf + (size_t)ebuf_i * 4096;
+          uint8_t* dst = lbuf + (size_t)lane * 128;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            uint32_t lo[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) lo[t] = __float_as_uint(lo_part(__uint_as_float(words[4 * j + t])));
+            *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && row0 < M) {
+            tma_store_2d(&mp->c_lo, lbuf, col0, row0);
+            bulk_commit();
+          }
+          ebuf_i ^= 1;
+        }
+      }
+      if (epi == SE_LOSS && it + 1 == (unsigned int)p.steps) add_loss(loss);
+      publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all);
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      wk.advance();
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
+                 : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ host side
+
+// Tensor map of `dims` (innermost contiguous) with the 128-byte swizzle (atom32: in 32-byte atoms).
+bool encode(CUtensorMap* map, const void* base, int eb, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+            const cuuint32_t* box, bool atom32, bool store) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return false;
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank,
+             const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+             store ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// mn x k operand with `rows` of M or N per tile. One 3-D box per stage where the extents are whole
+// 128-byte columns (K for a K-contiguous operand, M/N otherwise), else 2-D boxes.
+bool make_operand(Operand& o, CUtensorMap& map, CUtensorMap& map_lo, const void* base, const void* lo, int eb,
+                  long long mn, long long k, long long ld, bool mn_major, int rows, int slabs) {
+  const int col = SLAB_BYTES / eb;
+  const cuuint64_t pitch = (cuuint64_t)ld * eb;
+  memset(&o, 0, sizeof o);
+  o.bytes = (uint32_t)rows * SLAB_BYTES * slabs;
+  auto both = [&](int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, bool atom32) {
+    if (!encode(&map, base, eb, rank, dims, strides, box, atom32, false)) return false;
+    if (!lo) { map_lo = map; return true; }
+    return encode(&map_lo, lo, eb, rank, dims, strides, box, atom32, false);
+  };
+  auto desc = [](uint32_t lbo, uint32_t sbo, uint32_t layout) {
+    return ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)layout << 61);
+  };
+  if (!mn_major) {
+    o.desc = desc(16, 8 * SLAB_BYTES, 2);
+    o.kstep16 = KSTEP_BYTES >> 4;
+    o.slab16 = (uint32_t)(rows * SLAB_BYTES) >> 4;
+    if (k % col == 0) {
+      const cuuint64_t dims[3] = {(cuuint64_t)col, (cuuint64_t)mn, (cuuint64_t)(k / col)};
+      const cuuint64_t strides[2] = {pitch, SLAB_BYTES};
+      const cuuint32_t box[3] = {(cuuint32_t)col, (cuuint32_t)rows, (cuuint32_t)slabs};
+      o.form = OP_K3D;
+      if (both(3, dims, strides, box, false)) return true;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)mn};
+    const cuuint32_t box[2] = {(cuuint32_t)col, (cuuint32_t)rows};
+    o.form = OP_K2D;
+    return both(2, dims, &pitch, box, false);
+  }
+  const bool atom32 = eb == 4;  // 32-bit M/N-contiguous operands: the swizzle of 32-byte atoms
+  const int block_k = slabs * col;
+  o.boxes = rows / col;
+  o.col_bytes = (uint32_t)block_k * SLAB_BYTES;
+  o.desc = desc(o.col_bytes, atom32 ? 512 : 1024, atom32 ? 1 : 2);
+  o.kstep16 = (uint32_t)((KSTEP_BYTES / eb) * SLAB_BYTES) >> 4;
+  o.slab16 = KSTEPS * o.kstep16;
+  if (mn % col == 0) {
+    const cuuint64_t dims[3] = {(cuuint64_t)col, (cuuint64_t)k, (cuuint64_t)(mn / col)};
+    const cuuint64_t strides[2] = {pitch, SLAB_BYTES};
+    const cuuint32_t box[3] = {(cuuint32_t)col, (cuuint32_t)block_k, (cuuint32_t)o.boxes};
+    o.form = OP_MN3D;
+    if (both(3, dims, strides, box, atom32)) return true;
+  }
+  const cuuint64_t dims[2] = {(cuuint64_t)mn, (cuuint64_t)k};
+  const cuuint32_t box[2] = {(cuuint32_t)col, (cuuint32_t)block_k};
+  o.form = OP_MN2D;
+  return both(2, dims, &pitch, box, atom32);
+}
+
+}  // namespace
+
+struct StepPlan {
+  StepMaps* maps_dev = nullptr;
+  int kind = KIND_BF16, grid = 0;
+  size_t smem = 0;
+  StepArgs args;  // counters, status, steps and learning rate are filled in per launch
+};
+
+int step_plan_counters(const StepSpec& s) {
+  int n = 0;
+  for (const StepGemm& g : s.gemms) n += (g.d.M + BLOCK_M - 1) / BLOCK_M + 1;
+  return n;
+}
+
+StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
+  const int nops = (int)s.gemms.size();
+  if (nops < 1 || nops > MAX_OPS) return nullptr;
+  const GemmDesc& d0 = s.gemms[0].d;
+  const int eb = d0.in_type == T_BF16 ? 2 : 4;
+  const bool x3 = d0.A_lo != nullptr;
+  const int slabs = x3 ? 1 : 2;
+  StepPlan* plan = new StepPlan();
+  memset(&plan->args, 0, sizeof plan->args);
+  StepArgs& args = plan->args;
+  StepOp* ops = args.op;
+  std::vector<StepMaps> maps(nops);
+  std::vector<int> row_base(nops), all_base(nops), ntiles(nops), row_add(nops);
+  std::vector<char> row_used(nops, 0), all_used(nops, 0);
+  auto refuse = [&]() -> StepPlan* {
+    step_plan_destroy(plan);
+    return nullptr;
+  };
+  int ncnt = 0, items = 0, max_bn = 64;
+  uint32_t slot = 0;
+  for (int i = 0; i < nops; ++i) {
+    const StepGemm& g = s.gemms[i];
+    const GemmDesc& d = g.d;
+    StepOp& o = ops[i];
+    StepMaps& mp = maps[i];
+    const int ob = d.out_type == T_BF16 ? 2 : 4;
+    o.M = d.M; o.N = d.N;
+    const int num_m = (d.M + BLOCK_M - 1) / BLOCK_M;
+    o.block_n = g.block_n;
+    o.num_n = (d.N + o.block_n - 1) / o.block_n;
+    const int block_k = slabs * SLAB_BYTES / eb;
+    o.num_kb = (d.K + block_k - 1) / block_k;
+    const bool narrow = g.role == STEP_LAST_FWD && d.N < 16;
+    if (narrow) {
+      if (d.sAk != 1 || d.sBk != 1 || d.sAm != d.sBn || d.sAm % (16 / eb) != 0 || o.num_n != 1) return refuse();
+      args.nar_a = d.A; args.nar_w = d.B; args.nar_y = static_cast<float*>(d.C);
+      args.nar_k = d.K; args.nar_lda = (int)d.sAm;
+    } else {
+      const bool a_mn = d.sAm == 1 && d.sAk != 1, b_mn = d.sBn == 1 && d.sBk != 1;
+      if (!make_operand(o.a, mp.a, mp.a_lo, d.A, d.A_lo, eb, d.M, d.K, a_mn ? d.sAk : d.sAm, a_mn, BLOCK_M, slabs) ||
+          !make_operand(o.b, mp.b, mp.b_lo, d.B, d.B_lo, eb, d.N, d.K, b_mn ? d.sBk : d.sBn, b_mn, o.block_n, slabs))
+        return refuse();
+      const cuuint64_t dims[2] = {(cuuint64_t)d.N, (cuuint64_t)d.M};
+      const cuuint64_t pitch = (cuuint64_t)d.ldc * ob;
+      const cuuint32_t box[2] = {(cuuint32_t)(128 / ob), 32};
+      if (!encode(&mp.c, d.C, ob, 2, dims, &pitch, box, false, true)) return refuse();
+      mp.c_lo = mp.c;
+      o.c_lo = d.C_lo != nullptr;
+      if (d.C_lo && !encode(&mp.c_lo, d.C_lo, 4, 2, dims, &pitch, box, false, true)) return refuse();
+      const uint32_t fmt = eb == 4 ? 2u : 1u;  // tf32 : bf16
+      o.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
+                ((uint32_t)(o.block_n >> 3) << 17) | ((uint32_t)(BLOCK_M >> 4) << 24);
+      o.tx_bytes = (o.a.bytes + o.b.bytes) * (x3 ? 2u : 1u);
+      if (o.tx_bytes > slot) slot = o.tx_bytes;
+      if (o.block_n > max_bn) max_bn = o.block_n;
+    }
+    o.out_bf16 = d.out_type == T_BF16;
+    o.epi = narrow ? SE_NARROW : g.role == STEP_LAST_FWD ? SE_LOSS : g.role == STEP_WGRAD ? SE_SGD
+            : d.epilogue == EPI_RELU ? SE_RELU : d.epilogue == EPI_MASK ? SE_MASK : SE_NONE;
+    if (o.epi == SE_MASK && !g.mask_in) return refuse();
+    o.mask_out = g.mask_out;
+    o.mask_in = g.mask_in;
+    o.ld_mask = (int)g.ld_mask;
+    o.ld = (int)d.ldc;
+    if (o.epi == SE_SGD) { o.w = g.w; o.w16 = g.w16; o.w_lo = g.w_lo; }
+    o.first_item = items;
+    ntiles[i] = num_m * (narrow ? 4 : o.num_n);
+    row_add[i] = 4 * (narrow ? 4 : o.num_n);  // every epilogue warp of a tile counts one
+    items += ntiles[i];
+    row_base[i] = ncnt;
+    all_base[i] = ncnt + num_m;
+    ncnt += num_m + 1;
+  }
+  for (int i = 0; i < nops; ++i) {
+    const StepGemm& g = s.gemms[i];
+    StepOp& o = ops[i];
+    // a dependency always points to an earlier entry of the list, or to a weight gradient of the step before
+    if (g.rows_of >= i || g.all_of >= i || g.update_after >= i) return refuse();
+    o.row_cnt = g.rows_of >= 0 ? row_base[g.rows_of] : -1;
+    o.row_target = g.rows_of >= 0 ? row_add[g.rows_of] : 0;
+    o.all_cnt = g.all_of >= 0 ? all_base[g.all_of] : -1;
+    o.all_target = g.all_of >= 0 ? 4 * ntiles[g.all_of] : 0;
+    o.upd_cnt = g.update_after >= 0 ? all_base[g.update_after] : -1;
+    o.upd_target = g.update_after >= 0 ? 4 * ntiles[g.update_after] : 0;
+    for (int k = 0; k < 2; ++k) {
+      o.prev_cnt[k] = g.prev_step[k] >= 0 ? all_base[g.prev_step[k]] : -1;
+      o.prev_target[k] = g.prev_step[k] >= 0 ? 4 * ntiles[g.prev_step[k]] : 0;
+    }
+    if (g.rows_of >= 0) row_used[g.rows_of] = 1;
+    for (int j : {g.all_of, g.update_after, g.prev_step[0], g.prev_step[1], g.role == STEP_WGRAD ? i : -1})
+      if (j >= 0) all_used[j] = 1;
+  }
+  for (int i = 0; i < nops; ++i) {
+    ops[i].sig_row = row_used[i] ? row_base[i] : -1;
+    ops[i].sig_all = all_used[i] ? all_base[i] : -1;
+    ops[i].own_target = 4 * ntiles[i];
+  }
+  plan->kind = x3 ? KIND_X3 : eb == 4 ? KIND_TF32 : KIND_BF16;
+  args.nops = nops;
+  args.items = items;
+  args.slot_bytes = slot;
+  args.tmem_cols = x3 ? 512 : 2 * max_bn;
+  args.target = s.target;
+  args.dz = s.dz;
+  args.dz_lo = s.dz_lo;
+  args.baseline = s.baseline;
+  args.inv_batch = s.inv_batch;
+  args.loss_scale = s.loss_scale;
+  args.loss = s.loss;
+  const size_t budget = 227 * 1024 - 1024 /* alignment slack */ - 512 /* static: barriers */;
+  args.stages = (int)((budget - EPI_BYTES) / slot);
+  if (args.stages > MAX_STAGES) args.stages = MAX_STAGES;
+  plan->smem = 1024 + (size_t)args.stages * slot + EPI_BYTES;
+  if (plan->smem < 140 * 1024) plan->smem = 140 * 1024;  // one CTA (one TMEM allocation) per SM
+  plan->grid = items < sm_count ? items : sm_count;
+  if (args.stages < 2 || cudaMalloc((void**)&plan->maps_dev, sizeof(StepMaps) * nops) != cudaSuccess ||
+      cudaMemcpy(plan->maps_dev, maps.data(), sizeof(StepMaps) * nops, cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaGetLastError();
+    return refuse();
+  }
+  args.maps = plan->maps_dev;
+  return plan;
+}
+
+void step_plan_destroy(StepPlan* p) {
+  if (!p) return;
+  cudaFree(p->maps_dev);
+  delete p;
+}
+
+cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
+                        cudaStream_t stream) {
+  void (*kernel)(const StepArgs) = plan->kind == KIND_BF16 ? step_kernel<KIND_BF16>
+                                   : plan->kind == KIND_TF32 ? step_kernel<KIND_TF32> : step_kernel<KIND_X3>;
+  // per launch: handles of several devices and threads share the library, and the call is cheap
+  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+  if (e != cudaSuccess) return e;
+  StepArgs a = plan->args;
+  a.counters = counters;
+  a.status = status;
+  a.steps = steps;
+  a.neg_lr = -lr;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(plan->grid);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = plan->smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+}  // namespace b2

@@ -1,0 +1,75 @@
+"""Whole steps as one launch (csrc/step_kernel.cu) against one launch per GEMM."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (widths, batch, options): one tile / several row blocks with a remainder / ragged widths of both operand majors /
+# more tiles than SMs / one layer / every output kind the epilogue has; "narrow": last layer on the CUDA cores
+NETS = [([96, 64], 40, {}), ([256] * 6, 256, {}), ([123, 77, 201, 33], 333, {}), ([784, 500, 300, 40], 1000, {}),
+        ([512, 384, 640, 128], 640, {"grad_bf16": True}), ([1024, 1536, 512], 1500, {}), ([64] * 22, 130, {}),
+        ([192, 160, 64], 200, {"ref": True}), ([192, 160, 64], 200, {"input_grad": False}),
+        ([160, 96, 10], 300, {}), ([256, 128, 1], 990, {"ref": True})]
+
+
+def states(O, K, nf, batch, prec, steps, opts, fed=False):
+    from tbb_test_b200.mlp import MLP
+    L = len(nf) - 1
+    mode = K.MODE_REF if opts.get("ref") else K.MODE_BASELINE
+    m = MLP(nf, batch, precision=prec, mode=mode, lr=1e-6 if opts.get("ref") else 0.01,
+            grad_bf16=opts.get("grad_bf16", False) and prec == K.PREC_BF16, input_grad=opts.get("input_grad", True))
+    for l in range(L):
+        a = (6.0 / nf[l]) ** 0.5
+        m.upload_weights(l, O.fill_uniform(nf[l + 1], nf[l], 5 + l, -a, a))
+    x = np.ascontiguousarray(O.fill_normal(batch, nf[0], 1))
+    t = np.ascontiguousarray(O.fill_sign(batch, nf[-1], 2))
+    if fed:
+        fp = C.POINTER(C.c_float)
+        for i in range(steps):
+            m.train_step_host_async(x.ctypes.data_as(fp), nf[0], t.ctypes.data_as(fp), nf[-1])
+            loss = m.wait_loss()
+    else:
+        m.upload_input(x)
+        m.upload_target(t)
+        m.step(steps)
+        loss = m.loss()
+    out = {"y": m.activation(L)}
+    for l in range(L):
+        out[f"w{l}"], out[f"dw{l}"], out[f"dz{l}"] = m.weights(l), m.weight_grad(l), m.dz(l)
+        if l:
+            out[f"act{l}"] = m.activation(l)
+    if opts.get("input_grad", True):
+        out["dinput"] = m.input_grad()
+    launches = m.launch_counts()[0]
+    m.close()
+    return out, loss, launches
+
+
+@pytest.mark.parametrize("prec", ["bf16", "tf32", "fp32tc"])
+@pytest.mark.parametrize("net", NETS, ids=lambda n: "x".join(map(str, n[0][:4])) + f"b{n[1]}" + "".join(n[2]))
+def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, prec):
+    """The same MMAs in the same k order and the same element-wise arithmetic: equal bits. A narrow last layer adds
+    its products in another order (fp32, K terms: 1e-5), which a bf16 store may turn into one unit in the last
+    place of a few elements (2^-8 each: 2e-3 of the tensors' norm, as for the other oracle that rounds alike)."""
+    from tbb_test_b200 import _capi as K
+    nf, batch, opts = net
+    P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32, "fp32tc": K.PREC_FP32_TC}[prec]
+    for steps in (1, 3):
+        monkeypatch.setenv("B2_STEP_KERNEL", "0")
+        a, la, na = states(oracle, K, nf, batch, P, steps, opts)
+        monkeypatch.setenv("B2_STEP_KERNEL", "1")
+        b, lb, nb = states(oracle, K, nf, batch, P, steps, opts)
+        f, lf, _ = states(oracle, K, nf, batch, P, steps, opts, fed=True)
+        if prec == "bf16":
+            assert nb < na  # one launch for all steps
+        tail = nf[-1] < 16
+        for k in a:
+            for o in (b, f):
+                if not tail:
+                    assert np.array_equal(a[k], o[k]), (k, steps)
+                else:
+                    d = np.linalg.norm((a[k] - o[k]).astype(np.float64))
+                    assert d <= (1e-5 if k == "y" and steps == 1 else 2e-3) * max(np.linalg.norm(a[k]), 1e-30), (k, steps)
+        assert abs(la - lb) <= 1e-5 * abs(la) and abs(la - lf) <= 1e-5 * abs(la)
