@@ -18,11 +18,14 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cctype>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/b200mlp.h"
@@ -116,6 +119,9 @@ struct b2_handle {
   float* y = nullptr;
   float* target = nullptr;
   void* dinput = nullptr;
+  // Page-locked buffers of download_rows, two per worker, made at the first large download
+  char* dl_buf = nullptr;
+  cudaEvent_t dl_ev[12] = {};
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
   // Per input slot: the loss accumulator (double) and, 16 bytes behind it, the tile counters of the step
@@ -313,6 +319,82 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
   return B2_OK;
 }
 
+// Device rows to host memory, done when it returns. A copy to pageable memory runs at the speed of one
+// thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
+// destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
+// buffers of their own, each moving one chunk while its next one is in flight, share that work.
+constexpr size_t DL_CHUNK = 512 << 10;
+constexpr int DL_WORKERS = 6;
+int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
+  const size_t width = (size_t)cols * 4;
+  cudaPointerAttributes attr;
+  bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  if (pageable && width <= DL_CHUNK && width * rows >= 4 * DL_CHUNK && !h->dl_buf) {
+    bool ok = cudaHostAlloc((void**)&h->dl_buf, 2 * DL_WORKERS * DL_CHUNK, cudaHostAllocDefault) == cudaSuccess;
+    if (!ok) h->dl_buf = nullptr;
+    for (int i = 0; ok && i < 2 * DL_WORKERS; ++i)
+      ok = h->dl_ev[i] || cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {  // no page-locked memory left: the plain copy
+      if (h->dl_buf) cudaFreeHost(h->dl_buf);
+      h->dl_buf = nullptr;
+      cudaGetLastError();
+    }
+  }
+  if (!pageable || width > DL_CHUNK || width * rows < 4 * DL_CHUNK || !h->dl_buf) {
+    CK(h, cudaMemcpy2DAsync(host, ld * 4, dev, pitch * 4, width, rows, cudaMemcpyDeviceToHost, h->s_main));
+    CK(h, cudaStreamSynchronize(h->s_main));
+    return B2_OK;
+  }
+  const int per = (int)(DL_CHUNK / width), chunks = (rows + per - 1) / per;
+  std::atomic<int> next{0}, error{(int)cudaSuccess};
+  auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(h->cfg.device);
+    int in_flight[2] = {-1, -1};  // chunk on its way into each of this worker's buffers
+    auto land = [&](int b) {      // wait for it and move it to its place
+      if (in_flight[b] < 0) return;
+      if (e == cudaSuccess) e = cudaEventSynchronize(h->dl_ev[2 * t + b]);
+      if (e == cudaSuccess) {
+        const char* src = h->dl_buf + (size_t)(2 * t + b) * DL_CHUNK;
+        const int r0 = in_flight[b] * per, n = std::min(per, rows - r0);
+        for (int r = 0; r < n; ++r) memcpy(host + (size_t)(r0 + r) * ld, src + width * r, width);
+      }
+      in_flight[b] = -1;
+    };
+    for (int b = 0; e == cudaSuccess && error.load() == (int)cudaSuccess; b ^= 1) {
+      const int c = next.fetch_add(1);
+      if (c >= chunks) break;
+      const int r0 = c * per, n = std::min(per, rows - r0);
+      e = copy_rows(h->dl_buf + (size_t)(2 * t + b) * DL_CHUNK, width,
+                    static_cast<const char*>(dev) + (size_t)r0 * pitch * 4, pitch * 4, width, (size_t)n,
+                    cudaMemcpyDeviceToHost, h->s_main);
+      if (e == cudaSuccess) e = cudaEventRecord(h->dl_ev[2 * t + b], h->s_main);
+      in_flight[b] = c;
+      land(b ^ 1);
+    }
+    land(0);
+    land(1);
+    if (e != cudaSuccess) error.store((int)e);
+  };
+  std::thread pool[DL_WORKERS];
+  int helpers = std::min(std::min(DL_WORKERS, (int)std::thread::hardware_concurrency()), chunks) - 1;
+  for (int i = 0; i < helpers; ++i) {
+    try {
+      pool[i] = std::thread(work, i + 1);
+    } catch (const std::system_error&) {  // no more threads to be had: those that run take all chunks
+      break;
+    }
+  }
+  work(0);
+  for (std::thread& th : pool)
+    if (th.joinable()) th.join();
+  if (error.load() != (int)cudaSuccess) {
+    cudaStreamSynchronize(h->s_main);  // copies into the buffers may still be in flight
+    return fail(h, B2_ERR_CUDA, "download: %s", cudaGetErrorString((cudaError_t)error.load()));
+  }
+  return B2_OK;
+}
+
 int download_matrix(b2_handle* h, const void* dev, int type, float* host, size_t ld, int rows, int cols, int pitch) {
   if (rows <= 0 || cols <= 0) return B2_OK;
   const void* src = dev;
@@ -322,10 +404,7 @@ int download_matrix(b2_handle* h, const void* dev, int type, float* host, size_t
     ++h->launches;
     src = h->stage;
   }
-  CK(h, cudaMemcpy2DAsync(host, ld * 4, src, (size_t)pitch * 4, (size_t)cols * 4, rows, cudaMemcpyDeviceToHost,
-                          h->s_main));
-  CK(h, cudaStreamSynchronize(h->s_main));
-  return B2_OK;
+  return download_rows(h, host, ld, src, (size_t)pitch, rows, cols);
 }
 
 int build_sites(b2_handle* h) {
@@ -919,6 +998,9 @@ void free_all(b2_handle* h) {
   cudaFree(h->target);
   cudaFree(h->dinput);
   cudaFree(h->stage);
+  if (h->dl_buf) cudaFreeHost(h->dl_buf);
+  for (cudaEvent_t ev : h->dl_ev)
+    if (ev) cudaEventDestroy(ev);
   cudaFree(h->sync_dev);
   for (StepPlan* p : h->step_plan) step_plan_destroy(p);
   cudaFree(h->act0_alt);
