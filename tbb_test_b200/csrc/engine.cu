@@ -323,14 +323,14 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
 // thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
 // destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
 // buffers of their own, each moving one chunk while its next one is in flight, share that work.
-constexpr size_t DL_CHUNK = 512 << 10;
+constexpr size_t DL_CHUNK = 128 << 10, DL_MIN_BYTES = 2 << 20;
 constexpr int DL_WORKERS = 6;
 int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
   const size_t width = (size_t)cols * 4;
   cudaPointerAttributes attr;
   bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
-  if (pageable && width <= DL_CHUNK && width * rows >= 4 * DL_CHUNK && !h->dl_buf) {
+  if (pageable && width <= DL_CHUNK && width * rows >= DL_MIN_BYTES && !h->dl_buf) {
     bool ok = cudaHostAlloc((void**)&h->dl_buf, 2 * DL_WORKERS * DL_CHUNK, cudaHostAllocDefault) == cudaSuccess;
     if (!ok) h->dl_buf = nullptr;
     for (int i = 0; ok && i < 2 * DL_WORKERS; ++i)
@@ -341,7 +341,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       cudaGetLastError();
     }
   }
-  if (!pageable || width > DL_CHUNK || width * rows < 4 * DL_CHUNK || !h->dl_buf) {
+  if (!pageable || width > DL_CHUNK || width * rows < DL_MIN_BYTES || !h->dl_buf) {
     CK(h, cudaMemcpy2DAsync(host, ld * 4, dev, pitch * 4, width, rows, cudaMemcpyDeviceToHost, h->s_main));
     CK(h, cudaStreamSynchronize(h->s_main));
     return B2_OK;

@@ -73,3 +73,50 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
                     d = np.linalg.norm((a[k] - o[k]).astype(np.float64))
                     assert d <= (1e-5 if k == "y" and steps == 1 else 2e-3) * max(np.linalg.norm(a[k]), 1e-30), (k, steps)
         assert abs(la - lb) <= 1e-5 * abs(la) and abs(la - lf) <= 1e-5 * abs(la)
+
+
+@pytest.mark.parametrize("prec", ["bf16"])
+def test_two_handles_in_two_threads(native, oracle, prec):
+    """Cooperative launches of two handles on one GPU, issued by two host threads at once, each keep their grid
+    resident: both finish with the weights they reach alone."""
+    import threading
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    P = {"bf16": K.PREC_BF16, "fp32": K.PREC_FP32}[prec]
+    nf, batch, L = [512] * 5, 512, 4
+
+    def make(seed):
+        m = MLP(nf, batch, precision=P, lr=0.01)
+        for l in range(L):
+            m.upload_weights(l, oracle.fill_uniform(nf[l + 1], nf[l], seed + l, -0.1, 0.1))
+        m.upload_input(oracle.fill_normal(batch, nf[0], seed + 20))
+        m.upload_target(oracle.fill_sign(batch, nf[-1], seed + 30))
+        return m
+
+    alone = []
+    for seed in (1, 100):
+        m = make(seed)
+        for _ in range(20):
+            m.step(5)
+        alone.append([m.weights(l) for l in range(L)])
+        m.close()
+    pair = [make(1), make(100)]
+    errors = []
+
+    def go(m):
+        try:
+            for _ in range(20):
+                m.step(5)
+        except Exception as e:  # reported below, on the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=go, args=(m,)) for m in pair]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for m, ref in zip(pair, alone):
+        for l in range(L):
+            assert np.array_equal(m.weights(l), ref[l])
+        m.close()
