@@ -272,17 +272,19 @@ __global__ void __launch_bounds__(512) gemm_short_kernel(GemmDesc g) {
   }
 }
 
-// Tile of gemm_simt_kernel: 0 = 128 x 128, 1 = 64 x 64, 2 = 32 x 32. A launch takes as long as its
-// fullest SM: rounds of the grid over the SMs times the tile's area, divided by the rate the tile
-// sustains (a smaller tile reads more shared memory per FMA).
+// Tile of gemm_simt_kernel, an index into SIMT_TILES. A launch takes as long as its fullest SM: rounds of the
+// grid over the SMs times the tile's area, divided by the rate the tile sustains (a smaller tile reads more
+// shared memory per FMA). Measured, us: 1024^3 as 64 x 64 74, as 64 x 32 105; 512 x 512 x 2048 (64 tiles of
+// 64 x 64 on 148 SMs) 94 and 72.
+struct SimtTile { int bm, bn; double rate; };
+constexpr SimtTile SIMT_TILES[4] = {{128, 128, 1.0}, {64, 64, 0.85}, {64, 32, 0.555}, {32, 32, 0.40}};
 int simt_tile(int M, int N, int sms) {
-  const int edge[3] = {128, 64, 32};
-  const double rate[3] = {1.0, 0.85, 0.40};
   int best = 0;
   double best_cost = 1e300;
-  for (int i = 0; i < 3; ++i) {
-    const long long T = (long long)((M + edge[i] - 1) / edge[i]) * ((N + edge[i] - 1) / edge[i]);
-    const double cost = (double)((T + sms - 1) / sms) * edge[i] * edge[i] / rate[i];
+  for (int i = 0; i < 4; ++i) {
+    const SimtTile& c = SIMT_TILES[i];
+    const long long T = (long long)((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
+    const double cost = (double)((T + sms - 1) / sms) * c.bm * c.bn / c.rate;
     if (cost < best_cost) { best_cost = cost; best = i; }
   }
   return best;
@@ -305,10 +307,11 @@ cudaError_t launch(const GemmDesc& g, cudaStream_t stream) {
   };
   const int va = vec(g.A, g.sAk == 1 ? g.sAm : g.sAk), vb = vec(g.B, g.sBk == 1 ? g.sBn : g.sBk);
   const int tile = simt_tile(g.M, g.N, 148);
-  const int edge = 128 >> tile;
-  const dim3 grid((g.N + edge - 1) / edge, (g.M + edge - 1) / edge);
+  const SimtTile& c = SIMT_TILES[tile];
+  const dim3 grid((g.N + c.bn - 1) / c.bn, (g.M + c.bm - 1) / c.bm);
   if (tile == 0) gemm_simt_kernel<TI, TO, 128, 128, 16, 8, 8><<<grid, 256, 0, stream>>>(g, va, vb);
   else if (tile == 1) gemm_simt_kernel<TI, TO, 64, 64, 32, 8, 4><<<grid, 128, 0, stream>>>(g, va, vb);
+  else if (tile == 2) gemm_simt_kernel<TI, TO, 64, 32, 32, 4, 4><<<grid, 128, 0, stream>>>(g, va, vb);
   else gemm_simt_kernel<TI, TO, 32, 32, 32, 4, 4><<<grid, 64, 0, stream>>>(g, va, vb);
   return cudaGetLastError();
 }

@@ -182,7 +182,7 @@ def test_optional_tile_schedules(dev, oracle, variant, monkeypatch):
 # Bound: the oracle adds in k order in fp32 as the tile kernel does (2e-5 covers the other order of the two
 # split-K forms: K terms, unit roundoff 6e-8, observed growth sqrt(K)).
 @pytest.mark.parametrize("shape", [(33, 65, 31), (129, 64, 64), (70, 1, 64), (70, 2, 63), (77, 16, 200), (77, 17, 200),
-                                   (1, 70, 64), (2, 96, 129), (16, 100, 321), (17, 100, 321), (1300, 1100, 20),
+                                   (1, 70, 64), (2, 96, 129), (16, 100, 321), (17, 100, 321), (1300, 1100, 20), (500, 509, 40),
                                    (5, 3, 1), (1000, 10, 300), (10, 300, 1000)], ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("form", list(FORMS))
 def test_cuda_core_dispatch_edges(dev, oracle, form, shape):
