@@ -138,6 +138,10 @@ cudaError_t p2p_allreduce_launch(const P2pParams& p, int cta_limit, cudaStream_t
 cudaError_t p2p_allreduce_emulated_launch(const P2pParams* ranks_dev, const P2pParams& any_rank, cudaStream_t stream);
 
 // Element-wise kernels.
+// For the current device: the kernels that prepare the next host-fed batch ask for the shared-memory split the GEMM
+// kernels run with, so that an SM need not drain before it takes them beside a running step. (The weight update
+// is not among them: with it 8 x 4096 layers, 1024 rows, bf16 took 1042 us per step against 1032.)
+cudaError_t elementwise_prepare();
 cudaError_t convert_f32_to_bf16(const float* src, __nv_bfloat16* dst, size_t n, cudaStream_t s);
 cudaError_t convert_bf16_to_f32(const __nv_bfloat16* src, float* dst, size_t n, cudaStream_t s);
 // dz = y (ref) or (y - t) * inv_batch (baseline); loss += 0.5 * sum(d^2) * loss_scale

@@ -219,6 +219,15 @@ int device_sms() {
 
 }  // namespace
 
+cudaError_t elementwise_prepare() {
+  const void* kernels[] = {(const void*)f32_to_bf16_kernel, (const void*)split_lo_kernel};
+  for (const void* k : kernels) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t sgd_launch(float* w, const void* g, int g_type, __nv_bfloat16* w16, size_t n, float lr,
                        int sm_count, cudaStream_t s, float* w_lo) {
   if (n == 0) return cudaSuccess;

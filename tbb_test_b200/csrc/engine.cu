@@ -1150,6 +1150,7 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     TRY(fail(h, B2_ERR_UNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a only", cfg->device,
              prop.major, prop.minor));
   h->sms = prop.multiProcessorCount;
+  TRYCK(elementwise_prepare());
   {
     const bool comm = cfg->world_size > 1 && cfg->allreduce && cfg->overlap;
     // default: 20 on 4 or more GPUs, none on 2 (measured there: 3.28 ms per step of configuration 4
@@ -1695,6 +1696,10 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
     void* land = h->op_type == T_BF16 ? (void*)h->xstage[slot] : act0;
     CK(h, copy_rows(land, p0 * 4, x + (size_t)h->b0 * ldx, ldx * 4, (size_t)f0 * 4, (size_t)rows,
                     cudaMemcpyHostToDevice, h->s_copy));
+    // both copies first: a kernel on this stream may have to wait for room beside the running step
+    if (t)
+      CK(h, copy_rows(slot ? h->target_alt : h->target, pl * 4, t + (size_t)h->b0 * ldt, ldt * 4, (size_t)fl * 4,
+                      (size_t)rows, cudaMemcpyHostToDevice, h->s_copy));
     if (h->op_type == T_BF16) {
       CK(h, convert_f32_to_bf16(h->xstage[slot], (__nv_bfloat16*)act0, (size_t)rows * p0, h->s_copy));
       ++h->launches;
@@ -1704,9 +1709,6 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
                             h->s_copy));
       ++h->launches;
     }
-    if (t)
-      CK(h, copy_rows(slot ? h->target_alt : h->target, pl * 4, t + (size_t)h->b0 * ldt, ldt * 4, (size_t)fl * 4,
-                      (size_t)rows, cudaMemcpyHostToDevice, h->s_copy));
   }
   CK(h, cudaEventRecord(h->ev_copied[slot], h->s_copy));
   CK(h, cudaStreamWaitEvent(h->s_main, h->ev_copied[slot], 0));
