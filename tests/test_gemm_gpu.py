@@ -196,3 +196,47 @@ def test_cuda_core_dispatch_edges(dev, oracle, form, shape):
     assert rel_fro(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_RELU), np.maximum(ref, 0)) <= 2 * TOL["fp32"]
     assert rel_fro(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_MASK, aux=aux),
                    ref * (aux > 0)) <= 2 * TOL["fp32"]
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("shape", [(128, 18, 60), (300, 33, 100), (256, 257, 61), (200, 1003, 64), (1, 301, 33), (700, 1302, 130),
+                                   (300, 64, 61)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("entry", ["fp32", "tf32", "noalloc"])
+def test_submatrices_of_larger_ones(dev, oracle, entry, form, shape):
+    """Operands and result with longer rows than the GEMM uses: what lies between the rows is neither read (NaN there)
+    nor written, also where rows end inside a 16-byte piece and where the values are not finite."""
+    import torch
+    from tbb_test_b200 import _capi as K
+    m, n, k = shape
+    ta, tb = FORMS[form]
+
+    def framed(rows, cols, seed):
+        t = torch.full((rows, (cols + 3) // 4 * 4 + 8), float("nan"))
+        t[:, :cols] = torch.from_numpy(oracle.fill_uniform(rows, cols, seed, -1.0, 1.0))
+        return t
+
+    if entry == "noalloc" and (m if ta else k) % 8 or entry == "noalloc" and (k if tb else n) % 8:
+        pytest.skip("rows the packed copies cannot have")
+    a, b = framed(k if ta else m, m if ta else k, 111), framed(n if tb else k, k if tb else n, 112)
+    for bad in (False, True):
+        if bad:
+            a[0, 0] = float("inf")
+        c = torch.full((m, (n + 3) // 4 * 4 + 4), 7.0)
+        ad, bd, cd = a.cuda(), b.cuda(), c.cuda()
+        torch.cuda.synchronize()
+        if entry == "noalloc":
+            rc = dev.lib.b2_gemm_bf16_noalloc(int(ta), int(tb), m, n, k, ad.data_ptr(), a.shape[1], bd.data_ptr(),
+                                              b.shape[1], cd.data_ptr(), c.shape[1], None)
+        else:
+            rc = dev.lib.b2_sgemm(dev._h, {"fp32": K.PREC_FP32, "tf32": K.PREC_TF32}[entry], int(ta), int(tb), m, n, k, 1.0,
+                                  ad.data_ptr(), a.shape[1], bd.data_ptr(), b.shape[1], 0.0, cd.data_ptr(), c.shape[1])
+        assert rc == K.OK and dev.lib.b2_sync(dev._h) == K.OK
+        got = cd.cpu().numpy()
+        assert (got[:, n:] == 7.0).all(), "columns behind the result were written"
+        if bad:
+            continue
+        ra, rb = a[:, :m if ta else k].double(), b[:, :k if tb else n].double()
+        if entry == "noalloc":
+            ra, rb = ra.float().bfloat16().double(), rb.float().bfloat16().double()
+        ref = ((ra.T if ta else ra) @ (rb.T if tb else rb)).numpy()
+        assert rel_fro(got[:, :n], ref) <= {"fp32": TOL["fp32"], "tf32": TOL["tf32"], "noalloc": TOL["bf16_f32out"]}[entry]
