@@ -145,9 +145,10 @@ cudaError_t p2p_allreduce_emulated_launch(const P2pParams* ranks_dev, const P2pP
 cudaError_t elementwise_prepare();
 cudaError_t convert_f32_to_bf16(const float* src, __nv_bfloat16* dst, size_t n, cudaStream_t s);
 cudaError_t convert_bf16_to_f32(const __nv_bfloat16* src, float* dst, size_t n, cudaStream_t s);
-// dz = y (ref) or (y - t) * inv_batch (baseline); loss += 0.5 * sum(d^2) * loss_scale
-cudaError_t loss_grad_launch(const float* y, const float* target, void* dz, int dz_type, size_t n,
-                             int baseline, float inv_batch, double loss_scale, double* loss,
+// dz = y (ref) or (y - t) * inv_batch (baseline); loss += 0.5 * sum(d^2) * loss_scale. Rows of `pitch` elements (a
+// multiple of 4 where it is not `cols`); dz is zero behind column cols.
+cudaError_t loss_grad_launch(const float* y, const float* target, void* dz, int dz_type, int rows, int cols,
+                             int pitch, int baseline, float inv_batch, double loss_scale, double* loss,
                              cudaStream_t s, float* dz_lo = nullptr);
 // w = fma(-lr, g, w); optional bf16 copy of the new weights, optional low-order twin w - tf32(w)
 cudaError_t sgd_launch(float* w, const void* g, int g_type, __nv_bfloat16* w_bf16, size_t n, float lr,

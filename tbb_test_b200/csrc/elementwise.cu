@@ -76,7 +76,8 @@ template <typename TO>
 __global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict__ y,
                                                         const float* __restrict__ t,
                                                         TO* __restrict__ dz, float* __restrict__ dz_lo, size_t n,
-                                                        int baseline, float inv_batch, double loss_scale,
+                                                        int cols, int pitch, int baseline, float inv_batch,
+                                                        double loss_scale,
                                                         double* __restrict__ loss) {
   // fp32 partial sums per thread (a few hundred terms each), double from the block level up
   float local = 0.f;
@@ -84,6 +85,13 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict_
   const size_t nvec = n / 4;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
     float4 d = __ldg(reinterpret_cast<const float4*>(y) + i);
+    if (pitch != cols) {  // padded rows: what the forward GEMM left behind the last column is 0 * operand, perhaps NaN
+      const int left = cols - (int)(4 * i % (size_t)pitch);
+      if (left < 1) d.x = 0.f;
+      if (left < 2) d.y = 0.f;
+      if (left < 3) d.z = 0.f;
+      if (left < 4) d.w = 0.f;
+    }
     float4 g = d;
     if (baseline) {
       const float4 tv = __ldg(reinterpret_cast<const float4*>(t) + i);
@@ -252,16 +260,17 @@ cudaError_t split_lo_launch(const float* src, float* dst, size_t n, cudaStream_t
   return cudaGetLastError();
 }
 
-cudaError_t loss_grad_launch(const float* y, const float* target, void* dz, int dz_type, size_t n,
-                             int baseline, float inv_batch, double loss_scale, double* loss,
+cudaError_t loss_grad_launch(const float* y, const float* target, void* dz, int dz_type, int rows, int cols,
+                             int pitch, int baseline, float inv_batch, double loss_scale, double* loss,
                              cudaStream_t s, float* dz_lo) {
+  const size_t n = (size_t)rows * pitch;
   if (n == 0) return cudaSuccess;
   int grid = grid_for(n / 4 + 1, device_sms(), 8);
   if (dz_type == T_BF16)
-    loss_grad_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(y, target, (__nv_bfloat16*)dz, nullptr, n, baseline,
+    loss_grad_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(y, target, (__nv_bfloat16*)dz, nullptr, n, cols, pitch, baseline,
                                                          inv_batch, loss_scale, loss);
   else
-    loss_grad_kernel<float><<<grid, 256, 0, s>>>(y, target, (float*)dz, dz_lo, n, baseline, inv_batch,
+    loss_grad_kernel<float><<<grid, 256, 0, s>>>(y, target, (float*)dz, dz_lo, n, cols, pitch, baseline, inv_batch,
                                                  loss_scale, loss);
   return cudaGetLastError();
 }

@@ -52,8 +52,10 @@ struct b2_handle {
   std::vector<int> nf;
   // Row pitch (elements) of every matrix with nf[l] columns: activations, gradients, weights of layer l.
   // With bf16 operands on the tensor cores it is nf[l] rounded up to 8, whole 16-byte pieces, which is what
-  // TMA can address; else rows are dense. The padding is zero from the allocation on and no kernel
-  // gives it another value (stores are clipped at nf[l]; 0 - lr * 0 in the updates), or it is never read.
+  // TMA can address; else rows are dense. The padding is zero from the allocation on, but nothing may rely on that: a
+  // store of a result takes whole 16-byte pieces along, and in a row that meets an Inf or a NaN the accumulators
+  // behind the last column are 0 * Inf. So every reader leaves the padding out, and that of the weights, which
+  // outlives a step, goes back to zero with an upload.
   std::vector<int> ld;
   int L = 0, b0 = 0, b1 = 0, bl = 0, sms = 148;
   int gemm_sms = 148;  // SMs the persistent GEMM kernels of the step occupy (sms - comm_sms)
@@ -822,12 +824,11 @@ int enqueue_step(b2_handle* h, bool timed, int slot = 0) {
     if (timed) CK(h, cudaEventRecord(phase_ev(h, l, B2_T_FWD, 1), sm));
   }
   {
-    const size_t n = (size_t)h->bl * h->ld[L];
     const bool baseline = h->cfg.mode == B2_MODE_BASELINE;
-    CK(h, loss_grad_launch(h->y, target, h->dz[L - 1], h->op_type, n, baseline ? 1 : 0,
+    CK(h, loss_grad_launch(h->y, target, h->dz[L - 1], h->op_type, h->bl, h->nf[L], h->ld[L], baseline ? 1 : 0,
                            1.0f / (float)h->cfg.batch, baseline ? 1.0 / (double)h->cfg.batch : 1.0, loss_acc, sm,
                            h->x3 ? h->dz_lo[L - 1] : nullptr));
-    if (n) ++h->launches;
+    if (h->bl) ++h->launches;
     if (wg) CK(h, cudaEventRecord(h->ev_dz_last, sm));
   }
   for (int l = L - 1; l >= 0; --l) {
@@ -1408,9 +1409,11 @@ int b2_upload_weights(b2_handle* h, int l, const float* host, size_t ld) {
   ENTER(h);
   LAYER_OK(h, l, h->L - 1);
   if (!host || ld < (size_t)h->nf[l]) return fail(h, B2_ERR_INVALID, "bad host matrix");
-  const int rows = h->nf[l + 1], cols = h->nf[l];
-  CK(h, cudaMemcpy2DAsync(h->w[l], (size_t)h->ld[l] * 4, host, ld * 4, (size_t)cols * 4, rows, cudaMemcpyHostToDevice,
+  const int rows = h->nf[l + 1], cols = h->nf[l], pitch = h->ld[l];
+  CK(h, cudaMemcpy2DAsync(h->w[l], (size_t)pitch * 4, host, ld * 4, (size_t)cols * 4, rows, cudaMemcpyHostToDevice,
                           h->s_main));
+  if (pitch != cols)  // a step that met an Inf or a NaN may have left one there
+    CK(h, cudaMemset2DAsync(h->w[l] + cols, (size_t)pitch * 4, 0, (size_t)(pitch - cols) * 4, rows, h->s_main));
   if (h->op_type == T_BF16) {
     CK(h, convert_f32_to_bf16(h->w[l], h->w16[l], layer_elems(h, l), h->s_main));
     ++h->launches;
@@ -2148,7 +2151,7 @@ int b2_weights_fingerprint(b2_handle* h, int l, unsigned long long* out) {
   const size_t n = layer_elems(h, l);
   CK(h, cudaStreamSynchronize(h->s_main));
   CK(h, cudaMemsetAsync(acc, 0, sizeof *acc, h->s_main));
-  if (h->op_type == T_BF16 && (h->nf[l] & 1))  // padded rows of odd length: pair the elements as in dense rows
+  if (h->op_type == T_BF16 && h->ld[l] != h->nf[l])  // the words of dense rows, without the padding
     CK(h, fingerprint_rows16_launch(h->w16[l], h->nf[l + 1], h->nf[l], h->ld[l], acc, h->s_main));
   else if (h->op_type == T_BF16)
     CK(h, fingerprint_launch(h->w16[l], n * 2, acc, h->s_main));

@@ -163,10 +163,16 @@ __device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap
   }
 }
 
-// Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic); t = targets.
+// Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic), `left` of them in front of the
+// row padding, where an accumulator is 0 * operand and NaN behind an Inf or a NaN; t = targets.
 template <bool BF16>
-__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t) {
+__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t, int left) {
   float4 d = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+  if (left < 4) {
+    if (left < 2) d.y = 0.f;
+    if (left < 3) d.z = 0.f;
+    d.w = 0.f;
+  }
   float4 g = d;
   if (p.baseline) {
     d.x -= t.x; d.y -= t.y; d.z -= t.z; d.w -= t.w;
@@ -205,10 +211,10 @@ __device__ __forceinline__ void load_chunk(float4 (&v)[8], const float* base, si
   }
 }
 
-// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats. Written by other SMs during this
-// launch: read past the L1.
+// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats, zero from element K on (the padding may
+// hold NaNs). Written by other SMs during this launch: read past the L1.
 template <bool BF16>
-__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k) {
+__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k, int K) {
   if (BF16) {
     const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(row) + k));
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -221,10 +227,14 @@ __device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const v
     const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k));
     v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
   }
+  if (k + (BF16 ? 8 : 4) > K) {
+#pragma unroll
+    for (int i = 1; i < (BF16 ? 8 : 4); ++i) v[i] = k + i < K ? v[i] : 0.f;
+  }
 }
 
 // Last layer with fewer than 16 outputs, too narrow for a tensor-core tile: eight rows per epilogue warp on the
-// CUDA cores, lanes split K (row padding is zero on both sides). Weight rows are loaded four at a time: one at
+// CUDA cores, lanes split K. Weight rows are loaded four at a time: one at
 // a time the L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
 template <bool BF16, int NMAX>
 __device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, int N, int ld, int lane) {
@@ -241,14 +251,16 @@ __device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, in
       float a[R][V];
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k);
+        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k,
+                             p.nar_k);
 #pragma unroll
       for (int n0 = 0; n0 < NMAX; n0 += 4) {
         if (n0 >= N) break;
         float b[4][V];
 #pragma unroll
         for (int n = 0; n < 4; ++n)
-          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k);
+          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k,
+                               p.nar_k);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -583,7 +595,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
               if (row0 + rr < M && gcol < N) {
                 const size_t at = (size_t)(row0 + rr) * ld + gcol;
                 if (epi == SE_LOSS)
-                  loss += loss_piece<!TF32>(p, at, v, cur[i]);
+                  loss += loss_piece<!TF32>(p, at, v, cur[i], N - gcol);
                 else
                   sgd_store(o, at,
                             sgd4(cur[i], __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),
