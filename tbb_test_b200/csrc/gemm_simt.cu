@@ -283,6 +283,7 @@ int simt_tile(int M, int N, int sms) {
   double best_cost = 1e300;
   for (int i = 0; i < 4; ++i) {
     const SimtTile& c = SIMT_TILES[i];
+    if (i > 0 && (M + c.bm - 1) / c.bm > 65535) continue;  // row blocks are gridDim.y
     const long long T = (long long)((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
     const double cost = (double)((T + sms - 1) / sms) * c.bm * c.bn / c.rate;
     if (cost < best_cost) { best_cost = cost; best = i; }

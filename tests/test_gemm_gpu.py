@@ -240,3 +240,24 @@ def test_submatrices_of_larger_ones(dev, oracle, entry, form, shape):
             ra, rb = ra.float().bfloat16().double(), rb.float().bfloat16().double()
         ref = ((ra.T if ta else ra) @ (rb.T if tb else rb)).numpy()
         assert rel_fro(got[:, :n], ref) <= {"fp32": TOL["fp32"], "tf32": TOL["tf32"], "noalloc": TOL["bf16_f32out"]}[entry]
+
+
+@pytest.mark.parametrize("m,n,transa", [(4_194_305, 32, False), (4_200_000, 17, True), (2_100_000, 20, False)])
+def test_cuda_core_gemm_of_very_many_rows(dev, m, n, transa):
+    """Row blocks are the grid's second dimension (65535 at most): from 4 194 241 rows on only the 128-row tile has few
+    enough, from 2 097 121 on the 32-row one has too many. Every row against a float64 sum (k = 16 terms, 2^-24 each)."""
+    import torch
+    from tbb_test_b200 import _capi as K
+    k = 16
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    a = torch.rand((k, m) if transa else (m, k), device="cuda", generator=g) - 0.5
+    b = torch.rand((k, n), device="cuda", generator=g) - 0.5
+    c = torch.full((m, n), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    rc = dev.lib.b2_sgemm(dev._h, K.PREC_FP32, int(transa), 0, m, n, k, 1.0, a.data_ptr(), a.shape[1], b.data_ptr(), n, 0.0,
+                          c.data_ptr(), n)
+    assert rc == K.OK and dev.lib.b2_sync(dev._h) == K.OK, dev.lib.b2_last_error(dev._h)
+    op = (a.T if transa else a).double()
+    ref, mag = op @ b.double(), op.abs() @ b.double().abs()
+    assert bool(((c.double() - ref).abs() <= 16 * 2.0 ** -24 * mag).all())
