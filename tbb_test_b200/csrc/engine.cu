@@ -132,6 +132,7 @@ struct b2_handle {
   size_t sync_bytes = 0;
   // Whole steps in one launch (step_kernel.cu), one plan per input slot; null: one launch per GEMM
   StepPlan* step_plan[2] = {nullptr, nullptr};
+  int launch_steps = 1;  // steps b2_step runs per launch
   unsigned int* status_dev = nullptr;
   unsigned long long* fp_dev = nullptr;  // accumulator of b2_weights_fingerprint
   float* tc_ws = nullptr;           // stream-K workspace shared by this handle's GEMMs (they
@@ -514,6 +515,19 @@ int build_sites(b2_handle* h) {
   return B2_OK;
 }
 
+// Steps per launch of the step kernel, so that a launch lasts about LAUNCH_US: it holds every SM, and work of other
+// handles, streams or processes gets its turn only between launches (64 steps of 20 x 512, batch 2048 in one launch were
+// 18.6 ms). A step is estimated as 5 us for each GEMM of the chain of layers plus all GEMMs at the rate the kernel
+// reaches: bf16, 5 x 1024, batch 1024 90 us (measured 107); 20 x 512, batch 2048 280 (290); 4 x 2048, batch 2048 298 (256).
+constexpr double LAUNCH_US = 2000.0;
+int steps_per_launch(const b2_handle* h) {
+  double flops = 0;
+  for (int l = 0; l < h->L; ++l) flops += 6.0 * h->bl * h->nf[l] * h->nf[l + 1];
+  const double rate = h->op_type == T_BF16 ? 800e6 : h->x3 ? 120e6 : 400e6;  // flops per us
+  const double n = LAUNCH_US / (5.0 * 2 * h->L + flops / rate);
+  return n < 1 ? 1 : n > 64 ? 64 : (int)n;
+}
+
 // Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken when every GEMM of the step
 // is at most two rounds of 128 x 128 tiles over the SMs, where the chain of layers is bound by latency; wider
 // layers keep the larger tiles of gemm_tc_kernel (per step, one launch per GEMM against one per step: 4 x 2048,
@@ -604,6 +618,7 @@ int build_step_plans(b2_handle* h) {
       return B2_OK;
     }
   }
+  h->launch_steps = steps_per_launch(h);
   return B2_OK;
 }
 
@@ -1590,9 +1605,8 @@ int b2_step(b2_handle* h, int iters) {
   }
   CK(h, cudaEventRecord(h->ev_t0, h->s_main));
   if (fused) {
-    // launches of a bounded number of steps, so that other work on the GPU gets its turn in between
-    for (int it = 0; it < iters; it += 64)
-      if ((rc = enqueue_fused(h, 0, iters - it < 64 ? iters - it : 64))) return rc;
+    for (int left = iters; left > 0; left -= h->launch_steps)
+      if ((rc = enqueue_fused(h, 0, std::min(left, h->launch_steps)))) return rc;
   }
   for (int it = 0; it < iters && !fused; ++it) {
     if (graph) {

@@ -120,3 +120,37 @@ def test_two_handles_in_two_threads(native, oracle, prec):
         for l in range(L):
             assert np.array_equal(m.weights(l), ref[l])
         m.close()
+
+
+@pytest.mark.parametrize("nf,batch,steps", [([512] * 21, 2048, 64), ([1024] * 6, 1024, 50), ([64, 64, 64], 64, 130)],
+                         ids=["deep", "c1", "small"])
+def test_steps_are_split_into_short_launches(native, oracle, monkeypatch, nf, batch, steps):
+    """b2_step holds the GPU for a few ms at a time at most (the limit is 2 ms by estimate; twice that here, for a slow
+    clock), whatever the number of steps, in few launches for short steps; and the split changes no bit."""
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    ws = [oracle.fill_uniform(nf[l + 1], nf[l], 5 + l, -0.1, 0.1) for l in range(len(nf) - 1)]
+    x, t = oracle.fill_normal(batch, nf[0], 1), oracle.fill_sign(batch, nf[-1], 2)
+
+    def run(fused):
+        monkeypatch.setenv("B2_STEP_KERNEL", fused)
+        m = MLP(nf, batch, precision=K.PREC_BF16, lr=1e-4)
+        for l, w in enumerate(ws):
+            m.upload_weights(l, w)
+        m.upload_input(x)
+        m.upload_target(t)
+        before = m.launch_counts()[0]
+        m.step(steps)
+        launches = m.launch_counts()[0] - before
+        loss, out = m.loss(), [m.weights(l) for l in range(len(ws))]
+        m.reset_timing()
+        m.step(steps)
+        ms = m.timing()[1]
+        m.close()
+        return launches, loss, out, ms
+
+    launches, loss, out, ms = run("1")
+    assert ms / launches <= 4.0, (ms, launches)
+    assert launches <= max(3, ms / 0.5)
+    _, loss0, out0, _ = run("0")
+    assert all(np.array_equal(a, b) for a, b in zip(out, out0)) and abs(loss - loss0) <= 1e-5 * abs(loss0)
