@@ -66,7 +66,8 @@ def build_host(force=False, verbose=False):
     srcs = sorted(glob.glob(os.path.join(HOST, "*.cc")))
     if not srcs:
         return None
-    deps = srcs + glob.glob(os.path.join(HOST, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    deps = srcs + glob.glob(os.path.join(HOST, "*.h")) + glob.glob(os.path.join(CSRC, "*.h")) + \
+        glob.glob(os.path.join(ROOT, "include", "*.h"))
     lib_srcs = [s for s in srcs if os.path.basename(s) != "mlp_cuda.cc"]
     flags = ["-std=c++17", "-O2", "-fPIC", "-Wall", "-I", os.path.join(ROOT, "include"), "-I", HOST]
     if force or _stale(HOST_LIB, deps):

@@ -37,6 +37,7 @@ struct GemmDesc {
   int in_type;   // ElemType of A, B and aux
   int out_type;  // ElemType of C
   int pad_writable;  // 1: the bytes between column N and the next 16-byte boundary of a row of C may be overwritten
+  int shared_sms;    // 1: another library's kernels may hold some of the SMs while this GEMM runs
   // Optional stream-K workspace of the tensor-core kernel (null = whole tiles per CTA):
   // TC_WS_SLOT_BYTES per SM and one zero-initialised flag word per SM. GEMMs that share a
   // workspace must not overlap on the GPU.

@@ -219,6 +219,7 @@ size_t layer_elems(const b2_handle* h, int l) { return (size_t)h->nf[l + 1] * h-
 int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
   s.d.ws = h->tc_ws;
   s.d.ws_flags = h->tc_ws_flags;
+  s.d.shared_sms = h->cfg.world_size > 1 && h->cfg.allreduce;
   s.d.pad_writable = 1;  // rows of b2_handle::ld elements
   s.active = s.d.M > 0 && s.d.N > 0 && s.d.K > 0;
   s.plan = nullptr;

@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include "tile_choice.h"
 
 namespace b2 {
 namespace {
@@ -1021,49 +1022,14 @@ TcPlan* gemm_tc_plan_create(const GemmDesc& g, int sm_count, char* err, size_t e
   p.M = g.M; p.N = g.N; p.K = g.K;
   // Tile shape: 256 x 256 per pair of SMs (cta_group::2: each SM holds 128 rows of A and half of B, two
   // accumulator stages), 256 x 256 per SM (two 128-row accumulators sharing each B slab, a single stage),
-  // 128 x 256, 128 x 128 or 128 x 64 (two stages). Chosen by a cost model: waves of the persistent grid times
-  // the time of one tile, its area per SM divided by the rate the shape sustains relative to 128 x 256
-  // (measured at 1024 x 4096 x 4096 and 8192 x 4096 x 4096, bf16 and tf32). Filling every SM is not the goal:
-  // 1024 x 4096 x 4096 bf16 takes 32 us as 64 pair tiles, 36 us as 128 x 256, 45 us as 128 x 128 on all SMs.
-  // Pair tiles against 256 x 256 per SM, us forward / weight / input gradient: 8192 x 4096 x 4096 bf16
-  // 179/185/178 against 192/195/192, tf32 359/357/354 against 372/365/370; 4096 x 4096 x 1024 tf32 57/56/56
-  // against 70/62/68; 2048 x 8192 x 8192 bf16 190/192/189 against 191/190/190.
+  // 128 x 256, 128 x 128 or 128 x 64 (two stages). The rule and its reasons: tile_choice.h.
   auto tiles = [&](int rows, int n) { return (long long)((g.M + rows - 1) / rows) * ((g.N + n - 1) / n); };
-  int bn = 256;
-  bool pair_best = false;
   const char* pe = getenv("B2_TC_PAIR");  // experiments: 0 never, 1 / 2 wherever the tile is 256 wide
   const char* sk = getenv("B2_TC_STREAMK");
-  {
-    struct Cand { int sub_m, bn; double rate; bool pair; };
-    const Cand cands[5] = {{2, 256, 1.08, true}, {2, 256, 1.0, false}, {1, 256, 1.0, false}, {1, 128, 0.74, false},
-                           {1, 64, 0.42, false}};
-    const bool pair_ok = !(pe && pe[0] == '0') && !(sk && sk[0] == '1') && sm_count >= 2 && g.M > BLOCK_M;
-    double best = 1e300;
-    int best_i = 4;
-    for (int i = 0; i < 5; ++i) {
-      const Cand& c = cands[i];
-      if (c.pair && !pair_ok) continue;
-      if (c.bn / 2 >= g.N && c.bn > 64) continue;  // tile wider than twice the matrix
-      if (x3 && (c.sub_m == 2 || c.bn == 256)) continue;  // twice the shared memory per stage: 128 x 128 at most
-      const long long T = tiles(c.sub_m * BLOCK_M, c.bn);
-      double waves, area = (double)(c.sub_m * BLOCK_M) * c.bn;
-      if (c.pair) {
-        waves = (double)((T + sm_count / 2 - 1) / (sm_count / 2));
-        area /= 2;
-      } else if (c.sub_m == 2) {
-        // the last partial wave is handed out as 128-row halves when that fits in one wave
-        const long long full = T / sm_count, rem = T % sm_count;
-        waves = (double)full + (rem == 0 ? 0.0 : (T > sm_count && rem * 2 <= sm_count ? 0.5 : 1.0));
-      } else {
-        waves = (double)((T + sm_count - 1) / sm_count);
-      }
-      const double cost = waves * area / c.rate;
-      if (cost < best * 0.999) { best = cost; best_i = i; }
-    }
-    bn = cands[best_i].bn;
-    p.sub_m = cands[best_i].sub_m;
-    pair_best = cands[best_i].pair;
-  }
+  const TileChoice tile = choose_tile(g.M, g.N, sm_count, x3, !(pe && pe[0] == '0') && !(sk && sk[0] == '1'), g.shared_sms != 0);
+  int bn = tile.bn;
+  p.sub_m = tile.sub_m;
+  const bool pair_best = tile.pair != 0;
   p.block_n = bn;
   if (const char* fb = getenv("B2_TC_BN")) {  // experiments: force the tile width
     const int v = atoi(fb);

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../csrc/bucket_plan.h"
+#include "../csrc/tile_choice.h"
 #include "HyperCubeAllReduce.h"
 #include "b2_rng.h"
 #include "TwistedHyperCube.h"
@@ -111,6 +112,12 @@ void b2h_plan_buckets_sharded(const size_t* layer_bytes, int nlayers, int world_
                               int* bucket_low, int* bucket_high) {
   b2::plan_gradient_buckets(layer_bytes, nlayers, world_size, true, ar_bucket_mb, growth, bucket_low, bucket_high);
   if (ar_bucket_mb < 0 && world_size > 1) b2::plan_split_lowest_layer(nlayers, bucket_low, bucket_high);
+}
+
+// Tile shape of the tensor-core GEMM (csrc/tile_choice.h): rows in 128s, columns, pair of SMs.
+void b2h_choose_tile(int m, int n, int sms, int x3, int pair_ok, int shared, int* out3) {
+  const b2::TileChoice t = b2::choose_tile(m, n, sms, x3 != 0, pair_ok != 0, shared != 0);
+  out3[0] = t.sub_m; out3[1] = t.bn; out3[2] = t.pair;
 }
 
 void b2h_ring_info(int nsock, int sid, int task, int* out3) {

@@ -226,3 +226,24 @@ def test_bench_reads_the_same_bucket_rule(host):
     assert bench.gradient_buckets([64 * mib] * 8, 2, -1) == [128 * mib] * 4
     assert bench.gradient_buckets([64 * mib] * 8, 4, -1) == [128 * mib, 192 * mib, 192 * mib]
     assert bench.gradient_buckets([64 * mib] * 8, 8, 0) == [64 * mib] * 8
+
+
+def test_tile_choice_beside_collectives(host):
+    """A GEMM that shares the GPU with collectives (csrc/tile_choice.h) gets no CTA-pair tile, whatever its size, and the
+    shapes the multi-GPU figures were measured with; alone, the wide ones get pairs."""
+    def tile(m, n, sms, x3=0, pair_ok=1, shared=0):
+        out = (C.c_int * 3)()
+        host.b2h_choose_tile(m, n, sms, x3, pair_ok, shared, out)
+        return tuple(out)
+
+    for m in (1, 100, 128, 129, 300, 512, 1000, 1024, 2048, 4096, 8192, 20000):
+        for n in (16, 64, 129, 512, 1000, 1024, 4096, 8192):
+            for sms in (148, 128, 1):
+                assert tile(m, n, sms, shared=1)[2] == 0
+                assert tile(m, n, sms, x3=1)[1] <= 128 and tile(m, n, sms, x3=1)[2] == 0
+                if m <= 128 or sms < 2:
+                    assert tile(m, n, sms)[2] == 0
+    # rows of one of 1, 2, 4, 8 GPUs x 4096, with and without SMs left to the collectives
+    assert [tile(m, 4096, s, shared=1) for m, s in ((8192, 148), (4096, 148), (2048, 128), (1024, 128))] == \
+        [(2, 256, 0), (2, 256, 0), (2, 256, 0), (1, 256, 0)]
+    assert [tile(m, 4096, 148) for m in (8192, 4096, 1024)] == [(2, 256, 1)] * 3
