@@ -163,16 +163,10 @@ __device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap
   }
 }
 
-// Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic), `left` of them in front of the
-// row padding, where an accumulator is 0 * operand and NaN behind an Inf or a NaN; t = targets.
+// Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic); t = targets.
 template <bool BF16>
-__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t, int left) {
+__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t) {
   float4 d = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-  if (left < 4) {
-    if (left < 2) d.y = 0.f;
-    if (left < 3) d.z = 0.f;
-    d.w = 0.f;
-  }
   float4 g = d;
   if (p.baseline) {
     d.x -= t.x; d.y -= t.y; d.z -= t.z; d.w -= t.w;
@@ -211,25 +205,21 @@ __device__ __forceinline__ void load_chunk(float4 (&v)[8], const float* base, si
   }
 }
 
-// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats, zero from element K on (the padding may
-// hold NaNs). Written by other SMs during this launch: read past the L1.
+// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats, the 16 bytes masked by `m` (the padding
+// behind the last column may hold NaNs). Written by other SMs during this launch: read past the L1.
 template <bool BF16>
-__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k, int K) {
+__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k, const uint32_t (&m)[4]) {
   if (BF16) {
     const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(row) + k));
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    const uint32_t w[4] = {u.x & m[0], u.y & m[1], u.z & m[2], u.w & m[3]};
 #pragma unroll
     for (int i = 0; i < (BF16 ? 4 : 2); ++i) {
       v[2 * i] = __uint_as_float(w[i] << 16);
       v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
     }
-  } else {
+  } else {  // rows of whole pieces
     const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k));
     v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-  }
-  if (k + (BF16 ? 8 : 4) > K) {
-#pragma unroll
-    for (int i = 1; i < (BF16 ? 8 : 4); ++i) v[i] = k + i < K ? v[i] : 0.f;
   }
 }
 
@@ -248,19 +238,23 @@ __device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, in
 #pragma unroll
       for (int n = 0; n < NMAX; ++n) acc[r][n] = 0.f;
     for (int k = lane * V; k < p.nar_k; k += 32 * V) {
+      uint32_t m[4];  // bf16: which halves of the piece lie in front of column K
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int left = p.nar_k - k - 2 * i;
+        m[i] = left > 1 ? 0xFFFFFFFFu : left == 1 ? 0xFFFFu : 0u;
+      }
       float a[R][V];
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k,
-                             p.nar_k);
+        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k, m);
 #pragma unroll
       for (int n0 = 0; n0 < NMAX; n0 += 4) {
         if (n0 >= N) break;
         float b[4][V];
 #pragma unroll
         for (int n = 0; n < 4; ++n)
-          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k,
-                               p.nar_k);
+          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k, m);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -588,6 +582,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
 #pragma unroll
             for (int i = 0; i < 8; ++i) cur[i] = pre[i];
             if (fetch && !last) load_chunk(pre, extra, ld, row0, M, gcol + 32, N, lane);
+            // behind the last column, in the row padding, an accumulator is 0 * operand: NaN after an Inf or a NaN
+            const uint32_t m1 = gcol + 1 < N ? ~0u : 0u, m2 = gcol + 2 < N ? ~0u : 0u, m3 = gcol + 3 < N ? ~0u : 0u;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int rr = 4 * i + (lane >> 3);
@@ -595,7 +591,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
               if (row0 + rr < M && gcol < N) {
                 const size_t at = (size_t)(row0 + rr) * ld + gcol;
                 if (epi == SE_LOSS)
-                  loss += loss_piece<!TF32>(p, at, v, cur[i], N - gcol);
+                  loss += loss_piece<!TF32>(p, at, make_uint4(v.x, v.y & m1, v.z & m2, v.w & m3), cur[i]);
                 else
                   sgd_store(o, at,
                             sgd4(cur[i], __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),
