@@ -41,7 +41,6 @@ namespace {
 
 enum StepEpi : int { SE_NONE = 0, SE_RELU = 1, SE_MASK = 2, SE_LOSS = 3, SE_SGD = 4, SE_NARROW = 5 };
 enum OpForm : int { OP_K2D = 0, OP_K3D = 1, OP_MN3D = 2, OP_MN2D = 3 };
-constexpr int MAX_OPS = 64;
 constexpr int EPI_BYTES = 4 * 2 * 4096;  // two chunk buffers of 32 rows x 128 bytes per epilogue warp
 
 // One operand of a GEMM: how its slabs are fetched and described to the tensor core.
@@ -77,9 +76,7 @@ struct StepOp {
   int sig_row, sig_all, own_target; // counters this op raises (-1: nobody waits for them)
 };
 
-// The scalars travel as kernel parameters, in the constant bank: read from global memory they cost an L2
-// round trip per cache line and tile, because every acquiring load of a counter drops the L1.
-struct StepArgs {
+struct StepHead {
   const StepMaps* maps;
   unsigned int* counters;
   unsigned int* status;
@@ -101,7 +98,17 @@ struct StepArgs {
   const void* nar_w;
   float* nar_y;
   int nar_k, nar_lda;
-  StepOp op[MAX_OPS];
+};
+// The scalars travel as kernel parameters, in the constant bank: read from global memory they cost an L2
+// round trip per cache line and tile, because every acquiring load of a counter drops the L1. So a step may
+// have as many GEMMs as fit into the 32 764 bytes of parameters a launch can take, about 50 layers. Every launch
+// copies its parameters, whatever part of them is used (3 small layers, one blocking step: 89 us with 32 KB
+// against 77 us with 14 KB), so there is a smaller table for the usual depths, up to 21 layers.
+constexpr int SMALL_OPS = 64;
+constexpr int MAX_OPS = (int)((32764 - sizeof(StepHead)) / sizeof(StepOp));
+template <int OPS>
+struct StepArgs : StepHead {
+  StepOp op[OPS];
 };
 
 __device__ __forceinline__ float lo_part(float v) {
@@ -112,7 +119,8 @@ __device__ __forceinline__ float lo_part(float v) {
 struct Walk {
   int w, it, op;
   __device__ __forceinline__ void begin() { w = blockIdx.x; it = 0; op = 0; }
-  __device__ __forceinline__ bool settle(const StepArgs& p) {
+  template <int OPS>
+  __device__ __forceinline__ bool settle(const StepArgs<OPS>& p) {
     while (w >= p.items) { w -= p.items; ++it; op = 0; }
     if (it >= p.steps) return false;
     while (op + 1 < p.nops && w >= p.op[op + 1].first_item) ++op;
@@ -165,7 +173,7 @@ __device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap
 
 // Output gradient and loss of four consecutive columns (loss_grad_kernel's arithmetic); t = targets.
 template <bool BF16>
-__device__ __forceinline__ float loss_piece(const StepArgs& p, size_t at, const uint4& v, const float4& t) {
+__device__ __forceinline__ float loss_piece(const StepHead& p, size_t at, const uint4& v, const float4& t) {
   float4 d = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
   float4 g = d;
   if (p.baseline) {
@@ -227,7 +235,7 @@ __device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const v
 // CUDA cores, lanes split K. Weight rows are loaded four at a time: one at
 // a time the L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
 template <bool BF16, int NMAX>
-__device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, int N, int ld, int lane) {
+__device__ __noinline__ float narrow_rows(const StepHead& p, int row0, int M, int N, int ld, int lane) {
   constexpr int V = BF16 ? 8 : 4, R = NMAX <= 4 ? 8 : 4;  // rows at a time, as registers allow
   const size_t row_bytes = (size_t)p.nar_lda * (BF16 ? 2 : 4);
   float loss = 0.f;
@@ -292,8 +300,8 @@ __device__ __noinline__ float narrow_rows(const StepArgs& p, int row0, int M, in
   return loss;
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_constant__ StepArgs p) {
+template <int KIND, int OPS>
+__global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_constant__ StepArgs<OPS> p) {
   constexpr bool TF32 = KIND != KIND_BF16, X3 = KIND == KIND_X3;
   constexpr int SLABS = X3 ? 1 : 2;
   constexpr int SLAB_K = TF32 ? 32 : 64, COL_LOG2 = TF32 ? 5 : 6;
@@ -731,7 +739,7 @@ struct StepPlan {
   StepMaps* maps_dev = nullptr;
   int kind = KIND_BF16, grid = 0;
   size_t smem = 0;
-  StepArgs args;  // counters, status, steps and learning rate are filled in per launch
+  StepArgs<MAX_OPS> args;  // counters, status, steps and learning rate are filled in per launch
 };
 
 int step_plan_counters(const StepSpec& s) {
@@ -749,7 +757,7 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
   const int slabs = x3 ? 1 : 2;
   StepPlan* plan = new StepPlan();
   memset(&plan->args, 0, sizeof plan->args);
-  StepArgs& args = plan->args;
+  StepArgs<MAX_OPS>& args = plan->args;
   StepOp* ops = args.op;
   std::vector<StepMaps> maps(nops);
   std::vector<int> row_base(nops), all_base(nops), ntiles(nops), row_add(nops);
@@ -870,15 +878,18 @@ void step_plan_destroy(StepPlan* p) {
   delete p;
 }
 
-cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
-                        cudaStream_t stream) {
-  void (*kernel)(const StepArgs) = plan->kind == KIND_BF16 ? step_kernel<KIND_BF16>
-                                   : plan->kind == KIND_TF32 ? step_kernel<KIND_TF32> : step_kernel<KIND_X3>;
+template <int OPS>
+static cudaError_t launch_ops(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
+                              cudaStream_t stream) {
+  void (*kernel)(const StepArgs<OPS>) = plan->kind == KIND_BF16 ? step_kernel<KIND_BF16, OPS>
+                                        : plan->kind == KIND_TF32 ? step_kernel<KIND_TF32, OPS> : step_kernel<KIND_X3, OPS>;
   // per launch: handles of several devices and threads share the library, and the call is cheap
   cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
   if (e != cudaSuccess) return e;
-  StepArgs a = plan->args;
+  StepArgs<OPS> a;
+  static_cast<StepHead&>(a) = plan->args;
+  memcpy(a.op, plan->args.op, sizeof a.op);
   a.counters = counters;
   a.status = status;
   a.steps = steps;
@@ -894,6 +905,12 @@ cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int*
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
+                        cudaStream_t stream) {
+  return plan->args.nops <= SMALL_OPS ? launch_ops<SMALL_OPS>(plan, steps, lr, counters, status, stream)
+                                      : launch_ops<MAX_OPS>(plan, steps, lr, counters, status, stream);
 }
 
 }  // namespace b2

@@ -10,6 +10,7 @@ pytestmark = pytest.mark.gpu
 # more tiles than SMs / one layer / every output kind the epilogue has; "narrow": last layer on the CUDA cores
 NETS = [([96, 64], 40, {}), ([256] * 6, 256, {}), ([123, 77, 201, 33], 333, {}), ([784, 500, 300, 40], 1000, {}),
         ([512, 384, 640, 128], 640, {"grad_bf16": True}), ([1024, 1536, 512], 1500, {}), ([64] * 22, 130, {}),
+        ([96] * 51, 200, {"lr": 1e-5}), ([64] * 53, 64, {"lr": 1e-5}), ([64] * 24, 130, {"input_grad": False}),
         ([192, 160, 64], 200, {"ref": True}), ([192, 160, 64], 200, {"input_grad": False}),
         ([160, 96, 10], 300, {}), ([256, 128, 1], 990, {"ref": True})]
 
@@ -18,7 +19,7 @@ def states(O, K, nf, batch, prec, steps, opts, fed=False):
     from tbb_test_b200.mlp import MLP
     L = len(nf) - 1
     mode = K.MODE_REF if opts.get("ref") else K.MODE_BASELINE
-    m = MLP(nf, batch, precision=prec, mode=mode, lr=1e-6 if opts.get("ref") else 0.01,
+    m = MLP(nf, batch, precision=prec, mode=mode, lr=1e-6 if opts.get("ref") else opts.get("lr", 0.01),
             grad_bf16=opts.get("grad_bf16", False) and prec == K.PREC_BF16, input_grad=opts.get("input_grad", True))
     for l in range(L):
         a = (6.0 / nf[l]) ** 0.5
@@ -62,7 +63,7 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
         monkeypatch.setenv("B2_STEP_KERNEL", "1")
         b, lb, nb = states(oracle, K, nf, batch, P, steps, opts)
         f, lf, _ = states(oracle, K, nf, batch, P, steps, opts, fed=True)
-        if prec == "bf16":
+        if prec == "bf16" and len(nf) <= 51:  # as many layers as the kernel's table holds
             assert nb < na  # one launch for all steps
         tail = nf[-1] < 16
         for k in a:
