@@ -23,8 +23,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -386,7 +386,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
   for (int i = 0; i < helpers; ++i) {
     try {
       pool[i] = std::thread(work, i + 1);
-    } catch (const std::system_error&) {  // no more threads to be had: those that run take all chunks
+    } catch (const std::exception&) {  // no more threads, or no memory for one: those that run take all chunks
       break;
     }
   }

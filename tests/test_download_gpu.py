@@ -1,6 +1,10 @@
 """Large downloads, which several threads share (download_rows in csrc/engine.cu)."""
 import ctypes as C
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -23,3 +27,33 @@ def test_large_downloads(native, oracle, shape, extra):
         assert rc == K.OK
         assert np.array_equal(got[:, :cols], w) and (got[:, cols:] == 7.0).all()
         m.close()
+
+
+OUT_OF_MEMORY = """
+import ctypes as C, sys
+import numpy as np
+from tbb_test_b200 import _capi as K
+from tbb_test_b200.mlp import MLP
+fake = C.CDLL(sys.argv[1])
+w = np.random.default_rng(1).standard_normal((1000, 1003), dtype=np.float32)
+m = MLP([1003, 1000], 8)
+m.upload_weights(0, w)
+got = np.full(w.shape, 7.0, np.float32)
+C.c_int.in_dll(fake, "fail_new").value = 1
+rc = m.lib.b2_download_weights(m._h, 0, got.ctypes.data_as(C.POINTER(C.c_float)), 1003)
+C.c_int.in_dll(fake, "fail_new").value = 0
+assert C.c_int.in_dll(fake, "failed").value > 0, "nothing was allocated"
+assert rc == K.OK and np.array_equal(got, w)
+print("all there")
+"""
+
+
+def test_large_download_without_memory_for_threads(native, tmp_path):
+    """Where a helper thread cannot be started for want of host memory, the calling thread does the work: no exception
+    leaves the C entry point, and every element arrives."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    so = str(tmp_path / "failing_new.so")
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-o", so, os.path.join(here, "fake", "failing_new.cc")], check=True)
+    env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=os.path.dirname(here))
+    r = subprocess.run([sys.executable, "-c", OUT_OF_MEMORY, so], env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "all there" in r.stdout, r.stderr[-2000:]
