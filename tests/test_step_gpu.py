@@ -173,6 +173,33 @@ def test_schedule_variants_agree(native, oracle, kw):
     check(out, TOL["fp32"], skip=("dinput",) if kw.get("input_grad") is False else ())
 
 
+@pytest.mark.parametrize("prec", ["bf16", "tf32", "fp32tc"])
+@pytest.mark.parametrize("nf,batch", [([128, 256, 128], 300), ([512, 2048, 2048], 4096)], ids=["small", "pairs"])
+def test_graph_replay_of_tensor_core_steps(native, oracle, monkeypatch, nf, batch, prec):
+    """One CUDA graph per step of tensor-core GEMMs (CTA-pair tiles in the wide layers): the same bits as plain
+    launches, before and after the learning rate, which the graph holds, changes."""
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    monkeypatch.setenv("B2_STEP_KERNEL", "0")
+    P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32, "fp32tc": K.PREC_FP32_TC}[prec]
+    ws = [oracle.fill_uniform(nf[l + 1], nf[l], 5 + l, -0.05, 0.05) for l in range(len(nf) - 1)]
+    x, t = oracle.fill_normal(batch, nf[0], 1), oracle.fill_sign(batch, nf[-1], 2)
+    got = []
+    for graph in (False, True):
+        m = MLP(nf, batch, precision=P, lr=0.01, use_graph=graph)
+        for l, w in enumerate(ws):
+            m.upload_weights(l, w)
+        m.upload_input(x)
+        m.upload_target(t)
+        m.step(3)
+        m.set_lr(0.002)
+        m.step(2)
+        got.append(([m.weights(l) for l in range(len(ws))] + [m.activation(len(ws))], m.loss(), m.launch_counts()))
+        m.close()
+    assert all(np.array_equal(a, b) for a, b in zip(got[0][0], got[1][0]))
+    assert abs(got[0][1] - got[1][1]) <= 1e-12 * abs(got[0][1]) and got[0][2] == got[1][2]
+
+
 def test_allreduce_sgd_known_answer(native, oracle):
     """The reference's self-check (mlp_omp.cc:325-373) for one socket: grad = i + j,
     w = i*j, alpha = 1 -> w = i*j - (i + j), exact in fp32."""

@@ -26,6 +26,7 @@ def states(O, K, nf, batch, prec, steps, opts, fed=False):
         m.upload_weights(l, O.fill_uniform(nf[l + 1], nf[l], 5 + l, -a, a))
     x = np.ascontiguousarray(O.fill_normal(batch, nf[0], 1))
     t = np.ascontiguousarray(O.fill_sign(batch, nf[-1], 2))
+    before = m.launch_counts()[0]
     if fed:
         fp = C.POINTER(C.c_float)
         for i in range(steps):
@@ -34,8 +35,10 @@ def states(O, K, nf, batch, prec, steps, opts, fed=False):
     else:
         m.upload_input(x)
         m.upload_target(t)
+        before = m.launch_counts()[0]
         m.step(steps)
         loss = m.loss()
+    launches = m.launch_counts()[0] - before
     out = {"y": m.activation(L)}
     for l in range(L):
         out[f"w{l}"], out[f"dw{l}"], out[f"dz{l}"] = m.weights(l), m.weight_grad(l), m.dz(l)
@@ -43,7 +46,6 @@ def states(O, K, nf, batch, prec, steps, opts, fed=False):
             out[f"act{l}"] = m.activation(l)
     if opts.get("input_grad", True):
         out["dinput"] = m.input_grad()
-    launches = m.launch_counts()[0]
     m.close()
     return out, loss, launches
 
@@ -62,9 +64,14 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
         a, la, na = states(oracle, K, nf, batch, P, steps, opts)
         monkeypatch.setenv("B2_STEP_KERNEL", "1")
         b, lb, nb = states(oracle, K, nf, batch, P, steps, opts)
-        f, lf, _ = states(oracle, K, nf, batch, P, steps, opts, fed=True)
-        if prec == "bf16" and len(nf) <= 51:  # as many layers as the kernel's table holds
-            assert nb < na  # one launch for all steps
+        f, lf, nfed = states(oracle, K, nf, batch, P, steps, opts, fed=True)
+        # every GEMM but a narrow last one on the tensor cores, and no more layers than the kernel's table holds
+        if (prec == "bf16" or all(n % 4 == 0 for n in nf)) and len(nf) <= 51:
+            assert nb == 1, "not one launch for all steps"
+            # per host-fed step, in both input slots: the launch, and the conversion of the input or its twin
+            assert nfed == steps * (1 if prec == "tf32" else 2)
+        else:
+            assert nb == na and na >= steps * (3 * len(nf) - 4), "one launch per GEMM"
         tail = nf[-1] < 16
         for k in a:
             for o in (b, f):
@@ -76,14 +83,14 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
         assert abs(la - lb) <= 1e-5 * abs(la) and abs(la - lf) <= 1e-5 * abs(la)
 
 
-@pytest.mark.parametrize("prec", ["bf16"])
+@pytest.mark.parametrize("prec", ["bf16", "tf32"])
 def test_two_handles_in_two_threads(native, oracle, prec):
     """Cooperative launches of two handles on one GPU, issued by two host threads at once, each keep their grid
     resident: both finish with the weights they reach alone."""
     import threading
     from tbb_test_b200 import _capi as K
     from tbb_test_b200.mlp import MLP
-    P = {"bf16": K.PREC_BF16, "fp32": K.PREC_FP32}[prec]
+    P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32}[prec]
     nf, batch, L = [512] * 5, 512, 4
 
     def make(seed):
@@ -123,8 +130,8 @@ def test_two_handles_in_two_threads(native, oracle, prec):
         m.close()
 
 
-@pytest.mark.parametrize("nf,batch,steps", [([512] * 21, 2048, 64), ([1024] * 6, 1024, 50), ([64, 64, 64], 64, 130)],
-                         ids=["deep", "c1", "small"])
+@pytest.mark.parametrize("nf,batch,steps", [([512] * 21, 2048, 64), ([1024] * 6, 1024, 50), ([64, 64, 64], 64, 130),
+                                            ([64, 64, 64], 64, 65)], ids=["deep", "c1", "small", "one-more"])
 def test_steps_are_split_into_short_launches(native, oracle, monkeypatch, nf, batch, steps):
     """b2_step holds the GPU for a few ms at a time at most (the limit is 2 ms by estimate; twice that here, for a slow
     clock), whatever the number of steps, in few launches for short steps; and the split changes no bit."""
