@@ -226,13 +226,18 @@ def measured_peaks():
         return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}, "fallback"
 
 
-def profiled_traffic(precision, rows, nf):
+def gemm_kernel(world):
+    """The kernel most GEMMs of wide layers run in: CTA pairs, unless collectives share the GPU (tile_choice.h)."""
+    return "gemm_tc_pair_kernel" if world == 1 else "gemm_tc_kernel"
+
+
+def profiled_traffic(kernel, precision, rows, nf):
     """DRAM bytes (read + write) per GEMM launch from the ncu summary kept for this shape under
     profiles/ (a line `dram_bytes_per_launch: fwd=.. wgrad=.. dgrad=..`), mean over the three
     forms, or None when the shape was not profiled."""
     if not all(f == nf[0] for f in nf):
         return None, "no ncu capture for this shape"
-    name = f"gemm_tc_kernel_{rows}x{nf[0]}x{nf[0]}_{precision}_ncu.md"
+    name = f"{kernel}_{rows}x{nf[0]}x{nf[0]}_{precision}_ncu.md"
     path = os.path.join(ROOT, "profiles", name)
     try:
         with open(path) as f:
@@ -567,9 +572,9 @@ def main():
     peak_burst = peaks.get("bf16_tflops", 1590.0)
     peak_sust = peaks.get("bf16_tflops_sustained", 1400.0)
     n_params = sum(nf[l] * nf[l + 1] for l in range(L))
-    traffic, traffic_note = profiled_traffic(args.precision, bl, nf)
+    traffic, traffic_note = profiled_traffic(gemm_kernel(world), args.precision, bl, nf)
     roofline = {"bound": "tensor",
-                "kernel": "gemm_tc_kernel (fwd + wgrad + dgrad launches; flops / time with a GEMM running, "
+                "kernel": gemm_kernel(world) + " (fwd + wgrad + dgrad launches; flops / time with a GEMM running, "
                           f"{phase_steps}-step run with per-phase events)",
                 "achieved": achieved_tf, "peak": peak_burst, "unit": "TFLOP/s",
                 "frac": achieved_tf / peak_burst if peak_burst else None,

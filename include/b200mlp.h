@@ -51,10 +51,12 @@ typedef enum {
   B2_PREC_FP32 = 0, /* fp32 operands, CUDA-core FMA (parity mode) */
   B2_PREC_TF32 = 1, /* fp32 storage, tcgen05 kind::tf32 */
   B2_PREC_BF16 = 2, /* bf16 operands (activations, gradients, a bf16 weight copy),
-                       tcgen05 kind::f16 */
+                       tcgen05 kind::f16: layers of any width, on rows padded to 16 bytes (but for
+                       the forward GEMM of a layer with fewer than 16 outputs), so sums are added
+                       by the tensor core, which truncates when it adds, not by fp32 FMAs */
   B2_PREC_FP32_TC = 3 /* fp32 storage and fp32-class results on the tensor cores: every operand x
                        is kept with its low-order twin x - tf32(x), and each k-step issues three
-                       kind::tf32 MMAs (A*B + A*B_lo + A_lo*B) into the same fp32 accumulator;
+                       kind::tf32 MMAs (A*B, and A*B_lo + A_lo*B) into two fp32 accumulators;
                        same tolerance class as B2_PREC_FP32 (the reference's sgemm), about a
                        third of the TF32 rate */
 } b2_precision;
@@ -81,7 +83,8 @@ typedef struct {
   int input_grad;           /* 1 = also compute dA[0] like the reference (mlp_omp.cc:656) */
   int collect_timing;       /* 1 = per-phase CUDA-event timing (sum_times, mlp_bench_common.h:35) */
   int use_graph;            /* 1 = replay each step as one CUDA graph (refused with B2_ERR_UNSUPPORTED
-                               when world_size > 1 and allreduce = 1) */
+                               when world_size > 1 and allreduce = 1). No graph is made where b2_step
+                               runs whole steps in one launch anyway */
   int force_simt;           /* 1 = never use the tensor-core kernels (debugging aid) */
   int comm_sms;             /* SMs the persistent GEMM kernels leave free for the collective's CTAs
                                while allreduce and GEMMs overlap (the counterpart of the threads the
@@ -351,9 +354,9 @@ int b2_write_trace(b2_handle* h, const char* path);
 
 /* Which kernel serves the GEMM sites of the step (three per layer, plus the second input slot's):
  * in the tensor-core precisions a site whose shape or alignment the tensor-core kernel cannot
- * address (a leading dimension that is not a multiple of 16 bytes, fewer than 16 output columns,
+ * address (TF32 and FP32_TC: a width that is not a multiple of 4; fewer than 16 output columns,
  * such as the 1-wide tail layer of the reference's topology, mlp_bench_common.h:26) falls to the
- * CUDA-core kernel, about 30 times slower. The counts and the reason given for the first such
+ * CUDA-core kernels, which are many times slower for wide layers. The counts and the reason given for the first such
  * site make that visible; with B2_VERBOSE set in the environment it is also printed once. */
 int b2_site_report(const b2_handle* h, int* tensor_core_sites, int* cuda_core_sites, char* first_reason,
                    size_t reason_len);

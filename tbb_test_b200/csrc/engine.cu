@@ -519,7 +519,8 @@ int build_sites(b2_handle* h) {
 // Steps per launch of the step kernel, so that a launch lasts about LAUNCH_US: it holds every SM, and work of other
 // handles, streams or processes gets its turn only between launches (64 steps of 20 x 512, batch 2048 in one launch were
 // 18.6 ms). A step is estimated as 5 us for each GEMM of the chain of layers plus all GEMMs at the rate the kernel
-// reaches: bf16, 5 x 1024, batch 1024 90 us (measured 107); 20 x 512, batch 2048 280 (290); 4 x 2048, batch 2048 298 (256).
+// reaches: bf16, 5 x 1024, batch 1024 90 us (measured 113); 20 x 512, batch 2048 280 (300); 4 x 2048, batch 2048 298 (270).
+// Splitting costs nothing that shows: fp32-class 5 x 1024 292 us per step in 22 launches as in 2 for 128 steps.
 constexpr double LAUNCH_US = 2000.0;
 int steps_per_launch(const b2_handle* h) {
   double flops = 0;
@@ -531,9 +532,9 @@ int steps_per_launch(const b2_handle* h) {
 
 // Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken when every GEMM of the step
 // is at most two rounds of 128 x 128 tiles over the SMs, where the chain of layers is bound by latency; wider
-// layers keep the larger tiles of gemm_tc_kernel (per step, one launch per GEMM against one per step: 4 x 2048,
-// batch 2048, bf16 283 -> 256 us; 1536-768-1536-1024, batch 3000, tf32 240 -> 172 us; but 3 x 4096, batch 1024,
-// bf16 433 -> 473 us and tf32 612 -> 709 us).
+// layers keep the larger tiles of gemm_tc_kernel (per step, one launch per GEMM against one for the step: 4 x 2048,
+// batch 2048, bf16 272 -> 270 us, fp32-class 1078 -> 988 us; 1536-768-1536-1024, batch 3000, tf32 253 -> 179 us; but
+// 3 x 4096, batch 1024, bf16 407 -> 500 us and tf32 600 -> 783 us).
 int build_step_plans(b2_handle* h) {
   const int L = h->L;
   const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
@@ -575,8 +576,9 @@ int build_step_plans(b2_handle* h) {
       }
     }
     // Backward: the chain of input gradients, and the weight gradients one layer behind it, so that an SM
-    // does not hold a chain tile back behind a weight gradient that became ready at the same moment
-    // (20 x 512, batch 2048: 313 us per step against 388 side by side; 4 x 2048: 275 against 291).
+    // does not hold a chain tile back behind a weight gradient that became ready at the same moment (bf16, 20 x 512,
+    // batch 2048: 303 us per step against 373 side by side and 316 with all of them at the end; 4 x 2048: 271, 285, 273;
+    // fp32-class, 20 x 512: 786, 891, 751).
     const int lag = 1;
     std::vector<int> dz_of(L, L - 1), dg(L, -1);  // the GEMMs that produced dz[l] and that read W[l]
     for (int t = L - 1; t >= -lag; --t) {

@@ -26,8 +26,8 @@
 // What bounds it: the latency of one layer after another. In-kernel stamps of a 1024 x 1024 layer at batch
 // 1024: 1.2 us from "dependency met" to the first operands, 2.8 us for 16 k-blocks (137 GB/s into each SM),
 // 1.3 us epilogue, 1.0 us until the stores are visible to the other SMs. bf16, per step, launch per GEMM ->
-// here: 5 x 1024, batch 1024 174 -> 106 us; 20 x 512, batch 2048 628 -> 291 us; 784-500-300-40,
-// batch 1000 83 -> 48 us.
+// here: 5 x 1024, batch 1024 173 -> 113 us; 20 x 512, batch 2048 629 -> 300 us; 784-500-300-40,
+// batch 1000 78 -> 50 us.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>

@@ -11,10 +11,10 @@ struct TileChoice {
 
 // Cost of a shape = waves of the persistent grid over `sms` SMs times a tile's area per SM divided by the rate the shape
 // sustains relative to 128 x 256 (measured at 1024 x 4096 x 4096 and 8192 x 4096 x 4096, bf16 and tf32). Filling every SM
-// is not the goal: 1024 x 4096 x 4096 bf16 takes 32 us as 64 pair tiles, 36 us as 128 x 256, 45 us as 128 x 128 on all SMs.
-// Pair tiles against 256 x 256 per SM, us forward / weight / input gradient: 8192 x 4096 x 4096 bf16 179/185/178 against
-// 192/195/192, tf32 359/357/354 against 372/365/370; 4096 x 4096 x 1024 tf32 57/56/56 against 70/62/68; 2048 x 8192 x 8192
-// bf16 190/192/189 against 191/190/190.
+// is not the goal: 1024 x 4096 x 4096 bf16 takes 31 us as 64 pair tiles, 35 us as 128 x 256, 41 us as 128 x 128 on all SMs.
+// Pair tiles against 256 x 256 per SM, us forward / weight / input gradient: 8192 x 4096 x 4096 bf16 179/195/178 against
+// 193/191/193, tf32 359/375/359 against 372/362/371; 1024 x 4096 x 4096 tf32 53/55/53 against 63/60/60 (128 x 256);
+// 2048 x 8192 x 8192 bf16 191/182/190 against 190/189/190.
 //
 // `shared`: kernels of another library may sit on some of the SMs while this one runs (a step whose gradients are
 // exchanged). A pair needs both SMs of a TPC, so each such SM can cost one, and a GEMM of one wave then takes two.
