@@ -603,6 +603,7 @@ int build_step_plans(b2_handle* h) {
     for (int l = 0; l < L; ++l) {
       spec.gemms[l].prev_step[0] = wg[l];
       if (l + 1 < L) spec.gemms[l].prev_step[1] = wg[l + 1];
+      if (dg[l] >= 0) spec.gemms[dg[l]].prev_step[0] = wg[l];  // its weights are fetched before its gradient exists
     }
     const bool baseline = h->cfg.mode == B2_MODE_BASELINE;
     spec.target = slot ? h->target_alt : h->target;

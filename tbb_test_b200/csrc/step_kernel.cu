@@ -41,7 +41,8 @@ namespace {
 
 enum StepEpi : int { SE_NONE = 0, SE_RELU = 1, SE_MASK = 2, SE_LOSS = 3, SE_SGD = 4, SE_NARROW = 5 };
 enum OpForm : int { OP_K2D = 0, OP_K3D = 1, OP_MN3D = 2, OP_MN2D = 3 };
-constexpr int EPI_BYTES = 4 * 2 * 4096;  // two chunk buffers of 32 rows x 128 bytes per epilogue warp
+constexpr int STEP_THREADS = 64 + 2 * 128;   // producer warp, MMA warp, two groups of four epilogue warps
+constexpr int EPI_BYTES = 8 * 4096;          // a chunk buffer of 32 rows x 128 bytes per epilogue warp
 
 // One operand of a GEMM: how its slabs are fetched and described to the tensor core.
 struct Operand {
@@ -75,6 +76,8 @@ struct StepOp {
   int upd_cnt, upd_target;          // weight gradient: input gradient of the same layer (reads the old weights)
   int sig_row, sig_all, own_target; // counters this op raises (-1: nobody waits for them)
 };
+
+constexpr int EARLY_POLLS = 1 << 16;  // polls (about 0.5 us each) of the loop that loads weights ahead of a dependency
 
 struct StepHead {
   const StepMaps* maps;
@@ -201,107 +204,117 @@ __device__ __forceinline__ void sgd_store(const StepOp& o, size_t at, float4 v) 
   if (o.w_lo)
     *reinterpret_cast<float4*>(o.w_lo + at) = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
 }
+// 16-byte piece `piece` of row `row` of a chunk (128-byte swizzle).
+__device__ __forceinline__ const uint8_t* chunk_piece(const uint8_t* chunk, int row, int piece) {
+  return chunk + row * 128 + ((piece ^ (row & 7)) << 4);
+}
+// at += step, opaque to the compiler, which would otherwise hold the addresses of all eight rows at once
+__device__ __forceinline__ void step_row(size_t& at, size_t step) {
+  at += step;
+  asm volatile("" : "+l"(at));
+}
+
 // The fp32 values (weights or targets) that belong to a chunk of 32 rows x 32 columns, in the order in which
 // the element-wise part of the epilogue takes the chunk's pieces: lanes 8i .. 8i+7 cover one row.
 __device__ __forceinline__ void load_chunk(float4 (&v)[8], const float* base, size_t ld, int row0, int M, int gcol, int N,
                                            int lane) {
+  const int rows = gcol < N ? M - row0 - (lane >> 3) : 0;
+  size_t at = (size_t)(row0 + (lane >> 3)) * ld + gcol;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int r = row0 + 4 * i + (lane >> 3);
-    v[i] = (r < M && gcol < N) ? __ldcg(reinterpret_cast<const float4*>(base + (size_t)r * ld + gcol))
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i] = 4 * i < rows ? __ldcg(reinterpret_cast<const float4*>(base + at)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    step_row(at, 4 * ld);
   }
 }
 
-// Eight consecutive elements of a bf16 row, four of an fp32 row, as floats, the 16 bytes masked by `m` (the padding
-// behind the last column may hold NaNs). Written by other SMs during this launch: read past the L1.
+// Eight consecutive elements of a bf16 row, four of an fp32 row, the 16 bytes masked by `m` (the padding behind the
+// last column may hold NaNs). Written by other SMs during this launch: read past the L1.
 template <bool BF16>
-__device__ __forceinline__ void load_row_piece(float (&v)[BF16 ? 8 : 4], const void* row, int k, const uint32_t (&m)[4]) {
-  if (BF16) {
-    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(row) + k));
-    const uint32_t w[4] = {u.x & m[0], u.y & m[1], u.z & m[2], u.w & m[3]};
-#pragma unroll
-    for (int i = 0; i < (BF16 ? 4 : 2); ++i) {
-      v[2 * i] = __uint_as_float(w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-  } else {  // rows of whole pieces
-    const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k));
-    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-  }
+__device__ __forceinline__ uint4 load_row_piece(const void* row, int k, const uint32_t (&m)[4]) {
+  if (!BF16) return __ldcg(reinterpret_cast<const uint4*>(static_cast<const float*>(row) + k));  // rows of whole pieces
+  const uint4 u = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(row) + k));
+  return make_uint4(u.x & m[0], u.y & m[1], u.z & m[2], u.w & m[3]);
+}
+template <bool BF16>
+__device__ __forceinline__ float row_elem(const uint4& u, int i) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  if (!BF16) return __uint_as_float(w[i & 3]);
+  return __uint_as_float(i & 1 ? w[i >> 1] & 0xFFFF0000u : w[i >> 1] << 16);
 }
 
-// Last layer with fewer than 16 outputs, too narrow for a tensor-core tile: eight rows per epilogue warp on the
-// CUDA cores, lanes split K. Weight rows are loaded four at a time: one at
-// a time the L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
+// Last layer with fewer than 16 outputs, too narrow for a tensor-core tile: two rows per epilogue warp on the
+// CUDA cores, lanes split K. The weight rows come eight at a time, all loads before the first use: one at a time the
+// L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
+constexpr int NARROW_R = 2, NARROW_ROWS = 4 * NARROW_R;  // rows of a warp and of an item
+constexpr int NARROW_ITEMS = BLOCK_M / NARROW_ROWS;         // items of a row block
 template <bool BF16, int NMAX>
-__device__ __noinline__ float narrow_rows(const StepHead& p, int row0, int M, int N, int ld, int lane) {
-  constexpr int V = BF16 ? 8 : 4, R = NMAX <= 4 ? 8 : 4;  // rows at a time, as registers allow
+__device__ __forceinline__ float narrow_rows(const StepHead& p, int row0, int M, int N, int ld, int lane) {
+  constexpr int V = BF16 ? 8 : 4, R = NARROW_R, NB = NMAX < 8 ? NMAX : 8;
   const size_t row_bytes = (size_t)p.nar_lda * (BF16 ? 2 : 4);
   float loss = 0.f;
-  for (int g = 0; g < 8 && row0 + g < M; g += R) {
-    float acc[R][NMAX];
+  if (row0 >= M) return loss;
+  float acc[R][NMAX];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int n = 0; n < NMAX; ++n) acc[r][n] = 0.f;
+  for (int k = lane * V; k < p.nar_k; k += 32 * V) {
+    uint32_t m[4];  // bf16: which halves of the piece lie in front of column K
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int left = p.nar_k - k - 2 * i;
+      m[i] = left > 1 ? 0xFFFFFFFFu : left == 1 ? 0xFFFFu : 0u;
+    }
+    uint4 a[R];
 #pragma unroll
     for (int r = 0; r < R; ++r)
+      a[r] = load_row_piece<BF16>(static_cast<const char*>(p.nar_a) + (size_t)min(row0 + r, M - 1) * row_bytes, k, m);
 #pragma unroll
-      for (int n = 0; n < NMAX; ++n) acc[r][n] = 0.f;
-    for (int k = lane * V; k < p.nar_k; k += 32 * V) {
-      uint32_t m[4];  // bf16: which halves of the piece lie in front of column K
+    for (int n0 = 0; n0 < NMAX; n0 += NB) {
+      if (n0 >= N) break;
+      uint4 b[NB];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int left = p.nar_k - k - 2 * i;
-        m[i] = left > 1 ? 0xFFFFFFFFu : left == 1 ? 0xFFFFu : 0u;
-      }
-      float a[R][V];
+      for (int n = 0; n < NB; ++n)
+        b[n] = load_row_piece<BF16>(static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k, m);
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        load_row_piece<BF16>(a[r], static_cast<const char*>(p.nar_a) + (size_t)min(row0 + g + r, M - 1) * row_bytes, k, m);
+      for (int n = 0; n < NB; ++n)
 #pragma unroll
-      for (int n0 = 0; n0 < NMAX; n0 += 4) {
-        if (n0 >= N) break;
-        float b[4][V];
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
-          load_row_piece<BF16>(b[n], static_cast<const char*>(p.nar_w) + (size_t)min(n0 + n, N - 1) * row_bytes, k, m);
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int i = 0; i < V; ++i) acc[r][n0 + n] = fmaf(a[r][i], b[n][i], acc[r][n0 + n]);
-      }
+          for (int i = 0; i < V; ++i)
+            acc[r][n0 + n] = fmaf(row_elem<BF16>(a[r], i), row_elem<BF16>(b[n], i), acc[r][n0 + n]);
     }
+  }
 #pragma unroll
-    for (int n = 0; n < NMAX; ++n) {
-      if (n >= N) break;
+  for (int n = 0; n < NMAX; ++n) {
+    if (n >= N) break;
 #pragma unroll
-      for (int s = 16; s > 0; s >>= 1)
+    for (int s = 16; s > 0; s >>= 1)
 #pragma unroll
-        for (int r = 0; r < R; ++r) acc[r][n] += __shfl_xor_sync(0xFFFFFFFFu, acc[r][n], s);
-      float y = acc[0][n];  // lane r finishes row r
+      for (int r = 0; r < R; ++r) acc[r][n] += __shfl_xor_sync(0xFFFFFFFFu, acc[r][n], s);
+    float y = acc[0][n];  // lane r finishes row r
 #pragma unroll
-      for (int r = 1; r < R; ++r) y = lane == r ? acc[r][n] : y;
-      const int row = row0 + g + lane;
-      if (lane < R && row < M) {
-        const size_t at = (size_t)row * ld + n;
-        p.nar_y[at] = y;
-        const float d = p.baseline ? y - __ldg(p.target + at) : y;
-        const float gr = p.baseline ? d * p.inv_batch : y;
-        if (BF16) {
-          static_cast<__nv_bfloat16*>(p.dz)[at] = __float2bfloat16_rn(gr);
-        } else {
-          static_cast<float*>(p.dz)[at] = gr;
-          if (p.dz_lo) p.dz_lo[at] = lo_part(gr);
-        }
-        loss += 0.5f * d * d;
+    for (int r = 1; r < R; ++r) y = lane == r ? acc[r][n] : y;
+    const int row = row0 + lane;
+    if (lane < R && row < M) {
+      const size_t at = (size_t)row * ld + n;
+      p.nar_y[at] = y;
+      const float d = p.baseline ? y - __ldg(p.target + at) : y;
+      const float gr = p.baseline ? d * p.inv_batch : y;
+      if (BF16) {
+        static_cast<__nv_bfloat16*>(p.dz)[at] = __float2bfloat16_rn(gr);
+      } else {
+        static_cast<float*>(p.dz)[at] = gr;
+        if (p.dz_lo) p.dz_lo[at] = lo_part(gr);
       }
+      loss += 0.5f * d * d;
     }
   }
   return loss;
 }
 
-template <int KIND, int OPS>
-__global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_constant__ StepArgs<OPS> p) {
+template <int KIND, int OPS, bool NARROW>
+__global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_constant__ StepArgs<OPS> p) {
   constexpr bool TF32 = KIND != KIND_BF16, X3 = KIND == KIND_X3;
   constexpr int SLABS = X3 ? 1 : 2;
   constexpr int SLAB_K = TF32 ? 32 : 64, COL_LOG2 = TF32 ? 5 : 6;
@@ -353,7 +366,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
       const uint32_t slot = p.slot_bytes;
       while (ok && wk.settle(p)) {
         const StepOp& o = p.op[wk.op];
-        if (o.epi == SE_NARROW) { wk.advance(); continue; }
+        if (NARROW && o.epi == SE_NARROW) { wk.advance(); continue; }
         const StepMaps* mp = p.maps + wk.op;
         asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->b) : "memory");
@@ -366,11 +379,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
         const Operand oa = o.a, ob = o.b;
         const uint32_t a_bytes = oa.bytes, b_bytes = ob.bytes;
         const unsigned int it = (unsigned int)wk.it;
-        // operands of this step
-        if (o.row_cnt >= 0)
-          ok = wait_counter(p.counters + o.row_cnt + mb, (it + 1) * (unsigned int)o.row_target, abort_flag, p.status, 6u);
-        if (ok && o.all_cnt >= 0)
-          ok = wait_counter(p.counters + o.all_cnt, (it + 1) * (unsigned int)o.all_target, abort_flag, p.status, 7u);
         if (it > 0) {
           // weights updated by the previous step; with them all readers of the buffers this tile overwrites are done
 #pragma unroll
@@ -378,19 +386,48 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
             if (ok && o.prev_cnt[i] >= 0)
               ok = wait_counter(p.counters + o.prev_cnt[i], it * (unsigned int)o.prev_target[i], abort_flag, p.status, 8u);
         }
+        int early = 0;  // stages whose B slabs are on their way before A exists
+        int estage = stage;
+        uint32_t ephase = phase;
+        int polls = 0;
+        if (ok && o.row_cnt >= 0) {
+          // B holds weights: while the tiles that produce A are computed, its slabs may already fill the ring
+          const unsigned int target = (it + 1) * (unsigned int)o.row_target;
+          const unsigned int* const cnt = p.counters + o.row_cnt + mb;
+          const int most = min(stages, nkb);
+          if (it > 0) fence_proxy_async_all();
+          while (early < most && ld_acquire_u32(cnt) < target) {
+            if (!mbar_test_wait(empty0 + 8u * estage, ephase ^ 1)) {
+              if (++polls > EARLY_POLLS) break;  // the bounded waits below take over
+              continue;
+            }
+            const uint32_t full = full0 + 8u * estage;
+            const uint32_t sb = ring0 + (uint32_t)estage * slot + a_bytes * (X3 ? 2u : 1u);
+            mbar_expect_tx(full, tx);
+            load_operand<SLABS>(ob, &mp->b, full, sb, early, SLAB_K, n0, COL_LOG2);
+            if (X3) load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, early, SLAB_K, n0, COL_LOG2);
+            ++early;
+            if (++estage == stages) { estage = 0; ephase ^= 1; }
+          }
+          ok = wait_counter(cnt, target, abort_flag, p.status, 6u);
+        }
+        if (ok && o.all_cnt >= 0)
+          ok = wait_counter(p.counters + o.all_cnt, (it + 1) * (unsigned int)o.all_target, abort_flag, p.status, 7u);
         if (!ok) break;
         fence_proxy_async_all();  // the acquired data is read through the async proxy next
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
           const uint32_t full = full0 + 8u * stage;
           const uint32_t sa = ring0 + (uint32_t)stage * slot;
           const uint32_t sb = sa + a_bytes * (X3 ? 2u : 1u);
-          mbar_expect_tx(full, tx);
+          if (kb >= early) {
+            if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
+            mbar_expect_tx(full, tx);
+          }
           load_operand<SLABS>(oa, &mp->a, full, sa, kb, SLAB_K, m0, COL_LOG2);
-          load_operand<SLABS>(ob, &mp->b, full, sb, kb, SLAB_K, n0, COL_LOG2);
-          if (X3) {  // the low-order twins
-            load_operand<SLABS>(oa, &mp->a_lo, full, sa + a_bytes, kb, SLAB_K, m0, COL_LOG2);
-            load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, kb, SLAB_K, n0, COL_LOG2);
+          if (X3) load_operand<SLABS>(oa, &mp->a_lo, full, sa + a_bytes, kb, SLAB_K, m0, COL_LOG2);
+          if (kb >= early) {
+            load_operand<SLABS>(ob, &mp->b, full, sb, kb, SLAB_K, n0, COL_LOG2);
+            if (X3) load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, kb, SLAB_K, n0, COL_LOG2);
           }
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -414,7 +451,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
       const int stages = p.stages;
       while (ok && wk.settle(p)) {
         const StepOp& o = p.op[wk.op];
-        if (o.epi == SE_NARROW) { wk.advance(); continue; }
+        if (NARROW && o.epi == SE_NARROW) { wk.advance(); continue; }
         const int nkb = o.num_kb;
         const uint32_t idesc = o.idesc;
         const uint32_t a16 = o.a.bytes >> 4, b16 = o.b.bytes >> 4;
@@ -443,10 +480,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    int acc = 0;
+    const int group = (warp - 2) >> 2;  // takes every other tile: those in TMEM accumulator `group`
+    const int acc = group;
+    int turn = 0, narrow_turn = 0;
     uint32_t acc_phase = 0;
-    uint8_t* ebuf = smem + (size_t)p.stages * p.slot_bytes + (size_t)(warp - 2) * (2 * 4096);
-    int ebuf_i = 0;
+    uint8_t* const cbuf = smem + (size_t)p.stages * p.slot_bytes + (size_t)(warp - 2) * 4096;
     const uint32_t swz = (uint32_t)(lane & 7);
     // the loss reported is the last step's
     auto add_loss = [&](float loss) {
@@ -470,16 +508,21 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
       const StepOp& o = p.op[wk.op];
       const int idx = wk.w - o.first_item;
       const int num_n = o.num_n, M = o.M, N = o.N, epi = o.epi;
-      if (epi == SE_NARROW) {  // an item is 32 rows here, four to a row block
-        bool ok = o.row_cnt < 0 || wait_counter(p.counters + o.row_cnt + (idx >> 2), (wk.it + 1u) * o.row_target,
+      int& t = NARROW && epi == SE_NARROW ? narrow_turn : turn;
+      const bool mine = t == group;
+      t ^= 1;
+      if (!mine) { wk.advance(); continue; }
+      if (NARROW && epi == SE_NARROW) {  // an item is NARROW_ROWS rows here
+        const int block = idx / NARROW_ITEMS;
+        bool ok = o.row_cnt < 0 || wait_counter(p.counters + o.row_cnt + block, (wk.it + 1u) * o.row_target,
                                                 abort_flag, p.status, 6u);
         if (ok && wk.it > 0 && o.prev_cnt[0] >= 0)
           ok = wait_counter(p.counters + o.prev_cnt[0], (unsigned int)wk.it * o.prev_target[0], abort_flag, p.status, 8u);
         if (!__all_sync(0xFFFFFFFFu, ok)) break;
-        const int r8 = idx * 32 + (warp - 2) * 8;
-        const float part = N <= 4 ? narrow_rows<!TF32, 4>(p, r8, M, N, o.ld, lane) : narrow_rows<!TF32, 16>(p, r8, M, N, o.ld, lane);
+        const int r0 = idx * NARROW_ROWS + ((warp - 2) & 3) * NARROW_R;
+        const float part = N <= 4 ? narrow_rows<!TF32, 4>(p, r0, M, N, o.ld, lane) : narrow_rows<!TF32, 16>(p, r0, M, N, o.ld, lane);
         if (wk.it + 1 == p.steps) add_loss(part);
-        publish(o.sig_row >= 0 ? o.sig_row + (idx >> 2) : -1, o.sig_all);
+        publish(o.sig_row >= 0 ? o.sig_row + block : -1, o.sig_all);
         wk.advance();
         continue;
       }
@@ -513,16 +556,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
         const int col0 = n0 + ch * chunk_cols;
         if (col0 >= N) break;  // uniform across the warp; the first chunk of a tile always lies inside
         const bool last = (ch == nchunks - 1) || (col0 + chunk_cols >= N);
-        uint32_t words[32];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (half == 1 && !out_bf16) break;
+        uint8_t* const dst = cbuf + (size_t)lane * 128;
+        uint32_t r[32];
+        // 32 columns at a time, and no more of them in registers than those: a value spilled to local memory costs
+        // a round trip to the L2 here, because every acquiring load of a counter drops the L1
+#pragma unroll 1
+        for (int half = 0; half < (out_bf16 ? 2 : 1); ++half) {
           const int c0 = col0 + half * 32;
-          uint32_t r[32];
-          tmem_ld32(taddr + (uint32_t)(ch * chunk_cols + half * 32), r);
+          const uint32_t tcol = taddr + (uint32_t)(ch * chunk_cols + half * 32);
+          tmem_ld32(tcol, r);
           if (X3) {
             uint32_t r2[32];
-            tmem_ld32(taddr + X3_CORR_COLS + (uint32_t)(ch * chunk_cols + half * 32), r2);
+            tmem_ld32(tcol + X3_CORR_COLS, r2);
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           }
@@ -540,39 +585,39 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = (mask >> j) & 1u ? r[j] : 0u;
           }
+          if (half == 0) {
+            if (lane == 0) bulk_wait_read<0>();  // the store before has read the buffer
+            __syncwarp();
+          }
           uint32_t part[4] = {0, 0, 0, 0};
           if (out_bf16) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              words[half * 16 + j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            for (int j = 0; j < 16; ++j) r[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
             if (mask_out) {  // bit = the stored half is non-zero (it is not negative)
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                const uint32_t m = ((words[half * 16 + j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u;
+                const uint32_t m = ((r[j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u;
                 part[j & 3] |= (((m >> 15) | (m >> 30)) & 3u) << (2 * j);
               }
             }
-          } else {
+            const uint32_t piece0 = (uint32_t)half << 2;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) words[j] = r[j];
+            for (int j = 0; j < 4; ++j)  // 128-byte swizzle: piece j of row `lane` at slot j ^ (lane & 7)
+              *reinterpret_cast<uint4*>(dst + (((piece0 + j) ^ swz) << 4)) =
+                  make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          } else {
             if (mask_out) {
 #pragma unroll
               for (int j = 0; j < 32; ++j)
                 if (__uint_as_float(r[j]) > 0.f) part[j & 3] |= 1u << j;
             }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) =
+                  make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           }
           if (mask_out && row < M && c0 < N)
             mask_out[(long long)row * ld_mask + (c0 >> 5)] = (part[0] | part[1]) | (part[2] | part[3]);
-        }
-        if (lane == 0) bulk_wait_read<1>();  // the store issued two chunks ago has read its buffer
-        __syncwarp();
-        uint8_t* cbuf = ebuf + (size_t)ebuf_i * 4096;
-        {
-          uint8_t* dst = cbuf + (size_t)lane * 128;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)  // 128-byte swizzle: piece j of row `lane` at slot j ^ (lane & 7)
-            *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) =
-                make_uint4(words[4 * j], words[4 * j + 1], words[4 * j + 2], words[4 * j + 3]);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -580,76 +625,68 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) step_kernel(const __grid_const
           tma_store_2d(&mp->c, cbuf, col0, row0);
           bulk_commit();
         }
-        ebuf_i ^= 1;
         if (epi >= SE_LOSS) {
           // element-wise work on the finished chunk, read back so that a warp instruction covers four whole
           // 128-byte rows: lanes 8i .. 8i+7 take the 16-byte pieces of one row
           const int gcol = col0 + piece * (out_bf16 ? 8 : 4);
           if (!out_bf16) {
-            float4 cur[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) cur[i] = pre[i];
-            if (fetch && !last) load_chunk(pre, extra, ld, row0, M, gcol + 32, N, lane);
             // behind the last column, in the row padding, an accumulator is 0 * operand: NaN after an Inf or a NaN
             const uint32_t m1 = gcol + 1 < N ? ~0u : 0u, m2 = gcol + 2 < N ? ~0u : 0u, m3 = gcol + 3 < N ? ~0u : 0u;
+            const int rows = gcol < N ? M - row0 - (lane >> 3) : 0;  // row 4 * i of this lane's is inside if 4 * i < rows
+            size_t at = (size_t)(row0 + (lane >> 3)) * ld + gcol;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const int rr = 4 * i + (lane >> 3);
-              const uint4 v = *reinterpret_cast<const uint4*>(cbuf + rr * 128 + ((piece ^ (rr & 7)) << 4));
-              if (row0 + rr < M && gcol < N) {
-                const size_t at = (size_t)(row0 + rr) * ld + gcol;
+              const uint4 v = *reinterpret_cast<const uint4*>(chunk_piece(cbuf, 4 * i + (lane >> 3), piece));
+              if (4 * i < rows) {
                 if (epi == SE_LOSS)
-                  loss += loss_piece<!TF32>(p, at, make_uint4(v.x, v.y & m1, v.z & m2, v.w & m3), cur[i]);
+                  loss += loss_piece<!TF32>(p, at, make_uint4(v.x, v.y & m1, v.z & m2, v.w & m3), pre[i]);
                 else
                   sgd_store(o, at,
-                            sgd4(cur[i], __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),
+                            sgd4(pre[i], __uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z),
                                  __uint_as_float(v.w), p.neg_lr));
               }
+              step_row(at, 4 * ld);
             }
+            if (fetch && !last) load_chunk(pre, extra, ld, row0, M, gcol + 32, N, lane);
           } else {  // bf16 gradients: the update uses the stored (rounded) values
-            float4 w0[8], w1[8];
-            load_chunk(w0, o.w, ld, row0, M, gcol, N, lane);
-            load_chunk(w1, o.w + 4, ld, row0, M, gcol, N, lane);
+            const int rows = gcol < N ? M - row0 - (lane >> 3) : 0;
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+              load_chunk(pre, o.w + 4 * e, ld, row0, M, gcol, N, lane);
+              size_t at = (size_t)(row0 + (lane >> 3)) * ld + gcol + 4 * e;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int rr = 4 * i + (lane >> 3);
-              const uint4 v = *reinterpret_cast<const uint4*>(cbuf + rr * 128 + ((piece ^ (rr & 7)) << 4));
-              if (row0 + rr < M && gcol < N) {
-                const size_t at = (size_t)(row0 + rr) * ld + gcol;
-                sgd_store(o, at,
-                          sgd4(w0[i], __uint_as_float(v.x << 16), __uint_as_float(v.x & 0xFFFF0000u),
-                               __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xFFFF0000u), p.neg_lr));
-                sgd_store(o, at + 4,
-                          sgd4(w1[i], __uint_as_float(v.z << 16), __uint_as_float(v.z & 0xFFFF0000u),
-                               __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xFFFF0000u), p.neg_lr));
+              for (int i = 0; i < 8; ++i) {
+                const uint2 v = *reinterpret_cast<const uint2*>(chunk_piece(cbuf, 4 * i + (lane >> 3), piece) + 8 * e);
+                if (4 * i < rows)
+                  sgd_store(o, at,
+                            sgd4(pre[i], __uint_as_float(v.x << 16), __uint_as_float(v.x & 0xFFFF0000u),
+                                 __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xFFFF0000u), p.neg_lr));
+                step_row(at, 4 * ld);
               }
             }
           }
+          __syncwarp();  // the next chunk overwrites what other lanes read
         }
         if (X3 && o.c_lo) {  // the low-order twin of the chunk
-          if (lane == 0) bulk_wait_read<1>();
+          if (lane == 0) bulk_wait_read<0>();
           __syncwarp();
-          uint8_t* lbuf = ebuf + (size_t)ebuf_i * 4096;
-          uint8_t* dst = lbuf + (size_t)lane * 128;
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            uint32_t lo[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) lo[t] = __float_as_uint(lo_part(__uint_as_float(words[4 * j + t])));
-            *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            float4* const at = reinterpret_cast<float4*>(dst + ((j ^ swz) << 4));
+            const float4 v = *at;
+            *at = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
           }
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && row0 < M) {
-            tma_store_2d(&mp->c_lo, lbuf, col0, row0);
+            tma_store_2d(&mp->c_lo, cbuf, col0, row0);
             bulk_commit();
           }
-          ebuf_i ^= 1;
         }
       }
       if (epi == SE_LOSS && it + 1 == (unsigned int)p.steps) add_loss(loss);
       publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all);
-      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      acc_phase ^= 1;
       wk.advance();
     }
     if (lane == 0) bulk_wait_all();
@@ -814,8 +851,8 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     o.ld = (int)d.ldc;
     if (o.epi == SE_SGD) { o.w = g.w; o.w16 = g.w16; o.w_lo = g.w_lo; }
     o.first_item = items;
-    ntiles[i] = num_m * (narrow ? 4 : o.num_n);
-    row_add[i] = 4 * (narrow ? 4 : o.num_n);  // every epilogue warp of a tile counts one
+    ntiles[i] = narrow ? num_m * NARROW_ITEMS : num_m * o.num_n;
+    row_add[i] = 4 * (narrow ? NARROW_ITEMS : o.num_n);  // every epilogue warp of a tile counts one
     items += ntiles[i];
     row_base[i] = ncnt;
     all_base[i] = ncnt + num_m;
@@ -881,8 +918,11 @@ void step_plan_destroy(StepPlan* p) {
 template <int OPS>
 static cudaError_t launch_ops(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
                               cudaStream_t stream) {
-  void (*kernel)(const StepArgs<OPS>) = plan->kind == KIND_BF16 ? step_kernel<KIND_BF16, OPS>
-                                        : plan->kind == KIND_TF32 ? step_kernel<KIND_TF32, OPS> : step_kernel<KIND_X3, OPS>;
+  using Kernel = void (*)(const StepArgs<OPS>);
+  static const Kernel kernels[3][2] = {{step_kernel<KIND_BF16, OPS, false>, step_kernel<KIND_BF16, OPS, true>},
+                                       {step_kernel<KIND_TF32, OPS, false>, step_kernel<KIND_TF32, OPS, true>},
+                                       {step_kernel<KIND_X3, OPS, false>, step_kernel<KIND_X3, OPS, true>}};
+  const Kernel kernel = kernels[plan->kind][plan->args.nar_a ? 1 : 0];
   // per launch: handles of several devices and threads share the library, and the call is cheap
   cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
@@ -896,7 +936,7 @@ static cudaError_t launch_ops(const StepPlan* plan, int steps, float lr, unsigne
   a.neg_lr = -lr;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(plan->grid);
-  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.blockDim = dim3(STEP_THREADS);
   cfg.dynamicSmemBytes = plan->smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
