@@ -89,6 +89,7 @@ struct StepGemm {
   int rows_of;       // a tile needs the same row block of that GEMM's result
   int all_of;        // a tile needs that GEMM's whole result
   int update_after;  // STEP_WGRAD: w may change once that GEMM (which reads it) is done
+  int mask_of;       // the GEMM that writes mask_in
   int prev_step[2];  // weight gradients of the previous step that must be done, update included
   uint32_t* mask_out;
   const uint32_t* mask_in;

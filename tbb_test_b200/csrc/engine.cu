@@ -561,7 +561,7 @@ int build_step_plans(b2_handle* h) {
       StepGemm g{};
       g.d = s.d;
       g.role = role;
-      g.rows_of = g.all_of = g.update_after = g.prev_step[0] = g.prev_step[1] = -1;
+      g.rows_of = g.all_of = g.update_after = g.mask_of = g.prev_step[0] = g.prev_step[1] = -1;
       // narrow tiles as long as the GEMM fits one round of the grid: shorter tiles, more SMs at work
       g.block_n = tiles(s.d, 64) <= h->sms ? 64 : 128;
       spec.gemms.push_back(g);
@@ -586,6 +586,7 @@ int build_step_plans(b2_handle* h) {
         StepGemm& g = add(h->dgrad[t], STEP_GEMM);
         g.rows_of = dz_of[t];
         g.mask_in = h->relu_bits[t];
+        g.mask_of = t - 1;
         g.ld_mask = (h->nf[t] + 31) / 32;
         dg[t] = (int)spec.gemms.size() - 1;
         if (t > 0) dz_of[t - 1] = dg[t];

@@ -53,27 +53,37 @@ struct Operand {
   uint64_t desc;          // descriptor without its address
 };
 struct StepMaps {
-  CUtensorMap a, b, c, a_lo, b_lo, c_lo;
+  CUtensorMap a, b, c, a_lo, b_lo;  // c: output and weight gradients
 };
 struct StepOp {
   Operand a, b;
   int M, N, num_n, num_kb, block_n;
   int first_item;
   uint32_t idesc, tx_bytes;
-  int epi, out_bf16, c_lo;
+  int epi, out_bf16, wide;          // wide: rows of the result start on 32-byte boundaries
   int ld;                           // row pitch of C and, element for element, of w, w16, w_lo, target, dz
   int ld_mask;
   uint32_t* mask_out;
   const uint32_t* mask_in;
-  float* w;                         // weight update
+  union {
+    float* w;                       // weight update
+    void* c;                        // hidden layer: result
+  };
   __nv_bfloat16* w16;
-  float* w_lo;
+  union {
+    float* w_lo;
+    float* c_lo;                    // low-order twin of the result
+  };
   // What has to be finished before a tile may load: indices into the counters (-1: nothing) and the counts a
   // step adds to them (every epilogue warp of a tile adds one).
   int row_cnt, row_target;          // counter of row block 0 of the operand's producer
   int all_cnt, all_target;          // all tiles of the producer (weight gradient)
   int prev_cnt[2], prev_target[2];  // weight updates of the previous step: this layer's and the next one's
-  int upd_cnt, upd_target;          // weight gradient: input gradient of the same layer (reads the old weights)
+  union {
+    int upd_cnt;                    // weight gradient: input gradient of the same layer (reads the old weights)
+    int mask_cnt;                   // input gradient: row block 0 of the GEMM that writes mask_in
+  };
+  union { int upd_target, mask_target; };
   int sig_row, sig_all, own_target; // counters this op raises (-1: nobody waits for them)
 };
 
@@ -156,6 +166,22 @@ __device__ __forceinline__ void count_up(unsigned int* c) {  // after a fence
   asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
 }
 
+// A slab of K in the fp32-class mode: A*B, A*B_lo and A_lo*B as two MMAs per k-step. B and its twin lie one behind the
+// other in the stage, so that A meets both as one operand of 2N columns (main sum | corrections): every MMA reads its
+// operands from shared memory, which bounds this loop, and A is the larger one (128 x 64 tiles: 18 -> 14 KB per k-step).
+// The terms enter each accumulator in the order of issue_ksteps.
+__device__ __forceinline__ void issue_ksteps_x3(uint32_t tmem_d, uint64_t adesc0, uint64_t bdesc0, uint32_t a_step16,
+                                                uint32_t b_step16, uint32_t idesc, int block_n, uint32_t accumulate0,
+                                                uint32_t alo16) {
+  const uint32_t idesc2 = idesc + ((uint32_t)(block_n >> 3) << 17);  // N is twice as large
+#pragma unroll
+  for (int ks = 0; ks < KSTEPS; ++ks) {
+    const uint64_t a = adesc0 + (uint64_t)(ks * a_step16), b = bdesc0 + (uint64_t)(ks * b_step16);
+    mma_issue<true, false>(tmem_d, a, b, idesc2, ks == 0 ? accumulate0 : 1u);
+    mma_issue<true, false>(tmem_d + (uint32_t)block_n, a + (uint64_t)alo16, b, idesc, 1u);
+  }
+}
+
 template <int SLABS>
 __device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap* map, uint32_t bar, uint32_t dst,
                                              int kb, int slab_k, int mn0, int col_log2) {
@@ -204,6 +230,19 @@ __device__ __forceinline__ void sgd_store(const StepOp& o, size_t at, float4 v) 
   if (o.w_lo)
     *reinterpret_cast<float4*>(o.w_lo + at) = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
 }
+// 32 bytes of a row to global memory: one store where rows start on 32-byte boundaries, else a 16-byte piece at a time
+// (`pieces` = how many of the two lie in the matrix).
+__device__ __forceinline__ void store32(void* at, const uint32_t* r, bool wide, int pieces) {
+  if (wide && pieces == 2) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+    return;
+  }
+  if (pieces > 0) *reinterpret_cast<uint4*>(at) = make_uint4(r[0], r[1], r[2], r[3]);
+  if (pieces > 1) *(reinterpret_cast<uint4*>(at) + 1) = make_uint4(r[4], r[5], r[6], r[7]);
+}
+
 // 16-byte piece `piece` of row `row` of a chunk (128-byte swizzle).
 __device__ __forceinline__ const uint8_t* chunk_piece(const uint8_t* chunk, int row, int piece) {
   return chunk + row * 128 + ((piece ^ (row & 7)) << 4);
@@ -351,7 +390,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
-  const uint32_t acc_cols = X3 ? 128u : (uint32_t)p.tmem_cols / 2;  // TMEM columns of one accumulator
+  const uint32_t acc_cols = (uint32_t)p.tmem_cols / 2;  // TMEM columns of one accumulator (fp32-class: and its corrections)
   Walk wk;
   wk.begin();
 
@@ -454,7 +493,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
         if (NARROW && o.epi == SE_NARROW) { wk.advance(); continue; }
         const int nkb = o.num_kb;
         const uint32_t idesc = o.idesc;
-        const uint32_t a16 = o.a.bytes >> 4, b16 = o.b.bytes >> 4;
+        const uint32_t a16 = o.a.bytes >> 4;
         const uint32_t a_step = o.a.kstep16, b_step = o.b.kstep16, a_slab = o.a.slab16, b_slab = o.b.slab16;
         const uint64_t a0 = o.a.desc + ring16, b0 = o.b.desc + ring16 + a16 * (X3 ? 2u : 1u);
         if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 2u)) { ok = false; break; }
@@ -465,9 +504,13 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           tc_fence_after();
           const uint32_t off = (uint32_t)stage * slot16;
 #pragma unroll
-          for (int s = 0; s < SLABS; ++s)
-            issue_ksteps<1, TF32, false, X3, KSTEPS>(tmem_d, a0 + off + s * a_slab, b0 + off + s * b_slab, a_step, b_step,
-                                                     idesc, 0u, (s == 0 && kb == 0) ? 0u : 1u, 0u, a16, b16);
+          for (int s = 0; s < SLABS; ++s) {
+            if (X3)
+              issue_ksteps_x3(tmem_d, a0 + off, b0 + off, a_step, b_step, idesc, o.block_n, kb == 0 ? 0u : 1u, a16);
+            else
+              issue_ksteps<1, TF32, false, false, KSTEPS>(tmem_d, a0 + off + s * a_slab, b0 + off + s * b_slab, a_step,
+                                                          b_step, idesc, 0u, (s == 0 && kb == 0) ? 0u : 1u, 0u, 0u, 0u);
+          }
           tc_commit(empty0 + 8u * stage);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -494,11 +537,13 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       if (lane == 0) atomicAdd(p.loss, sum * p.loss_scale);
     };
     // this warp's part of a tile is stored: complete the stores, then the counters
-    auto publish = [&](int sig_row, int sig_all) {
+    auto publish = [&](int sig_row, int sig_all, bool bulk) {
       __syncwarp();
       if (lane == 0) {
-        bulk_wait_all();
-        fence_proxy_async_all();
+        if (bulk) {
+          bulk_wait_all();
+          fence_proxy_async_all();
+        }
         __threadfence();  // one fence for both counters
         if (sig_row >= 0) count_up(p.counters + sig_row);
         if (sig_all >= 0) count_up(p.counters + sig_all);
@@ -522,24 +567,115 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
         const int r0 = idx * NARROW_ROWS + ((warp - 2) & 3) * NARROW_R;
         const float part = N <= 4 ? narrow_rows<!TF32, 4>(p, r0, M, N, o.ld, lane) : narrow_rows<!TF32, 16>(p, r0, M, N, o.ld, lane);
         if (wk.it + 1 == p.steps) add_loss(part);
-        publish(o.sig_row >= 0 ? o.sig_row + block : -1, o.sig_all);
+        publish(o.sig_row >= 0 ? o.sig_row + block : -1, o.sig_all, true);
         wk.advance();
         continue;
       }
       const int mb = idx / num_n, nb = idx - mb * num_n;
       const int row0 = mb * BLOCK_M + q * 32, row = row0 + lane, n0 = nb * o.block_n;
       const bool out_bf16 = o.out_bf16 != 0;
+      const size_t ld = (size_t)o.ld;
+      const unsigned int it = (unsigned int)wk.it;
+      if (epi < SE_LOSS) {
+        // A hidden layer's result goes straight from registers to global memory, a row per lane. Through shared
+        // memory and a TMA store the chain of layers paid 1.2 us to stage a tile and 1.8 us until it was visible.
+        uint32_t mask[4] = {0, 0, 0, 0};
+        bool ok = true;
+        if (epi == SE_MASK) {  // written by other SMs during this launch: after their counter, and past the L1
+          ok = wait_counter(p.counters + o.mask_cnt + mb, (it + 1) * (unsigned int)o.mask_target, abort_flag, p.status, 11u);
+          const uint32_t* const m = o.mask_in + (long long)row * o.ld_mask + (n0 >> 5);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (ok && row < M && 32 * j < o.block_n && n0 + 32 * j < N) mask[j] = __ldcg(m + j);
+        }
+        ok = ok && mbar_wait(&acc_full_bar[acc], acc_phase, abort_flag, p.status, 4u);
+        if (!__all_sync(0xFFFFFFFFu, ok)) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols;
+        const bool wide = o.wide != 0;
+        const int cols = min(o.block_n, N - n0);
+        uint32_t bits = 0;
+#pragma unroll 1
+        for (int c = 0; c < cols; c += 32) {
+          uint32_t r[32];
+          tmem_ld32(taddr + (uint32_t)c, r);
+          if (X3) {
+            uint32_t r2[32];
+            tmem_ld32(taddr + (uint32_t)(o.block_n + c), r2);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+          }
+          if (c + 32 >= cols) {  // last read of the accumulator: the next tile may have it
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
+          }
+          if (epi == SE_RELU) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(fmaxf(__uint_as_float(r[j]), 0.f));
+          } else if (epi == SE_MASK) {
+            const uint32_t mk = c < 64 ? (c < 32 ? mask[0] : mask[1]) : (c < 96 ? mask[2] : mask[3]);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = (mk >> j) & 1u ? r[j] : 0u;
+          }
+          uint32_t part[4] = {0, 0, 0, 0};
+          const size_t at = (size_t)row * ld + n0 + c;
+          if (out_bf16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            if (epi == SE_RELU) {  // bit = the stored half is non-zero (it is not negative)
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint32_t m = ((r[j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u;
+                part[j & 3] |= (((m >> 15) | (m >> 30)) & 3u) << (2 * j);
+              }
+            }
+            if (row < M) {
+              __nv_bfloat16* const dst = static_cast<__nv_bfloat16*>(o.c) + at;
+#pragma unroll
+              for (int j = 0; j < 2; ++j) store32(dst + 16 * j, r + 8 * j, wide, (cols - c - 16 * j + 7) >> 3);
+            }
+          } else {
+            if (epi == SE_RELU) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (__uint_as_float(r[j]) > 0.f) part[j & 3] |= 1u << j;
+            }
+            if (row < M) {
+              float* const dst = static_cast<float*>(o.c) + at;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) store32(dst + 8 * j, r + 8 * j, wide, (cols - c - 8 * j + 3) >> 2);
+              if (X3 && o.c_lo) {  // the low-order twin
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(lo_part(__uint_as_float(r[j])));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) store32(o.c_lo + at + 8 * j, r + 8 * j, wide, (cols - c - 8 * j + 3) >> 2);
+              }
+            }
+          }
+          if (epi == SE_RELU && o.mask_out) {
+            const uint32_t b = (part[0] | part[1]) | (part[2] | part[3]);
+            uint32_t* const m = o.mask_out + (long long)row * o.ld_mask + ((n0 + c) >> 5);
+            const bool odd = (c & 32) != 0;
+            if (row < M) {  // two words at a time where that is an aligned pair
+              if (o.ld_mask & 1) *m = b;
+              else if (odd) *reinterpret_cast<uint2*>(m - 1) = make_uint2(bits, b);
+              else if (c + 32 >= cols) *m = b;
+            }
+            bits = b;
+          }
+        }
+        publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all, false);
+        acc_phase ^= 1;
+        wk.advance();
+        continue;
+      }
       const int chunk_cols = out_bf16 ? 64 : 32;  // 128 bytes of C per row and chunk
       const int nchunks = o.block_n / chunk_cols;
-      const size_t ld = (size_t)o.ld;
       const StepMaps* mp = p.maps + wk.op;
       const int piece = lane & 7;  // 16-byte piece of a row this lane takes in the element-wise part
-      const unsigned int it = (unsigned int)wk.it;
       float loss = 0.f;
-      uint32_t* const mask_out = epi == SE_RELU ? o.mask_out : nullptr;
-      const uint32_t* const mask_in = o.mask_in;
-      const long long ld_mask = o.ld_mask;
-      const float* const extra = epi == SE_SGD ? o.w : epi == SE_LOSS && p.baseline ? p.target : nullptr;
+      const float* const extra = epi == SE_SGD ? o.w : p.baseline ? p.target : nullptr;
       const bool fetch = extra && !out_bf16;
       float4 pre[8];  // weights or targets of the next chunk, on their way while the MMAs run
       bool ok = true;
@@ -562,12 +698,11 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
         // a round trip to the L2 here, because every acquiring load of a counter drops the L1
 #pragma unroll 1
         for (int half = 0; half < (out_bf16 ? 2 : 1); ++half) {
-          const int c0 = col0 + half * 32;
           const uint32_t tcol = taddr + (uint32_t)(ch * chunk_cols + half * 32);
           tmem_ld32(tcol, r);
           if (X3) {
             uint32_t r2[32];
-            tmem_ld32(tcol + X3_CORR_COLS, r2);
+            tmem_ld32(tcol + (uint32_t)o.block_n, r2);
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           }
@@ -576,48 +711,24 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
           }
-          if (epi == SE_RELU) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(fmaxf(__uint_as_float(r[j]), 0.f));
-          } else if (epi == SE_MASK) {
-            // written by other SMs during this launch: read past the L1
-            const uint32_t mask = (row < M && c0 < N) ? __ldcg(mask_in + (long long)row * ld_mask + (c0 >> 5)) : 0u;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = (mask >> j) & 1u ? r[j] : 0u;
-          }
           if (half == 0) {
             if (lane == 0) bulk_wait_read<0>();  // the store before has read the buffer
             __syncwarp();
           }
-          uint32_t part[4] = {0, 0, 0, 0};
           if (out_bf16) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) r[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-            if (mask_out) {  // bit = the stored half is non-zero (it is not negative)
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const uint32_t m = ((r[j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u;
-                part[j & 3] |= (((m >> 15) | (m >> 30)) & 3u) << (2 * j);
-              }
-            }
             const uint32_t piece0 = (uint32_t)half << 2;
 #pragma unroll
             for (int j = 0; j < 4; ++j)  // 128-byte swizzle: piece j of row `lane` at slot j ^ (lane & 7)
               *reinterpret_cast<uint4*>(dst + (((piece0 + j) ^ swz) << 4)) =
                   make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           } else {
-            if (mask_out) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (__uint_as_float(r[j]) > 0.f) part[j & 3] |= 1u << j;
-            }
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               *reinterpret_cast<uint4*>(dst + ((j ^ swz) << 4)) =
                   make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           }
-          if (mask_out && row < M && c0 < N)
-            mask_out[(long long)row * ld_mask + (c0 >> 5)] = (part[0] | part[1]) | (part[2] | part[3]);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -625,7 +736,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           tma_store_2d(&mp->c, cbuf, col0, row0);
           bulk_commit();
         }
-        if (epi >= SE_LOSS) {
+        {
           // element-wise work on the finished chunk, read back so that a warp instruction covers four whole
           // 128-byte rows: lanes 8i .. 8i+7 take the 16-byte pieces of one row
           const int gcol = col0 + piece * (out_bf16 ? 8 : 4);
@@ -667,25 +778,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           }
           __syncwarp();  // the next chunk overwrites what other lanes read
         }
-        if (X3 && o.c_lo) {  // the low-order twin of the chunk
-          if (lane == 0) bulk_wait_read<0>();
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4* const at = reinterpret_cast<float4*>(dst + ((j ^ swz) << 4));
-            const float4 v = *at;
-            *at = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0 && row0 < M) {
-            tma_store_2d(&mp->c_lo, cbuf, col0, row0);
-            bulk_commit();
-          }
-        }
       }
       if (epi == SE_LOSS && it + 1 == (unsigned int)p.steps) add_loss(loss);
-      publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all);
+      publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all, true);
       acc_phase ^= 1;
       wk.advance();
     }
@@ -831,9 +926,9 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
       const cuuint64_t pitch = (cuuint64_t)d.ldc * ob;
       const cuuint32_t box[2] = {(cuuint32_t)(128 / ob), 32};
       if (!encode(&mp.c, d.C, ob, 2, dims, &pitch, box, false, true)) return refuse();
-      mp.c_lo = mp.c;
-      o.c_lo = d.C_lo != nullptr;
-      if (d.C_lo && !encode(&mp.c_lo, d.C_lo, 4, 2, dims, &pitch, box, false, true)) return refuse();
+      o.c = d.C;
+      o.c_lo = static_cast<float*>(d.C_lo);
+      o.wide = pitch % 32 == 0 && reinterpret_cast<uintptr_t>(d.C) % 32 == 0 && reinterpret_cast<uintptr_t>(d.C_lo) % 32 == 0;
       const uint32_t fmt = eb == 4 ? 2u : 1u;  // tf32 : bf16
       o.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
                 ((uint32_t)(o.block_n >> 3) << 17) | ((uint32_t)(BLOCK_M >> 4) << 24);
@@ -862,7 +957,7 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     const StepGemm& g = s.gemms[i];
     StepOp& o = ops[i];
     // a dependency always points to an earlier entry of the list, or to a weight gradient of the step before
-    if (g.rows_of >= i || g.all_of >= i || g.update_after >= i) return refuse();
+    if (g.rows_of >= i || g.all_of >= i || g.update_after >= i || g.mask_of >= i) return refuse();
     o.row_cnt = g.rows_of >= 0 ? row_base[g.rows_of] : -1;
     o.row_target = g.rows_of >= 0 ? row_add[g.rows_of] : 0;
     o.all_cnt = g.all_of >= 0 ? all_base[g.all_of] : -1;
@@ -872,6 +967,12 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     for (int k = 0; k < 2; ++k) {
       o.prev_cnt[k] = g.prev_step[k] >= 0 ? all_base[g.prev_step[k]] : -1;
       o.prev_target[k] = g.prev_step[k] >= 0 ? 4 * ntiles[g.prev_step[k]] : 0;
+    }
+    if (o.epi == SE_MASK) {
+      if (g.mask_of < 0) return refuse();
+      o.mask_cnt = row_base[g.mask_of];
+      o.mask_target = row_add[g.mask_of];
+      row_used[g.mask_of] = 1;
     }
     if (g.rows_of >= 0) row_used[g.rows_of] = 1;
     for (int j : {g.all_of, g.update_after, g.prev_step[0], g.prev_step[1], g.role == STEP_WGRAD ? i : -1})
