@@ -85,7 +85,7 @@ enum StepRole : int { STEP_GEMM = 0, STEP_LAST_FWD = 1, STEP_WGRAD = 2 };
 struct StepGemm {
   GemmDesc d;
   int role;          // STEP_LAST_FWD: the epilogue also writes dz and the loss; STEP_WGRAD: it also updates w
-  int block_n;       // tile width, 64 or 128
+  int block_n;       // tile width, 64 or 128 (128 for pairs)
   int rows_of;       // a tile needs the same row block of that GEMM's result
   int all_of;        // a tile needs that GEMM's whole result
   int update_after;  // STEP_WGRAD: w may change once that GEMM (which reads it) is done
@@ -100,6 +100,7 @@ struct StepGemm {
 };
 struct StepSpec {
   std::vector<StepGemm> gemms;
+  bool pair;  // tiles of 256 x 128 by CTA pairs
   const float* target;
   void* dz;
   float* dz_lo;

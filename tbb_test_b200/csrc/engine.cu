@@ -554,16 +554,31 @@ int build_step_plans(b2_handle* h) {
       if (!(e && e[0] == '1') && tiles(s->d, 128) > 2 * h->sms) return B2_OK;
     }
   }
+  // CTA pairs (256 x 128 tiles, two thirds of the operand traffic) once the layers are as many 128 x 128 tiles as fill the
+  // SMs, a little earlier where operands are 32 bits wide; below that a step waits for latency, and smaller tiles on more
+  // SMs are shorter. us per step, one CTA per tile -> pairs, by tiles of an average layer: 256 tiles (6 x 512, batch
+  // 8192) bf16 219 -> 171, tf32 411 -> 285; 256 (4 x 2048, batch 2048) bf16 222 -> 212, fp32-class 886 -> 804; 192 (6 x 1024,
+  // batch 3000) bf16 175 -> 156; 144 (4 x 1536, batch 1536) bf16 125 -> 129, tf32 195 -> 186; 128 (4 x 2048, batch 1024)
+  // bf16 156 -> 159, tf32 240 -> 222; 76 (3072-1024-2048-512, batch 700) tf32 119 -> 121; 64 (5 x 1024, batch 1024)
+  // bf16 90 -> 95, fp32-class 233 -> 268.
+  long long chain = 0, width = 0;
+  for (int l = 0; l < L; ++l) {
+    chain += tiles(h->fwd[l].d, 128) + tiles(h->dgrad[l].d, 128);
+    width += h->nf[l];
+  }
+  const char* pe = getenv("B2_STEP_PAIR");  // experiments: 0 never, 1 whatever the size
+  const bool pair = pe ? pe[0] == '1' : chain > 2LL * L * h->sms * (h->op_type == T_BF16 ? 3 : 2) / 3;
   for (int slot = 0; slot < 2; ++slot) {
     StepSpec spec;
+    spec.pair = pair;
     std::vector<int> wg(L, -1);
     auto add = [&](const Site& s, int role) -> StepGemm& {
       StepGemm g{};
       g.d = s.d;
       g.role = role;
       g.rows_of = g.all_of = g.update_after = g.mask_of = g.prev_step[0] = g.prev_step[1] = -1;
-      // narrow tiles as long as the GEMM fits one round of the grid: shorter tiles, more SMs at work
-      g.block_n = tiles(s.d, 64) <= h->sms ? 64 : 128;
+      // one CTA per tile: narrow tiles as long as the GEMM fits one round of the grid, shorter tiles on more SMs
+      g.block_n = !pair && tiles(s.d, 64) <= h->sms ? 64 : 128;
       spec.gemms.push_back(g);
       return spec.gemms.back();
     };
@@ -576,10 +591,11 @@ int build_step_plans(b2_handle* h) {
       }
     }
     // Backward: the chain of input gradients, and the weight gradients one layer behind it, so that an SM
-    // does not hold a chain tile back behind a weight gradient that became ready at the same moment (bf16, 20 x 512,
-    // batch 2048: 303 us per step against 373 side by side and 316 with all of them at the end; 4 x 2048: 271, 285, 273;
-    // fp32-class, 20 x 512: 786, 891, 751).
-    const int lag = 1;
+    // does not hold a chain tile back behind a weight gradient that became ready at the same moment; two layers behind
+    // where the weight gradients' sums (over the batch) are long against the chain's (over the width). us per step side by
+    // side, one behind, two behind: 5 x 1024, batch 1024, bf16 92, 90, 91, fp32-class 229, 233, 237; 20 x 512, batch 2048, bf16
+    // 267, 246, 243, fp32-class 716, 633, 595; as pairs 6 x 512, batch 8192, tf32 -, 285, 263.
+    const int lag = (long long)h->bl * L >= 4 * width ? 2 : 1;
     std::vector<int> dz_of(L, L - 1), dg(L, -1);  // the GEMMs that produced dz[l] and that read W[l]
     for (int t = L - 1; t >= -lag; --t) {
       if (t >= 0 && h->dgrad[t].active) {

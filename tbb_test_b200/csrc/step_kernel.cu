@@ -6,7 +6,7 @@
 // most SMs idle (a 1024 x 1024 layer is 64 tiles of 128 x 128). Here one persistent CTA per SM walks a
 // fixed list of output tiles of all GEMMs of the step:
 //
-//   fwd(0) .. fwd(L-1), then for l = L-1 .. 0: dgrad(l) and, one layer behind, wgrad(l+1)
+//   fwd(0) .. fwd(L-1), then for l = L-1 .. 0: dgrad(l) and, one or two layers behind, wgrad
 //
 // round-robin over the grid, and a tile starts as soon as the tiles that produce its operands are
 // done: a forward or input-gradient tile waits for the row block it reads, a weight-gradient tile for
@@ -20,14 +20,21 @@
 // bounded as in gemm_tc_kernel.
 //
 // Roles per CTA as in gemm_tc_kernel: warp 0 TMA producer (also waits for the dependencies), warp 1 MMA
-// issuer, warps 2-5 epilogue; two TMEM accumulators. A stage holds two 128-byte slabs of K (one in the
-// fp32-class mode): the issuing threads' instructions per stage bound these short k-loops.
+// issuer, warps 2-9 epilogue in two groups of four; two TMEM accumulators. A stage holds two 128-byte slabs of K
+// (one in the fp32-class mode): the issuing threads' instructions per stage bound these short k-loops. While a tile
+// waits for the tiles that produce its A, its weights already fill the ring.
 //
-// What bounds it: the latency of one layer after another. In-kernel stamps of a 1024 x 1024 layer at batch
-// 1024: 1.2 us from "dependency met" to the first operands, 2.8 us for 16 k-blocks (137 GB/s into each SM),
-// 1.3 us epilogue, 1.0 us until the stores are visible to the other SMs. bf16, per step, launch per GEMM ->
-// here: 5 x 1024, batch 1024 173 -> 113 us; 20 x 512, batch 2048 629 -> 300 us; 784-500-300-40,
-// batch 1000 78 -> 50 us.
+// Two forms: a CTA per tile (128 x 64 or 128 x 128), and CTA pairs (cta_group::2, 256 x 128, each CTA holds 128 rows of
+// A and half of B) for networks whose layers fill the GPU.
+//
+// What bounds it: with a CTA per tile the latency of one layer after another. In-kernel stamps of a 1024 x 1024 layer at
+// batch 1024: 1.1 us from "dependency met" to the first operands, 2.5 us for 16 k-blocks, 1.2 us epilogue (weight
+// update 3.6 us, loss 3.3 us), 1.2 us until the stores are visible to the other SMs, 0.8 us until the next tile's
+// producer has seen the counter; in the backward pass, where two GEMMs per layer run, the L2 (11-13 TB/s into all
+// SMs). Pairs: L2 and shared memory. Nothing may spill to local memory here: the acquiring loads of the counters drop
+// the L1, and each reload is an L2 round trip (two spilling epilogue groups: 110 -> 135 us per step, without spills 97).
+// bf16, us per step, launch per GEMM -> here: 5 x 1024, batch 1024 170 -> 90; 20 x 512, batch 2048 589 -> 243;
+// 784-500-300-10, batch 1000 87 -> 48; 6 x 512, batch 8192 -> 166 (pairs).
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -131,7 +138,7 @@ __device__ __forceinline__ float lo_part(float v) {
 // Walks this CTA's items: step `it`, op `op`, item `w` of the step's list.
 struct Walk {
   int w, it, op;
-  __device__ __forceinline__ void begin() { w = blockIdx.x; it = 0; op = 0; }
+  __device__ __forceinline__ void begin(int unit) { w = unit; it = 0; op = 0; }
   template <int OPS>
   __device__ __forceinline__ bool settle(const StepArgs<OPS>& p) {
     while (w >= p.items) { w -= p.items; ++it; op = 0; }
@@ -139,7 +146,7 @@ struct Walk {
     while (op + 1 < p.nops && w >= p.op[op + 1].first_item) ++op;
     return true;
   }
-  __device__ __forceinline__ void advance() { w += gridDim.x; }
+  __device__ __forceinline__ void advance(int units) { w += units; }
 };
 
 __device__ __forceinline__ bool wait_counter(const unsigned int* c, unsigned int target, volatile int* abort_flag,
@@ -182,21 +189,21 @@ __device__ __forceinline__ void issue_ksteps_x3(uint32_t tmem_d, uint64_t adesc0
   }
 }
 
-template <int SLABS>
+template <int SLABS, bool PAIR>
 __device__ __forceinline__ void load_operand(const Operand& o, const CUtensorMap* map, uint32_t bar, uint32_t dst,
                                              int kb, int slab_k, int mn0, int col_log2) {
   const int k0 = kb * SLABS * slab_k;
   if (o.form == OP_K3D) {
-    tma_load_3d<false>(map, bar, dst, 0, mn0, kb * SLABS);
+    tma_load_3d<PAIR>(map, bar, dst, 0, mn0, kb * SLABS);
   } else if (o.form == OP_MN3D) {
-    tma_load_3d<false>(map, bar, dst, 0, k0, mn0 >> col_log2);
+    tma_load_3d<PAIR>(map, bar, dst, 0, k0, mn0 >> col_log2);
   } else if (o.form == OP_K2D) {
 #pragma unroll
     for (int s = 0; s < SLABS; ++s)
-      tma_load_2d<false>(map, bar, dst + (uint32_t)s * (o.bytes / SLABS), k0 + s * slab_k, mn0);
+      tma_load_2d<PAIR>(map, bar, dst + (uint32_t)s * (o.bytes / SLABS), k0 + s * slab_k, mn0);
   } else {
     for (int c = 0; c < o.boxes; ++c)
-      tma_load_2d<false>(map, bar, dst + (uint32_t)c * o.col_bytes, mn0 + (c << col_log2), k0);
+      tma_load_2d<PAIR>(map, bar, dst + (uint32_t)c * o.col_bytes, mn0 + (c << col_log2), k0);
   }
 }
 
@@ -285,7 +292,7 @@ __device__ __forceinline__ float row_elem(const uint4& u, int i) {
 // CUDA cores, lanes split K. The weight rows come eight at a time, all loads before the first use: one at a time the
 // L2's latency per row added up (10 outputs of 300: 75 us). Returns this lane's share of the loss.
 constexpr int NARROW_R = 2, NARROW_ROWS = 4 * NARROW_R;  // rows of a warp and of an item
-constexpr int NARROW_ITEMS = BLOCK_M / NARROW_ROWS;         // items of a row block
+constexpr int NARROW_ITEMS = BLOCK_M / NARROW_ROWS;         // items of a row block, of one CTA or of a pair
 template <bool BF16, int NMAX>
 __device__ __forceinline__ float narrow_rows(const StepHead& p, int row0, int M, int N, int ld, int lane) {
   constexpr int V = BF16 ? 8 : 4, R = NARROW_R, NB = NMAX < 8 ? NMAX : 8;
@@ -352,10 +359,11 @@ __device__ __forceinline__ float narrow_rows(const StepHead& p, int row0, int M,
   return loss;
 }
 
-template <int KIND, int OPS, bool NARROW>
+template <int KIND, int OPS, bool PAIR>
 __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_constant__ StepArgs<OPS> p) {
   constexpr bool TF32 = KIND != KIND_BF16, X3 = KIND == KIND_X3;
   constexpr int SLABS = X3 ? 1 : 2;
+  constexpr int ROWS = PAIR ? 2 * BLOCK_M : BLOCK_M;  // rows of a tile
   constexpr int SLAB_K = TF32 ? 32 : 64, COL_LOG2 = TF32 ? 5 : 6;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
@@ -368,6 +376,8 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &abort_s;
+  const int rank = PAIR ? (int)cluster_ctarank() : 0;
+  const int unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
   if (threadIdx.x == 0) {
     abort_s = 0;
     for (int s = 0; s < p.stages; ++s) {
@@ -376,23 +386,32 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full_bar[a], 1);
-      mbar_init(&acc_empty_bar[a], 4);
+      mbar_init(&acc_empty_bar[a], PAIR ? 16 : 4);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
-                 "r"((uint32_t)p.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                   "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                   "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // no remote arrival before the barriers exist
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
-  const uint32_t acc_cols = (uint32_t)p.tmem_cols / 2;  // TMEM columns of one accumulator (fp32-class: and its corrections)
+  // TMEM columns of one accumulator (fp32-class: with its corrections behind it, of a pair behind both accumulators)
+  const uint32_t acc_cols = X3 && PAIR ? 128u : (uint32_t)p.tmem_cols / 2;
   Walk wk;
-  wk.begin();
+  wk.begin(unit);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -400,12 +419,13 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), ring0 = smem_u32(smem);
+      const uint32_t full_own = smem_u32(full_bar), empty0 = smem_u32(empty_bar), ring0 = smem_u32(smem);
+      const uint32_t full0 = PAIR ? map_to_cta(full_own, 0) : full_own;  // the leader's counts the bytes of both CTAs
       const int stages = p.stages;
       const uint32_t slot = p.slot_bytes;
       while (ok && wk.settle(p)) {
         const StepOp& o = p.op[wk.op];
-        if (NARROW && o.epi == SE_NARROW) { wk.advance(); continue; }
+        if (o.epi == SE_NARROW) { wk.advance(units); continue; }
         const StepMaps* mp = p.maps + wk.op;
         asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&mp->b) : "memory");
@@ -413,8 +433,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
         const int idx = wk.w - o.first_item;
         const int num_n = o.num_n, nkb = o.num_kb;
         const int mb = idx / num_n, nb = idx - mb * num_n;
-        const int m0 = mb * BLOCK_M, n0 = nb * o.block_n;
-        const uint32_t tx = o.tx_bytes;
+        const int m0 = mb * ROWS + rank * BLOCK_M;                        // this CTA's rows of A
+        const int n0 = nb * o.block_n + (PAIR ? rank * (o.block_n >> 1) : 0);  // and of B
+        const uint32_t tx = o.tx_bytes * (PAIR ? 2u : 1u);
         const Operand oa = o.a, ob = o.b;
         const uint32_t a_bytes = oa.bytes, b_bytes = ob.bytes;
         const unsigned int it = (unsigned int)wk.it;
@@ -442,9 +463,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
             }
             const uint32_t full = full0 + 8u * estage;
             const uint32_t sb = ring0 + (uint32_t)estage * slot + a_bytes * (X3 ? 2u : 1u);
-            mbar_expect_tx(full, tx);
-            load_operand<SLABS>(ob, &mp->b, full, sb, early, SLAB_K, n0, COL_LOG2);
-            if (X3) load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, early, SLAB_K, n0, COL_LOG2);
+            if (rank == 0) mbar_expect_tx(full_own + 8u * estage, tx);
+            load_operand<SLABS, PAIR>(ob, &mp->b, full, sb, early, SLAB_K, n0, COL_LOG2);
+            if (X3) load_operand<SLABS, PAIR>(ob, &mp->b_lo, full, sb + b_bytes, early, SLAB_K, n0, COL_LOG2);
             ++early;
             if (++estage == stages) { estage = 0; ephase ^= 1; }
           }
@@ -460,17 +481,17 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           const uint32_t sb = sa + a_bytes * (X3 ? 2u : 1u);
           if (kb >= early) {
             if (!mbar_wait(empty0 + 8u * stage, phase ^ 1, abort_flag, p.status, 1u)) { ok = false; break; }
-            mbar_expect_tx(full, tx);
+            if (rank == 0) mbar_expect_tx(full_own + 8u * stage, tx);
           }
-          load_operand<SLABS>(oa, &mp->a, full, sa, kb, SLAB_K, m0, COL_LOG2);
-          if (X3) load_operand<SLABS>(oa, &mp->a_lo, full, sa + a_bytes, kb, SLAB_K, m0, COL_LOG2);
+          load_operand<SLABS, PAIR>(oa, &mp->a, full, sa, kb, SLAB_K, m0, COL_LOG2);
+          if (X3) load_operand<SLABS, PAIR>(oa, &mp->a_lo, full, sa + a_bytes, kb, SLAB_K, m0, COL_LOG2);
           if (kb >= early) {
-            load_operand<SLABS>(ob, &mp->b, full, sb, kb, SLAB_K, n0, COL_LOG2);
-            if (X3) load_operand<SLABS>(ob, &mp->b_lo, full, sb + b_bytes, kb, SLAB_K, n0, COL_LOG2);
+            load_operand<SLABS, PAIR>(ob, &mp->b, full, sb, kb, SLAB_K, n0, COL_LOG2);
+            if (X3) load_operand<SLABS, PAIR>(ob, &mp->b_lo, full, sb + b_bytes, kb, SLAB_K, n0, COL_LOG2);
           }
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
-        wk.advance();
+        wk.advance(units);
       }
       if (!ok) {  // give copies already in flight a bounded time to land before the CTA retires
         const unsigned long long t0 = globaltimer();
@@ -478,8 +499,8 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // -------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
+    // ------------------------------------------- MMA issuer (of a pair: the leader's)
+    if (rank == 0 && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -490,10 +511,10 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       const int stages = p.stages;
       while (ok && wk.settle(p)) {
         const StepOp& o = p.op[wk.op];
-        if (NARROW && o.epi == SE_NARROW) { wk.advance(); continue; }
+        if (o.epi == SE_NARROW) { wk.advance(units); continue; }
         const int nkb = o.num_kb;
         const uint32_t idesc = o.idesc;
-        const uint32_t a16 = o.a.bytes >> 4;
+        const uint32_t a16 = o.a.bytes >> 4, b16 = o.b.bytes >> 4;
         const uint32_t a_step = o.a.kstep16, b_step = o.b.kstep16, a_slab = o.a.slab16, b_slab = o.b.slab16;
         const uint64_t a0 = o.a.desc + ring16, b0 = o.b.desc + ring16 + a16 * (X3 ? 2u : 1u);
         if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 2u)) { ok = false; break; }
@@ -505,28 +526,46 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           const uint32_t off = (uint32_t)stage * slot16;
 #pragma unroll
           for (int s = 0; s < SLABS; ++s) {
-            if (X3)
+            if (X3 && PAIR)
+              issue_ksteps<1, true, true, true, KSTEPS>(tmem_d, a0 + off, b0 + off, a_step, b_step, idesc, 0u,
+                                                        kb == 0 ? 0u : 1u, 0u, a16, b16);
+            else if (X3)
               issue_ksteps_x3(tmem_d, a0 + off, b0 + off, a_step, b_step, idesc, o.block_n, kb == 0 ? 0u : 1u, a16);
             else
-              issue_ksteps<1, TF32, false, false, KSTEPS>(tmem_d, a0 + off + s * a_slab, b0 + off + s * b_slab, a_step,
+              issue_ksteps<1, TF32, PAIR, false, KSTEPS>(tmem_d, a0 + off + s * a_slab, b0 + off + s * b_slab, a_step,
                                                           b_step, idesc, 0u, (s == 0 && kb == 0) ? 0u : 1u, 0u, 0u, 0u);
           }
-          tc_commit(empty0 + 8u * stage);
+          if (PAIR) tc_commit_pair(empty0 + 8u * stage); else tc_commit(empty0 + 8u * stage);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit(acc_full0 + 8u * acc);
+        if (PAIR) tc_commit_pair(acc_full0 + 8u * acc); else tc_commit(acc_full0 + 8u * acc);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
-        wk.advance();
+        wk.advance(units);
       }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    const int group = (warp - 2) >> 2;  // takes every other tile: those in TMEM accumulator `group`
-    const int acc = group;
-    int turn = 0, narrow_turn = 0;
+    // One CTA: a group takes every other tile, those in TMEM accumulator `group`, so that an input gradient does not wait
+    // behind the long epilogue of a weight gradient. A pair has half as many tiles, twice as large: a group takes half of
+    // the columns of each.
+    const int group = (warp - 2) >> 2;
+    int acc = PAIR ? 0 : group;
     uint32_t acc_phase = 0;
+    int turn = 0, narrow_turn = 0;
+    const auto free_acc = [&]() {  // last read of the accumulator: the next tile may have it
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(map_to_cta(smem_u32(&acc_empty_bar[acc]), 0));
+        else mbar_arrive(&acc_empty_bar[acc]);
+      }
+    };
+    const auto next_acc = [&]() {
+      if (PAIR) acc ^= 1;
+      if (!PAIR || acc == 0) acc_phase ^= 1;
+    };
     uint8_t* const cbuf = smem + (size_t)p.stages * p.slot_bytes + (size_t)(warp - 2) * 4096;
     const uint32_t swz = (uint32_t)(lane & 7);
     // the loss reported is the last step's
@@ -553,26 +592,30 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       const StepOp& o = p.op[wk.op];
       const int idx = wk.w - o.first_item;
       const int num_n = o.num_n, M = o.M, N = o.N, epi = o.epi;
-      int& t = NARROW && epi == SE_NARROW ? narrow_turn : turn;
-      const bool mine = t == group;
-      t ^= 1;
-      if (!mine) { wk.advance(); continue; }
-      if (NARROW && epi == SE_NARROW) {  // an item is NARROW_ROWS rows here
+      if (!PAIR || epi == SE_NARROW) {
+        int& t = epi == SE_NARROW ? narrow_turn : turn;
+        const bool mine = t == group;
+        t ^= 1;
+        if (!mine) { wk.advance(units); continue; }
+      }
+      if (epi == SE_NARROW) {  // an item is NARROW_ROWS rows here
         const int block = idx / NARROW_ITEMS;
         bool ok = o.row_cnt < 0 || wait_counter(p.counters + o.row_cnt + block, (wk.it + 1u) * o.row_target,
                                                 abort_flag, p.status, 6u);
         if (ok && wk.it > 0 && o.prev_cnt[0] >= 0)
           ok = wait_counter(p.counters + o.prev_cnt[0], (unsigned int)wk.it * o.prev_target[0], abort_flag, p.status, 8u);
         if (!__all_sync(0xFFFFFFFFu, ok)) break;
-        const int r0 = idx * NARROW_ROWS + ((warp - 2) & 3) * NARROW_R;
+        const int r0 = block * ROWS + rank * BLOCK_M + (idx - block * NARROW_ITEMS) * NARROW_ROWS + ((warp - 2) & 3) * NARROW_R;
         const float part = N <= 4 ? narrow_rows<!TF32, 4>(p, r0, M, N, o.ld, lane) : narrow_rows<!TF32, 16>(p, r0, M, N, o.ld, lane);
         if (wk.it + 1 == p.steps) add_loss(part);
         publish(o.sig_row >= 0 ? o.sig_row + block : -1, o.sig_all, true);
-        wk.advance();
+        wk.advance(units);
         continue;
       }
       const int mb = idx / num_n, nb = idx - mb * num_n;
-      const int row0 = mb * BLOCK_M + q * 32, row = row0 + lane, n0 = nb * o.block_n;
+      const int row0 = mb * ROWS + rank * BLOCK_M + q * 32, row = row0 + lane;
+      const int width = PAIR ? o.block_n >> 1 : o.block_n, part0 = PAIR ? group * width : 0;  // this group's columns
+      const int n0 = nb * o.block_n + part0;
       const bool out_bf16 = o.out_bf16 != 0;
       const size_t ld = (size_t)o.ld;
       const unsigned int it = (unsigned int)wk.it;
@@ -586,14 +629,15 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           const uint32_t* const m = o.mask_in + (long long)row * o.ld_mask + (n0 >> 5);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (ok && row < M && 32 * j < o.block_n && n0 + 32 * j < N) mask[j] = __ldcg(m + j);
+            if (ok && row < M && 32 * j < width && n0 + 32 * j < N) mask[j] = __ldcg(m + j);
         }
         ok = ok && mbar_wait(&acc_full_bar[acc], acc_phase, abort_flag, p.status, 4u);
         if (!__all_sync(0xFFFFFFFFu, ok)) break;
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols;
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols + (uint32_t)part0;
         const bool wide = o.wide != 0;
-        const int cols = min(o.block_n, N - n0);
+        const int cols = min(width, N - n0);
+        if (PAIR && cols <= 0) free_acc();
         uint32_t bits = 0;
 #pragma unroll 1
         for (int c = 0; c < cols; c += 32) {
@@ -601,15 +645,11 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           tmem_ld32(taddr + (uint32_t)c, r);
           if (X3) {
             uint32_t r2[32];
-            tmem_ld32(taddr + (uint32_t)(o.block_n + c), r2);
+            tmem_ld32(taddr + (PAIR ? X3_CORR_COLS : (uint32_t)o.block_n) + (uint32_t)c, r2);
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           }
-          if (c + 32 >= cols) {  // last read of the accumulator: the next tile may have it
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
-          }
+          if (c + 32 >= cols) free_acc();
           if (epi == SE_RELU) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(fmaxf(__uint_as_float(r[j]), 0.f));
@@ -666,12 +706,12 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           }
         }
         publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all, false);
-        acc_phase ^= 1;
-        wk.advance();
+        next_acc();
+        wk.advance(units);
         continue;
       }
       const int chunk_cols = out_bf16 ? 64 : 32;  // 128 bytes of C per row and chunk
-      const int nchunks = o.block_n / chunk_cols;
+      const int nchunks = width / chunk_cols;
       const StepMaps* mp = p.maps + wk.op;
       const int piece = lane & 7;  // 16-byte piece of a row this lane takes in the element-wise part
       float loss = 0.f;
@@ -687,10 +727,11 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       ok = ok && mbar_wait(&acc_full_bar[acc], acc_phase, abort_flag, p.status, 4u);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols;
+      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * acc_cols + (uint32_t)part0;
+      if (PAIR && n0 >= N) free_acc();
       for (int ch = 0; ch < nchunks; ++ch) {
         const int col0 = n0 + ch * chunk_cols;
-        if (col0 >= N) break;  // uniform across the warp; the first chunk of a tile always lies inside
+        if (col0 >= N) break;  // uniform across the warp
         const bool last = (ch == nchunks - 1) || (col0 + chunk_cols >= N);
         uint8_t* const dst = cbuf + (size_t)lane * 128;
         uint32_t r[32];
@@ -702,15 +743,11 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
           tmem_ld32(tcol, r);
           if (X3) {
             uint32_t r2[32];
-            tmem_ld32(tcol + (uint32_t)o.block_n, r2);
+            tmem_ld32(tcol + (PAIR ? X3_CORR_COLS : (uint32_t)o.block_n), r2);
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           }
-          if (last && (half == 1 || !out_bf16)) {  // last read of the accumulator: the next tile may have it
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty_bar[acc]);
-          }
+          if (last && (half == 1 || !out_bf16)) free_acc();
           if (half == 0) {
             if (lane == 0) bulk_wait_read<0>();  // the store before has read the buffer
             __syncwarp();
@@ -781,8 +818,8 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
       }
       if (epi == SE_LOSS && it + 1 == (unsigned int)p.steps) add_loss(loss);
       publish(o.sig_row >= 0 ? o.sig_row + mb : -1, o.sig_all, true);
-      acc_phase ^= 1;
-      wk.advance();
+      next_acc();
+      wk.advance(units);
     }
     if (lane == 0) bulk_wait_all();
   }
@@ -790,10 +827,15 @@ __global__ void __launch_bounds__(STEP_THREADS, 1) step_kernel(const __grid_cons
   __syncwarp();
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // both CTAs are done with each other's shared memory and TMEM
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
-                 : "memory");
+    if (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)p.tmem_cols)
+                   : "memory");
   }
 }
 
@@ -870,9 +912,53 @@ bool make_operand(Operand& o, CUtensorMap& map, CUtensorMap& map_lo, const void*
 struct StepPlan {
   StepMaps* maps_dev = nullptr;
   int kind = KIND_BF16, grid = 0;
+  bool pair = false;
   size_t smem = 0;
   StepArgs<MAX_OPS> args;  // counters, status, steps and learning rate are filled in per launch
 };
+
+template <int OPS>
+using StepKernel = void (*)(const StepArgs<OPS>);
+template <int OPS>
+static cudaError_t pick_kernel(const StepPlan* plan, StepKernel<OPS>* kernel) {
+  static const StepKernel<OPS> kernels[3][2] = {{step_kernel<KIND_BF16, OPS, false>, step_kernel<KIND_BF16, OPS, true>},
+                                                {step_kernel<KIND_TF32, OPS, false>, step_kernel<KIND_TF32, OPS, true>},
+                                                {step_kernel<KIND_X3, OPS, false>, step_kernel<KIND_X3, OPS, true>}};
+  *kernel = kernels[plan->kind][plan->pair ? 1 : 0];
+  // per launch: handles of several devices and threads share the library, and the call is cheap
+  return cudaFuncSetAttribute(reinterpret_cast<const void*>(*kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+}
+
+template <int OPS>
+static void launch_config(const StepPlan* plan, cudaStream_t stream, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg->gridDim = dim3(plan->grid);
+  cfg->blockDim = dim3(STEP_THREADS);
+  cfg->dynamicSmemBytes = plan->smem;
+  cfg->stream = stream;
+  cfg->attrs = attr;
+  cfg->numAttrs = plan->pair ? 2 : 1;
+}
+
+// Pairs that fit on the GPU at once: its SMs come in clusters that need not all hold whole pairs.
+template <int OPS>
+static int resident_pairs(const StepPlan* plan) {
+  StepKernel<OPS> kernel;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  launch_config<OPS>(plan, nullptr, &cfg, attr);
+  int n = 0;
+  if (pick_kernel<OPS>(plan, &kernel) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kernel), &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
 
 int step_plan_counters(const StepSpec& s) {
   int n = 0;
@@ -887,12 +973,14 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
   const int eb = d0.in_type == T_BF16 ? 2 : 4;
   const bool x3 = d0.A_lo != nullptr;
   const int slabs = x3 ? 1 : 2;
+  const bool pair = s.pair;
+  const int rows = pair ? 2 * BLOCK_M : BLOCK_M;
   StepPlan* plan = new StepPlan();
   memset(&plan->args, 0, sizeof plan->args);
   StepArgs<MAX_OPS>& args = plan->args;
   StepOp* ops = args.op;
   std::vector<StepMaps> maps(nops);
-  std::vector<int> row_base(nops), all_base(nops), ntiles(nops), row_add(nops);
+  std::vector<int> row_base(nops), all_base(nops), ntiles(nops), per_item(nops), row_add(nops);
   std::vector<char> row_used(nops, 0), all_used(nops, 0);
   auto refuse = [&]() -> StepPlan* {
     step_plan_destroy(plan);
@@ -907,7 +995,7 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     StepMaps& mp = maps[i];
     const int ob = d.out_type == T_BF16 ? 2 : 4;
     o.M = d.M; o.N = d.N;
-    const int num_m = (d.M + BLOCK_M - 1) / BLOCK_M;
+    const int num_m = (d.M + rows - 1) / rows;
     o.block_n = g.block_n;
     o.num_n = (d.N + o.block_n - 1) / o.block_n;
     const int block_k = slabs * SLAB_BYTES / eb;
@@ -920,7 +1008,8 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     } else {
       const bool a_mn = d.sAm == 1 && d.sAk != 1, b_mn = d.sBn == 1 && d.sBk != 1;
       if (!make_operand(o.a, mp.a, mp.a_lo, d.A, d.A_lo, eb, d.M, d.K, a_mn ? d.sAk : d.sAm, a_mn, BLOCK_M, slabs) ||
-          !make_operand(o.b, mp.b, mp.b_lo, d.B, d.B_lo, eb, d.N, d.K, b_mn ? d.sBk : d.sBn, b_mn, o.block_n, slabs))
+          !make_operand(o.b, mp.b, mp.b_lo, d.B, d.B_lo, eb, d.N, d.K, b_mn ? d.sBk : d.sBn, b_mn,
+                        pair ? o.block_n / 2 : o.block_n, slabs))
         return refuse();
       const cuuint64_t dims[2] = {(cuuint64_t)d.N, (cuuint64_t)d.M};
       const cuuint64_t pitch = (cuuint64_t)d.ldc * ob;
@@ -931,7 +1020,7 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
       o.wide = pitch % 32 == 0 && reinterpret_cast<uintptr_t>(d.C) % 32 == 0 && reinterpret_cast<uintptr_t>(d.C_lo) % 32 == 0;
       const uint32_t fmt = eb == 4 ? 2u : 1u;  // tf32 : bf16
       o.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
-                ((uint32_t)(o.block_n >> 3) << 17) | ((uint32_t)(BLOCK_M >> 4) << 24);
+                ((uint32_t)(o.block_n >> 3) << 17) | ((uint32_t)(rows >> 4) << 24);
       o.tx_bytes = (o.a.bytes + o.b.bytes) * (x3 ? 2u : 1u);
       if (o.tx_bytes > slot) slot = o.tx_bytes;
       if (o.block_n > max_bn) max_bn = o.block_n;
@@ -947,7 +1036,9 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     if (o.epi == SE_SGD) { o.w = g.w; o.w16 = g.w16; o.w_lo = g.w_lo; }
     o.first_item = items;
     ntiles[i] = narrow ? num_m * NARROW_ITEMS : num_m * o.num_n;
-    row_add[i] = 4 * (narrow ? NARROW_ITEMS : o.num_n);  // every epilogue warp of a tile counts one
+    // every epilogue warp counts one for each item it takes part in
+    per_item[i] = pair ? (narrow ? 8 : 16) : 4;
+    row_add[i] = per_item[i] * (narrow ? NARROW_ITEMS : o.num_n);
     items += ntiles[i];
     row_base[i] = ncnt;
     all_base[i] = ncnt + num_m;
@@ -961,12 +1052,12 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
     o.row_cnt = g.rows_of >= 0 ? row_base[g.rows_of] : -1;
     o.row_target = g.rows_of >= 0 ? row_add[g.rows_of] : 0;
     o.all_cnt = g.all_of >= 0 ? all_base[g.all_of] : -1;
-    o.all_target = g.all_of >= 0 ? 4 * ntiles[g.all_of] : 0;
+    o.all_target = g.all_of >= 0 ? per_item[g.all_of] * ntiles[g.all_of] : 0;
     o.upd_cnt = g.update_after >= 0 ? all_base[g.update_after] : -1;
-    o.upd_target = g.update_after >= 0 ? 4 * ntiles[g.update_after] : 0;
+    o.upd_target = g.update_after >= 0 ? per_item[g.update_after] * ntiles[g.update_after] : 0;
     for (int k = 0; k < 2; ++k) {
       o.prev_cnt[k] = g.prev_step[k] >= 0 ? all_base[g.prev_step[k]] : -1;
-      o.prev_target[k] = g.prev_step[k] >= 0 ? 4 * ntiles[g.prev_step[k]] : 0;
+      o.prev_target[k] = g.prev_step[k] >= 0 ? per_item[g.prev_step[k]] * ntiles[g.prev_step[k]] : 0;
     }
     if (o.epi == SE_MASK) {
       if (g.mask_of < 0) return refuse();
@@ -981,12 +1072,13 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
   for (int i = 0; i < nops; ++i) {
     ops[i].sig_row = row_used[i] ? row_base[i] : -1;
     ops[i].sig_all = all_used[i] ? all_base[i] : -1;
-    ops[i].own_target = 4 * ntiles[i];
+    ops[i].own_target = per_item[i] * ntiles[i];
   }
   plan->kind = x3 ? KIND_X3 : eb == 4 ? KIND_TF32 : KIND_BF16;
   args.nops = nops;
   args.items = items;
   args.slot_bytes = slot;
+  plan->pair = pair;
   args.tmem_cols = x3 ? 512 : 2 * max_bn;
   args.target = s.target;
   args.dz = s.dz;
@@ -1001,6 +1093,14 @@ StepPlan* step_plan_create(const StepSpec& s, int sm_count) {
   plan->smem = 1024 + (size_t)args.stages * slot + EPI_BYTES;
   if (plan->smem < 140 * 1024) plan->smem = 140 * 1024;  // one CTA (one TMEM allocation) per SM
   plan->grid = items < sm_count ? items : sm_count;
+  if (pair) {
+    int pairs = items < sm_count / 2 ? items : sm_count / 2;
+    plan->grid = 2 * pairs;
+    const int fit = nops <= SMALL_OPS ? resident_pairs<SMALL_OPS>(plan) : resident_pairs<MAX_OPS>(plan);
+    if (fit < pairs) pairs = fit;
+    if (pairs < 1) return refuse();
+    plan->grid = 2 * pairs;
+  }
   if (args.stages < 2 || cudaMalloc((void**)&plan->maps_dev, sizeof(StepMaps) * nops) != cudaSuccess ||
       cudaMemcpy(plan->maps_dev, maps.data(), sizeof(StepMaps) * nops, cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
@@ -1019,14 +1119,8 @@ void step_plan_destroy(StepPlan* p) {
 template <int OPS>
 static cudaError_t launch_ops(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
                               cudaStream_t stream) {
-  using Kernel = void (*)(const StepArgs<OPS>);
-  static const Kernel kernels[3][2] = {{step_kernel<KIND_BF16, OPS, false>, step_kernel<KIND_BF16, OPS, true>},
-                                       {step_kernel<KIND_TF32, OPS, false>, step_kernel<KIND_TF32, OPS, true>},
-                                       {step_kernel<KIND_X3, OPS, false>, step_kernel<KIND_X3, OPS, true>}};
-  const Kernel kernel = kernels[plan->kind][plan->args.nar_a ? 1 : 0];
-  // per launch: handles of several devices and threads share the library, and the call is cheap
-  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+  StepKernel<OPS> kernel;
+  cudaError_t e = pick_kernel<OPS>(plan, &kernel);
   if (e != cudaSuccess) return e;
   StepArgs<OPS> a;
   static_cast<StepHead&>(a) = plan->args;
@@ -1036,15 +1130,8 @@ static cudaError_t launch_ops(const StepPlan* plan, int steps, float lr, unsigne
   a.steps = steps;
   a.neg_lr = -lr;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(plan->grid);
-  cfg.blockDim = dim3(STEP_THREADS);
-  cfg.dynamicSmemBytes = plan->smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  launch_config<OPS>(plan, stream, &cfg, attr);
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 

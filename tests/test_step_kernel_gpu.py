@@ -83,6 +83,32 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
         assert abs(la - lb) <= 1e-5 * abs(la) and abs(la - lf) <= 1e-5 * abs(la)
 
 
+# One tile of a pair with its second CTA empty / a remainder in rows and columns of either CTA / both input slots,
+# bf16 gradients / several rounds of the grid / narrow last layers / more layers than the small table holds
+PAIR_NETS = [([96, 64], 40, {}), ([256, 132, 388, 260], 130, {}), ([123, 77, 201, 33], 333, {}),
+             ([512, 384, 640, 128], 640, {"grad_bf16": True}), ([1024, 1536, 512], 3100, {}), ([64] * 24, 257, {"input_grad": False}),
+             ([160, 96, 10], 300, {}), ([256, 128, 1], 990, {"ref": True})]
+
+
+@pytest.mark.parametrize("prec", ["bf16", "tf32", "fp32tc"])
+@pytest.mark.parametrize("net", PAIR_NETS, ids=lambda n: "x".join(map(str, n[0][:4])) + f"b{n[1]}" + "".join(n[2]))
+def test_pair_tiles_match_single_cta_tiles(native, oracle, monkeypatch, net, prec):
+    """256 x 128 tiles of CTA pairs, and the tiles of one CTA, add every element's products in the same order: equal
+    bits, narrow last layers included."""
+    from tbb_test_b200 import _capi as K
+    nf, batch, opts = net
+    P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32, "fp32tc": K.PREC_FP32_TC}[prec]
+    monkeypatch.setenv("B2_STEP_KERNEL", "1")
+    for steps, fed in ((1, False), (3, False), (2, True)):
+        got = []
+        for pair in ("0", "1"):
+            monkeypatch.setenv("B2_STEP_PAIR", pair)
+            got.append(states(oracle, K, nf, batch, P, steps, opts, fed=fed))
+        (a, la, na), (b, lb, nb) = got
+        assert na == nb and abs(la - lb) <= 1e-5 * abs(la)
+        assert all(np.array_equal(a[k], b[k]) for k in a), (steps, fed)
+
+
 @pytest.mark.parametrize("prec", ["bf16", "tf32"])
 def test_two_handles_in_two_threads(native, oracle, prec):
     """Cooperative launches of two handles on one GPU, issued by two host threads at once, each keep their grid
