@@ -516,31 +516,43 @@ int build_sites(b2_handle* h) {
   return B2_OK;
 }
 
-// Steps per launch of the step kernel, so that a launch lasts about LAUNCH_US: it holds every SM, and work of other
-// handles, streams or processes gets its turn only between launches (64 steps of 20 x 512, batch 2048 in one launch were
-// 18.6 ms). A step is estimated as 5 us for each GEMM of the chain of layers plus all GEMMs at the rate the kernel
-// reaches: bf16, 5 x 1024, batch 1024 90 us (measured 113); 20 x 512, batch 2048 280 (300); 4 x 2048, batch 2048 298 (270).
-// Splitting costs nothing that shows: fp32-class 5 x 1024 292 us per step in 22 launches as in 2 for 128 steps.
-constexpr double LAUNCH_US = 2000.0;
-int steps_per_launch(const b2_handle* h) {
+// Flops of the GEMMs of a step, and its time as one launch: 4 us for each GEMM of the chain of layers plus all GEMMs at
+// the rate the kernel reaches. us, estimated and measured: bf16 5 x 1024, batch 1024 80 and 90; 20 x 512, batch 2048 241 and
+// 244; 4 x 2048, batch 2048 238 and 210; fp32-class 5 x 1024 201 and 233; 2 layers of 103 GFLOP GEMMs 3108 and 2423.
+double step_flops(const b2_handle* h) {
   double flops = 0;
   for (int l = 0; l < h->L; ++l) flops += 6.0 * h->bl * h->nf[l] * h->nf[l + 1];
-  const double rate = h->op_type == T_BF16 ? 800e6 : h->x3 ? 120e6 : 400e6;  // flops per us
-  const double n = LAUNCH_US / (5.0 * 2 * h->L + flops / rate);
+  return flops;
+}
+double step_us(const b2_handle* h) {
+  const double rate = h->op_type == T_BF16 ? 1000e6 : h->x3 ? 200e6 : 500e6;  // flops per us
+  return 4.0 * 2 * h->L + step_flops(h) / rate;
+}
+
+// Steps per launch of the step kernel, so that a launch lasts about LAUNCH_US: it holds every SM, and work of other
+// handles, streams or processes gets its turn only between launches (64 steps of 20 x 512, batch 2048 in one launch were
+// 18.6 ms). Splitting costs nothing that shows: fp32-class 5 x 1024 292 us per step in 22 launches as in 2 for 128 steps.
+constexpr double LAUNCH_US = 2000.0;
+int steps_per_launch(const b2_handle* h) {
+  const double n = LAUNCH_US / step_us(h);
   return n < 1 ? 1 : n > 64 ? 64 : (int)n;
 }
 
-// Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken when every GEMM of the step
-// is at most two rounds of 128 x 128 tiles over the SMs, where the chain of layers is bound by latency; wider
-// layers keep the larger tiles of gemm_tc_kernel (per step, one launch per GEMM against one for the step: 4 x 2048,
-// batch 2048, bf16 272 -> 270 us, fp32-class 1078 -> 988 us; 1536-768-1536-1024, batch 3000, tf32 253 -> 179 us; but
-// 3 x 4096, batch 1024, bf16 407 -> 500 us and tf32 600 -> 783 us).
+// Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken up to the size of an average GEMM
+// from which on the larger tiles of gemm_tc_kernel (256 x 256 by CTA pairs; 128 x 128 in the fp32-class mode) outweigh the
+// launch, fill and drain of every GEMM, and for steps of a few ms, since a launch holds every SM. us per step, one launch per
+// GEMM -> one for the step, by GFLOP of a GEMM: bf16 9 (800 wide, batch 8192) 292 -> 173, 17 (1024, batch 8192) 436 -> 319,
+// 25 (3072, batch 1300) 288 -> 263, 34 (2560, batch 2560) 316 -> 294, 34 (2048, batch 4096) 470 -> 473, 58 (3072, batch 3072)
+// 426 -> 474; tf32 17 (4096, batch 512) 456 -> 381, 24 (2304, batch 2304) 439 -> 386 but 25 (3072, batch 1300) 404 -> 439, 34
+// (2560, batch 2560) 501 -> 527; fp32-class 34 (2560) 1376 -> 1200, 69 (2048, batch 8192) 2753 -> 2427, 103 2793 -> 2423.
 int build_step_plans(b2_handle* h) {
   const int L = h->L;
   const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
   if (e && e[0] == '0') return B2_OK;
   const bool has_ar = h->cfg.world_size > 1 && h->cfg.allreduce;
   if (!use_tc(h) || has_ar || !h->cfg.overlap || h->bl < 1) return B2_OK;
+  const double most = h->op_type == T_BF16 ? 35e9 : h->x3 ? 110e9 : 21e9;
+  if (!(e && e[0] == '1') && (step_flops(h) > most * 3 * h->L || step_us(h) > 2 * LAUNCH_US)) return B2_OK;
   auto tiles = [](const GemmDesc& d, int bn) { return (long long)((d.M + 127) / 128) * ((d.N + bn - 1) / bn); };
   for (int l = 0; l < L; ++l) {
     for (const Site* s : {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]}) {
@@ -551,7 +563,6 @@ int build_step_plans(b2_handle* h) {
       // a last layer of fewer than 16 outputs stays on the CUDA cores, inside the step kernel
       const bool narrow = s == &h->fwd[L - 1] && s->d.N < 16 && s->d.sAm % (16 / (int)esize(s->d.in_type)) == 0;
       if (!s->plan && !narrow) return B2_OK;
-      if (!(e && e[0] == '1') && tiles(s->d, 128) > 2 * h->sms) return B2_OK;
     }
   }
   // CTA pairs (256 x 128 tiles, two thirds of the operand traffic) once the layers are as many 128 x 128 tiles as fill the

@@ -109,6 +109,20 @@ def test_pair_tiles_match_single_cta_tiles(native, oracle, monkeypatch, net, pre
         assert all(np.array_equal(a[k], b[k]) for k in a), (steps, fed)
 
 
+@pytest.mark.parametrize("prec", ["bf16", "tf32", "fp32tc"])
+@pytest.mark.parametrize("nf,batch", [([800, 800, 800], 8192), ([64, 8000, 64], 300), ([64, 64, 64], 20000), ([2304, 2304], 1500)],
+                         ids=["many-tiles", "wide-middle", "long-sums", "large"])
+def test_layers_of_many_tiles(native, oracle, monkeypatch, nf, batch, prec):
+    """Layers of many more tiles than SMs run as one launch by default, with the bits of one launch per GEMM."""
+    from tbb_test_b200 import _capi as K
+    P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32, "fp32tc": K.PREC_FP32_TC}[prec]
+    a, la, na = states(oracle, K, nf, batch, P, 2, {"lr": 1e-5})
+    monkeypatch.setenv("B2_STEP_KERNEL", "0")
+    b, lb, nb = states(oracle, K, nf, batch, P, 2, {"lr": 1e-5})
+    assert na <= 2 < nb and abs(la - lb) <= 1e-5 * abs(la)
+    assert all(np.array_equal(a[k], b[k]) for k in a)
+
+
 @pytest.mark.parametrize("prec", ["bf16", "tf32"])
 def test_two_handles_in_two_threads(native, oracle, prec):
     """Cooperative launches of two handles on one GPU, issued by two host threads at once, each keep their grid
