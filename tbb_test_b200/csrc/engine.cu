@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <sched.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -123,7 +124,8 @@ struct b2_handle {
   void* dinput = nullptr;
   // Page-locked buffers of download_rows, two per worker, made at the first large download
   char* dl_buf = nullptr;
-  cudaEvent_t dl_ev[12] = {};
+  size_t dl_bytes = 0;
+  cudaEvent_t dl_ev[24] = {};
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
   // Per input slot: the loss accumulator (double) and, 16 bytes behind it, the tile counters of the step
@@ -327,31 +329,49 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
 // Device rows to host memory, done when it returns. A copy to pageable memory runs at the speed of one
 // thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
 // destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
-// buffers of their own, each moving one chunk while its next one is in flight, share that work.
-constexpr size_t DL_CHUNK = 128 << 10, DL_MIN_BYTES = 2 << 20;
-constexpr int DL_WORKERS = 6;
+// buffers of their own, each moving one chunk while its next one is in flight, share that work. A chunk costs
+// about 8 us whatever its size, so chunks grow with the matrix, and so do the buffers; starting a thread takes 10 us, so
+// a few MB get half of them. To fresh memory, us, six threads with 128 KB chunks -> now: 4096 x 4096 4475 -> 2158, 8192 x 8192
+// 25434 -> 12356.
+constexpr size_t DL_MIN_CHUNK = 128 << 10, DL_MAX_CHUNK = 1 << 20, DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20;
+constexpr int DL_WORKERS = 12;
 int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
-  const size_t width = (size_t)cols * 4;
+  const size_t width = (size_t)cols * 4, total = width * rows;
   cudaPointerAttributes attr;
   bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
-  if (pageable && width <= DL_CHUNK && width * rows >= DL_MIN_BYTES && !h->dl_buf) {
-    bool ok = cudaHostAlloc((void**)&h->dl_buf, 2 * DL_WORKERS * DL_CHUNK, cudaHostAllocDefault) == cudaSuccess;
+  const int workers = total >= DL_MANY_BYTES ? DL_WORKERS : DL_WORKERS / 2;
+  size_t chunk = DL_MIN_CHUNK;
+  while (chunk < DL_MAX_CHUNK && 4 * chunk * workers <= total) chunk *= 2;
+  bool shared = pageable && width <= chunk && total >= DL_MIN_BYTES;
+  if (shared && h->dl_bytes < 2 * workers * chunk) {
+    if (h->dl_buf) cudaFreeHost(h->dl_buf);
+    h->dl_buf = nullptr;
+    h->dl_bytes = 2 * workers * chunk;
+    bool ok = cudaHostAlloc((void**)&h->dl_buf, h->dl_bytes, cudaHostAllocDefault) == cudaSuccess;
     if (!ok) h->dl_buf = nullptr;
     for (int i = 0; ok && i < 2 * DL_WORKERS; ++i)
       ok = h->dl_ev[i] || cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {  // no page-locked memory left: the plain copy
       if (h->dl_buf) cudaFreeHost(h->dl_buf);
       h->dl_buf = nullptr;
+      h->dl_bytes = 0;
       cudaGetLastError();
     }
   }
-  if (!pageable || width > DL_CHUNK || width * rows < DL_MIN_BYTES || !h->dl_buf) {
+  if (!shared || !h->dl_buf) {
+    // Pages of fresh memory in one call instead of a fault each (1 MB 443 -> 350 us); it changes nothing but that they
+    // are there, and where the kernel does not know the request the copy takes the faults.
+    if (pageable && ld == (size_t)cols) {
+      const uintptr_t page = 4096, from = (reinterpret_cast<uintptr_t>(host) + page - 1) & ~(page - 1);
+      const uintptr_t to = (reinterpret_cast<uintptr_t>(host) + total) & ~(page - 1);
+      if (to > from && total >= 64 * 1024) madvise(reinterpret_cast<void*>(from), to - from, 23 /* MADV_POPULATE_WRITE */);
+    }
     CK(h, cudaMemcpy2DAsync(host, ld * 4, dev, pitch * 4, width, rows, cudaMemcpyDeviceToHost, h->s_main));
     CK(h, cudaStreamSynchronize(h->s_main));
     return B2_OK;
   }
-  const int per = (int)(DL_CHUNK / width), chunks = (rows + per - 1) / per;
+  const int per = (int)(chunk / width), chunks = (rows + per - 1) / per;
   std::atomic<int> next{0}, error{(int)cudaSuccess};
   auto work = [&](int t) {
     cudaError_t e = cudaSetDevice(h->cfg.device);
@@ -360,7 +380,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       if (in_flight[b] < 0) return;
       if (e == cudaSuccess) e = cudaEventSynchronize(h->dl_ev[2 * t + b]);
       if (e == cudaSuccess) {
-        const char* src = h->dl_buf + (size_t)(2 * t + b) * DL_CHUNK;
+        const char* src = h->dl_buf + (size_t)(2 * t + b) * chunk;
         const int r0 = in_flight[b] * per, n = std::min(per, rows - r0);
         for (int r = 0; r < n; ++r) memcpy(host + (size_t)(r0 + r) * ld, src + width * r, width);
       }
@@ -370,7 +390,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       const int c = next.fetch_add(1);
       if (c >= chunks) break;
       const int r0 = c * per, n = std::min(per, rows - r0);
-      e = copy_rows(h->dl_buf + (size_t)(2 * t + b) * DL_CHUNK, width,
+      e = copy_rows(h->dl_buf + (size_t)(2 * t + b) * chunk, width,
                     static_cast<const char*>(dev) + (size_t)r0 * pitch * 4, pitch * 4, width, (size_t)n,
                     cudaMemcpyDeviceToHost, h->s_main);
       if (e == cudaSuccess) e = cudaEventRecord(h->dl_ev[2 * t + b], h->s_main);
@@ -382,7 +402,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
     if (e != cudaSuccess) error.store((int)e);
   };
   std::thread pool[DL_WORKERS];
-  int helpers = std::min(std::min(DL_WORKERS, (int)std::thread::hardware_concurrency()), chunks) - 1;
+  int helpers = std::min(std::min(workers, (int)std::thread::hardware_concurrency()), chunks) - 1;
   for (int i = 0; i < helpers; ++i) {
     try {
       pool[i] = std::thread(work, i + 1);

@@ -29,6 +29,28 @@ def test_large_downloads(native, oracle, shape, extra):
         m.close()
 
 
+@pytest.mark.parametrize("shape,extra", [((257, 513), 0), ((1024, 512), 0), ((1800, 2050), 0), ((1800, 2050), 7), ((4100, 4099), 0),
+                                         ((300, 20000), 3)])
+def test_chunks_grow_with_the_matrix(native, oracle, shape, extra):
+    """Sizes on both sides of each step in threads and chunk size, one handle growing its buffers: fresh destinations
+    (pages that do not exist yet) and pitched ones, every element in place, nothing written between the rows."""
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    rows, cols = shape
+    m = MLP([cols, rows, 700, 800], 8)
+    ws = [oracle.fill_uniform(rows, cols, 3, -1, 1), oracle.fill_uniform(700, rows, 4, -1, 1), oracle.fill_uniform(800, 700, 5, -1, 1)]
+    for l, w in enumerate(ws):
+        m.upload_weights(l, w)
+    for l in (2, 1, 0, 2):
+        r, c = ws[l].shape
+        got = np.empty((r, c + extra), np.float32)
+        if extra:
+            got[:] = 7.0
+        assert m.lib.b2_download_weights(m._h, l, got.ctypes.data_as(C.POINTER(C.c_float)), c + extra) == K.OK
+        assert np.array_equal(got[:, :c], ws[l]) and (got[:, c:] == 7.0).all()
+    m.close()
+
+
 OUT_OF_MEMORY = """
 import ctypes as C, sys
 import numpy as np
