@@ -38,6 +38,7 @@ struct GemmDesc {
   int out_type;  // ElemType of C
   int pad_writable;  // 1: the bytes between column N and the next 16-byte boundary of a row of C may be overwritten
   int shared_sms;    // 1: another library's kernels may hold some of the SMs while this GEMM runs
+  int large_tiles;   // 1: CUDA-core GEMM: not the kernel for small grids
   // Optional stream-K workspace of the tensor-core kernel (null = whole tiles per CTA):
   // TC_WS_SLOT_BYTES per SM and one zero-initialised flag word per SM. GEMMs that share a
   // workspace must not overlap on the GPU.
@@ -65,6 +66,10 @@ constexpr size_t TC_WS_SLOT_BYTES = 2 * 128 * 256 * sizeof(float);
 
 // CUDA-core GEMM for any shape, stride and alignment (fp32 accumulate).
 cudaError_t gemm_simt_launch(const GemmDesc& g, cudaStream_t stream);
+// Kernel for small grids (gemm_f32.cu), which gemm_simt_launch takes where it serves and large_tiles is not set.
+bool gemm_f32_serves(const GemmDesc& g);
+cudaError_t gemm_f32_launch(const GemmDesc& g, cudaStream_t stream);
+bool gemm_simt_small(const GemmDesc& g);  // served by one of its kernels for small grids (unless large_tiles)
 
 // Tensor-core (tcgen05 + TMA + TMEM) GEMM. in_type T_BF16 -> kind::f16 (bf16),
 // in_type T_F32 -> kind::tf32. Returns cudaErrorNotSupported when the shape or

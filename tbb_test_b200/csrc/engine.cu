@@ -520,6 +520,15 @@ int build_sites(b2_handle* h) {
       make_site(h, h->wgrad0_alt, tc, wg_sms);
     }
   }
+  // CUDA-core GEMMs: the kernel for small grids only where it serves all GEMMs of the step. Weight and input gradient of
+  // a layer run side by side, and beside a large GEMM's kernel a small one's warps take the issue slots that the chain of
+  // layers waits for (us per step, one kernel for all -> each GEMM its own: 6 x 512, batch 1024 458 -> 729;
+  // 123-777-345-999, batch 1700 509 -> 697).
+  std::vector<Site*> sites = {&h->fwd0_alt, &h->wgrad0_alt};
+  for (int l = 0; l < L; ++l) sites.insert(sites.end(), {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]});
+  bool small = true;
+  for (const Site* s : sites) small = small && (!s->active || s->plan || gemm_simt_small(s->d));
+  for (Site* s : sites) s->d.large_tiles = !small;
   // ReLU bit planes: used for a layer only if both its producer (forward of the layer below) and
   // its consumer (input gradient of the layer itself) run on the tensor-core kernel
   for (int l = 1; l < L; ++l) {

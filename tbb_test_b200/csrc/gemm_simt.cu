@@ -4,11 +4,12 @@
 //
 // Stand in for the reference's cblas_sgemm calls (mlp_omp.cc:474,566,657):
 // C = alpha * op(A) * op(B) + beta * C with fp32 accumulation. Three kernels:
-//   gemm_simt_kernel    any shape; every sum runs in k order, one FMA per term
+//   gemm_simt_kernel    any shape; every sum runs in k order, one FMA per term (small grids: gemm_f32.cu)
 //   gemm_narrow_kernel  N <= 16 with K contiguous in both operands (the forward GEMM of a
 //                       narrow output layer): lanes split K
 //   gemm_short_kernel   M <= 16 with N contiguous in B (the weight gradient of that layer): warps split K
 #include "common.cuh"
+#include "simt_tile.h"
 
 namespace b2 {
 namespace {
@@ -272,37 +273,27 @@ __global__ void __launch_bounds__(512) gemm_short_kernel(GemmDesc g) {
   }
 }
 
-// Tile of gemm_simt_kernel, an index into SIMT_TILES. A launch takes as long as its fullest SM: rounds of the
-// grid over the SMs times the tile's area, divided by the rate the tile sustains (a smaller tile reads more
-// shared memory per FMA). Measured, us: 1024^3 as 64 x 64 74, as 64 x 32 105; 512 x 512 x 2048 (64 tiles of
-// 64 x 64 on 148 SMs) 94 and 72.
-struct SimtTile { int bm, bn; double rate; };
+// Tile of gemm_simt_kernel, an index into SIMT_TILES. Measured, us: 1024^3 as 64 x 64 74, as 64 x 32 105; 512 x 512 x 2048
+// (64 tiles of 64 x 64 on 148 SMs) 94 and 72.
 constexpr SimtTile SIMT_TILES[4] = {{128, 128, 1.0}, {64, 64, 0.85}, {64, 32, 0.555}, {32, 32, 0.40}};
-int simt_tile(int M, int N, int sms) {
-  int best = 0;
-  double best_cost = 1e300;
-  for (int i = 0; i < 4; ++i) {
-    const SimtTile& c = SIMT_TILES[i];
-    if (i > 0 && (M + c.bm - 1) / c.bm > 65535) continue;  // row blocks are gridDim.y
-    const long long T = (long long)((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn);
-    const double cost = (double)((T + sms - 1) / sms) * c.bm * c.bn / c.rate;
-    if (cost < best_cost) { best_cost = cost; best = i; }
-  }
-  return best;
-}
+int simt_tile(int M, int N, int sms) { return fastest_tile(SIMT_TILES, 4, M, N, sms); }
+
+bool narrow_form(const GemmDesc& g) { return g.N <= 16 && g.K >= 64 && g.sAk == 1 && g.sBk == 1; }
+bool short_form(const GemmDesc& g) { return g.M <= 16 && g.K >= 64 && g.sBn == 1; }
 
 template <typename TI, typename TO>
 cudaError_t launch(const GemmDesc& g, cudaStream_t stream) {
-  if (g.N <= 16 && g.K >= 64 && g.sAk == 1 && g.sBk == 1) {
+  if (narrow_form(g)) {
     if (g.N <= 2) gemm_narrow_kernel<TI, TO, 2, 1><<<(g.M + 3) / 4, 128, 0, stream>>>(g);
     else gemm_narrow_kernel<TI, TO, 16, 2><<<(g.M + 7) / 8, 128, 0, stream>>>(g);
     return cudaGetLastError();
   }
-  if (g.M <= 16 && g.K >= 64 && g.sBn == 1) {
+  if (short_form(g)) {
     if (g.M <= 2) gemm_short_kernel<TI, TO, 2><<<(g.N + 31) / 32, 512, 0, stream>>>(g);
     else gemm_short_kernel<TI, TO, 16><<<(g.N + 31) / 32, 512, 0, stream>>>(g);
     return cudaGetLastError();
   }
+  if (!g.large_tiles && gemm_f32_serves(g)) return gemm_f32_launch(g, stream);
   auto vec = [](const void* p, long long ld) {
     return sizeof(TI) == 4 && reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0 ? 1 : 0;
   };
@@ -318,6 +309,8 @@ cudaError_t launch(const GemmDesc& g, cudaStream_t stream) {
 }
 
 }  // namespace
+
+bool gemm_simt_small(const GemmDesc& g) { return narrow_form(g) || short_form(g) || gemm_f32_serves(g); }
 
 cudaError_t gemm_simt_launch(const GemmDesc& g, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0) return cudaSuccess;

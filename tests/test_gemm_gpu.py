@@ -198,6 +198,21 @@ def test_cuda_core_dispatch_edges(dev, oracle, form, shape):
                    ref * (aux > 0)) <= 2 * TOL["fp32"]
 
 
+# fp32 on the CUDA cores at small grids and with rows that are not whole 16-byte pieces: one and several slabs of 32 k with
+# remainders, tiles of every size with remainders, against sums in float64. Bound per element: K roundings of the sum of
+# magnitudes, 2^-24 each.
+@pytest.mark.parametrize("shape", [(33, 18, 1), (65, 33, 31), (64, 96, 32), (31, 100, 33), (300, 301, 95), (129, 257, 97), (640, 900, 64),
+                                   (1001, 1300, 70), (1537, 1003, 65)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("form", list(FORMS))
+def test_fp32_small_grids(dev, oracle, form, shape):
+    from tbb_test_b200 import _capi as K
+    m, n, k = shape
+    ta, tb, a, b = operands(oracle, form, m, n, k, 121)
+    c = dev.sgemm_host(K.PREC_FP32, ta, tb, a, b).astype(np.float64)
+    ra, rb = (a.T if ta else a).astype(np.float64), (b.T if tb else b).astype(np.float64)
+    assert (np.abs(c - ra @ rb) <= k * 2.0 ** -24 * (np.abs(ra) @ np.abs(rb)) + 1e-30).all()
+
+
 @pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("shape", [(128, 18, 60), (300, 33, 100), (256, 257, 61), (200, 1003, 64), (1, 301, 33), (700, 1302, 130),
                                    (300, 64, 61)], ids=lambda s: "x".join(map(str, s)))
