@@ -125,7 +125,7 @@ struct b2_handle {
   // Page-locked buffers of download_rows, two per worker, made at the first large download
   char* dl_buf = nullptr;
   size_t dl_bytes = 0;
-  cudaEvent_t dl_ev[24] = {};
+  cudaEvent_t dl_ev[12] = {};
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
   // Per input slot: the loss accumulator (double) and, 16 bytes behind it, the tile counters of the step
@@ -329,28 +329,30 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
 // Device rows to host memory, done when it returns. A copy to pageable memory runs at the speed of one
 // thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
 // destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
-// buffers of their own, each moving one chunk while its next one is in flight, share that work. A chunk costs
-// about 8 us whatever its size, so chunks grow with the matrix, and so do the buffers; starting a thread takes 10 us, so
-// a few MB get half of them. To fresh memory, us, six threads with 128 KB chunks -> now: 4096 x 4096 4475 -> 2158, 8192 x 8192
-// 25434 -> 12356.
-constexpr size_t DL_MIN_CHUNK = 128 << 10, DL_MAX_CHUNK = 1 << 20, DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20;
+// buffers of their own share that work. A chunk costs about 8 us whatever its size, starting a thread 10 us, and a MB of
+// page-locked memory 1.1 ms, once. So a few MB get six threads with two buffers of 128 KB each; from 12 MB on twelve
+// threads share the same 1.5 MB, one buffer each (2048 x 2048 to fresh memory 1901 -> 1491 us); and from 32 MB on buffers of
+// 512 KB pay for themselves within the first matrices (4096 x 4096 4395 -> 3116 us, 8192 x 8192 25298 -> 13700 us; with 24 MB
+// of buffers 2253 and 12421, but 25 ms for the buffers).
+constexpr size_t DL_CHUNK = 128 << 10, DL_LARGE_CHUNK = 512 << 10;
+constexpr size_t DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20, DL_LARGE_BYTES = 32 << 20;
 constexpr int DL_WORKERS = 12;
 int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
   const size_t width = (size_t)cols * 4, total = width * rows;
   cudaPointerAttributes attr;
   bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
-  const int workers = total >= DL_MANY_BYTES ? DL_WORKERS : DL_WORKERS / 2;
-  size_t chunk = DL_MIN_CHUNK;
-  while (chunk < DL_MAX_CHUNK && 4 * chunk * workers <= total) chunk *= 2;
+  const bool many = total >= DL_MANY_BYTES;
+  const int workers = many ? DL_WORKERS : DL_WORKERS / 2, bufs = many ? 1 : 2;  // threads, buffers of each
+  const size_t chunk = total >= DL_LARGE_BYTES ? DL_LARGE_CHUNK : DL_CHUNK;
   bool shared = pageable && width <= chunk && total >= DL_MIN_BYTES;
-  if (shared && h->dl_bytes < 2 * workers * chunk) {
+  if (shared && h->dl_bytes < DL_WORKERS * chunk) {
     if (h->dl_buf) cudaFreeHost(h->dl_buf);
     h->dl_buf = nullptr;
-    h->dl_bytes = 2 * workers * chunk;
+    h->dl_bytes = DL_WORKERS * chunk;
     bool ok = cudaHostAlloc((void**)&h->dl_buf, h->dl_bytes, cudaHostAllocDefault) == cudaSuccess;
     if (!ok) h->dl_buf = nullptr;
-    for (int i = 0; ok && i < 2 * DL_WORKERS; ++i)
+    for (int i = 0; ok && i < DL_WORKERS; ++i)
       ok = h->dl_ev[i] || cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {  // no page-locked memory left: the plain copy
       if (h->dl_buf) cudaFreeHost(h->dl_buf);
@@ -378,24 +380,24 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
     int in_flight[2] = {-1, -1};  // chunk on its way into each of this worker's buffers
     auto land = [&](int b) {      // wait for it and move it to its place
       if (in_flight[b] < 0) return;
-      if (e == cudaSuccess) e = cudaEventSynchronize(h->dl_ev[2 * t + b]);
+      if (e == cudaSuccess) e = cudaEventSynchronize(h->dl_ev[bufs * t + b]);
       if (e == cudaSuccess) {
-        const char* src = h->dl_buf + (size_t)(2 * t + b) * chunk;
+        const char* src = h->dl_buf + (size_t)(bufs * t + b) * chunk;
         const int r0 = in_flight[b] * per, n = std::min(per, rows - r0);
         for (int r = 0; r < n; ++r) memcpy(host + (size_t)(r0 + r) * ld, src + width * r, width);
       }
       in_flight[b] = -1;
     };
-    for (int b = 0; e == cudaSuccess && error.load() == (int)cudaSuccess; b ^= 1) {
+    for (int b = 0; e == cudaSuccess && error.load() == (int)cudaSuccess; b = (b + 1) % bufs) {
       const int c = next.fetch_add(1);
       if (c >= chunks) break;
       const int r0 = c * per, n = std::min(per, rows - r0);
-      e = copy_rows(h->dl_buf + (size_t)(2 * t + b) * chunk, width,
+      e = copy_rows(h->dl_buf + (size_t)(bufs * t + b) * chunk, width,
                     static_cast<const char*>(dev) + (size_t)r0 * pitch * 4, pitch * 4, width, (size_t)n,
                     cudaMemcpyDeviceToHost, h->s_main);
-      if (e == cudaSuccess) e = cudaEventRecord(h->dl_ev[2 * t + b], h->s_main);
+      if (e == cudaSuccess) e = cudaEventRecord(h->dl_ev[bufs * t + b], h->s_main);
       in_flight[b] = c;
-      land(b ^ 1);
+      land((b + 1) % bufs);
     }
     land(0);
     land(1);
