@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../csrc/bucket_plan.h"
+#include "../csrc/row_pieces.h"
 #include "../csrc/tile_choice.h"
 #include "HyperCubeAllReduce.h"
 #include "b2_rng.h"
@@ -119,6 +120,9 @@ void b2h_choose_tile(int m, int n, int sms, int x3, int pair_ok, int shared, int
   const b2::TileChoice t = b2::choose_tile(m, n, sms, x3 != 0, pair_ok != 0, shared != 0);
   out3[0] = t.sub_m; out3[1] = t.bn; out3[2] = t.pair;
 }
+
+// 16-byte pieces of a 32-byte group of a result row that are stored (csrc/row_pieces.h).
+int b2h_pieces_of_32(int left, int per) { return b2::pieces_of_32(left, per); }
 
 void b2h_ring_info(int nsock, int sid, int task, int* out3) {
   nsockets = nsock;

@@ -247,3 +247,13 @@ def test_tile_choice_beside_collectives(host):
     assert [tile(m, 4096, s, shared=1) for m, s in ((8192, 148), (4096, 148), (2048, 128), (1024, 128))] == \
         [(2, 256, 0), (2, 256, 0), (2, 256, 0), (1, 256, 0)]
     assert [tile(m, 4096, 148) for m in (8192, 4096, 1024)] == [(2, 256, 1)] * 3
+
+
+@pytest.mark.parametrize("per", [8, 4], ids=["bf16", "fp32"])
+def test_groups_of_a_result_row(host, per):
+    """Every 32-byte group of a row (csrc/row_pieces.h) that lies in the matrix with both its 16-byte pieces counts two,
+    wherever it is in the row; the last one of a ragged row counts what the row has, and nothing lies behind the end."""
+    for cols in list(range(1, 129)):
+        got = [host.b2h_pieces_of_32(cols - at, per) for at in range(0, 128, 2 * per)]
+        whole = -(-cols // per)  # pieces of the row, the last one padded
+        assert got == [max(0, min(2, whole - 2 * i)) for i in range(len(got))], cols
