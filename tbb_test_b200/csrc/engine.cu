@@ -31,6 +31,7 @@
 
 #include "../../include/b200mlp.h"
 #include "bucket_plan.h"
+#include "step_choice.h"
 #include "common.cuh"
 #include "nccl_dyn.h"
 
@@ -547,26 +548,9 @@ int build_sites(b2_handle* h) {
   return B2_OK;
 }
 
-// Flops of the GEMMs of a step, and its time as one launch: 4 us for each GEMM of the chain of layers plus all GEMMs at
-// the rate the kernel reaches. us, estimated and measured: bf16 5 x 1024, batch 1024 80 and 90; 20 x 512, batch 2048 241 and
-// 244; 4 x 2048, batch 2048 238 and 210; fp32-class 5 x 1024 201 and 233; 2 layers of 103 GFLOP GEMMs 3108 and 2423.
-double step_flops(const b2_handle* h) {
-  double flops = 0;
-  for (int l = 0; l < h->L; ++l) flops += 6.0 * h->bl * h->nf[l] * h->nf[l + 1];
-  return flops;
-}
-double step_us(const b2_handle* h) {
-  const double rate = h->op_type == T_BF16 ? 1000e6 : h->x3 ? 200e6 : 500e6;  // flops per us
-  return 4.0 * 2 * h->L + step_flops(h) / rate;
-}
-
-// Steps per launch of the step kernel, so that a launch lasts about LAUNCH_US: it holds every SM, and work of other
-// handles, streams or processes gets its turn only between launches (64 steps of 20 x 512, batch 2048 in one launch were
-// 18.6 ms). Splitting costs nothing that shows: fp32-class 5 x 1024 292 us per step in 22 launches as in 2 for 128 steps.
-constexpr double LAUNCH_US = 2000.0;
-int steps_per_launch(const b2_handle* h) {
-  const double n = LAUNCH_US / step_us(h);
-  return n < 1 ? 1 : n > 64 ? 64 : (int)n;
+StepShape step_shape(const b2_handle* h) {
+  return {h->nf.data(), h->L, h->bl, h->op_type == T_BF16 ? STEP_BF16 : h->x3 ? STEP_X3 : STEP_TF32, h->sms,
+          h->cfg.input_grad != 0};
 }
 
 // Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken up to the size of an average GEMM
@@ -583,7 +567,8 @@ int build_step_plans(b2_handle* h) {
   const bool has_ar = h->cfg.world_size > 1 && h->cfg.allreduce;
   if (!use_tc(h) || has_ar || !h->cfg.overlap || h->bl < 1) return B2_OK;
   const double most = h->op_type == T_BF16 ? 35e9 : h->x3 ? 110e9 : 21e9;
-  if (!(e && e[0] == '1') && (step_flops(h) > most * 3 * h->L || step_us(h) > 2 * LAUNCH_US)) return B2_OK;
+  const StepShape shape = step_shape(h);
+  if (!(e && e[0] == '1') && (step_flops(shape) > most * 3 * L || 4.0 * 2 * L + step_flops_us(shape) > 2 * LAUNCH_US)) return B2_OK;
   auto tiles = [](const GemmDesc& d, int bn) { return (long long)((d.M + 127) / 128) * ((d.N + bn - 1) / bn); };
   for (int l = 0; l < L; ++l) {
     for (const Site* s : {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]}) {
@@ -681,7 +666,7 @@ int build_step_plans(b2_handle* h) {
       return B2_OK;
     }
   }
-  h->launch_steps = steps_per_launch(h);
+  h->launch_steps = steps_per_launch(shape);
   return B2_OK;
 }
 

@@ -257,3 +257,27 @@ def test_groups_of_a_result_row(host, per):
         got = [host.b2h_pieces_of_32(cols - at, per) for at in range(0, 128, 2 * per)]
         whole = -(-cols // per)  # pieces of the row, the last one padded
         assert got == [max(0, min(2, whole - 2 * i)) for i in range(len(got))], cols
+
+
+BF16, TF32, X3 = 0, 1, 2
+
+
+def step_choice(host, nf, rows, prec, sms=148, input_grad=True):
+    host.b2h_step_choice.restype = C.c_double
+    out = (C.c_int * 1)()
+    us = host.b2h_step_choice((C.c_int * len(nf))(*nf), len(nf) - 1, rows, prec, sms, int(input_grad), out)
+    return us, list(out)
+
+
+# us per step as measured on a B200
+@pytest.mark.parametrize("nf,rows,prec,us", [
+    ([1024] * 6, 1024, BF16, 89), ([1024] * 6, 1024, X3, 227), ([512] * 21, 2048, BF16, 234), ([64] * 5, 200000, BF16, 838),
+    ([64] * 5, 200000, TF32, 1444), ([64] * 5, 200000, X3, 3063), ([256] * 5, 100000, BF16, 637), ([512] * 4, 60000, X3, 1756),
+    ([8192] * 3, 64, BF16, 613), ([4096] * 3, 128, X3, 396), ([2048] * 17, 2048, X3, 3154), ([784, 500, 300, 10], 1000, BF16, 47)])
+def test_steps_per_launch(host, nf, rows, prec, us):
+    """Launches of the step kernel (csrc/step_choice.h) of about 2 ms, 4 at most, where a step is shorter than that: long
+    sums over the batch and many weights count, not only the flops."""
+    est, (steps,) = step_choice(host, nf, rows, prec)
+    assert 0.6 <= us / est <= 1.7
+    assert 1 <= steps <= 64 and (steps == 1 or steps * us <= 4000)
+    assert steps == 64 or (steps + 1) * est > 2000

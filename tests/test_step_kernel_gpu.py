@@ -171,7 +171,8 @@ def test_two_handles_in_two_threads(native, oracle, prec):
 
 
 @pytest.mark.parametrize("nf,batch,steps", [([512] * 21, 2048, 64), ([1024] * 6, 1024, 50), ([64, 64, 64], 64, 130),
-                                            ([64, 64, 64], 64, 65)], ids=["deep", "c1", "small", "one-more"])
+                                            ([64, 64, 64], 64, 65), ([64] * 5, 200000, 12), ([4096] * 3, 64, 48)],
+                         ids=["deep", "c1", "small", "one-more", "long-sums", "many-weights"])
 def test_steps_are_split_into_short_launches(native, oracle, monkeypatch, nf, batch, steps):
     """b2_step holds the GPU for a few ms at a time at most (the limit is 2 ms by estimate; twice that here, for a slow
     clock), whatever the number of steps, in few launches for short steps; and the split changes no bit."""
