@@ -553,22 +553,15 @@ StepShape step_shape(const b2_handle* h) {
           h->cfg.input_grad != 0};
 }
 
-// Whether whole steps run as one launch (step_kernel.cu), and the plans for it. Taken up to the size of an average GEMM
-// from which on the larger tiles of gemm_tc_kernel (256 x 256 by CTA pairs; 128 x 128 in the fp32-class mode) outweigh the
-// launch, fill and drain of every GEMM, and for steps of a few ms, since a launch holds every SM. us per step, one launch per
-// GEMM -> one for the step, by GFLOP of a GEMM: bf16 9 (800 wide, batch 8192) 292 -> 173, 17 (1024, batch 8192) 436 -> 319,
-// 25 (3072, batch 1300) 288 -> 263, 34 (2560, batch 2560) 316 -> 294, 34 (2048, batch 4096) 470 -> 473, 58 (3072, batch 3072)
-// 426 -> 474; tf32 17 (4096, batch 512) 456 -> 381, 24 (2304, batch 2304) 439 -> 386 but 25 (3072, batch 1300) 404 -> 439, 34
-// (2560, batch 2560) 501 -> 527; fp32-class 34 (2560) 1376 -> 1200, 69 (2048, batch 8192) 2753 -> 2427, 103 2793 -> 2423.
+// The plans of the networks whose whole steps run as one launch (step_kernel.cu; the rules: step_choice.h).
 int build_step_plans(b2_handle* h) {
   const int L = h->L;
   const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
   if (e && e[0] == '0') return B2_OK;
   const bool has_ar = h->cfg.world_size > 1 && h->cfg.allreduce;
   if (!use_tc(h) || has_ar || !h->cfg.overlap || h->bl < 1) return B2_OK;
-  const double most = h->op_type == T_BF16 ? 35e9 : h->x3 ? 110e9 : 21e9;
   const StepShape shape = step_shape(h);
-  if (!(e && e[0] == '1') && (step_flops(shape) > most * 3 * L || 4.0 * 2 * L + step_flops_us(shape) > 2 * LAUNCH_US)) return B2_OK;
+  if (!(e && e[0] == '1') && !step_serves(shape)) return B2_OK;
   auto tiles = [](const GemmDesc& d, int bn) { return (long long)((d.M + 127) / 128) * ((d.N + bn - 1) / bn); };
   for (int l = 0; l < L; ++l) {
     for (const Site* s : {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]}) {

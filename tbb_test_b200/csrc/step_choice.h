@@ -56,4 +56,29 @@ inline int steps_per_launch(const StepShape& s) {
   return n < 1 ? 1 : n > 64 ? 64 : (int)n;
 }
 
+// Whether steps run as one launch. Always where every GEMM is at most two rounds of 128 x 128 tiles over the SMs, however many
+// layers there are (us per step, one launch per GEMM -> one for the step, fp32-class, 2048 wide, batch 2048: 16 layers 3853 ->
+// 3154, 20 layers 4809 -> 3967). With larger GEMMs among them up to the size of an average GEMM from which on the larger
+// tiles of gemm_tc_kernel (256 x 256 by CTA pairs; 128 x 128 in the fp32-class mode) outweigh the launch, fill and drain of
+// every GEMM, and for steps of a few ms, since a launch holds every SM. By GFLOP of a GEMM: bf16 9 (800 wide, batch 8192) 292
+// -> 173, 17 (1024, batch 8192) 436 -> 319, 25 (3072, batch 1300) 288 -> 263, 34 (2560, batch 2560) 316 -> 294, 34 (2048, batch
+// 4096) 470 -> 473, 58 (3072, batch 3072) 426 -> 474; tf32 17 (4096, batch 512) 456 -> 381, 24 (2304, batch 2304) 439 -> 386
+// but 25 (3072, batch 1300) 404 -> 439, 34 (2560, batch 2560) 501 -> 527; fp32-class 34 (2560) 1376 -> 1200, 69 (2048, batch
+// 8192) 2753 -> 2427, 103 2793 -> 2423. One wide layer among narrow ones follows the average too: a 4096 x 4096 layer among
+// ten of 64, batch 8192, bf16 1064 -> 892, among seven of 1024, batch 4096, 758 -> 701; an 8192 x 8192 layer among twenty of 256,
+// batch 2048, 1218 -> 1179, tf32 1919 -> 1927; 4096 x 4096 among 24 of 512, batch 4096, tf32 2126 -> 1474.
+inline bool step_serves(const StepShape& s) {
+  bool short_gemms = true;
+  for (int l = 0; l < s.layers; ++l) {
+    const int in = s.nf[l], out = s.nf[l + 1];
+    const long long most = 2LL * s.sms;
+    if (step_tiles(s.rows, out, 128, 128) > most || step_tiles(out, in, 128, 128) > most ||
+        ((l > 0 || s.input_grad) && step_tiles(s.rows, in, 128, 128) > most))
+      short_gemms = false;
+  }
+  if (short_gemms) return true;
+  const double most = s.prec == STEP_BF16 ? 35e9 : s.prec == STEP_X3 ? 110e9 : 21e9;
+  return step_flops(s) <= most * 3 * s.layers && 4.0 * 2 * s.layers + step_flops_us(s) <= 2 * LAUNCH_US;
+}
+
 }  // namespace b2

@@ -264,7 +264,7 @@ BF16, TF32, X3 = 0, 1, 2
 
 def step_choice(host, nf, rows, prec, sms=148, input_grad=True):
     host.b2h_step_choice.restype = C.c_double
-    out = (C.c_int * 1)()
+    out = (C.c_int * 2)()
     us = host.b2h_step_choice((C.c_int * len(nf))(*nf), len(nf) - 1, rows, prec, sms, int(input_grad), out)
     return us, list(out)
 
@@ -277,7 +277,23 @@ def step_choice(host, nf, rows, prec, sms=148, input_grad=True):
 def test_steps_per_launch(host, nf, rows, prec, us):
     """Launches of the step kernel (csrc/step_choice.h) of about 2 ms, 4 at most, where a step is shorter than that: long
     sums over the batch and many weights count, not only the flops."""
-    est, (steps,) = step_choice(host, nf, rows, prec)
+    est, (steps, _) = step_choice(host, nf, rows, prec)
     assert 0.6 <= us / est <= 1.7
     assert 1 <= steps <= 64 and (steps == 1 or steps * us <= 4000)
     assert steps == 64 or (steps + 1) * est > 2000
+
+
+# networks measured on both paths, faster (or no slower) as whole steps, and slower
+STEPS = [([2048] * 17, 2048, X3), ([2048] * 21, 2048, X3), ([2048] * 50, 2048, TF32), ([2048] * 50, 2048, X3), ([512] * 21, 2048, TF32),
+         ([800] * 5, 8192, BF16), ([3072] * 5, 1300, BF16), ([2048] * 4, 8192, X3), ([64] * 5, 200000, X3),
+         ([64] * 5 + [4096, 4096] + [64] * 5, 8192, BF16), ([512] * 13 + [4096, 4096] + [512] * 12, 4096, TF32)]
+NO_STEPS = [([3072] * 5, 3072, BF16), ([4096] * 9, 8192, BF16), ([4096] * 9, 1024, TF32), ([3072] * 5, 1300, TF32), ([8192] * 3, 2048, BF16),
+            ([4096] * 9, 8192, X3)]
+
+
+@pytest.mark.parametrize("nets,want", [(STEPS, 1), (NO_STEPS, 0)], ids=["steps", "no-steps"])
+def test_networks_of_the_step_kernel(host, nets, want):
+    """The rule by which whole steps become one launch (csrc/step_choice.h), on networks measured on both paths: GEMMs of
+    at most two rounds of tiles in any number, larger ones by their average."""
+    for nf, rows, prec in nets:
+        assert step_choice(host, nf, rows, prec)[1][1] == want, (nf, rows, prec)
