@@ -56,6 +56,23 @@ inline int steps_per_launch(const StepShape& s) {
   return n < 1 ? 1 : n > 64 ? 64 : (int)n;
 }
 
+// What the long sums of the chain leave idle: the terms of a sum times the share of SMs without a tile (128 x 64), over the
+// forward and input-gradient GEMMs in the mean.
+inline double step_idle_terms(const StepShape& s) {
+  double idle = 0;
+  int n = 0;
+  auto gemm = [&](int cols, int sum) {
+    const double share = 1.0 - (double)step_tiles(s.rows, cols, 128, 64) / s.sms;
+    if (share > 0) idle += sum * share;
+    ++n;
+  };
+  for (int l = 0; l < s.layers; ++l) {
+    gemm(s.nf[l + 1], s.nf[l]);
+    if (l > 0 || s.input_grad) gemm(s.nf[l], s.nf[l + 1]);
+  }
+  return n > 0 ? idle / n : 0;
+}
+
 // Whether steps run as one launch. Always where every GEMM is at most two rounds of 128 x 128 tiles over the SMs, however many
 // layers there are (us per step, one launch per GEMM -> one for the step, fp32-class, 2048 wide, batch 2048: 16 layers 3853 ->
 // 3154, 20 layers 4809 -> 3967). With larger GEMMs among them up to the size of an average GEMM from which on the larger
@@ -67,6 +84,12 @@ inline int steps_per_launch(const StepShape& s) {
 // 8192) 2753 -> 2427, 103 2793 -> 2423. One wide layer among narrow ones follows the average too: a 4096 x 4096 layer among
 // ten of 64, batch 8192, bf16 1064 -> 892, among seven of 1024, batch 4096, 758 -> 701; an 8192 x 8192 layer among twenty of 256,
 // batch 2048, 1218 -> 1179, tf32 1919 -> 1927; 4096 x 4096 among 24 of 512, batch 4096, tf32 2126 -> 1474.
+// Not where few tiles with long sums hold up the chain of layers (step_idle_terms): an SM that walks one takes its share of
+// the weight gradients only afterwards, while separate launches let them fill the other SMs. By idle terms: bf16 6300 (1024-
+// 16000-1024, batch 256) 273 -> 264, 7100 (batch 128) 252 -> 264, 9400 (2048-24000-2048, batch 128) 565 -> 606, 17800 (1024-
+// 40000-1024, batch 128) 559 -> 653; tf32 5400 (1024-16000-1024, batch 300) 406 -> 388, 7100 371 -> 365, 9400 695 -> 770, 17800
+// 895 -> 896; fp32-class 550 (4096, batch 256) 434 -> 397, 1100 (3072, batch 256) 298 -> 279, 2100 (batch 128) 265 -> 279, 2300
+// (4096, batch 128) 375 -> 395, 3500 (1024-8000-1024, batch 128) 323 -> 342, 17800 1509 -> 1664.
 inline bool step_serves(const StepShape& s) {
   bool short_gemms = true;
   for (int l = 0; l < s.layers; ++l) {
@@ -78,6 +101,7 @@ inline bool step_serves(const StepShape& s) {
   }
   if (short_gemms) return true;
   const double most = s.prec == STEP_BF16 ? 35e9 : s.prec == STEP_X3 ? 110e9 : 21e9;
+  if (step_idle_terms(s) > (s.prec == STEP_X3 ? 2000 : 7000)) return false;
   return step_flops(s) <= most * 3 * s.layers && 4.0 * 2 * s.layers + step_flops_us(s) <= 2 * LAUNCH_US;
 }
 
