@@ -83,7 +83,11 @@ inline double step_idle_terms(const StepShape& s) {
 // but 25 (3072, batch 1300) 404 -> 439, 34 (2560, batch 2560) 501 -> 527; fp32-class 34 (2560) 1376 -> 1200, 69 (2048, batch
 // 8192) 2753 -> 2427, 103 2793 -> 2423. One wide layer among narrow ones follows the average too: a 4096 x 4096 layer among
 // ten of 64, batch 8192, bf16 1064 -> 892, among seven of 1024, batch 4096, 758 -> 701; an 8192 x 8192 layer among twenty of 256,
-// batch 2048, 1218 -> 1179, tf32 1919 -> 1927; 4096 x 4096 among 24 of 512, batch 4096, tf32 2126 -> 1474.
+// batch 2048, 1218 -> 1179, tf32 1919 -> 1927; 4096 x 4096 among 24 of 512, batch 4096, tf32 2126 -> 1474. In bf16 the line is
+// lower for layers that are not whole 128-byte columns, whose operands come in more boxes: 13 (900, batch 8000) 411 -> 337, 17
+// (2040, batch 2040) 309 -> 302, but 23 (1700, batch 4000) 403 -> 431, 31 (2500, batch 2500) 386 -> 405, 30 (5000, batch 600) 550
+// -> 591, and two layers of 9000 among four of 256, batch 1000, 823 -> 917; tf32 17 (2040) 421 -> 390, fp32-class 31 (2500) 1738
+// -> 1581.
 // Not where few tiles with long sums hold up the chain of layers (step_idle_terms): an SM that walks one takes its share of
 // the weight gradients only afterwards, while separate launches let them fill the other SMs. By idle terms: bf16 6300 (1024-
 // 16000-1024, batch 256) 273 -> 264, 7100 (batch 128) 252 -> 264, 9400 (2048-24000-2048, batch 128) 565 -> 606, 17800 (1024-
@@ -100,9 +104,14 @@ inline bool step_serves(const StepShape& s) {
       short_gemms = false;
   }
   if (short_gemms) return true;
-  const double most = s.prec == STEP_BF16 ? 35e9 : s.prec == STEP_X3 ? 110e9 : 21e9;
+  double size = 0;  // of an average GEMM, 1 at the line
+  for (int l = 0; l < s.layers; ++l) {
+    const bool columns = s.nf[l] % 64 == 0 && s.nf[l + 1] % 64 == 0;
+    const double most = s.prec == STEP_BF16 ? (columns ? 35e9 : 18e9) : s.prec == STEP_X3 ? 110e9 : 21e9;
+    size += 2.0 * s.rows * s.nf[l] * s.nf[l + 1] / most / s.layers;
+  }
   if (step_idle_terms(s) > (s.prec == STEP_X3 ? 2000 : 7000)) return false;
-  return step_flops(s) <= most * 3 * s.layers && 4.0 * 2 * s.layers + step_flops_us(s) <= 2 * LAUNCH_US;
+  return size <= 1.0 && 4.0 * 2 * s.layers + step_flops_us(s) <= 2 * LAUNCH_US;
 }
 
 }  // namespace b2

@@ -286,17 +286,20 @@ def test_steps_per_launch(host, nf, rows, prec, us):
 # networks measured on both paths, faster (or no slower) as whole steps, and slower
 STEPS = [([2048] * 17, 2048, X3), ([2048] * 21, 2048, X3), ([2048] * 50, 2048, TF32), ([2048] * 50, 2048, X3), ([512] * 21, 2048, TF32),
          ([800] * 5, 8192, BF16), ([3072] * 5, 1300, BF16), ([2048] * 4, 8192, X3), ([64] * 5, 200000, X3),
+         ([900] * 5, 8000, BF16), ([2040] * 5, 2040, BF16), ([2500] * 4, 2500, X3), ([256] * 2 + [4008] * 2 + [256] * 2, 1500, BF16),
          ([1024, 16000, 1024], 256, BF16), ([8192] * 3, 64, BF16), ([4096] * 3, 128, TF32), ([1024, 8000, 1024], 128, TF32),
          ([4096] * 3, 256, X3), ([2048] * 3, 64, X3), ([256, 16000, 256], 128, BF16), ([20000, 512, 512, 512], 512, TF32),
          ([64] * 5 + [4096, 4096] + [64] * 5, 8192, BF16), ([512] * 13 + [4096, 4096] + [512] * 12, 4096, TF32)]
 NO_STEPS = [([3072] * 5, 3072, BF16), ([4096] * 9, 8192, BF16), ([4096] * 9, 1024, TF32), ([3072] * 5, 1300, TF32), ([8192] * 3, 2048, BF16),
             ([4096] * 9, 8192, X3), ([1024, 40000, 1024], 128, BF16), ([1024, 16000, 1024], 128, BF16), ([2048, 24000, 2048], 128, TF32),
-            ([1024, 40000, 1024], 256, X3), ([4096] * 3, 128, X3), ([3072] * 7, 128, X3), ([1024, 6000, 1024], 256, X3)]
+            ([1024, 40000, 1024], 256, X3), ([4096] * 3, 128, X3), ([3072] * 7, 128, X3), ([1024, 6000, 1024], 256, X3),
+            ([1700] * 5, 4000, BF16), ([2500] * 4, 2500, BF16), ([3000] * 4, 1300, BF16), ([5000] * 4, 600, BF16),
+            ([256] * 3 + [9000] * 2 + [256] * 2, 1000, BF16), ([256] * 2 + [6008] * 2 + [256] * 2, 1500, BF16)]
 
 
 @pytest.mark.parametrize("nets,want", [(STEPS, 1), (NO_STEPS, 0)], ids=["steps", "no-steps"])
 def test_networks_of_the_step_kernel(host, nets, want):
     """The rule by which whole steps become one launch (csrc/step_choice.h), on networks measured on both paths: GEMMs of
-    at most two rounds of tiles in any number, larger ones by their average unless long sums hold up the chain of layers."""
+    at most two rounds of tiles in any number, larger ones by their average (bf16: and their widths) unless long sums hold up the chain of layers."""
     for nf, rows, prec in nets:
         assert step_choice(host, nf, rows, prec)[1][1] == want, (nf, rows, prec)
