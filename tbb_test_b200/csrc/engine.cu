@@ -574,20 +574,10 @@ int build_step_plans(b2_handle* h) {
       if (!s->plan && !narrow) return B2_OK;
     }
   }
-  // CTA pairs (256 x 128 tiles, two thirds of the operand traffic) once the layers are as many 128 x 128 tiles as fill the
-  // SMs, a little earlier where operands are 32 bits wide; below that a step waits for latency, and smaller tiles on more
-  // SMs are shorter. us per step, one CTA per tile -> pairs, by tiles of an average layer: 256 tiles (6 x 512, batch
-  // 8192) bf16 219 -> 171, tf32 411 -> 285; 256 (4 x 2048, batch 2048) bf16 222 -> 212, fp32-class 886 -> 804; 192 (6 x 1024,
-  // batch 3000) bf16 175 -> 156; 144 (4 x 1536, batch 1536) bf16 125 -> 129, tf32 195 -> 186; 128 (4 x 2048, batch 1024)
-  // bf16 156 -> 159, tf32 240 -> 222; 76 (3072-1024-2048-512, batch 700) tf32 119 -> 121; 64 (5 x 1024, batch 1024)
-  // bf16 90 -> 95, fp32-class 233 -> 268.
-  long long chain = 0, width = 0;
-  for (int l = 0; l < L; ++l) {
-    chain += tiles(h->fwd[l].d, 128) + tiles(h->dgrad[l].d, 128);
-    width += h->nf[l];
-  }
+  long long width = 0;
+  for (int l = 0; l < L; ++l) width += h->nf[l];
   const char* pe = getenv("B2_STEP_PAIR");  // experiments: 0 never, 1 whatever the size
-  const bool pair = pe ? pe[0] == '1' : chain > 2LL * L * h->sms * (h->op_type == T_BF16 ? 3 : 2) / 3;
+  const bool pair = pe ? pe[0] == '1' : step_pairs(shape);
   for (int slot = 0; slot < 2; ++slot) {
     StepSpec spec;
     spec.pair = pair;

@@ -114,4 +114,37 @@ inline bool step_serves(const StepShape& s) {
   return size <= 1.0 && 4.0 * 2 * s.layers + step_flops_us(s) <= 2 * LAUNCH_US;
 }
 
+// Whether the steps run on CTA pairs (256 x 128 tiles: a pair fetches 384 rows of operands where two 128 x 128 tiles fetch 512).
+// Forward and input-gradient GEMMs of as many 128 x 128 tiles as fill the SMs, a little earlier where operands are 32 bits
+// wide, gain by their flops; those of less than 48 tiles wait for latency, and smaller tiles on more SMs are shorter.
+// us per step, one CTA per tile -> pairs, by tiles of a GEMM: 256 tiles (6 x 512, batch 8192) bf16 219 -> 171, tf32 411 -> 285;
+// 256 (4 x 2048, batch 2048) bf16 222 -> 212, fp32-class 886 -> 804; 192 (6 x 1024, batch 3000) bf16 175 -> 156; 144 (4 x 1536,
+// batch 1536) bf16 125 -> 129, tf32 195 -> 186; 128 (4 x 2048, batch 1024) bf16 156 -> 159, tf32 240 -> 222; 64 (5 x 1024, batch
+// 1024) bf16 90 -> 95, fp32-class 233 -> 268. Mixed: 256 and 64 (2048-512-2048-512-2048, batch 2048) bf16 112 -> 105, tf32 173
+// -> 151; 192 and 24 (2048-256-..., batch 1500) bf16 93 -> 104, tf32 141 -> 149, fp32-class 261 -> 277; 384 among 20 of 24
+// (4096 x 4096 among layers of 256, batch 1500) bf16 288 -> 299, tf32 496 -> 484, fp32-class 1026 -> 988; 8192 x 8192 among
+// layers of 64, batch 700, tf32 929 -> 840.
+// Not where an odd number of row blocks, whose last pair is half empty, costs the chain a round over the SMs more: 12800 wide, batch
+// 128, fp32-class 2402 -> 3052; 5000, batch 300, tf32 557 -> 617; 6144, batch 384, fp32-class 893 -> 1029 (bf16 loses without one
+// at three blocks: 6400, batch 384 460 -> 486; five and more do not show: 4096, batch 640 331 -> 330).
+inline bool step_pairs(const StepShape& s) {
+  const int p = s.prec, blocks = (s.rows + 127) / 128;
+  const double gain[3] = {0.075, 0.45, 0.6}, cost[3] = {1.0, 1.0, 1.5};  // us per GFLOP, us per GEMM
+  if (s.sms < 2 || (p == STEP_BF16 && blocks == 3)) return false;
+  const int fill = p == STEP_BF16 ? s.sms : s.sms * 2 / 3;
+  double score = 0, single = 0, paired = 0;
+  auto gemm = [&](int cols, int sum) {
+    const long long tiles = step_tiles(s.rows, cols, 128, 128), pairs = step_tiles(s.rows, cols, 256, 128);
+    if (tiles > fill) score += 2e-9 * s.rows * cols * sum * gain[p];
+    else if (tiles < 48) score -= cost[p];
+    single += (double)sum * ((tiles + s.sms - 1) / s.sms);
+    paired += (double)sum * ((pairs + s.sms / 2 - 1) / (s.sms / 2));
+  };
+  for (int l = 0; l < s.layers; ++l) {
+    gemm(s.nf[l + 1], s.nf[l]);
+    if (l > 0 || s.input_grad) gemm(s.nf[l], s.nf[l + 1]);
+  }
+  return score > 0 && paired <= single;
+}
+
 }  // namespace b2

@@ -126,11 +126,12 @@ void b2h_choose_tile(int m, int n, int sms, int x3, int pair_ok, int shared, int
 int b2h_pieces_of_32(int left, int per) { return b2::pieces_of_32(left, per); }
 
 // Rules of the step kernel (csrc/step_choice.h) for one network: estimated us per step; steps per launch,
-// and whether whole steps run as one launch.
-double b2h_step_choice(const int* nf, int layers, int rows, int prec, int sms, int input_grad, int* out2) {
+// whether whole steps run as one launch, and whether on CTA pairs.
+double b2h_step_choice(const int* nf, int layers, int rows, int prec, int sms, int input_grad, int* out3) {
   const b2::StepShape s{nf, layers, rows, static_cast<b2::StepPrec>(prec), sms, input_grad != 0};
-  out2[0] = b2::steps_per_launch(s);
-  out2[1] = b2::step_serves(s);
+  out3[0] = b2::steps_per_launch(s);
+  out3[1] = b2::step_serves(s);
+  out3[2] = b2::step_pairs(s);
   return b2::step_us(s);
 }
 

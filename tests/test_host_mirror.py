@@ -264,7 +264,7 @@ BF16, TF32, X3 = 0, 1, 2
 
 def step_choice(host, nf, rows, prec, sms=148, input_grad=True):
     host.b2h_step_choice.restype = C.c_double
-    out = (C.c_int * 2)()
+    out = (C.c_int * 3)()
     us = host.b2h_step_choice((C.c_int * len(nf))(*nf), len(nf) - 1, rows, prec, sms, int(input_grad), out)
     return us, list(out)
 
@@ -277,7 +277,7 @@ def step_choice(host, nf, rows, prec, sms=148, input_grad=True):
 def test_steps_per_launch(host, nf, rows, prec, us):
     """Launches of the step kernel (csrc/step_choice.h) of about 2 ms, 4 at most, where a step is shorter than that: long
     sums over the batch and many weights count, not only the flops."""
-    est, (steps, _) = step_choice(host, nf, rows, prec)
+    est, (steps, _, _) = step_choice(host, nf, rows, prec)
     assert 0.6 <= us / est <= 1.7
     assert 1 <= steps <= 64 and (steps == 1 or steps * us <= 4000)
     assert steps == 64 or (steps + 1) * est > 2000
@@ -303,3 +303,23 @@ def test_networks_of_the_step_kernel(host, nets, want):
     at most two rounds of tiles in any number, larger ones by their average (bf16: and their widths) unless long sums hold up the chain of layers."""
     for nf, rows, prec in nets:
         assert step_choice(host, nf, rows, prec)[1][1] == want, (nf, rows, prec)
+
+
+# networks measured in both forms of the step kernel: faster as pairs of CTAs, and as one CTA per tile
+PAIRS = [([512] * 7, 8192, BF16), ([512] * 7, 8192, TF32), ([2048] * 5, 2048, X3), ([1024] * 7, 3000, BF16), ([1536] * 5, 1536, TF32),
+         ([2048] * 5, 1024, TF32), ([2048, 512, 2048, 512, 2048], 2048, BF16), ([2304] * 5, 1152, TF32), ([4352] * 3, 384, X3),
+         ([256] * 3 + [4096] * 2 + [256] * 2, 700, X3), ([64] * 8 + [8192] * 2 + [64] * 8, 700, TF32), ([1024, 384] * 4, 4000, X3),
+         ([256] * 5 + [9000] * 2 + [256] * 5, 700, TF32), ([8192] * 3, 384, X3)]
+SINGLE = [([1024] * 6, 1024, BF16), ([1024] * 6, 1024, X3), ([512] * 21, 2048, BF16), ([1536] * 5, 1536, BF16), ([2048] * 5, 1024, BF16),
+          ([12800] * 3, 128, X3), ([6144] * 3, 384, X3), ([5000] * 4, 300, TF32), ([6400] * 3, 384, BF16), ([2048, 256] * 3, 1500, TF32),
+          ([2048, 256] * 3, 1500, X3), ([128] * 9 + [2560] * 2 + [128] * 9, 2560, TF32), ([256] * 5 + [4096] * 2 + [256] * 5, 1500, BF16),
+          ([8000, 64, 8000], 500, X3), ([64, 64], 1, X3)]
+
+
+@pytest.mark.parametrize("nets,want", [(PAIRS, 1), (SINGLE, 0)], ids=["pairs", "single"])
+def test_form_of_the_step_kernel(host, nets, want):
+    """The rule between the step kernel's two forms (csrc/step_choice.h), on networks measured in both: pairs where they
+    fill the SMs, not where half-empty pairs of an odd number of row blocks cost a round, nor for a GPU of one SM."""
+    for nf, rows, prec in nets:
+        assert step_choice(host, nf, rows, prec)[1][2] == want, (nf, rows, prec)
+        assert step_choice(host, nf, rows, prec, sms=1)[1][2] == 0
