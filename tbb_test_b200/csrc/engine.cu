@@ -31,6 +31,7 @@
 
 #include "../../include/b200mlp.h"
 #include "bucket_plan.h"
+#include "download_plan.h"
 #include "step_choice.h"
 #include "common.cuh"
 #include "nccl_dyn.h"
@@ -123,10 +124,8 @@ struct b2_handle {
   float* y = nullptr;
   float* target = nullptr;
   void* dinput = nullptr;
-  // Page-locked buffers of download_rows, two per worker, made at the first large download
-  char* dl_buf = nullptr;
-  size_t dl_bytes = 0;
-  cudaEvent_t dl_ev[12] = {};
+  DownloadBuffers dl;  // page-locked buffers of download_rows, made at the first large download
+  cudaEvent_t dl_ev[DL_WORKERS] = {};
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
   // Per input slot: the loss accumulator (double) and, 16 bytes behind it, the tile counters of the step
@@ -330,39 +329,31 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
 // Device rows to host memory, done when it returns. A copy to pageable memory runs at the speed of one
 // thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
 // destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
-// buffers of their own share that work. A chunk costs about 8 us whatever its size, starting a thread 10 us, and a MB of
-// page-locked memory 1.1 ms, once. So a few MB get six threads with two buffers of 128 KB each; from 12 MB on twelve
-// threads share the same 1.5 MB, one buffer each (2048 x 2048 to fresh memory 1901 -> 1491 us); and from 32 MB on buffers of
-// 512 KB pay for themselves within the first matrices (4096 x 4096 4395 -> 3116 us, 8192 x 8192 25298 -> 13700 us; with 24 MB
-// of buffers 2253 and 12421, but 25 ms for the buffers).
-constexpr size_t DL_CHUNK = 128 << 10, DL_LARGE_CHUNK = 512 << 10;
-constexpr size_t DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20, DL_LARGE_BYTES = 32 << 20;
-constexpr int DL_WORKERS = 12;
+// buffers of their own share that work (how many, and in what chunks: download_plan.h).
 int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
   const size_t width = (size_t)cols * 4, total = width * rows;
   cudaPointerAttributes attr;
   bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
-  const bool many = total >= DL_MANY_BYTES;
-  const int workers = many ? DL_WORKERS : DL_WORKERS / 2, bufs = many ? 1 : 2;  // threads, buffers of each
-  const size_t chunk = total >= DL_LARGE_BYTES ? DL_LARGE_CHUNK : DL_CHUNK;
-  bool shared = pageable && width <= chunk && total >= DL_MIN_BYTES;
-  if (shared && h->dl_bytes < DL_WORKERS * chunk) {
-    if (h->dl_buf) cudaFreeHost(h->dl_buf);
-    h->dl_buf = nullptr;
-    h->dl_bytes = DL_WORKERS * chunk;
-    bool ok = cudaHostAlloc((void**)&h->dl_buf, h->dl_bytes, cudaHostAllocDefault) == cudaSuccess;
-    if (!ok) h->dl_buf = nullptr;
-    for (int i = 0; ok && i < DL_WORKERS; ++i)
-      ok = h->dl_ev[i] || cudaEventCreateWithFlags(&h->dl_ev[i], cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) {  // no page-locked memory left: the plain copy
-      if (h->dl_buf) cudaFreeHost(h->dl_buf);
-      h->dl_buf = nullptr;
-      h->dl_bytes = 0;
+  DownloadPlan plan{};
+  if (pageable && total >= DL_MIN_BYTES) {
+    auto alloc = [](size_t bytes) {
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) p = nullptr;
       cudaGetLastError();
-    }
+      return static_cast<char*>(p);
+    };
+    cpu_set_t cpus;  // those this process may run on, which need not be all of the machine's
+    const int cores = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : (int)std::thread::hardware_concurrency();
+    plan = ready_download(width, (size_t)rows, cores, h->dl, alloc, [](char* p) { cudaFreeHost(p); });
+    for (cudaEvent_t& ev : h->dl_ev)
+      if (plan.threads > 0 && !ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+        ev = nullptr;
+        plan.threads = 0;
+        cudaGetLastError();
+      }
   }
-  if (!shared || !h->dl_buf) {
+  if (plan.threads == 0) {
     // Pages of fresh memory in one call instead of a fault each (1 MB 443 -> 350 us); it changes nothing but that they
     // are there, and where the kernel does not know the request the copy takes the faults.
     if (pageable && ld == (size_t)cols) {
@@ -374,6 +365,8 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
     CK(h, cudaStreamSynchronize(h->s_main));
     return B2_OK;
   }
+  const int bufs = plan.bufs;
+  const size_t chunk = plan.chunk;
   const int per = (int)(chunk / width), chunks = (rows + per - 1) / per;
   std::atomic<int> next{0}, error{(int)cudaSuccess};
   auto work = [&](int t) {
@@ -383,7 +376,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       if (in_flight[b] < 0) return;
       if (e == cudaSuccess) e = cudaEventSynchronize(h->dl_ev[bufs * t + b]);
       if (e == cudaSuccess) {
-        const char* src = h->dl_buf + (size_t)(bufs * t + b) * chunk;
+        const char* src = h->dl.at + (size_t)(bufs * t + b) * chunk;
         const int r0 = in_flight[b] * per, n = std::min(per, rows - r0);
         for (int r = 0; r < n; ++r) memcpy(host + (size_t)(r0 + r) * ld, src + width * r, width);
       }
@@ -393,7 +386,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       const int c = next.fetch_add(1);
       if (c >= chunks) break;
       const int r0 = c * per, n = std::min(per, rows - r0);
-      e = copy_rows(h->dl_buf + (size_t)(bufs * t + b) * chunk, width,
+      e = copy_rows(h->dl.at + (size_t)(bufs * t + b) * chunk, width,
                     static_cast<const char*>(dev) + (size_t)r0 * pitch * 4, pitch * 4, width, (size_t)n,
                     cudaMemcpyDeviceToHost, h->s_main);
       if (e == cudaSuccess) e = cudaEventRecord(h->dl_ev[bufs * t + b], h->s_main);
@@ -405,8 +398,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
     if (e != cudaSuccess) error.store((int)e);
   };
   std::thread pool[DL_WORKERS];
-  int helpers = std::min(std::min(workers, (int)std::thread::hardware_concurrency()), chunks) - 1;
-  for (int i = 0; i < helpers; ++i) {
+  for (int i = 0; i + 1 < plan.threads; ++i) {
     try {
       pool[i] = std::thread(work, i + 1);
     } catch (const std::exception&) {  // no more threads, or no memory for one: those that run take all chunks
@@ -1046,7 +1038,7 @@ void free_all(b2_handle* h) {
   cudaFree(h->target);
   cudaFree(h->dinput);
   cudaFree(h->stage);
-  if (h->dl_buf) cudaFreeHost(h->dl_buf);
+  if (h->dl.at) cudaFreeHost(h->dl.at);
   for (cudaEvent_t ev : h->dl_ev)
     if (ev) cudaEventDestroy(ev);
   cudaFree(h->sync_dev);

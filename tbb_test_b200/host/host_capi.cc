@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../csrc/bucket_plan.h"
+#include "../csrc/download_plan.h"
 #include "../csrc/row_pieces.h"
 #include "../csrc/step_choice.h"
 #include "../csrc/tile_choice.h"
@@ -133,6 +134,31 @@ double b2h_step_choice(const int* nf, int layers, int rows, int prec, int sms, i
   out3[1] = b2::step_serves(s);
   out3[2] = b2::step_pairs(s);
   return b2::step_us(s);
+}
+
+// One handle's downloads one after the other (csrc/download_plan.h), with `memory` bytes of page-locked memory to be had at
+// once: threads, buffers of each, KB of a chunk, KB held and allocations asked for, per download.
+void b2h_downloads(int n, const size_t* width, const size_t* rows, int cores, size_t memory, int* out5) {
+  b2::DownloadBuffers b;
+  std::vector<std::vector<char>> held;
+  for (int i = 0; i < n; ++i) {
+    int asked = 0;
+    auto alloc = [&](size_t bytes) -> char* {
+      ++asked;
+      size_t used = 0;
+      for (const auto& v : held) used += v.size();
+      if (used + bytes > memory) return nullptr;
+      held.emplace_back(bytes);
+      return held.back().data();
+    };
+    auto release = [&](char* p) {
+      for (auto it = held.begin(); it != held.end(); ++it)
+        if (it->data() == p) { held.erase(it); return; }
+    };
+    const b2::DownloadPlan p = b2::ready_download(width[i], rows[i], cores, b, alloc, release);
+    int* o = out5 + 5 * i;
+    o[0] = p.threads; o[1] = p.bufs; o[2] = (int)(p.chunk >> 10); o[3] = (int)(b.bytes >> 10); o[4] = asked;
+  }
 }
 
 void b2h_ring_info(int nsock, int sid, int task, int* out3) {

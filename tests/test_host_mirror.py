@@ -323,3 +323,26 @@ def test_form_of_the_step_kernel(host, nets, want):
     for nf, rows, prec in nets:
         assert step_choice(host, nf, rows, prec)[1][2] == want, (nf, rows, prec)
         assert step_choice(host, nf, rows, prec, sms=1)[1][2] == 0
+
+
+def downloads(host, shapes, cores=16, memory=1 << 30):
+    n = len(shapes)
+    sizes = [(C.c_size_t * n)(*(s[i] * (4 if i else 1) for s in shapes)) for i in (1, 0)]
+    out = (C.c_int * (5 * n))()
+    host.b2h_downloads.argtypes = [C.c_int, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t), C.c_int, C.c_size_t, C.POINTER(C.c_int)]
+    host.b2h_downloads(n, sizes[0], sizes[1], cores, memory, out)
+    return [tuple(out[5 * i:5 * i + 5]) for i in range(n)]
+
+
+def test_threads_and_buffers_of_a_download(host):
+    """Two buffers for each thread wherever few run, be it for the size or for want of cores, one for each of twelve; never
+    more buffers than there are, nor threads than cores or chunks; small matrices and rows longer than a chunk as one plain copy."""
+    for rows, cols in ((724, 724), (1024, 1024), (1800, 1700), (2048, 2048), (4096, 4096), (25, 32768), (100, 32768), (8, 1 << 20)):
+        for cores in (0, 1, 2, 4, 6, 7, 12, 64):
+            (threads, bufs, kb, _, _), = downloads(host, [(rows, cols)], cores)
+            if rows * cols * 4 < 2 << 20 or cols * 4 > kb << 10:
+                assert threads == 0
+                continue
+            chunks = -(-rows // ((kb << 10) // (cols * 4)))
+            assert threads == max(1, min(12 if rows * cols * 4 >= 12 << 20 and cores >= 12 else 6, cores, chunks))
+            assert bufs == (2 if threads <= 6 else 1) and threads * bufs <= 12
