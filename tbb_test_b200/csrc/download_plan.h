@@ -8,11 +8,14 @@ namespace b2 {
 constexpr int DL_WORKERS = 12;  // threads at most, and buffers
 constexpr size_t DL_CHUNK = 128 << 10, DL_LARGE_CHUNK = 512 << 10;
 constexpr size_t DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20, DL_LARGE_BYTES = 32 << 20;
+constexpr size_t DL_LARGE_AFTER = (size_t)256 << 20;
 
 // Page-locked buffers of a handle, DL_WORKERS chunks.
 struct DownloadBuffers {
   char* at = nullptr;
   size_t bytes = 0;
+  size_t large_read = 0;  // bytes of the matrices of DL_LARGE_BYTES and more read so far
+  bool no_large = false;  // there was no memory for the larger chunks: not asked for again
 };
 
 struct DownloadPlan {
@@ -25,11 +28,12 @@ struct DownloadPlan {
 // each (one copied to while the other is emptied), and from 12 MB on twelve threads share the same 1.5 MB, one buffer each
 // (us per matrix into fresh memory: 3072 x 3072 3490 -> 3040, 4096 x 4096 6050 -> 5150). Fewer than twelve cores run a thread
 // each, six at most, with two buffers: 2048 x 2048 and 4096 x 4096 on eight cores 1110 and 6000, as eight threads with one
-// buffer each 1160 and 6400; on four 1080 and 7100 (twelve threads 1300 and 8300), on two 1250 and 9600 (2200 and 12400). Chunks of
-// 512 KB from 32 MB on are faster still (3040 -> 2250, 5150 -> 3850, 8192 x 8192 19000 -> 12800).
-inline DownloadPlan plan_download(size_t width, size_t rows, int cores) {
+// buffer each 1160 and 6400; on four 1080 and 7100 (twelve threads 1300 and 8300), on two 1250 and 9600 (2200 and 12400). Chunks of 512 KB from 32 MB on are faster still (3040 -> 2250, 5150 -> 3850, 8192 x 8192 19000 -> 12800), but
+// their 6 MB of page-locked memory take 3 to 9 ms to make and 1.3 to give back: what was gained over some 256 MB, and only a
+// handle that has read as much makes them.
+inline DownloadPlan plan_download(size_t width, size_t rows, int cores, const DownloadBuffers& b) {
   const size_t total = width * rows;
-  const bool large = total >= DL_LARGE_BYTES;
+  const bool large = total >= DL_LARGE_BYTES && b.large_read >= DL_LARGE_AFTER && !b.no_large;
   DownloadPlan p{0, 0, large ? DL_LARGE_CHUNK : DL_CHUNK};
   if (total < DL_MIN_BYTES || width > p.chunk) return p;
   const size_t per = p.chunk / width, chunks = (rows + per - 1) / per;
@@ -40,19 +44,30 @@ inline DownloadPlan plan_download(size_t width, size_t rows, int cores) {
   return p;
 }
 
-// The plan of a download with its buffers made: the plain copy without memory for them. `alloc(bytes)` returns null when
-// there is none.
+// The plan of a download with its buffers made: without memory for larger chunks the ones that are there serve, without
+// memory for any the plain copy. `alloc(bytes)` returns null when there is none.
 template <class Alloc, class Free>
 DownloadPlan ready_download(size_t width, size_t rows, int cores, DownloadBuffers& b, Alloc alloc, Free release) {
-  DownloadPlan p = plan_download(width, rows, cores);
-  const size_t need = DL_WORKERS * p.chunk;
-  if (p.threads > 0 && b.bytes < need) {
-    if (b.at) release(b.at);
-    b.at = alloc(need);
-    b.bytes = b.at ? need : 0;
-    if (!b.at) p.threads = 0;
+  for (;;) {
+    DownloadPlan p = plan_download(width, rows, cores, b);
+    const size_t need = DL_WORKERS * p.chunk;
+    if (p.threads > 0 && b.bytes < need) {
+      char* fresh = alloc(need);
+      if (!fresh && p.chunk == DL_LARGE_CHUNK) {
+        b.no_large = true;
+        continue;
+      }
+      if (fresh) {
+        if (b.at) release(b.at);
+        b.at = fresh;
+        b.bytes = need;
+      } else {
+        p.threads = 0;
+      }
+    }
+    if (width * rows >= DL_LARGE_BYTES && b.large_read < DL_LARGE_AFTER) b.large_read += width * rows;
+    return p;
   }
-  return p;
 }
 
 }  // namespace b2

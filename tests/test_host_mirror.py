@@ -346,3 +346,15 @@ def test_threads_and_buffers_of_a_download(host):
             chunks = -(-rows // ((kb << 10) // (cols * 4)))
             assert threads == max(1, min(12 if rows * cols * 4 >= 12 << 20 and cores >= 12 else 6, cores, chunks))
             assert bufs == (2 if threads <= 6 else 1) and threads * bufs <= 12
+
+
+def test_buffers_of_large_downloads(host):
+    """6 MB of page-locked memory only for a handle that has read 256 MB of large matrices, 1.5 MB until then. Where they cannot be
+    had, the 1.5 MB stay in use and are not asked for again; where none can be had, a plain copy."""
+    got = downloads(host, [(4096, 4096)] * 6 + [(1024, 1024)])
+    assert [g[2] for g in got] == [128] * 4 + [512, 512, 128]
+    assert [g[3] for g in got] == [1536] * 4 + [6144] * 3 and [g[4] for g in got] == [1, 0, 0, 0, 1, 0, 0]
+    got = downloads(host, [(4096, 4096)] * 7, memory=7 << 20)  # no room for both at once
+    assert [g[2] for g in got] == [128] * 7 and [g[3] for g in got] == [1536] * 7
+    assert [g[4] for g in got] == [1, 0, 0, 0, 1, 0, 0] and all(g[0] == 12 for g in got)
+    assert all(g[0] == 0 and g[3] == 0 for g in downloads(host, [(4096, 4096)] * 6, memory=1 << 20))
