@@ -76,8 +76,8 @@ __device__ __forceinline__ void fetch4(float (&f)[4][T], const uint8_t* slab, in
 // per term, as in gemm_simt_kernel. A warp owns WM x WN elements, its lanes a grid of WM/TM by WN/TN. Bound by latency
 // where the grid is small: the copies of two slabs are in flight while one is multiplied, no thread holds a slab in
 // registers (71 to 163 of them, against 222), and small tiles put many warps on an SM. us, forward / weight
-// gradient / input gradient, gemm_simt_kernel -> here: 300 x 300 x 2000 105/118/113 -> 51/51/53; 700 x 900 x 600
-// 51/55/53 -> 37/37/41; 200 x 123 x 701 33/39/34 -> 25/23/27; 1536 x 1000 x 777 113/95/115 -> 100/77/93.
+// gradient / input gradient, gemm_simt_kernel -> here: 300 x 300 x 2000 105/118/113 -> 51/51/53; 200 x 123 x 701 33/39/34 ->
+// 25/23/27.
 template <int BM, int BN, int TM, int TN, int WM, int WN, bool AK, bool BK>
 __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32) gemm_f32_kernel(GemmDesc g, int vec_a, int vec_b) {
   constexpr int NT = (BM / WM) * (BN / WN) * 32, LM = WM / TM, LN = WN / TN, STAGES = 3;
@@ -158,30 +158,21 @@ cudaError_t launch_f32_tile(const GemmDesc& g, int tile, int va, int vb, cudaStr
   return launch_f32<32, 32, 4, 4, 16, 32, AK, BK>(g, va, vb, stream);
 }
 
-
 bool whole_pieces(const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; }
 bool whole_a(const GemmDesc& g) { return whole_pieces(g.A, g.sAk == 1 ? g.sAm : g.sAk); }
 bool whole_b(const GemmDesc& g) { return whole_pieces(g.B, g.sBk == 1 ? g.sBn : g.sBk); }
 
-// Tiles and their rates, the first one gemm_simt_kernel's. Measured, us: 1024^3 as 64 x 64 72, 64 x 32 78, 32 x 32 84; 512 x 512 x
-// 2048 86, 60 and 55.
-constexpr SimtTile F32_TILES[4] = {{128, 128, 1.0}, {64, 64, 0.85}, {64, 32, 0.79}, {32, 32, 0.635}};
-
-// Tile of gemm_f32_kernel, or 0: grids that 32 x 32 tiles serve best, and any small grid with rows that are not whole
-// 16-byte pieces. Larger ones keep gemm_simt_kernel, which needs fewer instructions per FMA.
-int f32_tile(const GemmDesc& g) {
+int tile_of(const GemmDesc& g) {
   if (g.in_type != T_F32 || g.out_type != T_F32 || (g.sAk != 1 && g.sAm != 1) || (g.sBk != 1 && g.sBn != 1)) return 0;
-  const int tile = fastest_tile(F32_TILES, 4, g.M, g.N, 148);
-  if (tile == 3) return tile;
-  return !(whole_a(g) && whole_b(g)) && (long long)((g.M + 63) / 64) * ((g.N + 63) / 64) <= 148 ? tile : 0;
+  return f32_tile(g.M, g.N, whole_a(g) && whole_b(g), 148);
 }
 
 }  // namespace
 
-bool gemm_f32_serves(const GemmDesc& g) { return f32_tile(g) > 0; }
+bool gemm_f32_serves(const GemmDesc& g) { return tile_of(g) > 0; }
 
 cudaError_t gemm_f32_launch(const GemmDesc& g, cudaStream_t stream) {
-  const int tile = f32_tile(g), va = whole_a(g), vb = whole_b(g);
+  const int tile = tile_of(g), va = whole_a(g), vb = whole_b(g);
   if (g.sAk == 1 && g.sBk == 1) return launch_f32_tile<true, true>(g, tile, va, vb, stream);
   if (g.sAk == 1) return launch_f32_tile<true, false>(g, tile, va, vb, stream);
   if (g.sBk == 1) return launch_f32_tile<false, true>(g, tile, va, vb, stream);

@@ -8,6 +8,7 @@
 #include "../csrc/bucket_plan.h"
 #include "../csrc/download_plan.h"
 #include "../csrc/row_pieces.h"
+#include "../csrc/simt_tile.h"
 #include "../csrc/step_choice.h"
 #include "../csrc/tile_choice.h"
 #include "HyperCubeAllReduce.h"
@@ -160,6 +161,9 @@ void b2h_downloads(int n, const size_t* width, const size_t* rows, int cores, si
     o[0] = p.threads; o[1] = p.bufs; o[2] = (int)(p.chunk >> 10); o[3] = (int)(b.bytes >> 10); o[4] = asked;
   }
 }
+
+// Tile of the CUDA-core GEMM for small fp32 grids (csrc/simt_tile.h), 0 where the general kernel serves.
+int b2h_f32_tile(int m, int n, int whole_pieces) { return b2::f32_tile(m, n, whole_pieces != 0, 148); }
 
 void b2h_ring_info(int nsock, int sid, int task, int* out3) {
   nsockets = nsock;

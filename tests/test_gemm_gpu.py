@@ -198,19 +198,40 @@ def test_cuda_core_dispatch_edges(dev, oracle, form, shape):
                    ref * (aux > 0)) <= 2 * TOL["fp32"]
 
 
-# fp32 on the CUDA cores at small grids and with rows that are not whole 16-byte pieces: one and several slabs of 32 k with
-# remainders, tiles of every size with remainders, against sums in float64. Bound per element: K roundings of the sum of
-# magnitudes, 2^-24 each.
-@pytest.mark.parametrize("shape", [(33, 18, 1), (65, 33, 31), (64, 96, 32), (31, 100, 33), (300, 301, 95), (129, 257, 97), (640, 900, 64),
-                                   (1001, 1300, 70), (1537, 1003, 65)], ids=lambda s: "x".join(map(str, s)))
+# fp32 on the CUDA cores at small grids and with rows that are not whole 16-byte pieces: (m, n, k) and the tile it takes
+# (csrc/simt_tile.h: 1 64 x 64, 2 64 x 32, 3 32 x 32, 0 the general kernel) with such rows. One and several slabs of 32 k with
+# remainders, every tile with remainders.
+SMALL_GRIDS = {(33, 18, 1): 3, (65, 33, 31): 3, (64, 96, 32): 3, (31, 100, 33): 3, (300, 301, 95): 3, (129, 257, 97): 3, (500, 509, 97): 2,
+               (333, 701, 31): 2, (449, 639, 1): 1, (400, 603, 1): 2, (577, 577, 33): 1, (300, 1003, 65): 1, (701, 803, 129): 1, (640, 900, 64): 0,
+               (1001, 1300, 70): 0, (1537, 1003, 65): 0}
+
+
+@pytest.mark.parametrize("shape", list(SMALL_GRIDS), ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("form", list(FORMS))
-def test_fp32_small_grids(dev, oracle, form, shape):
+def test_fp32_small_grids(dev, native, oracle, form, shape):
+    """Against sums in float64, with ReLU, mask and beta. Bound per element: K roundings of the sum of magnitudes, 2^-24 each,
+    and two more for alpha and beta."""
+    import ctypes as C
+    import torch
     from tbb_test_b200 import _capi as K
     m, n, k = shape
     ta, tb, a, b = operands(oracle, form, m, n, k, 121)
-    c = dev.sgemm_host(K.PREC_FP32, ta, tb, a, b).astype(np.float64)
+    whole = a.shape[1] % 4 == 0 and b.shape[1] % 4 == 0
+    host = C.CDLL(native.HOST_LIB)
+    assert host.b2h_f32_tile(m, n, 0) == SMALL_GRIDS[shape]
+    assert host.b2h_f32_tile(m, n, int(whole)) == (0 if whole and SMALL_GRIDS[shape] < 3 else SMALL_GRIDS[shape])
     ra, rb = (a.T if ta else a).astype(np.float64), (b.T if tb else b).astype(np.float64)
-    assert (np.abs(c - ra @ rb) <= k * 2.0 ** -24 * (np.abs(ra) @ np.abs(rb)) + 1e-30).all()
+    ref, mag = ra @ rb, np.abs(ra) @ np.abs(rb)
+    near = lambda got, want, extra=0.0: (np.abs(got.astype(np.float64) - want) <= (k + 2) * 2.0 ** -24 * (mag + extra) + 1e-30).all()  # noqa: E731
+    assert near(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b), ref)
+    assert near(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_RELU), np.maximum(ref, 0))
+    aux = oracle.fill_uniform(m, n, 122, -1.0, 1.0)
+    assert near(dev.sgemm_host(K.PREC_FP32, ta, tb, a, b, epilogue=K.EPI_MASK, aux=aux), ref * (aux > 0))
+    ad, bd, cd = (torch.from_numpy(np.ascontiguousarray(t)).cuda() for t in (a, b, aux))
+    torch.cuda.synchronize()
+    assert dev.lib.b2_sgemm(dev._h, K.PREC_FP32, int(ta), int(tb), m, n, k, 2.0, ad.data_ptr(), a.shape[1], bd.data_ptr(), b.shape[1],
+                            -0.5, cd.data_ptr(), n) == K.OK and dev.lib.b2_sync(dev._h) == K.OK
+    assert near(cd.cpu().numpy(), 2.0 * ref - 0.5 * aux, mag + np.abs(aux))
 
 
 @pytest.mark.parametrize("form", list(FORMS))
