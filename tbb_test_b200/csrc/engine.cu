@@ -642,6 +642,8 @@ int build_step_plans(b2_handle* h) {
     }
   }
   h->launch_steps = steps_per_launch(shape);
+  if (getenv("B2_VERBOSE"))
+    fprintf(stderr, "b200mlp: rank %d: whole steps in one launch, %s\n", h->cfg.rank, pair ? "CTA pairs" : "a CTA per tile");
   return B2_OK;
 }
 

@@ -83,29 +83,36 @@ def test_step_kernel_matches_launch_per_gemm(native, oracle, monkeypatch, net, p
         assert abs(la - lb) <= 1e-5 * abs(la) and abs(la - lf) <= 1e-5 * abs(la)
 
 
-# One tile of a pair with its second CTA empty / a remainder in rows and columns of either CTA / both input slots,
-# bf16 gradients / several rounds of the grid / narrow last layers / more layers than the small table holds
-PAIR_NETS = [([96, 64], 40, {}), ([256, 132, 388, 260], 130, {}), ([123, 77, 201, 33], 333, {}),
+# One tile of a pair with its second CTA empty / a remainder in rows and columns of either CTA / ragged widths (rows that
+# start on 16-byte boundaries only) / both input slots, bf16 gradients / several rounds of the grid / narrow last layers / more
+# layers than the small table holds. Odd widths run in bf16 alone, on padded rows.
+PAIR_NETS = [([96, 64], 40, {}), ([256, 132, 388, 260], 130, {}), ([124, 76, 204, 36], 333, {}), ([123, 77, 201, 33], 333, {}),
              ([512, 384, 640, 128], 640, {"grad_bf16": True}), ([1024, 1536, 512], 3100, {}), ([64] * 24, 257, {"input_grad": False}),
-             ([160, 96, 10], 300, {}), ([256, 128, 1], 990, {"ref": True})]
+             ([160, 96, 12], 300, {}), ([160, 96, 10], 300, {}), ([256, 128, 4], 990, {"ref": True}), ([256, 128, 1], 990, {"ref": True})]
 
 
-@pytest.mark.parametrize("prec", ["bf16", "tf32", "fp32tc"])
-@pytest.mark.parametrize("net", PAIR_NETS, ids=lambda n: "x".join(map(str, n[0][:4])) + f"b{n[1]}" + "".join(n[2]))
-def test_pair_tiles_match_single_cta_tiles(native, oracle, monkeypatch, net, prec):
+@pytest.mark.parametrize("prec,net", [(p, n) for n in PAIR_NETS for p in ("bf16", "tf32", "fp32tc")
+                                      if p == "bf16" or all(w % 4 == 0 for w in n[0])],
+                         ids=lambda v: v if isinstance(v, str) else "x".join(map(str, v[0][:4])) + f"b{v[1]}" + "".join(v[2]))
+def test_pair_tiles_match_single_cta_tiles(native, oracle, monkeypatch, capfd, net, prec):
     """256 x 128 tiles of CTA pairs, and the tiles of one CTA, add every element's products in the same order: equal
-    bits, narrow last layers included."""
+    bits, narrow last layers included. Each form is the one that runs, in one launch for all steps."""
     from tbb_test_b200 import _capi as K
     nf, batch, opts = net
     P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32, "fp32tc": K.PREC_FP32_TC}[prec]
     monkeypatch.setenv("B2_STEP_KERNEL", "1")
+    monkeypatch.setenv("B2_VERBOSE", "1")
     for steps, fed in ((1, False), (3, False), (2, True)):
         got = []
-        for pair in ("0", "1"):
+        for pair, form in (("0", "a CTA per tile"), ("1", "CTA pairs")):
             monkeypatch.setenv("B2_STEP_PAIR", pair)
+            capfd.readouterr()
             got.append(states(oracle, K, nf, batch, P, steps, opts, fed=fed))
+            assert f"whole steps in one launch, {form}\n" in capfd.readouterr().err
         (a, la, na), (b, lb, nb) = got
-        assert na == nb and abs(la - lb) <= 1e-5 * abs(la)
+        # per host-fed step the launch, and the conversion of the input or its twin
+        assert na == nb == (steps * (1 if prec == "tf32" else 2) if fed else 1)
+        assert abs(la - lb) <= 1e-5 * abs(la)
         assert all(np.array_equal(a[k], b[k]) for k in a), (steps, fed)
 
 
@@ -123,15 +130,17 @@ def test_layers_of_many_tiles(native, oracle, monkeypatch, nf, batch, prec):
     assert all(np.array_equal(a[k], b[k]) for k in a)
 
 
+@pytest.mark.parametrize("pair", ["0", "1"], ids=["single", "pairs"])
 @pytest.mark.parametrize("prec", ["bf16", "tf32"])
-def test_two_handles_in_two_threads(native, oracle, prec):
+def test_two_handles_in_two_threads(native, oracle, monkeypatch, prec, pair):
     """Cooperative launches of two handles on one GPU, issued by two host threads at once, each keep their grid
-    resident: both finish with the weights they reach alone."""
+    resident, in either form (a pair is a cluster of two CTAs): both finish with the weights they reach alone."""
     import threading
     from tbb_test_b200 import _capi as K
     from tbb_test_b200.mlp import MLP
+    monkeypatch.setenv("B2_STEP_PAIR", pair)
     P = {"bf16": K.PREC_BF16, "tf32": K.PREC_TF32}[prec]
-    nf, batch, L = [512] * 5, 512, 4
+    nf, batch, L = [512] * 5, 512 if pair == "0" else 5000, 4  # 80 pair tiles a GEMM: the grid is full
 
     def make(seed):
         m = MLP(nf, batch, precision=P, lr=0.01)
