@@ -349,12 +349,13 @@ def test_threads_and_buffers_of_a_download(host):
 
 
 def test_buffers_of_large_downloads(host):
-    """6 MB of page-locked memory only for a handle that has read 256 MB of large matrices, 1.5 MB until then. Where they cannot be
+    """6 MB of page-locked memory only from the matrix on that makes it 256 MB of large ones for a handle, 1.5 MB until then. Where they cannot be
     had, the 1.5 MB stay in use and are not asked for again; where none can be had, a plain copy."""
     got = downloads(host, [(4096, 4096)] * 6 + [(1024, 1024)])
-    assert [g[2] for g in got] == [128] * 4 + [512, 512, 128]
-    assert [g[3] for g in got] == [1536] * 4 + [6144] * 3 and [g[4] for g in got] == [1, 0, 0, 0, 1, 0, 0]
+    assert [g[2] for g in got] == [128] * 3 + [512] * 3 + [128]
+    assert [g[3] for g in got] == [1536] * 3 + [6144] * 4 and [g[4] for g in got] == [1, 0, 0, 1, 0, 0, 0]
+    assert downloads(host, [(8192, 8192)])[0][2] == 512
     got = downloads(host, [(4096, 4096)] * 7, memory=7 << 20)  # no room for both at once
     assert [g[2] for g in got] == [128] * 7 and [g[3] for g in got] == [1536] * 7
-    assert [g[4] for g in got] == [1, 0, 0, 0, 1, 0, 0] and all(g[0] == 12 for g in got)
+    assert [g[4] for g in got] == [1, 0, 0, 1, 0, 0, 0] and all(g[0] == 12 for g in got)
     assert all(g[0] == 0 and g[3] == 0 for g in downloads(host, [(4096, 4096)] * 6, memory=1 << 20))
