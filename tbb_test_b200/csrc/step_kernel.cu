@@ -28,13 +28,14 @@
 // A and half of B) for networks whose layers fill the GPU.
 //
 // What bounds it: with a CTA per tile the latency of one layer after another. In-kernel stamps of a 1024 x 1024 layer at
-// batch 1024: 1.1 us from "dependency met" to the first operands, 2.5 us for 16 k-blocks, 1.2 us epilogue (weight
-// update 3.6 us, loss 3.3 us), 1.2 us until the stores are visible to the other SMs, 0.8 us until the next tile's
-// producer has seen the counter; in the backward pass, where two GEMMs per layer run, the L2 (11-13 TB/s into all
-// SMs). Pairs: L2 and shared memory. Nothing may spill to local memory here: the acquiring loads of the counters drop
-// the L1, and each reload is an L2 round trip (two spilling epilogue groups: 110 -> 135 us per step, without spills 97).
-// bf16, us per step, launch per GEMM -> here: 5 x 1024, batch 1024 170 -> 90; 20 x 512, batch 2048 589 -> 243;
-// 784-500-300-10, batch 1000 87 -> 48; 6 x 512, batch 8192 -> 166 (pairs).
+// batch 1024, taken before the 32-byte stores: 1.1 us from "dependency met" to the first operands, 2.5 us for 16 k-blocks,
+// 1.2 us epilogue (weight update 3.6 us, loss 3.3 us), 1.2 us until the stores are visible to the other SMs, 0.8 us until
+// the next tile's producer has seen the counter. No unit is busy meanwhile (tensor pipe 16 %, L2 26 % of peak). The pair form
+// has no counters: a cooperative launch of clusters does not replay under the profiler. Loops must not spill to local
+// memory here: the acquiring loads of the counters drop the L1, and each reload is an L2 round trip (two spilling epilogue
+// groups: 110 -> 135 us per step, without spills 97; what is left are 4 to 16 bytes in three of the six kernels).
+// bf16, us per step, launch per GEMM -> here: 5 x 1024, batch 1024 170 -> 89; 20 x 512, batch 2048 589 -> 233;
+// 784-500-300-10, batch 1000 87 -> 47; 6 x 512, batch 8192 -> 158 (pairs).
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
