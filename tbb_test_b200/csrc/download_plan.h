@@ -28,9 +28,10 @@ struct DownloadPlan {
 // each (one copied to while the other is emptied), and from 12 MB on twelve threads share the same 1.5 MB, one buffer each
 // (us per matrix into fresh memory: 3072 x 3072 3490 -> 3040, 4096 x 4096 6050 -> 5150). Fewer than twelve cores run a thread
 // each, six at most, with two buffers: 2048 x 2048 and 4096 x 4096 on eight cores 1110 and 6000, as eight threads with one
-// buffer each 1160 and 6400; on four 1080 and 7100 (twelve threads 1300 and 8300), on two 1250 and 9600 (2200 and 12400). Chunks of 512 KB from 32 MB on are faster still (3040 -> 2250, 5150 -> 3850, 8192 x 8192 19000 -> 12800), but
-// their 6 MB of page-locked memory take 3 to 9 ms to make and 1.3 to give back: what is gained over some 256 MB, and only with
-// the matrix that makes it as much for a handle they are made.
+// buffer each 1160 and 6400; on four 1080 and 7100 (twelve threads 1300 and 8300), on two 1250 and 9600 (2200 and 12400).
+// Chunks of 512 KB from 32 MB on are faster still (3040 -> 2250, 5150 -> 3850, 8192 x 8192 19000 -> 12800), but their 6 MB of
+// page-locked memory take 3 to 9 ms to make and 1.3 to give back. That is gained over some 256 MB, so they are made with the
+// matrix that makes it as much for a handle.
 inline DownloadPlan plan_download(size_t width, size_t rows, int cores, const DownloadBuffers& b) {
   const size_t total = width * rows;
   const bool large = total >= DL_LARGE_BYTES && b.large_read + total >= DL_LARGE_AFTER && !b.no_large;
