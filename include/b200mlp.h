@@ -48,7 +48,10 @@ typedef enum {
 /* Arithmetic of the three GEMMs; accumulation is fp32 and the master weights and
  * the SGD update are fp32 in every case. */
 typedef enum {
-  B2_PREC_FP32 = 0, /* fp32 operands, CUDA-core FMA (parity mode) */
+  B2_PREC_FP32 = 0, /* fp32 operands at fp32 precision (parity mode): small GEMMs as CUDA-core FMAs in k order; large ones
+                       on the tensor cores as products of exact three-way bf16 splits whose sums are rounded in
+                       fp32, with a smaller error against 64-bit sums than the FMAs' and the same results where
+                       operands or sums are not finite (csrc/gemm_split.cu). With force_simt: FMAs only */
   B2_PREC_TF32 = 1, /* fp32 storage, tcgen05 kind::tf32 */
   B2_PREC_BF16 = 2, /* bf16 operands (activations, gradients, a bf16 weight copy),
                        tcgen05 kind::f16: layers of any width, on rows padded to 16 bytes (but for
@@ -356,14 +359,16 @@ int b2_write_trace(b2_handle* h, const char* path);
  * in the tensor-core precisions a site whose shape or alignment the tensor-core kernel cannot
  * address (TF32 and FP32_TC: a width that is not a multiple of 4; fewer than 16 output columns,
  * such as the 1-wide tail layer of the reference's topology, mlp_bench_common.h:26) falls to the
- * CUDA-core kernels, which are many times slower for wide layers. The counts and the reason given for the first such
+ * fp32 kernels (CUDA cores, or split operands as in B2_PREC_FP32), which are several times slower for wide layers, and
+ * counts as a CUDA-core site here. The counts and the reason given for the first such
  * site make that visible; with B2_VERBOSE set in the environment it is also printed once. */
 int b2_site_report(const b2_handle* h, int* tensor_core_sites, int* cuda_core_sites, char* first_reason,
                    size_t reason_len);
 
 /* Number of kernels of this library launched on the handle since creation, and
- * the number of GEMMs run by its tensor-core (tcgen05) kernels: one per GEMM launch; a
- * launch that computes whole training steps counts all tensor-core GEMMs of its steps. */
+ * the number of GEMMs run by the tensor-core (tcgen05) kernels of the TF32, BF16 and FP32_TC
+ * precisions: one per GEMM launch; a launch that computes whole training steps counts all
+ * tensor-core GEMMs of its steps. (GEMMs of B2_PREC_FP32 count in `total` only, on whichever unit they run.) */
 int b2_launch_counts(const b2_handle* h, long long* total, long long* tensor_core);
 
 #ifdef __cplusplus

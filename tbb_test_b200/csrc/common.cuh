@@ -71,6 +71,11 @@ bool gemm_f32_serves(const GemmDesc& g);
 cudaError_t gemm_f32_launch(const GemmDesc& g, cudaStream_t stream);
 bool gemm_simt_small(const GemmDesc& g);  // served by one of its kernels for small grids (unless large_tiles)
 
+// GEMM of fp32 matrices on the tensor cores at fp32 precision, any alignment (gemm_split.cu), where it is faster than
+// gemm_simt_launch; on at most `sms` SMs; `status` as for gemm_tc_launch.
+bool gemm_split_serves(const GemmDesc& g);
+cudaError_t gemm_split_launch(const GemmDesc& g, int sms, cudaStream_t stream, unsigned int* status);
+
 // Tensor-core (tcgen05 + TMA + TMEM) GEMM. in_type T_BF16 -> kind::f16 (bf16),
 // in_type T_F32 -> kind::tf32. Returns cudaErrorNotSupported when the shape or
 // alignment cannot be served (caller falls back to gemm_simt_launch).

@@ -44,7 +44,8 @@ thread_local std::string g_tls_error;
 
 struct Site {
   GemmDesc d;
-  TcPlan* plan = nullptr;  // null: CUDA-core kernel
+  TcPlan* plan = nullptr;
+  bool split = false;      // without a plan: fp32 operands cut into bf16 pieces (gemm_split.cu) instead of the CUDA cores
   bool active = false;
 };
 
@@ -225,6 +226,7 @@ int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
   s.d.pad_writable = 1;  // rows of b2_handle::ld elements
   s.active = s.d.M > 0 && s.d.N > 0 && s.d.K > 0;
   s.plan = nullptr;
+  s.split = s.active && !h->cfg.force_simt && gemm_split_serves(s.d);
   if (!s.active || !want_tc) return B2_OK;
   char why[128] = "";
   s.plan = gemm_tc_plan_create(s.d, sms > 0 ? sms : h->gemm_sms, why, sizeof why);
@@ -240,8 +242,14 @@ int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
     }
   } else {
     ++h->tensor_core_sites;
+    s.split = false;
   }
   return B2_OK;
+}
+
+// A GEMM that no plan serves.
+cudaError_t launch_unplanned(const b2_handle* h, const GemmDesc& d, bool split, cudaStream_t st) {
+  return split ? gemm_split_launch(d, h->gemm_sms, st, h->status_dev) : gemm_simt_launch(d, st);
 }
 
 int run_site(b2_handle* h, const Site& s, cudaStream_t st) {
@@ -251,7 +259,7 @@ int run_site(b2_handle* h, const Site& s, cudaStream_t st) {
     ++h->tc_launches;
     CK(h, gemm_tc_launch(s.plan, st, h->status_dev));
   } else {
-    CK(h, gemm_simt_launch(s.d, st));
+    CK(h, launch_unplanned(h, s.d, s.split, st));
     if (s.d.C_lo) {  // fp32-class mode: the CUDA-core kernel served this site, so its result's twin is made here
       CK(h, split_lo_launch(static_cast<const float*>(s.d.C), static_cast<float*>(s.d.C_lo), (size_t)s.d.M * s.d.N, st));
       ++h->launches;
@@ -522,7 +530,7 @@ int build_sites(b2_handle* h) {
   std::vector<Site*> sites = {&h->fwd0_alt, &h->wgrad0_alt};
   for (int l = 0; l < L; ++l) sites.insert(sites.end(), {&h->fwd[l], &h->wgrad[l], &h->dgrad[l]});
   bool small = true;
-  for (const Site* s : sites) small = small && (!s->active || s->plan || gemm_simt_small(s->d));
+  for (const Site* s : sites) small = small && (!s->active || s->plan || s->split || gemm_simt_small(s->d));
   for (Site* s : sites) s->d.large_tiles = !small;
   // ReLU bit planes: used for a layer only if both its producer (forward of the layer below) and
   // its consumer (input gradient of the layer itself) run on the tensor-core kernel
@@ -2289,7 +2297,7 @@ int b2_gemm_bench(b2_handle* h, int form, int m, int n, int k, int precision, in
         ++h->tc_launches;
         return gemm_tc_launch(s.plan, h->s_main, h->status_dev);
       }
-      return gemm_simt_launch(s.d, h->s_main);
+      return launch_unplanned(h, s.d, !h->cfg.force_simt && gemm_split_serves(s.d), h->s_main);
     };
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < warmup && e == cudaSuccess; ++i) e = run(i);
@@ -2414,7 +2422,7 @@ static int gemm_common(b2_handle* h, int precision, GemmDesc& d, cudaStream_t st
     e = gemm_tc_launch(plan, st, h->status_dev);
     gemm_tc_plan_destroy(plan);  // the tensor maps were passed by value at launch
   } else {
-    e = gemm_simt_launch(d, st);
+    e = launch_unplanned(h, d, !h->cfg.force_simt && gemm_split_serves(d), st);
   }
   if (e != cudaSuccess) return fail(h, B2_ERR_CUDA, "GEMM launch: %s", cudaGetErrorString(e));
   return B2_OK;

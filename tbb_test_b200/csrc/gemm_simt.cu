@@ -1,6 +1,6 @@
-// CUDA-core GEMMs: the fp32 parity path of the training step and the fallback for
-// shapes the tensor-core kernel does not take (unaligned leading dimensions, the
-// N = 1 tail layer of the reference topology, mlp_bench_common.h:26).
+// CUDA-core GEMMs: the small ones of the fp32 parity path of the training step (large ones: gemm_split.cu) and
+// the fallback for shapes the tensor-core kernels do not take (the N = 1 tail layer of the reference topology,
+// mlp_bench_common.h:26).
 //
 // Stand in for the reference's cblas_sgemm calls (mlp_omp.cc:474,566,657):
 // C = alpha * op(A) * op(B) + beta * C with fp32 accumulation. Three kernels:
