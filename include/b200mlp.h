@@ -173,8 +173,7 @@ int b2_set_lr(b2_handle* h, float lr);
 /* The loop body of mlp_omp.cc:435-737, `iters` times: forward GEMMs, output
  * gradient, then per layer (last to first) weight-gradient GEMM, gradient
  * allreduce + SGD on the side stream, input-gradient GEMM. Returns after both
- * streams have drained. Networks of small layers (tensor-core precisions, no gradient
- * exchange) run as launches of several whole steps that take all SMs for up to about 2 ms
+ * streams have drained. Networks of small layers (no gradient exchange) run as launches of several whole steps that take all SMs for up to about 2 ms
  * at a time (or for one step, where that takes longer): other work on the GPU gets its
  * turn between them. */
 int b2_step(b2_handle* h, int iters);

@@ -126,6 +126,32 @@ void step_plan_destroy(StepPlan* p);
 cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
                         cudaStream_t stream);
 
+// Whole steps of small fp32 networks as one cooperative launch (small_step.cu). Rows of all matrices are dense.
+constexpr int SMALL_LAYERS = 16;
+struct SmallLayer {
+  int fi, fo;
+  const float* in;  // batch x fi
+  float* out;       // batch x fo: the next layer's input, or the network's output
+  float* dz;        // batch x fo
+  float* dx;        // batch x fi: the layer's below dz, or the input gradient
+  float *w, *dw;    // fo x fi
+};
+struct SmallStep {
+  SmallLayer layer[SMALL_LAYERS];
+  int L, batch, baseline, input_grad;
+  const float* target;
+  float inv_batch;
+  double loss_scale;
+  double* loss;
+};
+bool small_step_serves(const SmallStep& s);
+int small_step_steps(const SmallStep& s);  // that one launch should take
+int small_step_blocks(const SmallStep& s, int sms);
+// Barriers of a launch: each adds `blocks` to *counter, which stands at `count` before the launch.
+int small_step_barriers(const SmallStep& s, int steps);
+cudaError_t small_step_launch(const SmallStep& s, int blocks, int steps, float lr, unsigned int count, unsigned int* counter,
+                              unsigned int* status, cudaStream_t stream);
+
 // Small-message allreduce over peer memory (p2p_allreduce.cu). Every rank's gradient slab and
 // flag block are addressable from every rank (peer access within a process, IPC mappings
 // between processes). A flag block is 2 * P2P_MAX_RANKS words, written by the peers: word

@@ -135,6 +135,10 @@ struct b2_handle {
   size_t sync_bytes = 0;
   // Whole steps in one launch (step_kernel.cu), one plan per input slot; null: one launch per GEMM
   StepPlan* step_plan[2] = {nullptr, nullptr};
+  // The same for small fp32 networks (small_step.cu); empty (no layers) where it does not serve
+  SmallStep small_step[2] = {};
+  int small_blocks = 0;
+  unsigned int small_count = 0;  // where the launches so far have brought the barriers' counter (behind the loss of slot 0)
   int launch_steps = 1;  // steps b2_step runs per launch
   unsigned int* status_dev = nullptr;
   unsigned long long* fp_dev = nullptr;  // accumulator of b2_weights_fingerprint
@@ -282,6 +286,8 @@ int check_status(b2_handle* h) {
   if (st != 0) {
     cudaMemset(h->status_dev, 0, sizeof st);
     if (h->tc_ws_flags) cudaMemset(h->tc_ws_flags, 0, (size_t)h->sms * sizeof(unsigned int));
+    cudaMemset(h->sync_dev + 16, 0, sizeof(unsigned int));
+    h->small_count = 0;
     if (st >= 100u) {  // a flag wait of the peer-memory allreduce: its call counters no longer agree
       h->p2p_ready = false;
       cudaMemset(h->p2p_ctas_done, 0, sizeof(unsigned int));
@@ -553,6 +559,43 @@ StepShape step_shape(const b2_handle* h) {
           h->cfg.input_grad != 0};
 }
 
+bool whole_steps(const b2_handle* h, int slot) { return h->step_plan[slot] || h->small_step[slot].L > 0; }
+
+// Small fp32 networks: the same on the CUDA cores (small_step.cu).
+void build_small_step(b2_handle* h) {
+  const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
+  const bool has_ar = h->cfg.world_size > 1 && h->cfg.allreduce;
+  if ((e && e[0] == '0') || h->cfg.precision != B2_PREC_FP32 || has_ar || !h->cfg.overlap || h->bl < 1 || h->L > SMALL_LAYERS)
+    return;
+  const bool baseline = h->cfg.mode == B2_MODE_BASELINE;
+  for (int slot = 0; slot < 2; ++slot) {
+    SmallStep s{};
+    for (int l = 0; l < h->L; ++l) {
+      SmallLayer& y = s.layer[l];
+      y.fi = h->nf[l];
+      y.fo = h->nf[l + 1];
+      y.in = static_cast<const float*>(l == 0 && slot ? h->act0_alt : h->act[l]);
+      y.out = l == h->L - 1 ? h->y : static_cast<float*>(h->act[l + 1]);
+      y.dz = static_cast<float*>(h->dz[l]);
+      y.dx = static_cast<float*>(l == 0 ? h->dinput : h->dz[l - 1]);
+      y.w = h->w[l];
+      y.dw = static_cast<float*>(h->dw[l]);
+    }
+    s.L = h->L;
+    s.batch = h->bl;
+    s.baseline = baseline ? 1 : 0;
+    s.input_grad = h->cfg.input_grad != 0;
+    s.target = slot ? h->target_alt : h->target;
+    s.inv_batch = 1.0f / (float)h->cfg.batch;
+    s.loss_scale = baseline ? 1.0 / (double)h->cfg.batch : 1.0;
+    s.loss = loss_ptr(h, slot);
+    if (!(e && e[0] == '1') && !small_step_serves(s)) return;
+    h->small_step[slot] = s;
+  }
+  h->small_blocks = small_step_blocks(h->small_step[0], h->sms);
+  h->launch_steps = small_step_steps(h->small_step[0]);
+}
+
 // The plans of the networks whose whole steps run as one launch (step_kernel.cu; the rules: step_choice.h).
 int build_step_plans(b2_handle* h) {
   const int L = h->L;
@@ -657,6 +700,13 @@ int build_step_plans(b2_handle* h) {
 
 // `steps` training steps on the main stream as one launch.
 int enqueue_fused(b2_handle* h, int slot, int steps) {
+  if (h->small_step[slot].L > 0) {
+    CK(h, small_step_launch(h->small_step[slot], h->small_blocks, steps, h->cfg.lr, h->small_count,
+                            reinterpret_cast<unsigned int*>(h->sync_dev + 16), h->status_dev, h->s_main));
+    h->small_count += (unsigned int)(small_step_barriers(h->small_step[slot], steps) * h->small_blocks);
+    ++h->launches;
+    return B2_OK;
+  }
   char* sync = h->sync_dev + (size_t)slot * h->sync_bytes;
   CK(h, cudaMemsetAsync(sync, 0, h->sync_bytes, h->s_main));
   CK(h, step_launch(h->step_plan[slot], steps, h->cfg.lr, reinterpret_cast<unsigned int*>(sync + 16), h->status_dev,
@@ -1426,6 +1476,7 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     }
   }
   TRY(build_sites(h));
+  build_small_step(h);
   TRY(build_step_plans(h));
   TRYCK(cudaDeviceSynchronize());
 #undef TRY
@@ -1609,7 +1660,7 @@ int b2_step(b2_handle* h, int iters) {
   if (h->async_issued != h->async_waited) return fail(h, B2_ERR_STATE, "pipelined steps in flight: b2_wait_loss first");
   if (iters == 0) return B2_OK;
   const bool timed = h->cfg.collect_timing != 0;
-  const bool fused = h->step_plan[0] && !timed;
+  const bool fused = whole_steps(h, 0) && !timed;
   const bool graph = h->cfg.use_graph && !timed && !fused;
   int rc;
   if (graph && !h->graph_exec) {
@@ -1763,7 +1814,7 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
   }
   CK(h, cudaEventRecord(h->ev_copied[slot], h->s_copy));
   CK(h, cudaStreamWaitEvent(h->s_main, h->ev_copied[slot], 0));
-  if ((rc = h->step_plan[slot] ? enqueue_fused(h, slot, 1) : enqueue_step(h, false, slot))) return rc;
+  if ((rc = whole_steps(h, slot) ? enqueue_fused(h, slot, 1) : enqueue_step(h, false, slot))) return rc;
   CK(h, cudaEventRecord(h->ev_slot_free[slot], h->s_main));
   h->slot_used[slot] = true;
   CK(h, cudaMemcpyAsync(h->loss_host + slot, loss_ptr(h, slot), sizeof(double), cudaMemcpyDeviceToHost,

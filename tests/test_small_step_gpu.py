@@ -1,0 +1,107 @@
+"""Whole steps of small fp32 networks in one launch (csrc/small_step.cu) against the launch-per-GEMM schedule of the same
+handle, at the edges of its tiles (16 x 32), groups of four k and layer table."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+# widths, batch, keywords; what makes them edges: one row; one column; one layer; tiles exactly and one more or less; rows of
+# whole 16-byte pieces and not; sums shorter than a group of four k; more tiles than the grid has blocks; the last layer count
+NETS = [([16, 32], 16, {}), ([1, 1], 1, {}), ([33, 17, 5], 7, {}), ([17, 31, 33, 1], 3, {}), ([64, 64, 64], 1, {}),
+        ([128, 256, 128, 64], 32, {}), ([36, 60, 4], 130, {}), ([512, 512, 512], 24, {}), ([300, 301, 95, 40], 60, {}),
+        ([20] * 17, 50, {}), ([40, 24], 2048, {}), ([64, 100, 10], 33, dict(input_grad=False))]
+
+
+def make(monkeypatch, nf, batch, whole, **kw):
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    monkeypatch.setenv("B2_STEP_KERNEL", "1" if whole else "0")
+    m = MLP(nf, batch, precision=K.PREC_FP32, lr=0.02, **kw)
+    monkeypatch.delenv("B2_STEP_KERNEL")
+    rng = np.random.default_rng(3)
+    for l in range(m.L):
+        m.upload_weights(l, rng.uniform(-1, 1, (nf[l + 1], nf[l])).astype(np.float32) * np.float32(nf[l] ** -0.5))
+    m.upload_input(rng.standard_normal((batch, nf[0])).astype(np.float32))
+    m.upload_target(np.sign(rng.standard_normal((batch, nf[-1]))).astype(np.float32))
+    return m
+
+
+def launches(m, f):
+    before = m.launch_counts()[0]
+    f()
+    return m.launch_counts()[0] - before
+
+
+@pytest.mark.parametrize("mode", ["baseline", "ref"])
+@pytest.mark.parametrize("net", NETS, ids=lambda n: f"{'-'.join(map(str, n[0][:4]))}x{len(n[0])}b{n[1]}")
+def test_one_step(native, monkeypatch, net, mode):
+    """Every tensor of one step. Both sides add fp32 FMAs or better in other orders: the bound of the single GEMMs (2e-5)
+    over the chain of at most 32 of them (sums of up to 2048 terms; seen: 5e-7)."""
+    from tbb_test_b200 import _capi as K
+    nf, batch, kw = net
+    kw = dict(kw, mode=K.MODE_REF if mode == "ref" else K.MODE_BASELINE)
+    a, b = make(monkeypatch, nf, batch, True, **kw), make(monkeypatch, nf, batch, False, **kw)
+    assert launches(a, lambda: a.step(1)) == 1 and launches(b, lambda: b.step(1)) >= 4 * a.L
+    for l in range(a.L + 1):
+        assert rel_fro(a.activation(l), b.activation(l)) <= 2e-5
+    for l in range(a.L):
+        for what in (a.dz, b.dz), (a.weight_grad, b.weight_grad), (a.weights, b.weights):
+            assert rel_fro(what[0](l), what[1](l)) <= 2e-5
+    if kw.get("input_grad", True):
+        assert rel_fro(a.input_grad(), b.input_grad()) <= 2e-5
+    assert abs(a.loss() - b.loss()) <= 1e-5 * abs(b.loss())
+    a.close()
+    b.close()
+
+
+def test_many_steps_in_few_launches(native, monkeypatch):
+    """100 steps in launches of at most 64, and the same steps one by one, from one handle's weights to the other's: equal
+    bits (sums have a fixed order; the loss's block sums have none)."""
+    nf, batch = [48, 64, 32], 20
+    a, b = make(monkeypatch, nf, batch, True), make(monkeypatch, nf, batch, True)
+    assert launches(a, lambda: a.step(100)) == 2
+    for _ in range(100):
+        b.step(1)
+    assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2)) and abs(a.loss() - b.loss()) <= 1e-12 * abs(b.loss())
+    a.set_timing(1)  # timed steps take the launch-per-GEMM schedule in between
+    assert launches(a, lambda: a.step(1)) > 1
+    a.set_timing(0)
+    assert launches(a, lambda: a.step(3)) == 1
+    b.step(4)
+    assert all(rel_fro(a.weights(l), b.weights(l)) <= 2e-5 for l in range(2))
+    a.close()
+    b.close()
+
+
+def test_host_fed_steps(native, monkeypatch):
+    """Both input slots: steps fed from the host, two in flight, against blocking ones."""
+    nf, batch = [40, 24, 12], 30
+    fp = C.POINTER(C.c_float)
+    rng = np.random.default_rng(4)
+    data = [(rng.standard_normal((batch, 40)).astype(np.float32), np.sign(rng.standard_normal((batch, 12))).astype(np.float32)) for _ in range(5)]
+    a, b = make(monkeypatch, nf, batch, True), make(monkeypatch, nf, batch, True)
+    got, want = [], []
+    for i, (x, t) in enumerate(data):
+        px, pt = x.ctypes.data_as(fp), t.ctypes.data_as(fp)
+        a.train_step_host_async(px, 40, pt, 12)
+        if i:
+            got.append(a.wait_loss())
+        want.append(b.train_step_host(px, 40, pt, 12))
+    got.append(a.wait_loss())
+    assert np.allclose(got, want, rtol=1e-12) and all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    a.close()
+    b.close()
+
+
+def test_what_it_does_not_serve(native, monkeypatch):
+    """More layers than its table, large networks, serial schedules and the tensor-core precisions keep their paths."""
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    for nf, batch, kw in (([20] * 18, 50, {}), ([1024, 1024], 256, {}), ([64, 64], 4096, {}), ([64, 64], 32, dict(overlap=False))):
+        m = MLP(nf, batch, precision=K.PREC_FP32, **kw)
+        assert launches(m, lambda: m.step(1)) > 1
+        m.close()
