@@ -10,7 +10,18 @@ constexpr size_t DL_CHUNK = 128 << 10, DL_LARGE_CHUNK = 512 << 10;
 constexpr size_t DL_MIN_BYTES = 2 << 20, DL_MANY_BYTES = 12 << 20, DL_LARGE_BYTES = 32 << 20;
 constexpr size_t DL_LARGE_AFTER = (size_t)256 << 20;
 
-// Page-locked buffers of a handle, DL_WORKERS chunks.
+// A matrix of up to 2.5 MB comes over in one copy into page-locked memory made with the handle (making any takes 1 to 4 ms
+// whatever its size up to here, so it is one block with the words that blocking calls read) and goes on to its place from there: in
+// one thread up to 1.5 MB, whose destination gets its pages meanwhile, else in six, which take the faults as they go (asking
+// for pages holds the others up). us per matrix into fresh memory, against the driver's copy or the chunks below: 128 KB 67 -> 22,
+// 512 KB 110 -> 58, 1 MB 350 -> 200, 2 MB 540 -> 245 (1 MB into pages that are there: 96 and 104). At 4 MB it gains nothing (515, 505) and making the block takes 2 ms longer.
+constexpr size_t DL_LANDING_BYTES = 5 << 19, DL_PIECE = 128 << 10;
+inline int landing_threads(size_t bytes, int cores) {
+  const int threads = bytes < 3 << 19 ? 1 : 6;
+  return threads < cores ? threads : cores > 1 ? cores : 1;
+}
+
+// Page-locked buffers of a handle for larger ones, DL_WORKERS chunks.
 struct DownloadBuffers {
   char* at = nullptr;
   size_t bytes = 0;

@@ -125,7 +125,16 @@ struct b2_handle {
   float* y = nullptr;
   float* target = nullptr;
   void* dinput = nullptr;
-  DownloadBuffers dl;  // page-locked buffers of download_rows, made at the first large download
+  // Page-locked block of the handle: the words that blocking calls wait for, and behind them where matrices of up to
+  // landing_bytes land on their way to the host
+  struct Mail {
+    double loss[2], last;  // of either input slot's step in flight, and what a blocking call asks for
+    unsigned int status;
+  };
+  Mail* mail = nullptr;
+  char* landing = nullptr;
+  size_t landing_bytes = 0;
+  DownloadBuffers dl;  // page-locked buffers of larger downloads, made at the first one
   cudaEvent_t dl_ev[DL_WORKERS] = {};
   float* stage = nullptr;  // fp32 staging for converted up/downloads
   size_t stage_elems = 0;
@@ -160,7 +169,6 @@ struct b2_handle {
   cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_slot_free[2] = {nullptr, nullptr},
               ev_loss[2] = {nullptr, nullptr};
   bool slot_used[2] = {false, false};
-  double* loss_host = nullptr;  // pinned, one value per slot
   long long async_issued = 0, async_waited = 0;
   ncclComm_t comm = nullptr;
   std::vector<double> phase_ms;
@@ -280,9 +288,13 @@ cudaEvent_t phase_ev(b2_handle* h, int l, int phase, int end) {
 
 int check_comm(b2_handle* h);
 
-int check_status(b2_handle* h) {
-  unsigned int st = 0;
-  CK(h, cudaMemcpy(&st, h->status_dev, sizeof st, cudaMemcpyDeviceToHost));
+// The status word on its way to the host behind the main stream's work, and what it says once that stream has been waited for.
+int fetch_status(b2_handle* h) {
+  CK(h, cudaMemcpyAsync(&h->mail->status, h->status_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->s_main));
+  return B2_OK;
+}
+int judge_status(b2_handle* h) {
+  const unsigned int st = h->mail->status;
   if (st != 0) {
     cudaMemset(h->status_dev, 0, sizeof st);
     if (h->tc_ws_flags) cudaMemset(h->tc_ws_flags, 0, (size_t)h->sms * sizeof(unsigned int));
@@ -297,6 +309,11 @@ int check_status(b2_handle* h) {
     return fail(h, B2_ERR_TIMEOUT, "tensor-core GEMM gave up waiting on a pipeline barrier (role %u)", st);
   }
   return check_comm(h);
+}
+int check_status(b2_handle* h) {
+  if (int rc = fetch_status(h)) return rc;
+  CK(h, cudaStreamSynchronize(h->s_main));
+  return judge_status(h);
 }
 
 // Asynchronous errors of the communicator (a peer process that died, a network fault): reported
@@ -340,6 +357,56 @@ int upload_matrix(b2_handle* h, void* dev, int type, const float* host, size_t l
   return B2_OK;
 }
 
+// Pages of fresh memory in one call instead of a fault each; it changes nothing but that they are there, and where the
+// kernel does not know the request the copy takes the faults.
+void make_pages(const void* at, size_t bytes) {
+  const uintptr_t page = 4096, from = (reinterpret_cast<uintptr_t>(at) + page - 1) & ~(page - 1);
+  const uintptr_t to = (reinterpret_cast<uintptr_t>(at) + bytes) & ~(page - 1);
+  if (to > from && bytes >= 64 * 1024) madvise(reinterpret_cast<void*>(from), to - from, 23 /* MADV_POPULATE_WRITE */);
+}
+
+int usable_cores() {  // those this process may run on, which need not be all of the machine's
+  cpu_set_t cpus;
+  return sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : (int)std::thread::hardware_concurrency();
+}
+
+// Matrices of up to landing_bytes, see download_plan.h.
+int download_landing(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
+  const size_t width = (size_t)cols * 4, total = width * rows;
+  CK(h, copy_rows(h->landing, width, dev, pitch * 4, width, (size_t)rows, cudaMemcpyDeviceToHost, h->s_main));
+  const int threads = landing_threads(total, usable_cores());
+  if (threads == 1 && ld == (size_t)cols) make_pages(host, total);
+  std::atomic<int> next{0}, landed{0};
+  const int per = (int)std::max<size_t>(1, threads == 1 ? rows : DL_PIECE / width);
+  auto work = [&] {
+    for (int w; (w = landed.load(std::memory_order_acquire)) <= 0;) {
+      if (w < 0) return;
+      std::this_thread::yield();
+    }
+    for (int r0; (r0 = next.fetch_add(per)) < rows;) {
+      const int n = std::min(per, rows - r0);
+      if (ld == (size_t)cols) memcpy(host + (size_t)r0 * ld, h->landing + width * r0, width * n);
+      else
+        for (int r = r0; r < r0 + n; ++r) memcpy(host + (size_t)r * ld, h->landing + width * r, width);
+    }
+  };
+  std::thread pool[DL_WORKERS];
+  for (int i = 0; i + 1 < threads; ++i) {
+    try {
+      pool[i] = std::thread(work);
+    } catch (const std::exception&) {  // no more threads, or no memory for one: those that run do it all
+      break;
+    }
+  }
+  const cudaError_t e = cudaStreamSynchronize(h->s_main);
+  landed.store(e == cudaSuccess ? 1 : -1, std::memory_order_release);
+  work();
+  for (std::thread& th : pool)
+    if (th.joinable()) th.join();
+  CK(h, e);
+  return B2_OK;
+}
+
 // Device rows to host memory, done when it returns. A copy to pageable memory runs at the speed of one
 // thread that moves it through the driver's own staging buffer and takes the page faults of a fresh
 // destination (4.7 GB/s here, 109 ms for the weights of 8 x 4096 layers); several threads with page-locked
@@ -349,6 +416,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
   cudaPointerAttributes attr;
   bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
+  if (pageable && total <= h->landing_bytes) return download_landing(h, host, ld, dev, pitch, rows, cols);
   DownloadPlan plan{};
   if (pageable && total >= DL_MIN_BYTES) {
     auto alloc = [](size_t bytes) {
@@ -357,9 +425,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       cudaGetLastError();
       return static_cast<char*>(p);
     };
-    cpu_set_t cpus;  // those this process may run on, which need not be all of the machine's
-    const int cores = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : (int)std::thread::hardware_concurrency();
-    plan = ready_download(width, (size_t)rows, cores, h->dl, alloc, [](char* p) { cudaFreeHost(p); });
+    plan = ready_download(width, (size_t)rows, usable_cores(), h->dl, alloc, [](char* p) { cudaFreeHost(p); });
     for (cudaEvent_t& ev : h->dl_ev)
       if (plan.threads > 0 && !ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
         ev = nullptr;
@@ -368,13 +434,7 @@ int download_rows(b2_handle* h, float* host, size_t ld, const void* dev, size_t 
       }
   }
   if (plan.threads == 0) {
-    // Pages of fresh memory in one call instead of a fault each (1 MB 443 -> 350 us); it changes nothing but that they
-    // are there, and where the kernel does not know the request the copy takes the faults.
-    if (pageable && ld == (size_t)cols) {
-      const uintptr_t page = 4096, from = (reinterpret_cast<uintptr_t>(host) + page - 1) & ~(page - 1);
-      const uintptr_t to = (reinterpret_cast<uintptr_t>(host) + total) & ~(page - 1);
-      if (to > from && total >= 64 * 1024) madvise(reinterpret_cast<void*>(from), to - from, 23 /* MADV_POPULATE_WRITE */);
-    }
+    if (pageable && ld == (size_t)cols) make_pages(host, total);
     CK(h, cudaMemcpy2DAsync(host, ld * 4, dev, pitch * 4, width, rows, cudaMemcpyDeviceToHost, h->s_main));
     CK(h, cudaStreamSynchronize(h->s_main));
     return B2_OK;
@@ -1107,7 +1167,7 @@ void free_all(b2_handle* h) {
   cudaFree(h->target_alt);
   cudaFree(h->xstage[0]);
   cudaFree(h->xstage[1]);
-  if (h->loss_host) cudaFreeHost(h->loss_host);
+  if (h->mail) cudaFreeHost(h->mail);
   gemm_tc_plan_destroy(h->fwd0_alt.plan);
   gemm_tc_plan_destroy(h->wgrad0_alt.plan);
   for (int i = 0; i < 2; ++i) {
@@ -1406,7 +1466,18 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     h->sync_bytes = (16 + words * sizeof(unsigned int) + 255) / 256 * 256;
     TRY(dev_alloc(h, &h->sync_dev, 2 * h->sync_bytes));
   }
-  TRYCK(cudaHostAlloc((void**)&h->loss_host, 2 * sizeof(double), cudaHostAllocDefault));
+  {
+    size_t most = 0;  // the largest matrix that lands in one piece
+    auto fits = [&](size_t bytes) {
+      if (bytes <= DL_LANDING_BYTES && bytes > most) most = bytes;
+    };
+    for (int l = 0; l < L; ++l) fits((size_t)h->nf[l] * h->nf[l + 1] * 4);
+    for (int l = 0; l <= L; ++l) fits(bl * h->nf[l] * 4);
+    TRYCK(cudaHostAlloc((void**)&h->mail, 4096 + most, cudaHostAllocDefault));
+    memset(h->mail, 0, sizeof *h->mail);
+    h->landing = reinterpret_cast<char*>(h->mail) + 4096;
+    h->landing_bytes = most;
+  }
   TRYCK(cudaStreamCreateWithFlags(&h->s_copy, cudaStreamNonBlocking));
   for (int i = 0; i < 2; ++i) {
     TRYCK(cudaEventCreateWithFlags(&h->ev_copied[i], cudaEventDisableTiming));
@@ -1654,8 +1725,8 @@ static long long launches_per_step(const b2_handle* h, long long* tc) {
   return n;
 }
 
-int b2_step(b2_handle* h, int iters) {
-  ENTER(h);
+// b2_step, and the loss of its last step with the same wait.
+static int run_steps(b2_handle* h, int iters, double* loss) {
   if (iters < 0) return fail(h, B2_ERR_INVALID, "iters < 0");
   if (h->async_issued != h->async_waited) return fail(h, B2_ERR_STATE, "pipelined steps in flight: b2_wait_loss first");
   if (iters == 0) return B2_OK;
@@ -1705,9 +1776,13 @@ int b2_step(b2_handle* h, int iters) {
   }
   if (!graph && !fused && (rc = join_streams(h))) return rc;
   CK(h, cudaEventRecord(h->ev_t1, h->s_main));
+  if ((rc = fetch_status(h))) return rc;
+  if (loss) CK(h, cudaMemcpyAsync(&h->mail->last, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
   CK(h, cudaStreamSynchronize(h->s_main));
-  CK(h, cudaStreamSynchronize(h->s_comm));
-  CK(h, cudaStreamSynchronize(h->s_upd));
+  if (!fused) {
+    CK(h, cudaStreamSynchronize(h->s_comm));
+    CK(h, cudaStreamSynchronize(h->s_upd));
+  }
   float ms = 0.f;
   CK(h, cudaEventElapsedTime(&ms, h->ev_t0, h->ev_t1));
   h->step_ms += ms;
@@ -1746,14 +1821,22 @@ int b2_step(b2_handle* h, int iters) {
     }
     if (cur_e >= 0.f) h->gemm_busy_ms += cur_e - cur_b;
   }
-  return check_status(h);
+  rc = judge_status(h);
+  if (rc == B2_OK && loss) *loss = h->mail->last;
+  return rc;
+}
+
+int b2_step(b2_handle* h, int iters) {
+  ENTER(h);
+  return run_steps(h, iters, nullptr);
 }
 
 int b2_loss(b2_handle* h, double* loss) {
   ENTER(h);
   if (!loss) return fail(h, B2_ERR_INVALID, "null output");
-  CK(h, cudaMemcpyAsync(loss, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
+  CK(h, cudaMemcpyAsync(&h->mail->last, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
   CK(h, cudaStreamSynchronize(h->s_main));
+  *loss = h->mail->last;
   return B2_OK;
 }
 
@@ -1774,9 +1857,7 @@ int b2_train_step_host(b2_handle* h, const float* x, size_t ldx, const float* t,
     if ((rc = upload_matrix(h, h->target, T_F32, t + (size_t)h->b0 * ldt, ldt, h->bl, h->nf[h->L], h->ld[h->L])))
       return rc;
   }
-  if ((rc = b2_step(h, 1))) return rc;
-  if (loss) return b2_loss(h, loss);
-  return B2_OK;
+  return run_steps(h, 1, loss);
 }
 
 int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const float* t, size_t ldt) {
@@ -1817,7 +1898,7 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
   if ((rc = whole_steps(h, slot) ? enqueue_fused(h, slot, 1) : enqueue_step(h, false, slot))) return rc;
   CK(h, cudaEventRecord(h->ev_slot_free[slot], h->s_main));
   h->slot_used[slot] = true;
-  CK(h, cudaMemcpyAsync(h->loss_host + slot, loss_ptr(h, slot), sizeof(double), cudaMemcpyDeviceToHost,
+  CK(h, cudaMemcpyAsync(h->mail->loss + slot, loss_ptr(h, slot), sizeof(double), cudaMemcpyDeviceToHost,
                         h->s_main));
   CK(h, cudaEventRecord(h->ev_loss[slot], h->s_main));
   ++h->async_issued;
@@ -1830,7 +1911,7 @@ int b2_wait_loss(b2_handle* h, double* loss) {
   if (h->async_waited >= h->async_issued) return fail(h, B2_ERR_STATE, "no step in flight");
   const int slot = (int)(h->async_waited & 1);
   CK(h, cudaEventSynchronize(h->ev_loss[slot]));
-  if (loss) *loss = h->loss_host[slot];
+  if (loss) *loss = h->mail->loss[slot];
   ++h->async_waited;
   if (h->async_waited == h->async_issued) {  // pipeline drained: also let the updates finish
     int rc = join_streams(h);

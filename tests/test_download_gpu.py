@@ -51,6 +51,25 @@ def test_chunks_grow_with_the_matrix(native, oracle, shape, extra):
     m.close()
 
 
+@pytest.mark.parametrize("shape,extra", [((1, 1), 0), ((3, 5), 2), ((127, 129), 0), ((400, 401), 7), ((700, 800), 0), ((700, 800), 1),
+                                         ((1, 655360), 0), ((1, 655361), 0)])
+def test_small_downloads(native, oracle, shape, extra):
+    """Matrices that land in the handle's page-locked block, up to its last byte and one element beyond: alone and in several
+    threads, into fresh and pitched memory, in two handles whose blocks differ."""
+    from tbb_test_b200.mlp import MLP
+    rows, cols = shape
+    w = oracle.fill_uniform(rows, cols, 3, -1, 1)
+    for other in (7, 300):
+        m = MLP([cols, rows, other], 4)
+        m.upload_weights(0, w)
+        for _ in range(2):
+            got = np.empty((rows, cols + extra), np.float32)
+            got[:, cols:] = 7.0
+            assert m.lib.b2_download_weights(m._h, 0, got.ctypes.data_as(C.POINTER(C.c_float)), cols + extra) == 0
+            assert np.array_equal(got[:, :cols], w) and (got[:, cols:] == 7.0).all()
+        m.close()
+
+
 OUT_OF_MEMORY = """
 import ctypes as C, sys
 import numpy as np
