@@ -121,22 +121,25 @@ struct ShareA {
   static __device__ __forceinline__ uint32_t offset(int w) {
     return ((uint32_t)((w & 3) * 32 + (KMAJOR ? (w >> 3) * 16 : 0)) << 16) + (uint32_t)((w >> 2 & 1) * A_HALF + (KMAJOR ? 0 : (w >> 3) * 8));
   }
-  // pieces v, w of parts 0 and 1
-  static __device__ __forceinline__ void store(uint32_t at, const uint32_t (&v)[3][4], const uint32_t (&w)[3][4]) {
+  // Half i of the elements to TMEM: four k of either row, or eight k. The four words of a piece are one store, in the order the
+  // cutting leaves them.
+  __device__ __forceinline__ void store(uint32_t at, int i) const {
+    uint32_t w[3][4];
     if (KMAJOR) {
-      asm volatile(
-          "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(at),
-          "r"(v[0][0]), "r"(v[0][1]), "r"(w[0][0]), "r"(w[0][1]), "r"(v[0][2]), "r"(v[0][3]), "r"(w[0][2]), "r"(w[0][3]),
-          "r"(v[1][0]), "r"(v[1][1]), "r"(w[1][0]), "r"(w[1][1]), "r"(v[1][2]), "r"(v[1][3]), "r"(w[1][2]), "r"(w[1][3])
-          : "memory");
-      asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(at + 32),
-                   "r"(v[2][0]), "r"(v[2][1]), "r"(w[2][0]), "r"(w[2][1]), "r"(v[2][2]), "r"(v[2][3]), "r"(w[2][2]), "r"(w[2][3])
-                   : "memory");
+      const float v[8] = {r[0][4 * i], r[0][4 * i + 1], r[0][4 * i + 2], r[0][4 * i + 3], r[1][4 * i], r[1][4 * i + 1], r[1][4 * i + 2], r[1][4 * i + 3]};
+      cut8(v, w);
     } else {
+      cut8(r[i], w);
+    }
 #pragma unroll
-      for (int p = 0; p < 3; ++p)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(at + 16 * p),
-                     "r"(v[p][0]), "r"(v[p][1]), "r"(v[p][2]), "r"(v[p][3]), "r"(w[p][0]), "r"(w[p][1]), "r"(w[p][2]), "r"(w[p][3])
+    for (int p = 0; p < 3; ++p) {
+      if (KMAJOR)
+        asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 16 * p + 8 * i), "r"(w[p][0]), "r"(w[p][1]),
+                     "r"(w[p][2]), "r"(w[p][3])
+                     : "memory");
+      else
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 16 * p + 4 * i), "r"(w[p][0]), "r"(w[p][1]),
+                     "r"(w[p][2]), "r"(w[p][3])
                      : "memory");
     }
   }
@@ -225,51 +228,42 @@ __device__ __forceinline__ void finish(const GemmDesc& g, int gm, int gn, float 
   if (g.epilogue == EPI_MASK) v = __ldg(static_cast<const float*>(g.aux) + (long long)gm * g.ldaux + gn) > 0.f ? v : 0.f;
   *c = v;
 }
-// Sixteen neighbouring elements of row gm from column gn on, this lane's; the warp has 32 rows.
-__device__ __forceinline__ void finish_row(const SplitParams& p, int gm, int gn, float* v) {
+// A warp's 32 rows of C from row m0 and 32 columns from n0 on, a lane a row in `v`, through shared memory of the warp's own, so
+// that a store writes four whole 128-byte lines (a lane storing its own row, 32 bytes at a time, took 3100 clocks per tile).
+constexpr int OUT_PITCH = 32 + 4;
+__device__ __forceinline__ void finish_part(const SplitParams& p, int m0, int n0, float* sh, int lane, const float (&v)[32]) {
   const GemmDesc& g = p.g;
-  const int left = gm < g.M ? g.N - gn : 0;
-  if (g.beta != 0.f) {
+  __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < left) finish(g, gm, gn + j, v[j]);
-    return;
-  }
-  float* const c = static_cast<float*>(g.C) + (long long)gm * g.ldc + gn;
-  const float* const x = static_cast<const float*>(g.aux) + (long long)gm * g.ldaux + gn;
+  for (int j = 0; j < 32; j += 4)
+    *reinterpret_cast<float4*>(sh + lane * OUT_PITCH + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  __syncwarp();
+  const int gn = n0 + (lane & 7) * 4;
+#pragma unroll 4
+  for (int i = 0; i < 32; i += 4) {
+    const int row = i + (lane >> 3), gm = m0 + row, left = gm < g.M ? g.N - gn : 0;
+    float4 w = *reinterpret_cast<const float4*>(sh + row * OUT_PITCH + (lane & 7) * 4);
+    if (g.beta != 0.f || left < 4 || !p.vec_c || (g.epilogue == EPI_MASK && !p.vec_x)) {
+      const float e[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-  for (int j0 = 0; j0 < 16; j0 += 8) {
-    float* const w = v + j0;
-    if (g.alpha != 1.f)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] *= g.alpha;
+      for (int j = 0; j < 4; ++j)
+        if (j < left) finish(g, gm, gn + j, e[j]);
+      continue;
+    }
+    w.x *= g.alpha; w.y *= g.alpha; w.z *= g.alpha; w.w *= g.alpha;
     if (g.epilogue == EPI_RELU) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = fmaxf(w[j], 0.f);
+      w.x = fmaxf(w.x, 0.f); w.y = fmaxf(w.y, 0.f); w.z = fmaxf(w.z, 0.f); w.w = fmaxf(w.w, 0.f);
     } else if (g.epilogue == EPI_MASK) {
-      float a[8];
-      if (p.vec_x && left >= j0 + 8) read8<BY16>(x + j0, a, 8);
-      else read8<CHECKED>(x + j0, a, left - j0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = a[j] > 0.f ? w[j] : 0.f;
+      const float4 a = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(g.aux) + (long long)gm * g.ldaux + gn));
+      w.x = a.x > 0.f ? w.x : 0.f; w.y = a.y > 0.f ? w.y : 0.f; w.z = a.z > 0.f ? w.z : 0.f; w.w = a.w > 0.f ? w.w : 0.f;
     }
-    if (p.vec_c == 2 && left >= j0 + 8) {
-      asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(c + j0), "f"(w[0]), "f"(w[1]), "f"(w[2]),
-                   "f"(w[3]), "f"(w[4]), "f"(w[5]), "f"(w[6]), "f"(w[7])
-                   : "memory");
-    } else if (p.vec_c && left >= j0 + 8) {
-      *reinterpret_cast<float4*>(c + j0) = make_float4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<float4*>(c + j0 + 4) = make_float4(w[4], w[5], w[6], w[7]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j0 + j < left) c[j0 + j] = w[j];
-    }
+    *reinterpret_cast<float4*>(static_cast<float*>(g.C) + (long long)gm * g.ldc + gn) = w;
   }
 }
 
-// A warp's 32 rows of C from row m0 and 32 columns from n0 on by FMAs in k order, a lane a row; `sh` is the warp's own.
+// The same part of C by FMAs in k order, a lane a row.
 constexpr int PLAIN_A = 32 + 1, PLAIN_B = 32 + 4, PLAIN_BYTES = 32 * (PLAIN_A + PLAIN_B) * 4;
+static_assert(PLAIN_BYTES >= 32 * OUT_PITCH * 4, "finish_part's room");
 static_assert(SMEM_BYTES >= 1024 + STAGES * (int)B_STAGE + SUM_WARPS * PLAIN_BYTES, "shared memory");
 template <bool AK, bool BK>
 __device__ __forceinline__ void plain_rows(const GemmDesc& g, int m0, int n0, float* sh, int lane, float (&acc)[32]) {
@@ -317,10 +311,12 @@ __device__ __forceinline__ void plain_rows(const GemmDesc& g, int m0, int n0, fl
 // from TMEM, so that an MMA reads 2 KB of shared memory instead of 6 (with A in shared memory an MMA of 64 columns took 74
 // clocks, 42 so). Tiles of 64 columns: D0, D1, D2 and three stages of A fill TMEM, and 1024 x 1024 fills 128 SMs.
 // Bound by the instructions that cut the operands (8 per pair of floats) and the latency of a chunk from load to hand-over:
-// 0.77 us per chunk, of which the MMAs are 0.4. So sixteen warps cut, each a small part: with eight of twice the share a chunk took
-// 1.0 us, with the summing in the same warps 1.05, with the pieces of A in shared memory 1.1 (1.5 for 128 columns).
-// us, forward / weight / input gradient, against gemm_simt_kernel, operands in L2: 1024^3 23/25/23 against 72/64/68, 2048^3
-// 121/135/122 (142 TFLOP/s) against 435/424/428, 512^3 15/16/16 against 21/21/21. 5 x 1024, batch 1024: 312 us per step, 938 before.
+// 0.8 us per chunk, of which the MMAs are 0.4. So sixteen warps cut, each a small part: with eight of twice the share a chunk took
+// 1.0 us, with the summing in the same warps 1.05, with the pieces of A in shared memory 1.1 (1.5 for 128 columns). Beside its chunks a
+// tile takes 5.5 us of launch, first loads and epilogue (8 with checked first loads, the first chunk handed over behind the second
+// one's cut, and lanes storing their own rows).
+// us, forward / weight / input gradient, against gemm_simt_kernel, operands in L2: 1024^3 21/22/20 against 72/64/68, 2048^3
+// 115/126/112 (153 TFLOP/s) against 435/425/427, 512^3 13/14/13 against 21/21/21. 5 x 1024, batch 1024: 293 us per step, 938 before.
 template <bool AK, bool BK>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __grid_constant__ SplitParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -337,11 +333,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
     sa.begin(g, tile / p.n_blocks * 128, t);
     sb.begin(g, tile % p.n_blocks * BN, t);
   };
+  auto how = [&](int c) { return sb.inside && (c + 1) * CHUNK_K <= g.K ? p.how_ab : CHECKED; };
   if (warp < CUT_WARPS) {  // on its way while the block sets up
     begin(blockIdx.x);
-    sa.template load<CHECKED>(g, 0);
-    sa.template load<CHECKED>(g, 1);
-    sb.template load<CHECKED>(g);
+    auto load = [&](auto h) {
+      sa.template load<decltype(h)::value>(g, 0);
+      sa.template load<decltype(h)::value>(g, 1);
+      sb.template load<decltype(h)::value>(g);
+    };
+    if (how(0) == BY32) load(std::integral_constant<int, BY32>());
+    else load(std::integral_constant<int, CHECKED>());
   }
   if (t == MMA_WARP * 32) {
     abort_s = 0;
@@ -445,17 +446,15 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
       __syncwarp();
       if (lane == 0) mbar_arrive(&tile_empty);
       const int m0 = tile / p.n_blocks * 128 + (warp & 3) * 32, n0 = tile % p.n_blocks * BN + col;
-      bool bad = false;
+      bool bad = false;  // not finite
 #pragma unroll
       for (int j = 0; j < COLS; ++j) bad = bad || !(fabsf(acc[j]) <= 3.402823466e38f);
-      if (__any_sync(0xFFFFFFFFu, bad))
-        plain_rows<AK, BK>(g, m0, n0, reinterpret_cast<float*>(smem_raw + SMEM_BYTES - (warp - CUT_WARPS + 1) * PLAIN_BYTES), lane, acc);
-#pragma unroll
-      for (int h = 0; h < COLS; h += 16) finish_row(p, m0 + lane, n0 + h, acc + h);
+      float* const sh = reinterpret_cast<float*>(smem_raw + SMEM_BYTES - (warp - CUT_WARPS + 1) * PLAIN_BYTES);
+      if (__any_sync(0xFFFFFFFFu, bad)) plain_rows<AK, BK>(g, m0, n0, sh, lane, acc);
+      finish_part(p, m0, n0, sh, lane, acc);
     }
   } else {
     const uint32_t a_at = tmem + T_A + ShareA<AK>::offset(warp), b_at = smem + ShareB<BK, AK>::offset(t);
-    auto how = [&](int c) { return sb.inside && (c + 1) * CHUNK_K <= g.K ? p.how_ab : CHECKED; };
     // What has been stored of a chunk is there for the MMAs. Done when the first part of the next chunk has been cut: the
     // stores have arrived by then.
     auto hand_over = [&](int s) {
@@ -468,18 +467,19 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
     // The present chunk into stage s, and behind each part of it the same part of the next one from memory.
     auto store_and_load = [&](int s, int s_before, auto how) {
       constexpr int V = decltype(how)::value;
-      uint32_t v[3][4], w[3][4];
-      cut8(sa.r[0], v);
-      cut8(sa.r[1], w);
       if (s_before >= 0) hand_over(s_before);
-      sa.store(a_at + (uint32_t)s * A_STAGE, v, w);
-      sa.template load<V>(g, 0);
+      sa.store(a_at + (uint32_t)s * A_STAGE, 0);
+      if (!AK) sa.template load<V>(g, 0);
+      sa.store(a_at + (uint32_t)s * A_STAGE, 1);
+      if (AK) sa.template load<V>(g, 0);
       sa.template load<V>(g, 1);
-      cut8(sb.r, v);
-      sb.store(b_at + (uint32_t)s * B_STAGE, v);
+      uint32_t w[3][4];
+      cut8(sb.r, w);
+      sb.store(b_at + (uint32_t)s * B_STAGE, w);
       sb.template load<V>(g);
     };
-    int s = 0, s_before = -1;
+    int s = 0, s_before = -1;  // stage, and the one that is still to be handed over
+    bool before_first = true;
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
@@ -502,11 +502,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
           case FLOATS: store_and_load(s, s_before, std::integral_constant<int, FLOATS>()); break;
           default: store_and_load(s, s_before, std::integral_constant<int, CHECKED>());
         }
-        s_before = s;
+        if (before_first) {  // nothing is under way that would hide the wait
+          hand_over(s);
+          before_first = false;
+        } else {
+          s_before = s;
+        }
         if (++s == STAGES) { s = 0; phase ^= 1; }
       }
     }
-    if (ok) hand_over(s_before);
+    if (ok && s_before >= 0) hand_over(s_before);
   }
   __syncwarp();
   tc_fence_before();
@@ -548,7 +553,7 @@ cudaError_t launch(const SplitParams& p, int sms, cudaStream_t stream) {
 }  // namespace
 
 // By the time of either side, us, fitted to 110 shapes of 16 to 4096 rows, columns and k in the three forms of the step (the
-// faster one is missed by 2 % on average): here 7 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte
+// faster one is missed by 2 % on average): here 6 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte
 // pieces; gemm_simt.cu 4.5 and the longer of 24 (28) per 1000 k and the flops at 33 (30) TFLOP/s. Sums of fewer than 64 terms
 // stay there: neither faster here nor more precise.
 bool gemm_split_serves(const GemmDesc& g) {
@@ -558,7 +563,7 @@ bool gemm_split_serves(const GemmDesc& g) {
   if (tiles > 1 << 30) return false;
   const double rounds = (double)((tiles + SMS - 1) / SMS), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
   const bool whole = how_to_read(g) != FLOATS;
-  const double here = 7.0 + rounds * chunks * (whole ? 0.85 : 1.35);
+  const double here = 6.0 + rounds * chunks * (whole ? 0.85 : 1.35);
   return here <= 4.5 + std::max((whole ? 0.024 : 0.028) * g.K, (double)g.M * g.N * g.K / (whole ? 16.5e6 : 15e6));
 }
 
