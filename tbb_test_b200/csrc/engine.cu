@@ -243,14 +243,14 @@ int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
   char why[128] = "";
   s.plan = gemm_tc_plan_create(s.d, sms > 0 ? sms : h->gemm_sms, why, sizeof why);
   if (!s.plan) {
-    // the CUDA-core kernel serves this site (about 30 x slower): counted, the first reason kept
+    // the fp32 kernels serve this site (cut operands about 10 x slower than bf16, CUDA cores 30 x): counted, the first reason kept
     // for b2_site_report, and announced once per handle when B2_VERBOSE is set
     if (h->cuda_core_sites++ == 0) {
       char buf[256];
       snprintf(buf, sizeof buf, "GEMM %d x %d x %d: %s", s.d.M, s.d.N, s.d.K, why);
       h->cuda_core_reason = buf;
       if (getenv("B2_VERBOSE"))
-        fprintf(stderr, "b200mlp: rank %d: tensor-core kernel refused, CUDA-core kernel used: %s\n", h->cfg.rank, buf);
+        fprintf(stderr, "b200mlp: rank %d: tensor-core kernel refused, fp32 kernels used: %s\n", h->cfg.rank, buf);
     }
   } else {
     ++h->tensor_core_sites;
@@ -272,7 +272,7 @@ int run_site(b2_handle* h, const Site& s, cudaStream_t st) {
     CK(h, gemm_tc_launch(s.plan, st, h->status_dev));
   } else {
     CK(h, launch_unplanned(h, s.d, s.split, st));
-    if (s.d.C_lo) {  // fp32-class mode: the CUDA-core kernel served this site, so its result's twin is made here
+    if (s.d.C_lo) {  // fp32-class mode: the fp32 kernels served this site, so its result's twin is made here
       CK(h, split_lo_launch(static_cast<const float*>(s.d.C), static_cast<float*>(s.d.C_lo), (size_t)s.d.M * s.d.N, st));
       ++h->launches;
     }
