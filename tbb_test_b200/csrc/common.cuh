@@ -70,6 +70,7 @@ cudaError_t gemm_simt_launch(const GemmDesc& g, cudaStream_t stream);
 bool gemm_f32_serves(const GemmDesc& g);
 cudaError_t gemm_f32_launch(const GemmDesc& g, cudaStream_t stream);
 bool gemm_simt_small(const GemmDesc& g);  // served by one of its kernels for small grids (unless large_tiles)
+bool gemm_simt_short_sums(const GemmDesc& g);  // its sums are partial ones of K / 16 or K / 32 terms and not one in k order
 
 // GEMM of fp32 matrices on the tensor cores at fp32 precision, any alignment (gemm_split.cu), where it is faster than
 // gemm_simt_launch; on at most `sms` SMs; `status` as for gemm_tc_launch.
@@ -128,8 +129,10 @@ cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int*
 
 // Whole steps of small fp32 networks as one cooperative launch (small_step.cu). Rows of all matrices are dense.
 constexpr int SMALL_LAYERS = 16;
+enum SmallForm : int { SMALL_FWD = 0, SMALL_DGRAD = 1, SMALL_WGRAD = 2 };
 struct SmallLayer {
   int fi, fo;
+  bool short_sums[3];  // by form: gemm_simt_short_sums of the GEMM
   const float* in;  // batch x fi
   float* out;       // batch x fo: the next layer's input, or the network's output
   float* dz;        // batch x fo

@@ -634,6 +634,9 @@ void build_small_step(b2_handle* h) {
       SmallLayer& y = s.layer[l];
       y.fi = h->nf[l];
       y.fo = h->nf[l + 1];
+      y.short_sums[SMALL_FWD] = gemm_simt_short_sums(h->fwd[l].d);
+      y.short_sums[SMALL_DGRAD] = gemm_simt_short_sums(h->dgrad[l].d);
+      y.short_sums[SMALL_WGRAD] = gemm_simt_short_sums(h->wgrad[l].d);
       y.in = static_cast<const float*>(l == 0 && slot ? h->act0_alt : h->act[l]);
       y.out = l == h->L - 1 ? h->y : static_cast<float*>(h->act[l + 1]);
       y.dz = static_cast<float*>(h->dz[l]);

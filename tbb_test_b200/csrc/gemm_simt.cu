@@ -312,6 +312,8 @@ cudaError_t launch(const GemmDesc& g, cudaStream_t stream) {
 
 bool gemm_simt_small(const GemmDesc& g) { return narrow_form(g) || short_form(g) || gemm_f32_serves(g); }
 
+bool gemm_simt_short_sums(const GemmDesc& g) { return narrow_form(g) || short_form(g); }
+
 cudaError_t gemm_simt_launch(const GemmDesc& g, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0) return cudaSuccess;
   if (g.in_type == T_F32 && g.out_type == T_F32) return launch<float, float>(g, stream);

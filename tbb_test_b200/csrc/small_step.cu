@@ -1,6 +1,7 @@
 // Whole training steps of small fp32 networks in one launch.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -16,12 +17,13 @@ constexpr int PITCH = CHUNK + 4, A_FLOATS = TILE_M * PITCH, B_FLOATS = TILE_N * 
 static_assert(A_FLOATS >= CHUNK * TILE_M && B_FLOATS >= CHUNK * TILE_N, "either layout");
 constexpr int SMEM_BYTES = GROUPS * STAGES * STAGE * 4;
 
-enum Form : int { FWD = 0, DGRAD = 1, WGRAD = 2 };
+enum Form : int { FWD = SMALL_FWD, DGRAD = SMALL_DGRAD, WGRAD = SMALL_WGRAD };
 struct Gemm {
   int M, N, K;
   const float *A, *B;  // FWD: A m x k, B n x k; DGRAD: A m x k, B k x n; WGRAD: A k x m, B k x n; rows dense
   int form, layer;
-  bool vec;  // rows of both are whole 16-byte pieces
+  bool vec;    // rows of both are whole 16-byte pieces
+  bool short_sums;  // see tile_sums
   __device__ __forceinline__ int tiles() const { return ((M + TILE_M - 1) / TILE_M) * ((N + TILE_N - 1) / TILE_N); }
 };
 
@@ -44,15 +46,23 @@ __device__ __forceinline__ void copy_rows(uint32_t dst, int pitch, const float* 
   }
 }
 
-// Four sums of this thread, every one in k order, one FMA per term, as in gemm_simt.cu.
-template <int FORM>
+// Four sums of this thread. In k order, one FMA per term, like those of gemm_simt_kernel and gemm_f32_kernel. The GEMMs that
+// a launch of their own would give to gemm_narrow_kernel or gemm_short_kernel, whose sums are 32 or 16 partial ones
+// and a tree, are summed in blocks of eight terms instead (SHORT), and what an addition of a block loses is kept. That is fewer
+// roundings than in those kernels: 4.5 per term in the mean, in squares of their size relative to a term, against at least 5 and
+// a half for each of the k / 32 or k / 16 terms of a partial sum. Relative error against 64 bits in k order / in their kernel /
+// here: 512 signed terms 3.8e-7 / 9.1e-8 / 6.4e-8, 2048 positive ones 6.1e-7 / 4.6e-8 / 2.6e-8. us per step in k order, so, and in
+// separate launches: 512-10, batch 2000 59, 66, 115; 512-512-512, batch 8 45, 48, 147. (As pairs of floats in one instruction: 65, 52.)
+template <int FORM, bool SHORT>
 __device__ __forceinline__ void tile_sums(const Gemm& g, int m0, int n0, float* sh, int group, int t, float (&acc)[4]) {
+  constexpr int STEP = SHORT ? 8 : 4;
   const int warp = t >> 5, lane = t & 31, chunks = (g.K + CHUNK - 1) / CHUNK;
   const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(sh));
+  float rest[4] = {0.f, 0.f, 0.f, 0.f};  // SHORT: what acc has lost
   auto copy = [&](int c) {
     if (c < chunks) {
       const uint32_t a = at + (c % STAGES) * (STAGE * 4), b = a + A_FLOATS * 4;
-      const int k0 = c * CHUNK, ks = min(CHUNK, (g.K - k0 + 3) / 4 * 4);
+      const int k0 = c * CHUNK, ks = min(CHUNK, (g.K - k0 + STEP - 1) / STEP * STEP);
       if (FORM == WGRAD) copy_rows<TILE_M>(a, TILE_M, g.A, g.M, k0, ks, g.K, m0, g.M, g.vec, t);
       else copy_rows<CHUNK>(a, PITCH, g.A, g.K, m0, TILE_M, g.M, k0, g.K, g.vec, t);
       if (FORM == FWD) copy_rows<CHUNK>(b, PITCH, g.B, g.K, n0, TILE_N, g.N, k0, g.K, g.vec, t);
@@ -71,33 +81,54 @@ __device__ __forceinline__ void tile_sums(const Gemm& g, int m0, int n0, float* 
     const float* b = a + A_FLOATS;
     const int ks = min(CHUNK, g.K - c * CHUNK);
 #pragma unroll 4
-    for (int k = 0; k < ks; k += 4) {  // behind the last k there are zeros
-      float x[4][4], y[4];             // [row][k]
-      if (FORM == WGRAD) {
+    for (int k0 = 0; k0 < ks; k0 += STEP) {  // behind the last k there are zeros
+      float part[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 v = *reinterpret_cast<const float4*>(a + (k + j) * TILE_M + warp * 4);
-          x[0][j] = v.x; x[1][j] = v.y; x[2][j] = v.z; x[3][j] = v.w;
+      for (int i = 0; i < 4; ++i) part[i] = SHORT ? 0.f : acc[i];
+#pragma unroll
+      for (int k = k0; k < k0 + STEP; k += 4) {
+        float x[4][4], y[4];  // [row][k]
+        if (FORM == WGRAD) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(a + (k + j) * TILE_M + warp * 4);
+            x[0][j] = v.x; x[1][j] = v.y; x[2][j] = v.z; x[3][j] = v.w;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(a + (warp * 4 + i) * PITCH + k);
+            x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+          }
         }
-      } else {
+        if (FORM == FWD) {
+          const float4 v = *reinterpret_cast<const float4*>(b + lane * PITCH + k);
+          y[0] = v.x; y[1] = v.y; y[2] = v.z; y[3] = v.w;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 v = *reinterpret_cast<const float4*>(a + (warp * 4 + i) * PITCH + k);
-          x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w;
+          for (int j = 0; j < 4; ++j) y[j] = b[(k + j) * TILE_N + lane];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) part[i] = fmaf(x[i][j], y[j], part[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (SHORT) {  // the error of a sum of two, itself a float (Knuth)
+          const float s = acc[i] + part[i], p = s - acc[i];
+          rest[i] += (acc[i] - (s - p)) + (part[i] - p);
+          acc[i] = s;
+        } else {
+          acc[i] = part[i];
         }
       }
-      if (FORM == FWD) {
-        const float4 v = *reinterpret_cast<const float4*>(b + lane * PITCH + k);
-        y[0] = v.x; y[1] = v.y; y[2] = v.z; y[3] = v.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[j] = b[(k + j) * TILE_N + lane];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] = fmaf(x[i][j], y[j], acc[i]);
     }
+  }
+  if (SHORT) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (fabsf(rest[i]) <= 3.402823466e38f) acc[i] += rest[i];  // else the sum is not finite
   }
   sync();  // before the next tile's copies
 }
@@ -148,15 +179,15 @@ __global__ void __launch_bounds__(THREADS) small_step_kernel(const __grid_consta
   auto vec = [](int a, int b) { return a % 4 == 0 && b % 4 == 0; };
   auto fwd = [&](int l) {
     const SmallLayer& y = s.layer[l];
-    return Gemm{s.batch, y.fo, y.fi, y.in, y.w, FWD, l, vec(y.fi, y.fi)};
+    return Gemm{s.batch, y.fo, y.fi, y.in, y.w, FWD, l, vec(y.fi, y.fi), y.short_sums[FWD]};
   };
   auto dgrad = [&](int l) {
     const SmallLayer& y = s.layer[l];
-    return Gemm{s.batch, y.fi, y.fo, y.dz, y.w, DGRAD, l, vec(y.fo, y.fi)};
+    return Gemm{s.batch, y.fi, y.fo, y.dz, y.w, DGRAD, l, vec(y.fo, y.fi), y.short_sums[DGRAD]};
   };
   auto wgrad = [&](int l) {
     const SmallLayer& y = s.layer[l];
-    return Gemm{y.fo, y.fi, s.batch, y.dz, y.in, WGRAD, l, vec(y.fo, y.fi)};
+    return Gemm{y.fo, y.fi, s.batch, y.dz, y.in, WGRAD, l, vec(y.fo, y.fi), y.short_sums[WGRAD]};
   };
   float loss = 0.f;  // of the elements this thread finishes in the last forward phase
   // what an element's epilogue reads: its target, the activation it is masked by, its weight
@@ -194,9 +225,14 @@ __global__ void __launch_bounds__(THREADS) small_step_kernel(const __grid_consta
 #pragma unroll
       for (int j = 0; j < 4; ++j) x[j] = fetch(g, m + j, n);
       float* const sh = smem + group * STAGES * STAGE;
-      if (g.form == FWD) tile_sums<FWD>(g, mt, nt, sh, group, t, acc);
-      else if (g.form == DGRAD) tile_sums<DGRAD>(g, mt, nt, sh, group, t, acc);
-      else tile_sums<WGRAD>(g, mt, nt, sh, group, t, acc);
+      auto sums = [&](auto is_short) {
+        constexpr bool S = decltype(is_short)::value;
+        if (g.form == FWD) tile_sums<FWD, S>(g, mt, nt, sh, group, t, acc);
+        else if (g.form == DGRAD) tile_sums<DGRAD, S>(g, mt, nt, sh, group, t, acc);
+        else tile_sums<WGRAD, S>(g, mt, nt, sh, group, t, acc);
+      };
+      if (g.short_sums) sums(std::true_type());
+      else sums(std::false_type());
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (m + j < g.M && n < g.N) finish(g, m + j, n, acc[j], x[j]);

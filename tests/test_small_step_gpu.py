@@ -105,3 +105,35 @@ def test_what_it_does_not_serve(native, monkeypatch):
         m = MLP(nf, batch, precision=K.PREC_FP32, **kw)
         assert launches(m, lambda: m.step(1)) > 1
         m.close()
+
+
+@pytest.mark.parametrize("lo", [-1.0, 0.0], ids=["signed", "positive"])
+@pytest.mark.parametrize("net", [([512, 10], 2048), ([2048, 10], 64), ([300, 1], 100), ([512, 512, 9], 8), ([256, 512, 300], 16), ([33, 90, 5], 7),
+                                 ([1, 70, 16], 71), ([76, 65], 2)], ids=lambda n: f"{'-'.join(map(str, n[0]))}b{n[1]}")
+def test_short_sums_are_as_exact(native, monkeypatch, net, lo):
+    """The GEMMs of narrow layers and short batches, whose sums are many partial ones in a launch of their own: the error
+    against 64-bit sums of the same operands is no larger in a whole step (a tenth for the luck of the roundings)."""
+    from tbb_test_b200 import _capi as K
+    nf, batch = net
+    err = []
+    for whole in (True, False):
+        m = make(monkeypatch, nf, batch, whole, mode=K.MODE_REF)
+        rng = np.random.default_rng(5)
+        w = [rng.uniform(lo, 1, (nf[l + 1], nf[l])).astype(np.float32) for l in range(m.L)]
+        for l in range(m.L):
+            m.upload_weights(l, w[l])
+        m.upload_input(rng.uniform(lo, 1, (batch, nf[0])).astype(np.float32))
+        m.step(1)
+        act, dz = [m.activation(l).astype(np.float64) for l in range(m.L + 1)], [m.dz(l).astype(np.float64) for l in range(m.L)]
+        e = {}
+        for l in range(m.L):
+            fi, fo = nf[l], nf[l + 1]
+            if fi >= 64 and fo <= 16:
+                e["forward", l] = rel_fro(act[l + 1], act[l] @ w[l].T)
+            if batch >= 64 and fo <= 16:
+                e["weight gradient", l] = rel_fro(m.weight_grad(l), dz[l].T @ act[l])
+            if fo >= 64 and (batch <= 16 or fi == 1):
+                e["input gradient", l] = rel_fro(dz[l - 1] if l else m.input_grad(), dz[l] @ w[l])
+        err.append(e)
+        m.close()
+    assert err[0] and all(err[0][g] <= 1.1 * err[1][g] for g in err[0]), err
