@@ -127,6 +127,7 @@ void step_plan_destroy(StepPlan* p);
 cudaError_t step_launch(const StepPlan* plan, int steps, float lr, unsigned int* counters, unsigned int* status,
                         cudaStream_t stream);
 
+constexpr unsigned int STATUS_GRID_BARRIER = 16;  // the status word where a wait of small_step.cu gave up
 // Whole steps of small fp32 networks as one cooperative launch (small_step.cu). Rows of all matrices are dense.
 constexpr int SMALL_LAYERS = 16;
 enum SmallForm : int { SMALL_FWD = 0, SMALL_DGRAD = 1, SMALL_WGRAD = 2 };
@@ -150,7 +151,8 @@ struct SmallStep {
 bool small_step_serves(const SmallStep& s);
 int small_step_steps(const SmallStep& s);  // that one launch should take
 int small_step_blocks(const SmallStep& s, int sms);
-// Barriers of a launch: each adds `blocks` to *counter, which stands at `count` before the launch.
+// Barriers of a launch: each adds `blocks` to *counter, which stands at `count` before the launch. A launch that finds *status
+// set (a wait of an earlier one gave up, so the counter is behind) touches neither counter nor weights.
 int small_step_barriers(const SmallStep& s, int steps);
 cudaError_t small_step_launch(const SmallStep& s, int blocks, int steps, float lr, unsigned int count, unsigned int* counter,
                               unsigned int* status, cudaStream_t stream);

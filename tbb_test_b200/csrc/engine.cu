@@ -127,9 +127,12 @@ struct b2_handle {
   void* dinput = nullptr;
   // Page-locked block of the handle: the words that blocking calls wait for, and behind them where matrices of up to
   // landing_bytes land on their way to the host
+  struct Words {
+    double loss;
+    unsigned int status, unused;
+  };
   struct Mail {
-    double loss[2], last;  // of either input slot's step in flight, and what a blocking call asks for
-    unsigned int status;
+    Words slot[2], call;  // of either input slot's step in flight, and what a blocking call asks for
   };
   Mail* mail = nullptr;
   char* landing = nullptr;
@@ -288,32 +291,39 @@ cudaEvent_t phase_ev(b2_handle* h, int l, int phase, int end) {
 
 int check_comm(b2_handle* h);
 
-// The status word on its way to the host behind the main stream's work, and what it says once that stream has been waited for.
-int fetch_status(b2_handle* h) {
-  CK(h, cudaMemcpyAsync(&h->mail->status, h->status_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->s_main));
+// The loss of an input slot's last step and the status word on their way to the host behind the main stream's work, in one
+// copy of two rows (the status word lies behind both slots' blocks).
+int fetch_words(b2_handle* h, int slot, b2_handle::Words* to) {
+  static_assert(sizeof(b2_handle::Words) == 16, "two rows of 8 bytes");
+  CK(h, cudaMemcpy2DAsync(to, 8, loss_ptr(h, slot), (size_t)(2 - slot) * h->sync_bytes, 8, 2, cudaMemcpyDeviceToHost, h->s_main));
   return B2_OK;
 }
-int judge_status(b2_handle* h) {
-  const unsigned int st = h->mail->status;
-  if (st != 0) {
-    cudaMemset(h->status_dev, 0, sizeof st);
-    if (h->tc_ws_flags) cudaMemset(h->tc_ws_flags, 0, (size_t)h->sms * sizeof(unsigned int));
-    cudaMemset(h->sync_dev + 16, 0, sizeof(unsigned int));
-    h->small_count = 0;
-    if (st >= 100u) {  // a flag wait of the peer-memory allreduce: its call counters no longer agree
-      h->p2p_ready = false;
-      cudaMemset(h->p2p_ctas_done, 0, sizeof(unsigned int));
-      return fail(h, B2_ERR_TIMEOUT, "peer-memory allreduce gave up waiting for another rank (code %u); "
-                  "the peer path is switched off for this handle", st);
-    }
-    return fail(h, B2_ERR_TIMEOUT, "tensor-core GEMM gave up waiting on a pipeline barrier (role %u)", st);
+int status_error(b2_handle* h, unsigned int st) {
+  if (st >= 100u)
+    return fail(h, B2_ERR_TIMEOUT, "peer-memory allreduce gave up waiting for another rank (code %u); "
+                "the peer path is switched off for this handle", st);
+  if (st == STATUS_GRID_BARRIER) return fail(h, B2_ERR_TIMEOUT, "a launch of whole steps gave up waiting at a barrier between its blocks");
+  return fail(h, B2_ERR_TIMEOUT, "tensor-core GEMM gave up waiting on a pipeline barrier (role %u)", st);
+}
+// What a status word says that was fetched behind all work of the handle. What a wait that gave up left behind is set back
+// on the main stream, where the next work comes behind it.
+int judge_status(b2_handle* h, unsigned int st) {
+  if (st == 0) return check_comm(h);
+  CK(h, cudaMemsetAsync(h->status_dev, 0, sizeof st, h->s_main));
+  if (h->tc_ws_flags) CK(h, cudaMemsetAsync(h->tc_ws_flags, 0, (size_t)h->sms * sizeof(unsigned int), h->s_main));
+  CK(h, cudaMemsetAsync(h->sync_dev + 16, 0, sizeof(unsigned int), h->s_main));
+  h->small_count = 0;
+  if (st >= 100u) {  // a flag wait of the peer-memory allreduce: its call counters no longer agree
+    h->p2p_ready = false;
+    CK(h, cudaMemsetAsync(h->p2p_ctas_done, 0, sizeof(unsigned int), h->s_main));
   }
-  return check_comm(h);
+  CK(h, cudaStreamSynchronize(h->s_main));  // other streams' work too
+  return status_error(h, st);
 }
 int check_status(b2_handle* h) {
-  if (int rc = fetch_status(h)) return rc;
+  if (int rc = fetch_words(h, 0, &h->mail->call)) return rc;
   CK(h, cudaStreamSynchronize(h->s_main));
-  return judge_status(h);
+  return judge_status(h, h->mail->call.status);
 }
 
 // Asynchronous errors of the communicator (a peer process that died, a network fault): reported
@@ -656,6 +666,7 @@ void build_small_step(b2_handle* h) {
     h->small_step[slot] = s;
   }
   h->small_blocks = small_step_blocks(h->small_step[0], h->sms);
+  if (const char* ahead = getenv("B2_STEP_COUNT_AHEAD")) h->small_count = (unsigned int)atoi(ahead);  // tests: a wait that runs out
   h->launch_steps = small_step_steps(h->small_step[0]);
 }
 
@@ -1179,7 +1190,6 @@ void free_all(b2_handle* h) {
     if (h->ev_loss[i]) cudaEventDestroy(h->ev_loss[i]);
   }
   if (h->s_copy) cudaStreamDestroy(h->s_copy);
-  cudaFree(h->status_dev);
   cudaFree(h->fp_dev);
   cudaFree(h->tc_ws);
   cudaFree(h->tc_ws_flags);
@@ -1467,7 +1477,8 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     size_t words = 0;  // a counter per 128-row block and one per GEMM: fwd, dgrad (batch rows), wgrad (weight rows)
     for (int l = 0; l < L; ++l) words += 2 * ((bl + 127) / 128 + 1) + ((size_t)h->nf[l + 1] + 127) / 128 + 1;
     h->sync_bytes = (16 + words * sizeof(unsigned int) + 255) / 256 * 256;
-    TRY(dev_alloc(h, &h->sync_dev, 2 * h->sync_bytes));
+    TRY(dev_alloc(h, &h->sync_dev, 2 * h->sync_bytes + 256));  // and the status word
+    h->status_dev = reinterpret_cast<unsigned int*>(h->sync_dev + 2 * h->sync_bytes);
   }
   {
     size_t most = 0;  // the largest matrix that lands in one piece
@@ -1487,7 +1498,6 @@ int b2_create(const b2_config* cfg, b2_handle** out) {
     TRYCK(cudaEventCreateWithFlags(&h->ev_slot_free[i], cudaEventDisableTiming));
     TRYCK(cudaEventCreateWithFlags(&h->ev_loss[i], cudaEventDisableTiming));
   }
-  TRY(dev_alloc(h, &h->status_dev, sizeof(unsigned int)));
   TRY(dev_alloc(h, &h->fp_dev, sizeof(unsigned long long)));
   if (cfg->precision != B2_PREC_FP32 && !cfg->force_simt) {
     TRY(dev_alloc(h, &h->tc_ws, (size_t)h->sms * TC_WS_SLOT_BYTES));
@@ -1779,8 +1789,7 @@ static int run_steps(b2_handle* h, int iters, double* loss) {
   }
   if (!graph && !fused && (rc = join_streams(h))) return rc;
   CK(h, cudaEventRecord(h->ev_t1, h->s_main));
-  if ((rc = fetch_status(h))) return rc;
-  if (loss) CK(h, cudaMemcpyAsync(&h->mail->last, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
+  if ((rc = fetch_words(h, 0, &h->mail->call))) return rc;
   CK(h, cudaStreamSynchronize(h->s_main));
   if (!fused) {
     CK(h, cudaStreamSynchronize(h->s_comm));
@@ -1824,8 +1833,8 @@ static int run_steps(b2_handle* h, int iters, double* loss) {
     }
     if (cur_e >= 0.f) h->gemm_busy_ms += cur_e - cur_b;
   }
-  rc = judge_status(h);
-  if (rc == B2_OK && loss) *loss = h->mail->last;
+  rc = judge_status(h, h->mail->call.status);
+  if (rc == B2_OK && loss) *loss = h->mail->call.loss;
   return rc;
 }
 
@@ -1837,9 +1846,9 @@ int b2_step(b2_handle* h, int iters) {
 int b2_loss(b2_handle* h, double* loss) {
   ENTER(h);
   if (!loss) return fail(h, B2_ERR_INVALID, "null output");
-  CK(h, cudaMemcpyAsync(&h->mail->last, loss_ptr(h, 0), sizeof(double), cudaMemcpyDeviceToHost, h->s_main));
+  if (int rc = fetch_words(h, 0, &h->mail->call)) return rc;
   CK(h, cudaStreamSynchronize(h->s_main));
-  *loss = h->mail->last;
+  *loss = h->mail->call.loss;
   return B2_OK;
 }
 
@@ -1901,8 +1910,7 @@ int b2_train_step_host_async(b2_handle* h, const float* x, size_t ldx, const flo
   if ((rc = whole_steps(h, slot) ? enqueue_fused(h, slot, 1) : enqueue_step(h, false, slot))) return rc;
   CK(h, cudaEventRecord(h->ev_slot_free[slot], h->s_main));
   h->slot_used[slot] = true;
-  CK(h, cudaMemcpyAsync(h->mail->loss + slot, loss_ptr(h, slot), sizeof(double), cudaMemcpyDeviceToHost,
-                        h->s_main));
+  if ((rc = fetch_words(h, slot, &h->mail->slot[slot]))) return rc;
   CK(h, cudaEventRecord(h->ev_loss[slot], h->s_main));
   ++h->async_issued;
   ++h->steps;
@@ -1914,7 +1922,8 @@ int b2_wait_loss(b2_handle* h, double* loss) {
   if (h->async_waited >= h->async_issued) return fail(h, B2_ERR_STATE, "no step in flight");
   const int slot = (int)(h->async_waited & 1);
   CK(h, cudaEventSynchronize(h->ev_loss[slot]));
-  if (loss) *loss = h->mail->loss[slot];
+  const b2_handle::Words& words = h->mail->slot[slot];
+  if (loss) *loss = words.loss;
   ++h->async_waited;
   if (h->async_waited == h->async_issued) {  // pipeline drained: also let the updates finish
     int rc = join_streams(h);
@@ -1922,7 +1931,8 @@ int b2_wait_loss(b2_handle* h, double* loss) {
     CK(h, cudaStreamSynchronize(h->s_main));
     return check_status(h);
   }
-  return B2_OK;
+  // Set back once the step behind it has been waited for too, which finds the word as it is and fails in its turn.
+  return words.status ? status_error(h, words.status) : B2_OK;
 }
 
 int b2_host_alloc(void** ptr, size_t bytes) {

@@ -134,25 +134,25 @@ __device__ __forceinline__ void tile_sums(const Gemm& g, int m0, int n0, float* 
 }
 
 // All blocks (a cooperative launch) have come here: thread 0 of each counts itself in and waits, with a limit, until the
-// counter has gone `blocks` further. False when a wait gave up, here or elsewhere.
-__device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int until, unsigned int* status) {
+// counter has gone `blocks` further. False when a wait gave up, here or elsewhere, or `before` says that an earlier launch's
+// did: the counter is then behind the host's, and nothing is to be waited for until the host has set both back.
+__device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int until, unsigned int* status, unsigned int before) {
   __shared__ int ok_s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(counter, 1u);
+    bool ok = before == 0;
+    if (ok) {
+      __threadfence();
+      atomicAdd(counter, 1u);
+    }
     unsigned long long t0 = 0;
     unsigned int spins = 0;
-    bool ok = true;
-    while ((int)(ld_acquire_u32(counter) - until) < 0) {
+    while (ok && (int)(ld_acquire_u32(counter) - until) < 0) {
       if ((++spins & 0xFF) == 0) {
         const unsigned long long now = globaltimer();
         if (t0 == 0) t0 = now;
-        if (now - t0 > WAIT_LIMIT_NS) {
-          atomicCAS(status, 0u, 8u);
-          ok = false;
-          break;
-        }
+        if (now - t0 > WAIT_LIMIT_NS) atomicCAS(status, 0u, STATUS_GRID_BARRIER);
+        ok = ld_acquire_u32(status) == 0;
       }
     }
     ok_s = ok;
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(THREADS) small_step_kernel(const __grid_consta
         if (m + j < g.M && n < g.N) finish(g, m + j, n, acc[j], x[j]);
     }
   };
-  auto barrier = [&] { return grid_barrier(counter, count += blocks, status); };
+  const unsigned int before = threadIdx.x == 0 ? __ldcg(status) : 0;  // (no acquire: it would hold up the first copies)
+  auto barrier = [&] { return grid_barrier(counter, count += blocks, status, before); };
   for (int step = 0; step < steps; ++step) {
     if (rank == 0 && threadIdx.x == 0) *s.loss = 0.0;  // the additions follow behind a barrier
     if (L == 1 && !barrier()) return;

@@ -1,6 +1,7 @@
 """Whole steps of small fp32 networks in one launch (csrc/small_step.cu) against the launch-per-GEMM schedule of the same
 handle, at the edges of its tiles (16 x 32), groups of four k and layer table."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -93,6 +94,59 @@ def test_host_fed_steps(native, monkeypatch):
         want.append(b.train_step_host(px, 40, pt, 12))
     got.append(a.wait_loss())
     assert np.allclose(got, want, rtol=1e-12) and all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    a.close()
+    b.close()
+
+
+def late(monkeypatch, nf, batch):
+    """A handle that counts one more arrival at the barriers than there will be: the first wait of its first launch runs out."""
+    monkeypatch.setenv("B2_STEP_COUNT_AHEAD", "1")
+    m = make(monkeypatch, nf, batch, True)
+    monkeypatch.delenv("B2_STEP_COUNT_AHEAD")
+    return m
+
+
+def test_a_wait_that_runs_out(native, monkeypatch):
+    """One wait limit (2 s) for any number of launches queued behind the one that gave up; the call reports it, the weights
+    are as they were, and the next call runs."""
+    from tbb_test_b200 import _capi as K
+    nf, batch = [48, 64, 32], 20
+    a, b = late(monkeypatch, nf, batch), make(monkeypatch, nf, batch, True)
+    t0 = time.time()
+    with pytest.raises(K.B2Error) as e:
+        a.step(1000)
+    assert e.value.code == K.ERR_TIMEOUT and time.time() - t0 < 3.5
+    assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    a.step(130)
+    b.step(130)
+    assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    a.close()
+    b.close()
+
+
+def test_a_wait_that_runs_out_in_the_pipeline(native, monkeypatch):
+    """With steps in flight every wait reports it until the pipeline has been drained, and none passes for a step."""
+    from tbb_test_b200 import _capi as K
+    nf, batch = [48, 64, 32], 20
+    fp = C.POINTER(C.c_float)
+    a, b = late(monkeypatch, nf, batch), make(monkeypatch, nf, batch, True)
+    x, t = np.full((batch, 48), 0.25, np.float32), np.ones((batch, 32), np.float32)
+    args = x.ctypes.data_as(fp), 48, t.ctypes.data_as(fp), 32
+    t0 = time.time()
+    a.train_step_host_async(*args)
+    for _ in range(3):  # a loader that keeps two in flight
+        a.train_step_host_async(*args)
+        with pytest.raises(K.B2Error) as e:
+            a.wait_loss()
+        assert e.value.code == K.ERR_TIMEOUT
+    with pytest.raises(K.B2Error):
+        a.wait_loss()
+    assert time.time() - t0 < 3.5 and all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    for m in (a, b):
+        m.train_step_host_async(*args)
+        m.train_step_host_async(*args)
+        m.wait_loss(), m.wait_loss()
+    assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
     a.close()
     b.close()
 
