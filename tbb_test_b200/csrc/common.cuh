@@ -73,8 +73,8 @@ bool gemm_simt_small(const GemmDesc& g);  // served by one of its kernels for sm
 bool gemm_simt_short_sums(const GemmDesc& g);  // its sums are partial ones of K / 16 or K / 32 terms and not one in k order
 
 // GEMM of fp32 matrices on the tensor cores at fp32 precision, any alignment (gemm_split.cu), where it is faster than
-// gemm_simt_launch; on at most `sms` SMs; `status` as for gemm_tc_launch.
-bool gemm_split_serves(const GemmDesc& g);
+// gemm_simt_launch; on at most `sms` SMs, which decide that too; `status` as for gemm_tc_launch.
+bool gemm_split_serves(const GemmDesc& g, int sms);
 cudaError_t gemm_split_launch(const GemmDesc& g, int sms, cudaStream_t stream, unsigned int* status);
 
 // Tensor-core (tcgen05 + TMA + TMEM) GEMM. in_type T_BF16 -> kind::f16 (bf16),

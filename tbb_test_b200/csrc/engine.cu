@@ -46,6 +46,7 @@ struct Site {
   GemmDesc d;
   TcPlan* plan = nullptr;
   bool split = false;      // without a plan: fp32 operands cut into bf16 pieces (gemm_split.cu) instead of the CUDA cores
+  int sms = 0;             // that the tensor-core kernels may take
   bool active = false;
 };
 
@@ -241,10 +242,11 @@ int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
   s.d.pad_writable = 1;  // rows of b2_handle::ld elements
   s.active = s.d.M > 0 && s.d.N > 0 && s.d.K > 0;
   s.plan = nullptr;
-  s.split = s.active && !h->cfg.force_simt && gemm_split_serves(s.d);
+  s.sms = sms > 0 ? sms : h->gemm_sms;
+  s.split = s.active && !h->cfg.force_simt && gemm_split_serves(s.d, s.sms);
   if (!s.active || !want_tc) return B2_OK;
   char why[128] = "";
-  s.plan = gemm_tc_plan_create(s.d, sms > 0 ? sms : h->gemm_sms, why, sizeof why);
+  s.plan = gemm_tc_plan_create(s.d, s.sms, why, sizeof why);
   if (!s.plan) {
     // the fp32 kernels serve this site (cut operands about 10 x slower than bf16, CUDA cores 30 x): counted, the first reason kept
     // for b2_site_report, and announced once per handle when B2_VERBOSE is set
@@ -263,8 +265,8 @@ int make_site(b2_handle* h, Site& s, bool want_tc, int sms = 0) {
 }
 
 // A GEMM that no plan serves.
-cudaError_t launch_unplanned(const b2_handle* h, const GemmDesc& d, bool split, cudaStream_t st) {
-  return split ? gemm_split_launch(d, h->gemm_sms, st, h->status_dev) : gemm_simt_launch(d, st);
+cudaError_t launch_unplanned(const b2_handle* h, const GemmDesc& d, bool split, int sms, cudaStream_t st) {
+  return split ? gemm_split_launch(d, sms, st, h->status_dev) : gemm_simt_launch(d, st);
 }
 
 int run_site(b2_handle* h, const Site& s, cudaStream_t st) {
@@ -274,7 +276,7 @@ int run_site(b2_handle* h, const Site& s, cudaStream_t st) {
     ++h->tc_launches;
     CK(h, gemm_tc_launch(s.plan, st, h->status_dev));
   } else {
-    CK(h, launch_unplanned(h, s.d, s.split, st));
+    CK(h, launch_unplanned(h, s.d, s.split, s.sms, st));
     if (s.d.C_lo) {  // fp32-class mode: the fp32 kernels served this site, so its result's twin is made here
       CK(h, split_lo_launch(static_cast<const float*>(s.d.C), static_cast<float*>(s.d.C_lo), (size_t)s.d.M * s.d.N, st));
       ++h->launches;
@@ -2377,6 +2379,7 @@ int b2_gemm_bench(b2_handle* h, int form, int m, int n, int k, int precision, in
   const bool x3 = precision == B2_PREC_FP32_TC && !h->cfg.force_simt;
   int rc = B2_OK;
   const bool tc = precision != B2_PREC_FP32 && !h->cfg.force_simt;
+  const int grid_sms = sms > 0 && sms <= h->sms ? sms : h->sms;
   // B2_TC_TRACE=1: per-tile timeline of CTA 0 of the last timed launch, printed to stderr
   unsigned long long* trace_dev = nullptr;
   if (tc && getenv("B2_TC_TRACE")) {
@@ -2424,7 +2427,7 @@ int b2_gemm_bench(b2_handle* h, int form, int m, int n, int k, int precision, in
       d.trace = trace_dev;
       if (tc) {
         char why[128] = "";
-        s.plan = gemm_tc_plan_create(d, sms > 0 && sms <= h->sms ? sms : h->sms, why, sizeof why);
+        s.plan = gemm_tc_plan_create(d, grid_sms, why, sizeof why);
         if (!s.plan) rc = fail(h, B2_ERR_UNSUPPORTED, "tensor-core kernel refuses this GEMM: %s", why);
         // like the step: the ReLU bit plane (here: the first bytes of the auxiliary buffer) is written
         // by a forward epilogue and read by an input-gradient epilogue instead of the activation
@@ -2442,7 +2445,7 @@ int b2_gemm_bench(b2_handle* h, int form, int m, int n, int k, int precision, in
         ++h->tc_launches;
         return gemm_tc_launch(s.plan, h->s_main, h->status_dev);
       }
-      return launch_unplanned(h, s.d, !h->cfg.force_simt && gemm_split_serves(s.d), h->s_main);
+      return launch_unplanned(h, s.d, !h->cfg.force_simt && gemm_split_serves(s.d, grid_sms), grid_sms, h->s_main);
     };
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < warmup && e == cudaSuccess; ++i) e = run(i);
@@ -2567,7 +2570,7 @@ static int gemm_common(b2_handle* h, int precision, GemmDesc& d, cudaStream_t st
     e = gemm_tc_launch(plan, st, h->status_dev);
     gemm_tc_plan_destroy(plan);  // the tensor maps were passed by value at launch
   } else {
-    e = launch_unplanned(h, d, !h->cfg.force_simt && gemm_split_serves(d), st);
+    e = launch_unplanned(h, d, !h->cfg.force_simt && gemm_split_serves(d, h->sms), h->sms, st);
   }
   if (e != cudaSuccess) return fail(h, B2_ERR_CUDA, "GEMM launch: %s", cudaGetErrorString(e));
   return B2_OK;

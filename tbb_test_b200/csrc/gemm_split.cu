@@ -13,7 +13,6 @@ namespace {
 constexpr int BN = 64;       // columns of a tile; its rows are the 128 lanes of TMEM
 constexpr int CHUNK_K = 64;  // elements of K per stage
 constexpr int STAGES = 3;
-constexpr int SMS = 148;
 // warps: sixteen load, cut and store the operands, eight add up the chunks and store C, one thread of the last issues the MMAs
 constexpr int CUT_WARPS = 16, SUM_WARPS = 8, MMA_WARP = CUT_WARPS + SUM_WARPS, SPLIT_THREADS = (MMA_WARP + 1) * 32;
 constexpr uint32_t B_PLANE = BN * 128;  // bytes of one piece of B's chunk
@@ -556,12 +555,12 @@ cudaError_t launch(const SplitParams& p, int sms, cudaStream_t stream) {
 // faster one is missed by 2 % on average): here 6 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte
 // pieces; gemm_simt.cu 4.5 and the longer of 24 (28) per 1000 k and the flops at 33 (30) TFLOP/s. Sums of fewer than 64 terms
 // stay there: neither faster here nor more precise.
-bool gemm_split_serves(const GemmDesc& g) {
+bool gemm_split_serves(const GemmDesc& g, int sms) {
   if (g.in_type != T_F32 || g.out_type != T_F32 || g.M <= 16 || g.N <= 16 || g.K < 64) return false;
   if ((g.sAk != 1 && g.sAm != 1) || (g.sBk != 1 && g.sBn != 1)) return false;
   const long long tiles = (long long)((g.M + 127) / 128) * ((g.N + BN - 1) / BN);
   if (tiles > 1 << 30) return false;
-  const double rounds = (double)((tiles + SMS - 1) / SMS), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
+  const double rounds = (double)((tiles + sms - 1) / sms), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
   const bool whole = how_to_read(g) != FLOATS;
   const double here = 6.0 + rounds * chunks * (whole ? 0.85 : 1.35);
   return here <= 4.5 + std::max((whole ? 0.024 : 0.028) * g.K, (double)g.M * g.N * g.K / (whole ? 16.5e6 : 15e6));

@@ -97,3 +97,22 @@ def test_values_at_the_ends_of_the_range(devs, oracle, form, shape, kind):
         ref = (a.T if ta else a).astype(np.float64) @ (b.T if tb else b).astype(np.float64) + (0 if c is None else beta * c)
     if ok.any():
         assert np.linalg.norm(got[ok] - ref[ok]) <= np.linalg.norm(fma[ok] - ref[ok])
+
+
+def test_the_choice_counts_the_sms_of_the_launch(native, monkeypatch):
+    """A forward GEMM of 3 x 47 tiles and one chunk of k: one round on 148 SMs, where the tensor cores are estimated faster,
+    but two on the 128 that are left when 20 are reserved, where FMAs are."""
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    monkeypatch.setenv("B2_STEP_KERNEL", "0")
+    rng = np.random.default_rng(6)
+    w, x = (rng.uniform(-1, 1, s).astype(np.float32) for s in ((2945, 64), (257, 64)))
+    y = []
+    for kw in (dict(), dict(comm_sms=20), dict(force_simt=True)):
+        m = MLP([64, 2945], 257, precision=K.PREC_FP32, mode=K.MODE_REF, **kw)
+        m.upload_weights(0, w)
+        m.upload_input(x)
+        m.step(1)
+        y.append(m.activation(1))
+        m.close()
+    assert not np.array_equal(y[0], y[2]) and np.array_equal(y[1], y[2])
