@@ -70,11 +70,13 @@ cudaError_t gemm_simt_launch(const GemmDesc& g, cudaStream_t stream);
 bool gemm_f32_serves(const GemmDesc& g);
 cudaError_t gemm_f32_launch(const GemmDesc& g, cudaStream_t stream);
 bool gemm_simt_small(const GemmDesc& g);  // served by one of its kernels for small grids (unless large_tiles)
+double gemm_simt_us(const GemmDesc& g);  // estimate (fp32)
 bool gemm_simt_short_sums(const GemmDesc& g);  // its sums are partial ones of K / 16 or K / 32 terms and not one in k order
 
 // GEMM of fp32 matrices on the tensor cores at fp32 precision, any alignment (gemm_split.cu), where it is faster than
 // gemm_simt_launch; on at most `sms` SMs, which decide that too; `status` as for gemm_tc_launch.
 bool gemm_split_serves(const GemmDesc& g, int sms);
+double gemm_split_us(const GemmDesc& g, int sms);  // estimate
 cudaError_t gemm_split_launch(const GemmDesc& g, int sms, cudaStream_t stream, unsigned int* status);
 
 // Tensor-core (tcgen05 + TMA + TMEM) GEMM. in_type T_BF16 -> kind::f16 (bf16),
@@ -148,8 +150,8 @@ struct SmallStep {
   double loss_scale;
   double* loss;
 };
-bool small_step_serves(const SmallStep& s);
-int small_step_steps(const SmallStep& s);  // that one launch should take
+bool small_step_serves(const SmallStep& s, int sms, double launches_us);  // launches_us: a step as a launch per GEMM
+int small_step_steps(const SmallStep& s, int sms);  // that one launch should take
 int small_step_blocks(const SmallStep& s, int sms);
 // Barriers of a launch: each adds `blocks` to *counter, which stands at `count` before the launch. A launch that finds *status
 // set (a wait of an earlier one gave up, so the counter is behind) touches neither counter nor weights.

@@ -633,6 +633,16 @@ StepShape step_shape(const b2_handle* h) {
 
 bool whole_steps(const b2_handle* h, int slot) { return h->step_plan[slot] || h->small_step[slot].L > 0; }
 
+// Time of a step as a launch per GEMM in fp32, us: forward and input gradients in a chain, the weight gradients beside it and the
+// updates, by the kernels' own estimates. Within 0.82 and 1.23 of the time measured for 250 networks at batches above 16.
+double launches_us(const b2_handle* h) {
+  auto us = [&](const Site& s) { return !s.active ? 0.0 : s.split ? gemm_split_us(s.d, s.sms) : gemm_simt_us(s.d); };
+  double sum = 7.7;
+  for (int l = 0; l < h->L; ++l)
+    sum += 0.82 * (us(h->fwd[l]) + us(h->dgrad[l])) + 0.95 * us(h->wgrad[l]) + 4.8e-6 * (double)layer_elems(h, l);
+  return sum;
+}
+
 // Small fp32 networks: the same on the CUDA cores (small_step.cu).
 void build_small_step(b2_handle* h) {
   const char* e = getenv("B2_STEP_KERNEL");  // experiments: 0 never, 1 whatever the size
@@ -664,12 +674,12 @@ void build_small_step(b2_handle* h) {
     s.inv_batch = 1.0f / (float)h->cfg.batch;
     s.loss_scale = baseline ? 1.0 / (double)h->cfg.batch : 1.0;
     s.loss = loss_ptr(h, slot);
-    if (!(e && e[0] == '1') && !small_step_serves(s)) return;
+    if (!(e && e[0] == '1') && !small_step_serves(s, h->sms, launches_us(h))) return;
     h->small_step[slot] = s;
   }
   h->small_blocks = small_step_blocks(h->small_step[0], h->sms);
   if (const char* ahead = getenv("B2_STEP_COUNT_AHEAD")) h->small_count = (unsigned int)atoi(ahead);  // tests: a wait that runs out
-  h->launch_steps = small_step_steps(h->small_step[0]);
+  h->launch_steps = small_step_steps(h->small_step[0], h->sms);
 }
 
 // The plans of the networks whose whole steps run as one launch (step_kernel.cu; the rules: step_choice.h).

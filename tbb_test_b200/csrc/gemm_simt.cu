@@ -8,6 +8,8 @@
 //   gemm_narrow_kernel  N <= 16 with K contiguous in both operands (the forward GEMM of a
 //                       narrow output layer): lanes split K
 //   gemm_short_kernel   M <= 16 with N contiguous in B (the weight gradient of that layer): warps split K
+#include <algorithm>
+
 #include "common.cuh"
 #include "simt_tile.h"
 
@@ -311,6 +313,16 @@ cudaError_t launch(const GemmDesc& g, cudaStream_t stream) {
 }  // namespace
 
 bool gemm_simt_small(const GemmDesc& g) { return narrow_form(g) || short_form(g) || gemm_f32_serves(g); }
+
+// us: 4.5 and the longer of 24 (28 where rows are not whole 16-byte pieces) per 1000 k and the flops at 33 (30) TFLOP/s; narrow
+// and short forms 15 and 76 per 1000 k, roughly (their columns and rows count too).
+double gemm_simt_us(const GemmDesc& g) {
+  if (narrow_form(g)) return 4.5 + 0.015 * g.K;
+  if (short_form(g)) return 4.5 + 0.076 * g.K;
+  auto whole = [](const void* p, long long ld) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld % 4 == 0; };
+  const bool a = g.sAk != 1 || whole(g.A, g.sAm), b = whole(g.B, g.sBk == 1 ? g.sBn : g.sBk);
+  return 4.5 + std::max((a && b ? 0.024 : 0.028) * g.K, (double)g.M * g.N * g.K / (a && b ? 16.5e6 : 15e6));
+}
 
 bool gemm_simt_short_sums(const GemmDesc& g) { return narrow_form(g) || short_form(g); }
 

@@ -551,19 +551,21 @@ cudaError_t launch(const SplitParams& p, int sms, cudaStream_t stream) {
 
 }  // namespace
 
-// By the time of either side, us, fitted to 110 shapes of 16 to 4096 rows, columns and k in the three forms of the step (the
-// faster one is missed by 2 % on average): here 6 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte
-// pieces; gemm_simt.cu 4.5 and the longer of 24 (28) per 1000 k and the flops at 33 (30) TFLOP/s. Sums of fewer than 64 terms
-// stay there: neither faster here nor more precise.
+// us: 6 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte pieces.
+double gemm_split_us(const GemmDesc& g, int sms) {
+  const long long tiles = (long long)((g.M + 127) / 128) * ((g.N + BN - 1) / BN);
+  const double rounds = (double)((tiles + sms - 1) / sms), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
+  return 6.0 + rounds * chunks * (how_to_read(g) != FLOATS ? 0.85 : 1.35);
+}
+
+// By the estimates of both sides, fitted to 110 shapes of 16 to 4096 rows, columns and k in the three forms of the step (the
+// faster one is missed by 2 % on average). Sums of fewer than 64 terms stay on the CUDA cores: neither faster here nor more
+// precise.
 bool gemm_split_serves(const GemmDesc& g, int sms) {
   if (g.in_type != T_F32 || g.out_type != T_F32 || g.M <= 16 || g.N <= 16 || g.K < 64) return false;
   if ((g.sAk != 1 && g.sAm != 1) || (g.sBk != 1 && g.sBn != 1)) return false;
-  const long long tiles = (long long)((g.M + 127) / 128) * ((g.N + BN - 1) / BN);
-  if (tiles > 1 << 30) return false;
-  const double rounds = (double)((tiles + sms - 1) / sms), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
-  const bool whole = how_to_read(g) != FLOATS;
-  const double here = 6.0 + rounds * chunks * (whole ? 0.85 : 1.35);
-  return here <= 4.5 + std::max((whole ? 0.024 : 0.028) * g.K, (double)g.M * g.N * g.K / (whole ? 16.5e6 : 15e6));
+  if ((long long)((g.M + 127) / 128) * ((g.N + BN - 1) / BN) > 1 << 30) return false;
+  return gemm_split_us(g, sms) <= gemm_simt_us(g);
 }
 
 cudaError_t gemm_split_launch(const GemmDesc& g, int sms, cudaStream_t stream, unsigned int* status) {

@@ -1,5 +1,6 @@
 // Whole training steps of small fp32 networks in one launch.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 
@@ -278,8 +279,36 @@ __global__ void __launch_bounds__(THREADS) small_step_kernel(const __grid_consta
 
 int small_step_barriers(const SmallStep& s, int steps) { return steps * (2 * s.L + 1 + (s.L == 1)) - 1; }
 
+namespace {
+
+int tiles(int m, int n) { return ((m + TILE_M - 1) / TILE_M) * ((n + TILE_N - 1) / TILE_N); }
+
+// Time of a step, us: for each phase 1.6 and the longer of what its tiles take on all SMs, 0.59 and 0.0111 per k each, and what
+// a group of warps takes for its share of either GEMM's, 0.59 and 0.0172 per k a tile; 1.29 times the terms of k where rows are
+// not whole 16-byte pieces. Within 0.82 and 1.21 of the time measured for 400 networks of 1 to 16 layers, 1 to 8192 wide, batches
+// of 1 to 2048 (4 x 4096, batch 1 904 us, 1 ms estimated; the weights alone, read and written, are 2 x 67 MB each).
+double step_us(const SmallStep& s, int sms) {
+  struct Load { double all, longest; };
+  auto gemm = [&](int m, int n, int k, bool whole) {
+    const double of_k = k * (whole ? 1.0 : 1.29), n_tiles = tiles(m, n);
+    return Load{n_tiles * (0.59 + 0.0111 * of_k) / sms, std::ceil(n_tiles / (GROUPS * sms)) * (0.59 + 0.0172 * of_k)};
+  };
+  auto phase = [](Load a, Load b) { return 1.6 + std::max(a.all + b.all, std::max(a.longest, b.longest)); };
+  auto whole = [](int a, int b) { return a % 4 == 0 && b % 4 == 0; };
+  double us = 0;
+  Load above{0, 0};  // the weight gradient of the layer above
+  for (int l = s.L - 1; l >= 0; --l) {
+    const SmallLayer& y = s.layer[l];
+    us += phase(gemm(s.batch, y.fo, y.fi, whole(y.fi, y.fi)), Load{0, 0});
+    us += phase(l > 0 || s.input_grad ? gemm(s.batch, y.fi, y.fo, whole(y.fo, y.fi)) : Load{0, 0}, above);
+    above = gemm(y.fo, y.fi, s.batch, whole(y.fo, y.fi));
+  }
+  return us + phase(above, Load{0, 0});
+}
+
+}  // namespace
+
 int small_step_blocks(const SmallStep& s, int sms) {
-  auto tiles = [](int m, int n) { return ((m + TILE_M - 1) / TILE_M) * ((n + TILE_N - 1) / TILE_N); };
   int most = 1;
   for (int l = 0; l < s.L; ++l) {
     const SmallLayer& y = s.layer[l];
@@ -294,22 +323,23 @@ int small_step_blocks(const SmallStep& s, int sms) {
 // million) 127 and 152; 192-608-..., batch 699 (55) 348 and 380; 8 x 384, batch 436 (64) 307 and 258; others: 7 layers of 39 to 356,
 // batch 2044 (40) 438 and 569; 5 of 157 to 948, batch 303 (49) 202 and 239; 8 of 32 to 724, batch 924 (49) 376 and 335). A weight
 // gradient's sum walks the batch on one SM, and batches above 2048 have not been weighed.
-bool small_step_serves(const SmallStep& s) {
+// Below that, large layers among small ones, which a GEMM each serves better: where the estimate of a step is 1.15 times the one of
+// separate launches (`launches_us`), as both are that exact (2048-2048-32-..., 14 layers, batch 128 355 and 305; 541-493-2742-10,
+// batch 56 186 and 154; 64-5504, batch 82 107 and 89; left here: 64-1920-32-448-2912-1440, batch 37 275 and 228, the worst of 330).
+// Batches of up to 16 are always faster here, whatever the widths: gemm_short_kernel walks K with 16 warps (4 x 4096, batch 2
+// 906 and 1197; 4 x 2048, batch 8 362 and 1087).
+bool small_step_serves(const SmallStep& s, int sms, double launches_us) {
   double macs = 0;
   bool whole = true;
   for (int l = 0; l < s.L; ++l) {
     macs += (double)s.batch * s.layer[l].fi * s.layer[l].fo;
     whole = whole && s.layer[l].fi % 4 == 0 && s.layer[l].fo % 4 == 0;
   }
-  return s.batch <= 2048 && macs <= s.L * (whole ? 48e6 : 40e6);
+  return s.batch <= 2048 && macs <= s.L * (whole ? 48e6 : 40e6) && (s.batch <= 16 || step_us(s, sms) <= 1.15 * launches_us);
 }
 
-// Steps that take about 2 ms (a launch may hold every SM), by 2.9 us per phase and the GEMMs at 10 TFLOP/s.
-int small_step_steps(const SmallStep& s) {
-  double us = 2.9 * (2 * s.L + 1);
-  for (int l = 0; l < s.L; ++l) us += 6.0 * s.batch * s.layer[l].fi * s.layer[l].fo / 10e6;
-  return std::max(1, std::min(64, (int)(2000 / us)));
-}
+// Steps that take about 2 ms (a launch may hold every SM).
+int small_step_steps(const SmallStep& s, int sms) { return std::max(1, std::min(64, (int)(2000 / step_us(s, sms)))); }
 
 cudaError_t small_step_launch(const SmallStep& s, int blocks, int steps, float lr, unsigned int count, unsigned int* counter,
                               unsigned int* status, cudaStream_t stream) {

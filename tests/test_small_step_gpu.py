@@ -98,6 +98,19 @@ def test_host_fed_steps(native, monkeypatch):
     b.close()
 
 
+@pytest.mark.parametrize("net", [([4096] * 5, 1), ([2048] * 3, 8), ([16384, 256, 10], 4), ([64] * 10, 1), ([128, 256, 128, 64], 32)],
+                         ids=lambda n: f"{'-'.join(map(str, n[0][:3]))}b{n[1]}")
+def test_launches_last_about_2_ms(native, monkeypatch, net):
+    """A launch holds every SM. (64 steps at most; the estimate of a step is within 0.82 and 1.21 of its time.)"""
+    m = make(monkeypatch, *net, True)
+    n = launches(m, lambda: m.step(128))
+    m.reset_timing()
+    m.step(128)
+    launch_ms = m.timing()[1] / n
+    assert launch_ms <= 2.0 / 0.8 and (n == 2 or launch_ms >= 0.5), (n, launch_ms)
+    m.close()
+
+
 def late(monkeypatch, nf, batch):
     """A handle that counts one more arrival at the barriers than there will be: the first wait of its first launch runs out."""
     monkeypatch.setenv("B2_STEP_COUNT_AHEAD", "1")
@@ -152,10 +165,11 @@ def test_a_wait_that_runs_out_in_the_pipeline(native, monkeypatch):
 
 
 def test_what_it_does_not_serve(native, monkeypatch):
-    """More layers than its table, large networks, serial schedules and the tensor-core precisions keep their paths."""
+    """More layers than its table, large networks, a large layer among small ones and serial schedules keep their paths."""
     from tbb_test_b200 import _capi as K
     from tbb_test_b200.mlp import MLP
-    for nf, batch, kw in (([20] * 18, 50, {}), ([1024, 1024], 256, {}), ([64, 64], 4096, {}), ([64, 64], 32, dict(overlap=False))):
+    for nf, batch, kw in (([20] * 18, 50, {}), ([1024, 1024], 256, {}), ([64, 64], 4096, {}), ([2048] * 2 + [32] * 13, 128, {}),
+                       ([64, 64], 32, dict(overlap=False))):
         m = MLP(nf, batch, precision=K.PREC_FP32, **kw)
         assert launches(m, lambda: m.step(1)) > 1
         m.close()
