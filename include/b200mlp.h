@@ -51,7 +51,8 @@ typedef enum {
   B2_PREC_FP32 = 0, /* fp32 operands at fp32 precision (parity mode): small GEMMs as CUDA-core FMAs in k order; large ones
                        on the tensor cores as products of exact three-way bf16 splits whose sums are rounded in
                        fp32, with a smaller error against 64-bit sums than the FMAs' and the same results where
-                       operands or sums are not finite (csrc/gemm_split.cu). With force_simt: FMAs only */
+                       operands or sums are not finite (which take up to three times the FMAs' time, where they are
+                       many; csrc/gemm_split.cu). With force_simt: FMAs only */
   B2_PREC_TF32 = 1, /* fp32 storage, tcgen05 kind::tf32 */
   B2_PREC_BF16 = 2, /* bf16 operands (activations, gradients, a bf16 weight copy),
                        tcgen05 kind::f16: layers of any width, on rows padded to 16 bytes (but for

@@ -17,7 +17,7 @@ constexpr int STAGES = 3;
 constexpr int CUT_WARPS = 16, SUM_WARPS = 8, MMA_WARP = CUT_WARPS + SUM_WARPS, SPLIT_THREADS = (MMA_WARP + 1) * 32;
 constexpr uint32_t B_PLANE = BN * 128;  // bytes of one piece of B's chunk
 constexpr uint32_t B_STAGE = 3 * B_PLANE;
-constexpr int SMEM_BYTES = 146 * 1024;  // the stages and what plain_rows needs; one block per SM, whose whole TMEM it takes
+constexpr int SMEM_BYTES = 146 * 1024;  // the stages and what plain_part needs; one block per SM, whose whole TMEM it takes
 // TMEM columns: D0, D1, D2, then the pieces of A's chunk (32 columns of two bf16 each) per stage
 constexpr uint32_t T_D1 = BN, T_A = 3 * BN, A_HALF = 6 * 8, A_STAGE = 2 * A_HALF, T_ALL = 512;
 static_assert(T_A + STAGES * A_STAGE <= T_ALL, "TMEM");
@@ -227,16 +227,11 @@ __device__ __forceinline__ void finish(const GemmDesc& g, int gm, int gn, float 
   if (g.epilogue == EPI_MASK) v = __ldg(static_cast<const float*>(g.aux) + (long long)gm * g.ldaux + gn) > 0.f ? v : 0.f;
   *c = v;
 }
-// A warp's 32 rows of C from row m0 and 32 columns from n0 on, a lane a row in `v`, through shared memory of the warp's own, so
-// that a store writes four whole 128-byte lines (a lane storing its own row, 32 bytes at a time, took 3100 clocks per tile).
+// A warp's 32 rows of C from row m0 and 32 columns from n0 on, from shared memory of the warp's own, so that a store writes
+// four whole 128-byte lines (a lane storing its own row, 32 bytes at a time, took 3100 clocks per tile).
 constexpr int OUT_PITCH = 32 + 4;
-__device__ __forceinline__ void finish_part(const SplitParams& p, int m0, int n0, float* sh, int lane, const float (&v)[32]) {
+__device__ __forceinline__ void finish_part(const SplitParams& p, int m0, int n0, const float* sh, int lane) {
   const GemmDesc& g = p.g;
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 32; j += 4)
-    *reinterpret_cast<float4*>(sh + lane * OUT_PITCH + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-  __syncwarp();
   const int gn = n0 + (lane & 7) * 4;
 #pragma unroll 4
   for (int i = 0; i < 32; i += 4) {
@@ -260,41 +255,77 @@ __device__ __forceinline__ void finish_part(const SplitParams& p, int m0, int n0
   }
 }
 
-// The same part of C by FMAs in k order, a lane a row.
-constexpr int PLAIN_A = 32 + 1, PLAIN_B = 32 + 4, PLAIN_BYTES = 32 * (PLAIN_A + PLAIN_B) * 4;
+// The same part of C by FMAs in k order: 16 k of both operands at a time as k-rows of 32 by cp.async, the next ones under way
+// while these are multiplied; a lane has eight rows and four columns. Bound by the twelve floats that a lane reads for 32 FMAs
+// (more accumulators have no registers) and their latency. us, operands all NaN, forward / weight / input gradient, CUDA-core
+// kernels, here, and here with a lane to a row and no loads ahead: 1024^3 73/65/69, 125/116/120, 204/508/333; 2048^3 434/425/427,
+// 933/873/891, 1552/4026/2620. (All eight warps on one slab of 128 x 64: 113/112/110, but 1 to 3 % on finite operands.)
+constexpr int PLAIN_K = 16, PLAIN_STAGE = 2 * PLAIN_K * OUT_PITCH, PLAIN_BYTES = 2 * PLAIN_STAGE * 4;
 static_assert(PLAIN_BYTES >= 32 * OUT_PITCH * 4, "finish_part's room");
 static_assert(SMEM_BYTES >= 1024 + STAGES * (int)B_STAGE + SUM_WARPS * PLAIN_BYTES, "shared memory");
-template <bool AK, bool BK>
-__device__ __forceinline__ void plain_rows(const GemmDesc& g, int m0, int n0, float* sh, int lane, float (&acc)[32]) {
-  float* const sa = sh + 32 * PLAIN_B;
-  const float* const A = static_cast<const float*>(g.A);
-  const float* const B = static_cast<const float*>(g.B);
-#pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-#pragma unroll 1
-  for (int k0 = 0; k0 < g.K; k0 += 32) {
-    __syncwarp();
+template <bool KMAJOR>
+__device__ __forceinline__ void plain_copy(uint32_t dst, const void* base, long long s_mn, long long s_k, int mn0, int mn_end, int k0, int k_end,
+                                           int lane) {
+  // K contiguous: a lane has one k of every other row, else every k of one
+  int mn = mn0 + (KMAJOR ? lane >> 4 : lane), k = k0 + (KMAJOR ? lane & 15 : 0);
+  const float* p = static_cast<const float*>(base) + mn * s_mn + k * s_k;
+  uint32_t at = dst + (uint32_t)((k - k0) * OUT_PITCH + mn - mn0) * 4;
 #pragma unroll 4
-    for (int i = 0; i < 32; ++i) {
-      const int m = AK ? i : lane, ka = AK ? lane : i, n = BK ? i : lane, kb = BK ? lane : i;
-      sa[m * PLAIN_A + ka] = m0 + m < g.M && k0 + ka < g.K ? __ldg(A + (m0 + m) * g.sAm + (k0 + ka) * g.sAk) : 0.f;
-      sh[kb * PLAIN_B + n] = n0 + n < g.N && k0 + kb < g.K ? __ldg(B + (n0 + n) * g.sBn + (k0 + kb) * g.sBk) : 0.f;
-    }
-    __syncwarp();
-    const int end = min(32, g.K - k0);
-#pragma unroll 1
-    for (int k = 0; k < end; ++k) {
-      const float a = sa[lane * PLAIN_A + k];
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        const float4 b = *reinterpret_cast<const float4*>(sh + k * PLAIN_B + j);
-        acc[j] = fmaf(a, b.x, acc[j]);
-        acc[j + 1] = fmaf(a, b.y, acc[j + 1]);
-        acc[j + 2] = fmaf(a, b.z, acc[j + 2]);
-        acc[j + 3] = fmaf(a, b.w, acc[j + 3]);
-      }
+  for (int i = 0; i < 16; ++i) {
+    const bool in = mn < mn_end && k < k_end;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at), "l"(in ? p : static_cast<const float*>(base)), "r"(in ? 4 : 0) : "memory");
+    if (KMAJOR) {
+      mn += 2;
+      p += 2 * s_mn;
+      at += 2 * 4;
+    } else {
+      ++k;
+      p += s_k;
+      at += OUT_PITCH * 4;
     }
   }
+}
+template <bool AK, bool BK>
+__device__ __forceinline__ void plain_part(const GemmDesc& g, int m0, int n0, float* sh, int lane) {
+  const uint32_t at = smem_u32(sh);
+  auto copy = [&](int k0) {
+    if (k0 < g.K) {
+      const uint32_t to = at + (uint32_t)(k0 / PLAIN_K & 1) * (PLAIN_STAGE * 4);
+      plain_copy<AK>(to, g.A, g.sAm, g.sAk, m0, g.M, k0, g.K, lane);
+      plain_copy<BK>(to + PLAIN_K * OUT_PITCH * 4, g.B, g.sBn, g.sBk, n0, g.N, k0, g.K, lane);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int row = (lane >> 3) * 8, col = (lane & 7) * 4;
+  float acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  copy(0);
+#pragma unroll 1
+  for (int k0 = 0; k0 < g.K; k0 += PLAIN_K) {
+    copy(k0 + PLAIN_K);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const float* const a = sh + (k0 / PLAIN_K & 1) * PLAIN_STAGE + row;
+    const float* const b = sh + (k0 / PLAIN_K & 1) * PLAIN_STAGE + PLAIN_K * OUT_PITCH + col;
+    const int end = min(PLAIN_K, g.K - k0);
+#pragma unroll 2
+    for (int k = 0; k < end; ++k) {
+      const float4 u = *reinterpret_cast<const float4*>(a + k * OUT_PITCH), v = *reinterpret_cast<const float4*>(a + k * OUT_PITCH + 4);
+      const float4 w = *reinterpret_cast<const float4*>(b + k * OUT_PITCH);
+      const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w}, y[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+    }
+    __syncwarp();  // before the next copies
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    *reinterpret_cast<float4*>(sh + (row + i) * OUT_PITCH + col) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
 }
 
 // x = h + 2^-16 (m + l) with bf16 h, m, l, each rounded to nearest: 8 bits and a sign each, so nothing of x is lost, and the
@@ -449,8 +480,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
 #pragma unroll
       for (int j = 0; j < COLS; ++j) bad = bad || !(fabsf(acc[j]) <= 3.402823466e38f);
       float* const sh = reinterpret_cast<float*>(smem_raw + SMEM_BYTES - (warp - CUT_WARPS + 1) * PLAIN_BYTES);
-      if (__any_sync(0xFFFFFFFFu, bad)) plain_rows<AK, BK>(g, m0, n0, sh, lane, acc);
-      finish_part(p, m0, n0, sh, lane, acc);
+      __syncwarp();  // all lanes have read the part before
+      if (__any_sync(0xFFFFFFFFu, bad)) {
+        plain_part<AK, BK>(g, m0, n0, sh, lane);
+      } else {
+#pragma unroll
+        for (int j = 0; j < COLS; j += 4)
+          *reinterpret_cast<float4*>(sh + lane * OUT_PITCH + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+      }
+      __syncwarp();
+      finish_part(p, m0, n0, sh, lane);
     }
   } else {
     const uint32_t a_at = tmem + T_A + ShareA<AK>::offset(warp), b_at = smem + ShareB<BK, AK>::offset(t);
