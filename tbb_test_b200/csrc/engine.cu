@@ -385,8 +385,9 @@ int usable_cores() {  // those this process may run on, which need not be all of
 // Matrices of up to landing_bytes, see download_plan.h.
 int download_landing(b2_handle* h, float* host, size_t ld, const void* dev, size_t pitch, int rows, int cols) {
   const size_t width = (size_t)cols * 4, total = width * rows;
-  CK(h, copy_rows(h->landing, width, dev, pitch * 4, width, (size_t)rows, cudaMemcpyDeviceToHost, h->s_main));
   const int threads = landing_threads(total, usable_cores());
+  if (threads > 1) CK(h, cudaStreamSynchronize(h->s_main));  // work queued before: the threads look out for the copy only
+  CK(h, copy_rows(h->landing, width, dev, pitch * 4, width, (size_t)rows, cudaMemcpyDeviceToHost, h->s_main));
   if (threads == 1 && ld == (size_t)cols) make_pages(host, total);
   std::atomic<int> next{0}, landed{0};
   const int per = (int)std::max<size_t>(1, threads == 1 ? rows : DL_PIECE / width);

@@ -70,6 +70,26 @@ def test_small_downloads(native, oracle, shape, extra):
         m.close()
 
 
+def test_a_download_behind_queued_work_waits_in_one_thread(native):
+    """Six threads copy a matrix of 2.4 MB, but none of them burns a core while the GPU is still busy with earlier work: the
+    processor time of the call is that of one waiting thread."""
+    import time
+    import torch
+    from tbb_test_b200 import _capi as K
+    from tbb_test_b200.mlp import MLP
+    m, n = MLP([768, 768], 64), 4096
+    a, c = torch.ones(n, n, device="cuda"), torch.zeros(n, n, device="cuda")
+    torch.cuda.synchronize()
+    m.weights(0)
+    for _ in range(300):
+        m.lib.b2_sgemm(m._h, K.PREC_TF32, 0, 1, n, n, n, 1.0, a.data_ptr(), n, a.data_ptr(), n, 0.0, c.data_ptr(), n)
+    cpu, wall = time.process_time(), time.perf_counter()
+    m.weights(0)
+    cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+    assert wall > 0.02 and cpu <= 2.0 * wall, (cpu, wall)
+    m.close()
+
+
 OUT_OF_MEMORY = """
 import ctypes as C, sys
 import numpy as np
