@@ -78,6 +78,50 @@ def test_many_steps_in_few_launches(native, monkeypatch):
     b.close()
 
 
+@pytest.mark.parametrize("net", [([33, 17, 5], 7, {}), ([300, 301, 95, 40], 60, {}), ([45, 30], 70, {}), ([40, 24], 30, {}),
+                                 ([64, 100, 10], 33, dict(input_grad=False)), ([63, 64, 9], 20, dict(input_grad=False)), ([1024, 1024, 1001], 16, {})],
+                         ids=lambda n: f"{'-'.join(map(str, n[0]))}b{n[1]}")
+def test_many_steps_of_other_networks(native, monkeypatch, net):
+    """Rows that are not whole 16-byte pieces (copied through the L1, which the barriers have to empty), a single layer (a
+    barrier more per step), no input gradient, more tiles than groups of warps: several steps in each of several launches against
+    steps one by one (equal bits), and four steps in one launch against a launch per GEMM."""
+    nf, batch, kw = net
+    a, b, c = make(monkeypatch, nf, batch, True, **kw), make(monkeypatch, nf, batch, True, **kw), make(monkeypatch, nf, batch, False, **kw)
+    for m, n in ((a, 1), (c, 5)):
+        assert launches(m, lambda: m.step(4)) >= n
+    assert all(rel_fro(a.weights(l), c.weights(l)) <= 2e-5 and rel_fro(a.weight_grad(l), c.weight_grad(l)) <= 1e-4 for l in range(a.L))
+    assert 2 <= launches(a, lambda: a.step(150)) <= 75
+    for _ in range(154):
+        b.step(1)
+    assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(a.L)) and abs(a.loss() - b.loss()) <= 1e-12 * abs(b.loss())
+    for m in (a, b, c):
+        m.close()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3e38], ids=str)
+@pytest.mark.parametrize("net", [([128, 70, 90], 30), ([512, 9, 70], 8), ([80, 3], 100)], ids=lambda n: f"{'-'.join(map(str, n[0]))}b{n[1]}")
+def test_values_that_are_not_finite(native, monkeypatch, net, value):
+    """An input, a weight: the same elements of every tensor of a step end up infinite or not a number as with a launch per GEMM,
+    whichever way the sums go. (Where finite values overflow, which of the two is a matter of the order: partial sums of both signs
+    give no number.)"""
+    from tbb_test_b200 import _capi as K
+    nf, batch = net
+    out = []
+    for whole in (True, False):
+        m = make(monkeypatch, nf, batch, whole, mode=K.MODE_REF)
+        w, x = m.weights(0), np.linspace(-1, 1, batch * nf[0], dtype=np.float32).reshape(batch, nf[0])
+        w[2, 7], x[3, 5] = -value, value
+        m.upload_weights(0, w)
+        m.upload_input(x)
+        m.step(1)
+        out.append([m.activation(l) for l in range(m.L + 1)] + [f(l) for l in range(m.L) for f in (m.dz, m.weight_grad, m.weights)] + [m.input_grad()])
+        m.close()
+    for got, want in zip(*out):
+        assert np.array_equal(np.isfinite(got), np.isfinite(want))
+        bad = ~np.isfinite(want)
+        assert value == 3e38 or np.array_equal(got[bad], want[bad], equal_nan=True)
+
+
 def test_host_fed_steps(native, monkeypatch):
     """Both input slots: steps fed from the host, two in flight, against blocking ones."""
     nf, batch = [40, 24, 12], 30
