@@ -59,6 +59,26 @@ def test_one_step(native, monkeypatch, net, mode):
     b.close()
 
 
+@pytest.mark.parametrize("mode", ["baseline", "ref"])
+@pytest.mark.parametrize("net", [([128, 256, 128, 64], 32), ([33, 101, 70], 41), ([300, 301, 95, 40], 60), ([20] * 5, 17), ([64, 48], 200)],
+                         ids=lambda n: f"{'-'.join(map(str, n[0][:4]))}b{n[1]}")
+def test_sums_in_k_order_are_the_same_bits(native, monkeypatch, net, mode):
+    """Where no layer is as narrow and no batch as short as 16: every sum is one FMA per term in k order, as in gemm_simt_kernel
+    and gemm_f32_kernel, so three steps end in the bits of separate launches of those (force_simt)."""
+    from tbb_test_b200 import _capi as K
+    nf, batch = net
+    kw = dict(mode=K.MODE_REF if mode == "ref" else K.MODE_BASELINE)
+    a, b = make(monkeypatch, nf, batch, True, **kw), make(monkeypatch, nf, batch, False, force_simt=True, **kw)
+    a.step(3)
+    b.step(3)
+    for l in range(a.L):
+        for what in (a.weights, b.weights), (a.weight_grad, b.weight_grad), (a.dz, b.dz), (a.activation, b.activation):
+            assert np.array_equal(what[0](l), what[1](l))
+    assert np.array_equal(a.activation(a.L), b.activation(a.L)) and np.array_equal(a.input_grad(), b.input_grad())
+    a.close()
+    b.close()
+
+
 def test_many_steps_in_few_launches(native, monkeypatch):
     """100 steps in launches of at most 64, and the same steps one by one, from one handle's weights to the other's: equal
     bits (sums have a fixed order; the loss's block sums have none)."""
