@@ -48,11 +48,14 @@ typedef enum {
 /* Arithmetic of the three GEMMs; accumulation is fp32 and the master weights and
  * the SGD update are fp32 in every case. */
 typedef enum {
-  B2_PREC_FP32 = 0, /* fp32 operands at fp32 precision (parity mode): small GEMMs as CUDA-core FMAs in k order; large ones
-                       on the tensor cores as products of exact three-way bf16 splits whose sums are rounded in
-                       fp32, with a smaller error against 64-bit sums than the FMAs' and the same results where
-                       operands or sums are not finite (which take up to three times the FMAs' time, where they are
-                       many; csrc/gemm_split.cu). With force_simt: FMAs only */
+  B2_PREC_FP32 = 0, /* fp32 operands at fp32 precision (parity mode): small GEMMs as CUDA-core FMAs, in k order
+                       or (M or N of 16 at most) in partial sums; large ones on the tensor cores as products of
+                       exact three-way bf16 splits whose sums are rounded in fp32. Over a matrix of products of like
+                       size their error against 64-bit sums is smaller than that of FMAs in k order (they are
+                       6e-9 to 2e-8 of themselves small in the mean, as the tensor core truncates), but large terms
+                       that cancel take smaller ones among their 16 neighbours with them. Where operands or sums are
+                       not finite the results are the FMAs' (in up to three times their time, where that is most of a
+                       matrix; csrc/gemm_split.cu). With force_simt: FMAs only */
   B2_PREC_TF32 = 1, /* fp32 storage, tcgen05 kind::tf32 */
   B2_PREC_BF16 = 2, /* bf16 operands (activations, gradients, a bf16 weight copy),
                        tcgen05 kind::f16: layers of any width, on rows padded to 16 bytes (but for
@@ -174,9 +177,9 @@ int b2_set_lr(b2_handle* h, float lr);
 /* The loop body of mlp_omp.cc:435-737, `iters` times: forward GEMMs, output
  * gradient, then per layer (last to first) weight-gradient GEMM, gradient
  * allreduce + SGD on the side stream, input-gradient GEMM. Returns after both
- * streams have drained. Networks of small layers (no gradient exchange) run as launches of several whole steps that take all SMs for up to about 2 ms
- * at a time (or for one step, where that takes longer): other work on the GPU gets its
- * turn between them. */
+ * streams have drained. Networks of small layers (no gradient exchange) run as launches of
+ * several whole steps that take all SMs for up to about 2 ms at a time (or for one step, where
+ * that takes longer): other work on the GPU gets its turn between them. */
 int b2_step(b2_handle* h, int iters);
 
 /* One step fed from host memory: uploads this rank's rows of `x` (and `t`),

@@ -34,6 +34,11 @@ __device__ __forceinline__ uint32_t to_bf16x2(float lo, float hi) {  // rounded 
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
+__device__ __forceinline__ uint32_t to_six_bits(float lo, float hi) {  // to nearest: eight bits truncated and rounded once more
+  uint32_t r;
+  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return (r + 0x00020002u) & 0xFFFCFFFCu;
+}
 // (lo, hi) - s * the bf16 pair p, exactly; s as two bf16.
 __device__ __forceinline__ void take_off(float& lo, float& hi, uint32_t p, uint32_t minus_s) {
   asm("{\n\t.reg .b16 l, h, s, u;\n\tmov.b32 {l, h}, %2;\n\tmov.b32 {s, u}, %3;\n\t"
@@ -41,12 +46,12 @@ __device__ __forceinline__ void take_off(float& lo, float& hi, uint32_t p, uint3
       : "+f"(lo), "+f"(hi)
       : "r"(p), "r"(minus_s));
 }
-// Eight floats x as three bf16 pieces: x = h + 2^-16 (m + l).
+// Eight floats x as three bf16 pieces: x = h + 2^-16 (m + l), six bits in h and eight in m and l.
 __device__ __forceinline__ void cut8(const float (&v)[8], uint32_t (&w)[3][4]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     float x = v[2 * j], y = v[2 * j + 1];
-    w[0][j] = to_bf16x2(x, y);
+    w[0][j] = to_six_bits(x, y);
     asm("{\n\t.reg .b64 a, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 s, {0f47800000, 0f47800000};\n\tmul.rn.f32x2 a, a, s;\n\t"
         "mov.b64 {%0, %1}, a;\n\t}"
         : "+f"(x), "+f"(y));
@@ -328,25 +333,32 @@ __device__ __forceinline__ void plain_part(const GemmDesc& g, int m0, int n0, fl
     *reinterpret_cast<float4*>(sh + (row + i) * OUT_PITCH + col) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
 }
 
-// x = h + 2^-16 (m + l) with bf16 h, m, l, each rounded to nearest: 8 bits and a sign each, so nothing of x is lost, and the
+// x = h + 2^-16 (m + l) with bf16 h, m, l, each rounded to nearest: 6, 8 and 8 bits and a sign each, so nothing of x is lost, and the
 // scale keeps the low pieces of a small x away from the denormal numbers. C = D0 + 2^-16 D1 + 2^-32 D2 with
-//   D0 = sum h h'     D1 = sum h m' + m h' + h l' + l h'     D2 = sum m m'
-// What is dropped (m l' + l m' and smaller) is 2^-26 of a product. The tensor core truncates when it adds into an accumulator,
-// so D0 holds one chunk of 64 k only: the sum warps add it to the sum they keep in registers, rounding to nearest. D1 and
-// D2 run over all of K in TMEM, where a truncation is 2^-8 and 2^-16 of one in D0.
+//   D0 = sum h h'     D1 = sum h m' + m h' + h l' + l h'     D2 = sum m m' + m l' + l m'
+// What is dropped (l l') is 2^-32 of a product. The tensor core truncates when it adds into an accumulator, so D0 holds one
+// chunk of 64 k only: the sum warps add it to the sum they keep in registers, rounding to nearest. D1 and D2 run over all of K
+// in TMEM, where a truncation is 2^-6 and 2^-12 of one in D0. And h has six bits, not the eight that a bf16 holds: products of
+// twelve mostly fit whole into D0 beside larger ones, so that little is truncated. Truncation has one sign, and with eight bits in h sums
+// came out 3.8e-8 (operands signed) to 6.6e-8 (positive) of themselves small in the mean, now 5.7e-9 to 1.7e-8; a number made of
+// many results shows it (the loss of nine 538-wide layers without ReLU was off by 7.7e-7, now by 8e-8, with FMAs by 8e-8 to 1.5e-7).
+// It takes three instructions for every pair instead of one, m l' and l m' among the products, and 3 % of a step of 5 x 1024. Error
+// against 64 bits in the norm of the result, here / FMAs in k order, signed and positive: K = 64 4.0e-8 / 1.5e-7 and
+// 5.0e-8 / 1.2e-7, K = 4096 2.0e-7 / 1.2e-6 and 1.2e-7 / 8.5e-7. But products are added 16 at a time against the largest
+// of them: where large terms cancel early in k order, FMAs keep a small one that is rounded away here.
 // 32 x 32 elements with one that is not finite in the end (an Inf or a NaN among the operands, whose pieces are NaN, or numbers
 // from 2^112 on) are computed again by FMAs in k order, so they are what the CUDA-core kernels give.
 //
-// Per 16 k one thread issues h h', h m', h l' and l h' (BN columns each) and m [h'|m'] (into D1 and D2 side by side). A comes
+// Per 16 k one thread issues h h', h m', h l' and m l' (BN columns each), m [h'|m'] and l [h'|m'] (into D1 and D2 side by side). A comes
 // from TMEM, so that an MMA reads 2 KB of shared memory instead of 6 (with A in shared memory an MMA of 64 columns took 74
 // clocks, 42 so). Tiles of 64 columns: D0, D1, D2 and three stages of A fill TMEM, and 1024 x 1024 fills 128 SMs.
-// Bound by the instructions that cut the operands (8 per pair of floats) and the latency of a chunk from load to hand-over:
-// 0.8 us per chunk, of which the MMAs are 0.4. So sixteen warps cut, each a small part: with eight of twice the share a chunk took
+// Bound by the instructions that cut the operands (10 per pair of floats) and the latency of a chunk from load to hand-over:
+// 0.9 us per chunk, of which the MMAs are 0.65. So sixteen warps cut, each a small part: with eight of twice the share a chunk took
 // 1.0 us, with the summing in the same warps 1.05, with the pieces of A in shared memory 1.1 (1.5 for 128 columns). Beside its chunks a
 // tile takes 5.5 us of launch, first loads and epilogue (8 with checked first loads, the first chunk handed over behind the second
 // one's cut, and lanes storing their own rows).
-// us, forward / weight / input gradient, against gemm_simt_kernel, operands in L2: 1024^3 21/22/20 against 72/64/68, 2048^3
-// 115/126/112 (153 TFLOP/s) against 435/425/427, 512^3 13/14/13 against 21/21/21. 5 x 1024, batch 1024: 293 us per step, 938 before.
+// us, forward / weight / input gradient, against gemm_simt_kernel, operands in L2: 1024^3 24/24/22 against 74/65/69, 2048^3
+// 130/135/120 (143 TFLOP/s) against 435/426/428, 512^3 15/16/15 against 22/22/22. 5 x 1024, batch 1024: 298 us per step, 938 before.
 template <bool AK, bool BK>
 __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __grid_constant__ SplitParams p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -431,7 +443,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
             mma_ts(d1, piece(ks, 1), b + ks * B_STEP, two, c > 0 || ks > 0);
             mma_ts(d1, piece(ks, 0), b + BP + ks * B_STEP, one, 1u);
             mma_ts(d1, piece(ks, 0), b + 2 * BP + ks * B_STEP, one, 1u);
-            mma_ts(d1, piece(ks, 2), b + ks * B_STEP, one, 1u);
+            mma_ts(d1, piece(ks, 2), b + ks * B_STEP, two, 1u);
+            mma_ts(d1 + BN, piece(ks, 1), b + 2 * BP + ks * B_STEP, one, 1u);
           }
           tc_commit(smem_u32(&empty_bar[s]));
           if (++s == STAGES) { s = 0; phase ^= 1; }
@@ -493,8 +506,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
     }
   } else {
     const uint32_t a_at = tmem + T_A + ShareA<AK>::offset(warp), b_at = smem + ShareB<BK, AK>::offset(t);
-    // What has been stored of a chunk is there for the MMAs. Done when the first part of the next chunk has been cut: the
-    // stores have arrived by then.
+    // What has been stored of a chunk is there for the MMAs. Done before the next chunk is cut, behind the wait for its stage:
+    // the loads of it, which are on their way, hide the wait for the stores.
     auto hand_over = [&](int s) {
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       fence_proxy_async_smem();
@@ -590,11 +603,11 @@ cudaError_t launch(const SplitParams& p, int sms, cudaStream_t stream) {
 
 }  // namespace
 
-// us: 6 and 0.85 per chunk and round of the tiles, 1.35 where rows are not whole 16-byte pieces.
+// us: 6 and 0.88 per chunk and round of the tiles, 1.37 where rows are not whole 16-byte pieces.
 double gemm_split_us(const GemmDesc& g, int sms) {
   const long long tiles = (long long)((g.M + 127) / 128) * ((g.N + BN - 1) / BN);
   const double rounds = (double)((tiles + sms - 1) / sms), chunks = (g.K + CHUNK_K - 1) / CHUNK_K;
-  return 6.0 + rounds * chunks * (how_to_read(g) != FLOATS ? 0.85 : 1.35);
+  return 6.0 + rounds * chunks * (how_to_read(g) != FLOATS ? 0.88 : 1.37);
 }
 
 // By the estimates of both sides, fitted to 110 shapes of 16 to 4096 rows, columns and k in the three forms of the step (the

@@ -167,8 +167,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int
 // whose epilogue updates the weights that the phase before was the last to read. A phase is a list of 16 x 32 tiles.
 // Bound by the latency of a phase where there is little to multiply: a trip to L2 for the operands, 4 ns per k, the
 // stores, the barrier's fence, its atomic and the trip that notices it, 2.9 us together; else by shared memory reads (eight lines
-// for the 16 FMAs of four k), half the FMA rate. Us per step, against a launch per GEMM on four streams: 128-256-128-64, batch 32 38 and
-// 72; 6 x 48, batch 167 58 and 141; 3 x 512, batch 16 74 and 246; 9 x 162, batch 151 111 and 217; 8 x 416, batch 140 175 and 258.
+// for the 16 FMAs of four k), half the FMA rate. Us per step in a launch of its own (5 less in
+// launches of many), against a launch per GEMM on four streams: 128-256-128-64, batch 32 37 and 70; 6 x 48, batch 167 57 and 115;
+// 3 x 512, batch 16 76 and 243; 9 x 162, batch 151 109 and 216; 8 x 416, batch 140 175 and 227.
 // Tried: sums split over 16 warps, which meet in shared memory (the same in small batches, other bits); one
 // cluster of 16 SMs and its barrier (3.7 us per phase, and nine times fewer SMs: 88-232-288-504-144-88, batch 26 315, 73 here).
 __global__ void __launch_bounds__(THREADS) small_step_kernel(const __grid_constant__ SmallStep s, int steps, float lr, unsigned int count,

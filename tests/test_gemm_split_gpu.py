@@ -61,6 +61,19 @@ def test_against_float64(devs, oracle, form, shape, lo):
     assert (np.abs(got - (2.0 * ref - 0.5 * c)) <= units * 2.0 ** -24 * (2.0 * mag + np.abs(c))).all()
 
 
+@pytest.mark.parametrize("lo", [-1.0, 0.0], ids=["signed", "positive"])
+@pytest.mark.parametrize("k", [64, 538, 2048])
+def test_sums_do_not_shrink(devs, oracle, k, lo):
+    """The error along the result, which many results combined to one number do not average out. The tensor core truncates:
+    pieces of eight bits left sums 3.8e-8 (signed) to 6.6e-8 (positive) small, those of six 5.7e-9 to 1.7e-8 (so too a model of
+    it in numpy: sums of 16 exact products and the accumulator, truncated to 24 bits)."""
+    ta, tb, a, b = operands(oracle, "fwd_NT", 1500, 1600, k, 261, lo)
+    ref = a.astype(np.float64) @ b.astype(np.float64).T
+    got = sgemm(devs[0], ta, tb, a, b)
+    assert not np.array_equal(got, sgemm(devs[1], ta, tb, a, b))
+    assert abs(((got - ref) * ref).sum()) <= 2.2e-8 * (ref * ref).sum()
+
+
 @pytest.mark.parametrize("shape", [(300, 204, 1300), (129, 65, 1001)], ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("form", list(FORMS))
 def test_relu_and_mask(devs, oracle, form, shape):
