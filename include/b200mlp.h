@@ -139,7 +139,8 @@ int b2_nccl_unique_id(void* out_bytes);
 
 /* Allocation phase of main (mlp_omp.cc:390-409): device buffers for weights,
  * gradients and activations of this rank's batch shard, streams, events and the
- * communicator. */
+ * communicator; and up to 2.5 MB of page-locked host memory, as large as the largest matrix
+ * of the network within that, through which such matrices and the losses are read back. */
 int b2_create(const b2_config* cfg, b2_handle** out);
 int b2_destroy(b2_handle* h);
 
@@ -192,7 +193,9 @@ int b2_train_step_host(b2_handle* h, const float* x, size_t ldx, const float* t,
  * step's inputs (on a copy stream, into one of two input slots) and the step, and
  * returns without waiting, so that the copy of step i+1 overlaps the compute of
  * step i. At most two steps may be in flight; b2_wait_loss() blocks until the
- * oldest one has finished and returns its loss share. `x` and `t` must stay valid
+ * oldest one has finished and returns its loss share. A step that a wait which gave up
+ * kept from running makes its b2_wait_loss() fail (B2_ERR_TIMEOUT), and so do the steps in
+ * flight behind it: wait for all of them before going on. `x` and `t` must stay valid
  * and unchanged until that step's b2_wait_loss() returns, and should be pinned.
  * Needs collect_timing = 0 and use_graph = 0. The reference has no counterpart
  * (its inputs never change, mlp_bench_common.cc:18); this is the form a data-loader
