@@ -165,13 +165,14 @@ def test_host_fed_steps(native, monkeypatch):
 @pytest.mark.parametrize("net", [([4096] * 5, 1), ([2048] * 3, 8), ([16384, 256, 10], 4), ([64] * 10, 1), ([128, 256, 128, 64], 32)],
                          ids=lambda n: f"{'-'.join(map(str, n[0][:3]))}b{n[1]}")
 def test_launches_last_about_2_ms(native, monkeypatch, net):
-    """A launch holds every SM. (64 steps at most; the estimate of a step is within 0.82 and 1.21 of its time.)"""
+    """A launch holds every SM. (64 steps at most; the estimate of a step is within 0.82 and 1.21 of its time at 1965 MHz, and a GPU
+    at its power limit runs at two thirds of that.)"""
     m = make(monkeypatch, *net, True)
     n = launches(m, lambda: m.step(128))
     m.reset_timing()
     m.step(128)
     launch_ms = m.timing()[1] / n
-    assert launch_ms <= 2.0 / 0.8 and (n == 2 or launch_ms >= 0.5), (n, launch_ms)
+    assert launch_ms <= 2.0 / 0.8 * 1.5 and (n == 2 or launch_ms >= 0.5), (n, launch_ms)
     m.close()
 
 
@@ -192,7 +193,7 @@ def test_a_wait_that_runs_out(native, monkeypatch):
     t0 = time.time()
     with pytest.raises(K.B2Error) as e:
         a.step(1000)
-    assert e.value.code == K.ERR_TIMEOUT and time.time() - t0 < 3.5
+    assert e.value.code == K.ERR_TIMEOUT and time.time() - t0 < 6.0
     assert all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
     a.step(130)
     b.step(130)
@@ -218,7 +219,7 @@ def test_a_wait_that_runs_out_in_the_pipeline(native, monkeypatch):
         assert e.value.code == K.ERR_TIMEOUT
     with pytest.raises(K.B2Error):
         a.wait_loss()
-    assert time.time() - t0 < 3.5 and all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
+    assert time.time() - t0 < 6.0 and all(np.array_equal(a.weights(l), b.weights(l)) for l in range(2))
     for m in (a, b):
         m.train_step_host_async(*args)
         m.train_step_host_async(*args)
